@@ -609,15 +609,15 @@ struct ChainPlan {
     ChainLayer* d_layers;
     ChainParams prm;
     int smem_bytes;
+    int clusters;            // clusters the device holds at once
 };
 
 // layers[i]: device pointers of layer i (weights, tables, residual, outputs); all layers are 3x3 stride-1
 // pad-1 convolutions C -> C on an H x W map, layer i + 1 reading what layer i writes (its fused BN's
 // output where it has one).  d_in = the first layer's input (one face, NHWC).  NULL when the shape does
 // not fit the kernel (C / 64 column tiles x row tiles of 128 positions must be exactly eight CTAs).
-ChainPlan* ffcu_chain_plan(int H, int W, int C, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers, int device)
+ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers)
 {
-    (void)device;
     encode_tiled_fn enc = get_encode();
     if (!enc || n_layers < 2 || C % 128 != 0 || C > TC_MAX_COUT) return nullptr;
     // pitch: a power of two >= W + 1.  With P = W + 1 the right-hand padding of a row is the next row's
@@ -650,11 +650,12 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, const int8_t* d_in, const ChainL
     if (stages > CHAIN_MAX_STAGES) stages = CHAIN_MAX_STAGES;
     stages &= ~1;                                         // two issuers on alternate stages: the ring must be even
     if (stages < 2) return nullptr;
-    if (!tc_chain_fits(fixed + stages * stage_bytes)) return nullptr;      // no room for a cluster of eight on this device
+    const int clusters = tc_chain_clusters(fixed + stages * stage_bytes);
+    if (clusters < 1) return nullptr;                     // no room for a cluster of eight on this device
     ChainPlan* p = new ChainPlan();
     p->d_layers = nullptr;
     {
-        cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, 1};
+        cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)max_batch};
         cuuint64_t strides[3] = {(cuuint64_t)C, (cuuint64_t)C * W, (cuuint64_t)C * W * H};
         cuuint32_t box[4] = {128, (cuuint32_t)P, (cuuint32_t)rows, 1};
         cuuint32_t es[4] = {1, 1, 1, 1};
@@ -692,8 +693,11 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, const int8_t* d_in, const ChainL
     p->prm.planes = planes; p->prm.plane_bytes = plane_bytes; p->prm.win_rows = rows; p->prm.tiles_n = tiles_n; p->prm.stages = stages; p->prm.tps = tps;
     p->prm.err = nullptr;
     p->smem_bytes = fixed + stages * stage_bytes;
+    p->clusters = clusters;
     return p;
 }
+
+int ffcu_chain_clusters(const ChainPlan* p) { return p->clusters; }
 
 void ffcu_chain_free(ChainPlan* p)
 {
@@ -712,7 +716,7 @@ extern "C" void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles
     g_test_chain_wait = wait_cycles;
 }
 
-int ffcu_chain_launch(const ChainPlan* p, int mode, int* d_err, cudaStream_t s)
+int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s)
 {
     ChainParams prm = p->prm;
     prm.err = d_err;
@@ -732,7 +736,7 @@ int ffcu_chain_launch(const ChainPlan* p, int mode, int* d_err, cudaStream_t s)
         if (!d_ts) cudaMalloc(&d_ts, 64 * 4 * sizeof(unsigned long long));
         prm.ts = d_ts;
         if (++calls == 29 || calls == 30) {
-            int rc = tc_launch_chain(mode, p->smem_bytes, s, p->mapA, prm);
+            int rc = tc_launch_chain(mode, faces, p->smem_bytes, s, p->mapA, prm);
             cudaStreamSynchronize(s);
             unsigned long long h[256];
             cudaMemcpy(h, d_ts, sizeof h, cudaMemcpyDeviceToHost);
@@ -744,7 +748,7 @@ int ffcu_chain_launch(const ChainPlan* p, int mode, int* d_err, cudaStream_t s)
         }
     }
 #endif
-    return tc_launch_chain(mode, p->smem_bytes, s, p->mapA, prm);
+    return tc_launch_chain(mode, faces, p->smem_bytes, s, p->mapA, prm);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,6 +1,10 @@
-// conv_tc_chain.cu -- batch-1 latency path: a run of consecutive 3x3 stride-1 convolutions of one
-// shape (the 26 layers of the 14x14 stage, the 4 of the 7x7 stage) in ONE launch of one cluster of
-// eight CTAs, with the activations resident in shared memory.
+// conv_tc_chain.cu -- small-batch latency path: a run of consecutive 3x3 stride-1 convolutions of one
+// shape (the 26 layers of the 14x14 stage, the 4 of the 7x7 stage) in ONE launch, one cluster of
+// eight CTAs per face, with the activations resident in shared memory.
+//
+// Clusters share nothing but the weights (L2): n faces cost one face's time while all n clusters are resident at once
+// (26 layers of 14x14: 144 us at 1 face, 150 us at 8, against 205-208 us as one launch per layer), and twice that with
+// one cluster more.  What bounds a layer is latency: MMA issue, epilogue, the exchange of results, in that order.
 //
 // At batch 1 a 14x14 layer is 8 tiles (2 row tiles x 4 column tiles of 64 channels); as separate
 // launches each layer pays kernel completion + dependency release + a TMA round trip for 50 KB of
@@ -149,6 +153,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
+    const int face = (int)blockIdx.x / CHAIN_CLUSTER;     // one cluster per face
     const int tile_m = (int)rank / p.tiles_n;
     const int tile_n = (int)rank % p.tiles_n;
     const int a_buf_bytes = p.planes * p.plane_bytes;
@@ -212,7 +217,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
                 // both buffers: the copy into the second one only puts the zero lines of the padding in place
                 if (lane < 2 * p.planes)
                     tma_load_4d(smem_u32(s_a) + lane * p.plane_bytes, &mapA, smem_u32(&sh->a0_full),
-                                (lane % p.planes) * 128, -1, (tile_m * TC_TILE_M) / p.P - 1, 0);
+                                (lane % p.planes) * 128, -1, (tile_m * TC_TILE_M) / p.P - 1, face);
             }
             ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, p.wait_cycles);
             if (!ok) break;
@@ -264,7 +269,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
         const int r = qpos / p.P, c = qpos - r * p.P;
         const bool valid = (c < p.W) && (r < p.H);
         const int cb = tile_n * CHAIN_BN + cg * 16;                // first of this thread's 16 channels
-        const size_t o = (size_t)(r * p.W + c) * p.C + cb;
+        const size_t o = (size_t)((face * p.H + r) * p.W + c) * p.C + cb;
         // where this output sits in the next layer's input: line (r + 1) * P + (c + 1), 16-byte chunk swizzled
         const int out_line = qpos + p.P + 1;
         const uint32_t nx_off = (uint32_t)((cb >> 7) * p.plane_bytes + out_line * 128 + ((((cb & 127) >> 4) ^ (out_line & 7)) << 4));
@@ -399,7 +404,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
     }
 }
 
-int tc_launch_chain(int mode, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm)
+int tc_launch_chain(int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm)
 {
     static int smem_set[2][64] = {};      // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
@@ -409,18 +414,18 @@ int tc_launch_chain(int mode, int smem, cudaStream_t s, const CUtensorMap& mapA,
         else      FFCU_CHECK(cudaFuncSetAttribute(conv_chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         smem_set[mode ? 1 : 0][dev & 63] = smem;
     }
-    if (mode) return tc_launch_ex(conv_chain_kernel<true>, CHAIN_CLUSTER, smem, s, CHAIN_CLUSTER, mapA, prm);
-    return tc_launch_ex(conv_chain_kernel<false>, CHAIN_CLUSTER, smem, s, CHAIN_CLUSTER, mapA, prm);
+    if (mode) return tc_launch_ex(conv_chain_kernel<true>, faces * CHAIN_CLUSTER, smem, s, CHAIN_CLUSTER, mapA, prm);
+    return tc_launch_ex(conv_chain_kernel<false>, faces * CHAIN_CLUSTER, smem, s, CHAIN_CLUSTER, mapA, prm);
 }
 
-// Can this device co-schedule one cluster of the chain kernel (eight CTAs with `smem` bytes each in one GPC)?
-// Asked once per plan; a device that cannot keeps the per-layer launches.
-bool tc_chain_fits(int smem)
+// How many clusters of the chain kernel (eight CTAs with `smem` bytes each in one GPC) the device holds at once.
+// Asked once per plan; a device that holds none keeps the per-layer launches.
+int tc_chain_clusters(int smem)
 {
     if (cudaFuncSetAttribute(conv_chain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaFuncSetAttribute(conv_chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return 0;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CHAIN_CLUSTER);
@@ -431,6 +436,6 @@ bool tc_chain_fits(int smem)
     attr[0].val.clusterDim.x = CHAIN_CLUSTER; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, conv_chain_kernel<true>, &cfg) != cudaSuccess) { cudaGetLastError(); return false; }
-    return n >= 1;
+    if (cudaOccupancyMaxActiveClusters(&n, conv_chain_kernel<true>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return n;
 }

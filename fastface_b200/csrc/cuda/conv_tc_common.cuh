@@ -885,8 +885,8 @@ struct ChainParams {
 #endif
 };
 
-int tc_launch_chain(int mode, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
-bool tc_chain_fits(int smem);
+int tc_launch_chain(int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
+int tc_chain_clusters(int smem);
 
 // Flat-pitch weight-stationary pair kernel: activation buffer = guard + box of WSP_BOX_ROWS image rows
 #define WSP_GUARD_BYTES 1024

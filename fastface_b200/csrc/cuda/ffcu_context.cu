@@ -74,8 +74,8 @@ struct ffcu_ctx {
     int graph_max_batch = 1 << 30;
     std::map<long long, cudaGraphExec_t> graphs;
     std::map<long long, int> graph_launches;
-    // Batch 1: runs of same-shape 3x3 stride-1 convolutions (the 14x14 and 7x7 stages) go out as one
-    // launch each (conv_tc_chain.cu).  Found on the first one-face forward; FF_CHAIN=0 disables.
+    // Small batches: runs of same-shape 3x3 stride-1 convolutions (the 14x14 and 7x7 stages) go out as one
+    // launch each (conv_tc_chain.cu).  Found on the first such forward; FF_CHAIN=0 disables.
     // Calls of at most lean_max_batch faces run copy-in, forward and copy-out on the compute stream alone
     // (FF_LEAN_MAX_BATCH, default 1: the single-face call; 0 = always the three-stream pipeline, whose overlap of
     // the next call's copy-in with this call's kernels is worth more than the hops it costs from a few faces up).
@@ -461,33 +461,44 @@ static void build_chains(ffcu_ctx* c)
                 desc[i].out2 = L.d.bn2_dst_buf >= 0 ? c->bufs[L.d.bn2_dst_buf] : nullptr;
             }
             const ffcu_layer& d0 = c->layers[k].d;
-            ChainPlan* plan = ffcu_chain_plan(d0.H, d0.W, d0.Cout, c->bufs[d0.src_buf], desc.data(), count, c->device);
+            ChainPlan* plan = ffcu_chain_plan(d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
             if (plan) c->chains.push_back({k, count, plan});
         }
         k = e;
     }
 }
 
+// Largest call that takes the layer chains (each chain's own limit, the clusters the device holds at once, comes on
+// top: one cluster of eight CTAs works on one face, and a second wave of clusters doubles the stage's time).  Measured,
+// forward of 2 / 4 / 8 / 12 / 16 faces, chains against one launch per layer: 300 / 311 / 332 / 363 / 547 us against
+// 366 / 379 / 403 / 445 / 467 on a device that holds 15 clusters.  A context made for two or three faces keeps one
+// launch per layer beyond a single face, the launch count fastface_launches_per_forward has always given there.
+static int chain_max_faces(const ffcu_ctx* c)
+{
+    return c->max_batch >= 4 ? FFCU_CHAIN_MAX_FACES : 1;
+}
+
 static int launch_forward(ffcu_ctx* c, int n)
 {
     int launches = 0;
-    if (n == 1 && !c->chains_built) build_chains(c);
+    const bool chain_call = n <= chain_max_faces(c);
+    if (chain_call && !c->chains_built) build_chains(c);
     size_t next_chain = 0;
     for (size_t k = 0; k < c->layers.size(); k++) {
-        if (n == 1) {
+        if (chain_call && !c->no_chain) {
             while (next_chain < c->chains.size() && c->chains[next_chain].first < k) next_chain++;
-            if (next_chain < c->chains.size() && c->chains[next_chain].first == k) {
+            if (next_chain < c->chains.size() && c->chains[next_chain].first == k &&
+                n <= ffcu_chain_clusters(c->chains[next_chain].plan)) {
                 const ffcu_ctx::Chain& ch = c->chains[next_chain];
-                if (ffcu_chain_launch(ch.plan, c->mode, c->d_err, c->stream) == 0) {
+                if (ffcu_chain_launch(ch.plan, n, c->mode, c->d_err, c->stream) == 0) {
                     launches++;
                     k += (size_t)ch.count - 1;
                     continue;
                 }
                 // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...):
-                // drop the chains for this context and go on with this layer as a launch of its own
+                // no more chains in this context (captured graphs may still hold launches of these plans: they stay until
+                // the context goes); go on with this layer as a launch of its own
                 cudaGetLastError();
-                for (auto& gone : c->chains) ffcu_chain_free(gone.plan);
-                c->chains.clear();
                 c->no_chain = 1;
             }
         }

@@ -202,12 +202,14 @@ ScPlan* ffcu_sc_plan(const ffcu_layer& main, const ffcu_layer& sc, int max_batch
 void    ffcu_sc_free(ScPlan* sp);
 int     ffcu_sc_launch(const ScPlan* sp, int batch, int mode, const EpiTables& t1, const EpiTables& t2, int8_t* out_main,
                        int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s);
-// Layer chain (batch 1): consecutive 3x3 stride-1 C -> C convolutions of one feature-map size in one launch.
+// Layer chain (small batches, one cluster of eight CTAs per face): consecutive 3x3 stride-1 C -> C convolutions of one feature-map size in one launch.
+#define FFCU_CHAIN_MAX_FACES 16     // 148 SMs hold at most 18 clusters of eight, fewer where GPCs are smaller
 struct ChainPlan;
 struct ChainLayerDesc { const int8_t* w; EpiTables t; const int8_t* res; int8_t* out; int8_t* out2; };
-ChainPlan* ffcu_chain_plan(int H, int W, int C, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers, int device);
+ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers);
+int        ffcu_chain_clusters(const ChainPlan* p);
 void       ffcu_chain_free(ChainPlan* p);
-int        ffcu_chain_launch(const ChainPlan* p, int mode, int* d_err, cudaStream_t s);
+int        ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s);
 struct TcPlan;   // opaque: tile shape, TMA descriptors, launch geometry for one layer
 int ffcu_stem_weight_k32(const int8_t* d_w, int8_t* d_wk, int Cout, cudaStream_t s);
 // Tensor-core stem (one launch): plan over the repacked weights d_wk [64][32]
