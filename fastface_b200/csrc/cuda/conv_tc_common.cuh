@@ -366,6 +366,8 @@ struct TcParams {
 // compile time, which turns the per-element code into one straight-line block the scheduler
 // can interleave across elements (the run-time form branches per element and runs several
 // times slower).
+// Both epilogue orders have them: with only the run-time form the strict order's forward took 560 / 1762 / 9180 us at
+// 17 / 160 / 1024 faces against 479 / 1391 / 7480 (the contracted order's times within 2 %).
 enum { EPI_RUNTIME = 0, EPI_PLAIN = 1, EPI_SLOPE = 2, EPI_RES_BN = 3, EPI_RES = 4, EPI_SLOPE_BN = 5 };
 
 #define TC_MAX_STAGES 8

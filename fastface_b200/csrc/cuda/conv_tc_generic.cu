@@ -182,20 +182,26 @@ static int launch_g(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA,
     return tc_launch_ex(kern, grid, smem, s, 1, mapA, mapB, prm);
 }
 
+template <int BN, int KC, bool CONTRACT>
+static int launch_g_mode(int epi, bool f32, int grid, int smem, cudaStream_t s,
+                         const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
+{
+    if (f32) return launch_g<BN, KC, CONTRACT, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
+    switch (epi) {
+    case EPI_PLAIN: return launch_g<BN, KC, CONTRACT, false, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_SLOPE: return launch_g<BN, KC, CONTRACT, false, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES_BN:return launch_g<BN, KC, CONTRACT, false, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES:   return launch_g<BN, KC, CONTRACT, false, EPI_RES>(grid, smem, s, mapA, mapB, prm);
+    default:         return launch_g<BN, KC, CONTRACT, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
+    }
+}
+
 template <int BN, int KC>
 static int launch_g_bn(int mode, int epi, bool f32, int grid, int smem, cudaStream_t s,
                        const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
-    if (f32) return mode ? launch_g<BN, KC, true, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm)
-                         : launch_g<BN, KC, false, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
-    if (!mode) return launch_g<BN, KC, false, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
-    switch (epi) {
-    case EPI_PLAIN:  return launch_g<BN, KC, true, false, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_SLOPE:  return launch_g<BN, KC, true, false, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES_BN: return launch_g<BN, KC, true, false, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES:    return launch_g<BN, KC, true, false, EPI_RES>(grid, smem, s, mapA, mapB, prm);
-    default:         return launch_g<BN, KC, true, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
-    }
+    return mode ? launch_g_mode<BN, KC, true>(epi, f32, grid, smem, s, mapA, mapB, prm)
+                : launch_g_mode<BN, KC, false>(epi, f32, grid, smem, s, mapA, mapB, prm);
 }
 
 int tc_launch_generic(int bn, int kc, int mode, int epi, bool f32, int grid, int smem, cudaStream_t s,

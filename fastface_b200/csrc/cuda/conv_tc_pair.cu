@@ -199,25 +199,25 @@ static int launch_p(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA,
     return tc_launch_ex(kern, grid, smem, s, 2, mapA, mapB, prm);
 }
 
-template <int BN>
-static int launch_p_bn(int mode, int epi, bool f32, int grid, int smem, cudaStream_t s,
+template <int BN, bool CONTRACT>
+static int launch_p_bn(int epi, bool f32, int grid, int smem, cudaStream_t s,
                        const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
-    if (f32) return mode ? launch_p<BN, true, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm)
-                         : launch_p<BN, false, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
-    if (!mode) return launch_p<BN, false, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
+    if (f32) return launch_p<BN, CONTRACT, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
     switch (epi) {
-    case EPI_PLAIN:  return launch_p<BN, true, false, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_SLOPE:  return launch_p<BN, true, false, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES_BN: return launch_p<BN, true, false, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES:    return launch_p<BN, true, false, EPI_RES>(grid, smem, s, mapA, mapB, prm);
-    default:         return launch_p<BN, true, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
+    case EPI_PLAIN: return launch_p<BN, CONTRACT, false, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_SLOPE: return launch_p<BN, CONTRACT, false, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES_BN:return launch_p<BN, CONTRACT, false, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES:   return launch_p<BN, CONTRACT, false, EPI_RES>(grid, smem, s, mapA, mapB, prm);
+    default:         return launch_p<BN, CONTRACT, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
     }
 }
 
 int tc_launch_pair(int bn, int mode, int epi, bool f32, int grid, int smem, cudaStream_t s,
                    const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
-    if (bn == 256) return launch_p_bn<256>(mode, epi, f32, grid, smem, s, mapA, mapB, prm);
-    return launch_p_bn<128>(mode, epi, f32, grid, smem, s, mapA, mapB, prm);
+    if (bn == 256) return mode ? launch_p_bn<256, true>(epi, f32, grid, smem, s, mapA, mapB, prm)
+                               : launch_p_bn<256, false>(epi, f32, grid, smem, s, mapA, mapB, prm);
+    return mode ? launch_p_bn<128, true>(epi, f32, grid, smem, s, mapA, mapB, prm)
+                : launch_p_bn<128, false>(epi, f32, grid, smem, s, mapA, mapB, prm);
 }

@@ -213,11 +213,10 @@ int tc_launch_stem(int mode, int epi, int in_u8, int grid, int smem, cudaStream_
 {
 #define STEM_PICK(C_, E_) (in_u8 ? launch_stem<C_, E_, true>(grid, smem, s, mapB, prm, in_any, inv3) \
                                  : launch_stem<C_, E_, false>(grid, smem, s, mapB, prm, in_any, inv3))
-    if (!mode) return STEM_PICK(false, EPI_RUNTIME);
     switch (epi) {
-    case EPI_SLOPE_BN: return STEM_PICK(true, EPI_SLOPE_BN);
-    case EPI_SLOPE:    return STEM_PICK(true, EPI_SLOPE);
-    default:           return STEM_PICK(true, EPI_RUNTIME);
+    case EPI_SLOPE_BN: return mode ? STEM_PICK(true, EPI_SLOPE_BN) : STEM_PICK(false, EPI_SLOPE_BN);
+    case EPI_SLOPE:    return mode ? STEM_PICK(true, EPI_SLOPE) : STEM_PICK(false, EPI_SLOPE);
+    default:           return mode ? STEM_PICK(true, EPI_RUNTIME) : STEM_PICK(false, EPI_RUNTIME);
     }
 #undef STEM_PICK
 }

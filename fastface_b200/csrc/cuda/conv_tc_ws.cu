@@ -149,23 +149,24 @@ static int launch_w(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA,
     return tc_launch_ex(kern, grid, smem, s, 1, mapA, mapB, prm);
 }
 
-template <int BN>
-static int launch_w_bn(int mode, int epi, int grid, int smem, cudaStream_t s,
+template <int BN, bool CONTRACT>
+static int launch_w_bn(int epi, int grid, int smem, cudaStream_t s,
                        const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
-    if (!mode) return launch_w<BN, false, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
     switch (epi) {
-    case EPI_PLAIN:  return launch_w<BN, true, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_SLOPE:  return launch_w<BN, true, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES_BN: return launch_w<BN, true, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
-    case EPI_RES:    return launch_w<BN, true, EPI_RES>(grid, smem, s, mapA, mapB, prm);
-    default:         return launch_w<BN, true, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
+    case EPI_PLAIN: return launch_w<BN, CONTRACT, EPI_PLAIN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_SLOPE: return launch_w<BN, CONTRACT, EPI_SLOPE>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES_BN:return launch_w<BN, CONTRACT, EPI_RES_BN>(grid, smem, s, mapA, mapB, prm);
+    case EPI_RES:   return launch_w<BN, CONTRACT, EPI_RES>(grid, smem, s, mapA, mapB, prm);
+    default:         return launch_w<BN, CONTRACT, EPI_RUNTIME>(grid, smem, s, mapA, mapB, prm);
     }
 }
 
 int tc_launch_ws(int bn, int mode, int epi, int grid, int smem, cudaStream_t s,
                  const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
-    if (bn == 64) return launch_w_bn<64>(mode, epi, grid, smem, s, mapA, mapB, prm);
-    return launch_w_bn<128>(mode, epi, grid, smem, s, mapA, mapB, prm);
+    if (bn == 64) return mode ? launch_w_bn<64, true>(epi, grid, smem, s, mapA, mapB, prm)
+                              : launch_w_bn<64, false>(epi, grid, smem, s, mapA, mapB, prm);
+    return mode ? launch_w_bn<128, true>(epi, grid, smem, s, mapA, mapB, prm)
+                : launch_w_bn<128, false>(epi, grid, smem, s, mapA, mapB, prm);
 }

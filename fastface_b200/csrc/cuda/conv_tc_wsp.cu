@@ -199,15 +199,22 @@ static int launch_wsp(int grid, int smem, cudaStream_t s, const CUtensorMap& map
     return tc_launch_ex(kern, grid, smem, s, 2, mapA, mapB, prm);
 }
 
+template <bool CONTRACT>
+static int launch_wsp_mode(int epi, int grid, int smem, cudaStream_t s,
+                           const CUtensorMap& mapA, const CUtensorMap& mapB_half, const TcParams& prm)
+{
+    switch (epi) {
+    case EPI_PLAIN: return launch_wsp<CONTRACT, EPI_PLAIN>(grid, smem, s, mapA, mapB_half, prm);
+    case EPI_SLOPE: return launch_wsp<CONTRACT, EPI_SLOPE>(grid, smem, s, mapA, mapB_half, prm);
+    case EPI_RES_BN:return launch_wsp<CONTRACT, EPI_RES_BN>(grid, smem, s, mapA, mapB_half, prm);
+    case EPI_RES:   return launch_wsp<CONTRACT, EPI_RES>(grid, smem, s, mapA, mapB_half, prm);
+    default:         return launch_wsp<CONTRACT, EPI_RUNTIME>(grid, smem, s, mapA, mapB_half, prm);
+    }
+}
+
 int tc_launch_wsp(int mode, int epi, int grid, int smem, cudaStream_t s,
                   const CUtensorMap& mapA, const CUtensorMap& mapB_half, const TcParams& prm)
 {
-    if (!mode) return launch_wsp<false, EPI_RUNTIME>(grid, smem, s, mapA, mapB_half, prm);
-    switch (epi) {
-    case EPI_PLAIN:  return launch_wsp<true, EPI_PLAIN>(grid, smem, s, mapA, mapB_half, prm);
-    case EPI_SLOPE:  return launch_wsp<true, EPI_SLOPE>(grid, smem, s, mapA, mapB_half, prm);
-    case EPI_RES_BN: return launch_wsp<true, EPI_RES_BN>(grid, smem, s, mapA, mapB_half, prm);
-    case EPI_RES:    return launch_wsp<true, EPI_RES>(grid, smem, s, mapA, mapB_half, prm);
-    default:         return launch_wsp<true, EPI_RUNTIME>(grid, smem, s, mapA, mapB_half, prm);
-    }
+    return mode ? launch_wsp_mode<true>(epi, grid, smem, s, mapA, mapB_half, prm)
+                : launch_wsp_mode<false>(epi, grid, smem, s, mapA, mapB_half, prm);
 }
