@@ -273,7 +273,9 @@ void ffcu_tc_free(TcPlan* p) { delete p; }
 
 // Epilogue warps per set for a launch whose CTAs each see about tiles_per_cta tiles of bn columns.
 // Narrow tiles at large batch: four (per-tile bookkeeping spread over twice the elements); otherwise
-// eight (half the tile latency).  $FF_TC_WPS64 / $FF_TC_WPS128 = 4 or 8 override.
+// eight (half the tile latency).  $FF_TC_WPS64 / $FF_TC_WPS128 = 4 or 8 override.  A 256-column tile that is its CTA's
+// only one is shared by all sixteen: eight leave the other set idle (forward of 64 / 80 / 100 faces 834 / 901 / 1100 ->
+// 823 / 891 / 1094 us; from 128 faces up no difference, and 128-column tiles are 0.5 % slower that way).
 static int tc_epi_wps(int bn, int tiles_per_cta)
 {
     static int w64 = -1, w128 = -1;
@@ -281,7 +283,7 @@ static int tc_epi_wps(int bn, int tiles_per_cta)
     if (w128 < 0) { const char* e = getenv("FF_TC_WPS128"); w128 = (e && (atoi(e) == 4 || atoi(e) == 8)) ? atoi(e) : 0; }
     if (bn == 64) return w64 ? w64 : (tiles_per_cta >= 8 ? 4 : 8);
     if (bn == 128) return w128 ? w128 : 8;
-    return 8;
+    return tiles_per_cta <= 1 ? 16 : 8;
 }
 
 static int g_test_fc_drop_step = -1;

@@ -348,7 +348,7 @@ struct TcParams {
     int flat_P;              // > 0: flat-pitch tiles (weight-stationary pair kernel): a tile is 128 consecutive lines of
                              // an image laid out with a row pitch of flat_P = W + 2 lines (one zero column either side);
                              // the tile walk's digits are then (image, tile-in-image) instead of (w, h, batch) tiles
-    int epi_wps;             // epilogue warps per set, 4 or 8 (16 / epi_wps sets take alternate tiles)
+    int epi_wps;             // epilogue warps per set, 4, 8 or 16 (16 / epi_wps sets take alternate tiles)
     long long full_wait;     // cycle limit of the MMA issuer's wait for a pipeline stage's data (TC_WAIT_CYCLES)
     int drop_stage;          // >= 0: the producer neither arms nor loads this K step of its first tile, so the
                              // issuer's wait for it must run out (ffcu_test_arm_timeout; -1 in every other launch)
@@ -388,14 +388,22 @@ struct TcShared {                 // lives after the stage ring and the tables
     uint64_t acc_full[TC_MAX_ACC];
     uint64_t acc_empty[TC_MAX_ACC];
     uint64_t w_full;              // weight-stationary kernel: weights have landed
+    uint64_t lut_full;            // the fused BN's byte table has landed
     uint32_t tmem_base;
     int abort_flag;
 };
 
-__device__ __forceinline__ void tc_load_tables(float* tab, const TcParams& p)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// Per-channel tables -> shared memory, by threads tid, tid + n, ...
+__device__ __forceinline__ void tc_load_tables(float* tab, const TcParams& p, int tid, int n)
 {
 #pragma unroll 1
-    for (int i = threadIdx.x; i < p.Cout; i += TC_THREADS) {
+    for (int i = tid; i < p.Cout; i += n) {
         tab[0 * TC_MAX_COUT + i] = p.t.w_scale[i];
         tab[1 * TC_MAX_COUT + i] = p.t.bias[i];
         tab[2 * TC_MAX_COUT + i] = p.t.slope ? p.t.slope[i] : 0.0f;
@@ -410,15 +418,24 @@ __device__ __forceinline__ void tc_load_tables(float* tab, const TcParams& p)
     }
 }
 
-// The fused BN pass as a byte table in shared memory: lut[c * 256 + (uint8_t)q] for the BN
-// channels [c0, c0 + bn) of this CTA's column tile (a CTA keeps one column tile for its lifetime).
-__device__ __forceinline__ void tc_load_lut(uint8_t* lut, const TcParams& p, int c0, int bn)
+// What only the epilogue needs before its first tile, done by its sixteen warps while the first operands are on their
+// way: the per-channel tables, and the fused BN pass as a byte table (lut[c * 256 + (uint8_t)q] for the CTA's column tile of
+// channels [c0, c0 + bn); a CTA keeps one column tile for its lifetime).  The byte table is one bulk copy: fetched by
+// all threads through registers before the role split it held up the whole CTA for seven L2 round trips at 64 KB
+// (14x14 residual + BN layer at 17 / 64 faces 9.5 / 16.5 -> 8.8 / 14.6 us; forward of 17 / 32 / 64 / 80 / 256 faces
+// 479 / 622 / 833 / 900 / 2073 -> 448 / 581 / 782 / 834 / 2043 us, the shared epilogue of single wide tiles included).
+__device__ __forceinline__ bool tc_epi_prologue(float* tab, uint8_t* lut, const TcParams& p, TcShared* sh, int c0, int bn,
+                                                volatile int* abort_flag)
 {
-    if (!p.out2 || !p.lut_bytes) return;
-    const int4* src = (const int4*)(p.t.bn_lut + (size_t)c0 * 256);
-    int4* dst = (int4*)lut;
-#pragma unroll 1
-    for (int i = threadIdx.x; i < bn * 16; i += TC_THREADS) dst[i] = __ldg(src + i);
+    const int tid = (int)threadIdx.x - 64;                // epilogue warps are 2 .. 17
+    const bool has_lut = p.out2 && p.lut_bytes;
+    if (tid == 0 && has_lut) {
+        mbar_expect_tx(smem_u32(&sh->lut_full), (uint32_t)bn * 256u);
+        bulk_load(smem_u32(lut), p.t.bn_lut + (size_t)c0 * 256, (uint32_t)bn * 256u, smem_u32(&sh->lut_full));
+    }
+    tc_load_tables(tab, p, tid, 512);
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    return !has_lut || mbar_wait(smem_u32(&sh->lut_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
 }
 
 // 32-byte global accesses (sm_100 has 256-bit vector loads / stores): one full sector per
@@ -650,7 +667,7 @@ __device__ __forceinline__ void walk_next(TileWalk& w, const TcParams& p)
 // fused BN comes with its byte table, no accumulator dump is asked for; everything else runs the
 // EPI_RUNTIME variant.
 template <int BN, bool CONTRACT, bool OUT_F32, int EPI, bool ACC22 = false>
-__device__ __forceinline__ void tc_epilogue_role(const TcParams& p, const float* tab, const uint8_t* lut, TcShared* sh,
+__device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, uint8_t* lut, TcShared* sh,
                                                  uint32_t tmem_base, volatile int* abort_flag, int warp, int lane,
                                                  int first, int step, int total, int m_mul, int m_off,
                                                  uint32_t remote_acc_empty /* 0: local barrier */)
@@ -674,9 +691,10 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, const float*
     const bool check = (EPI == EPI_RUNTIME) && !p.t.no_overflow;
     const bool dump = (EPI == EPI_RUNTIME) && p.acc_out != nullptr;
     int local = set;
-    bool ok = true;
     const int tn = first % p.tiles_n;
     const int c0 = tn * BN + cg * cols;                   // first channel of this warp's range
+    bool ok = tc_epi_prologue(tab, lut, p, sh, tn * BN, BN, abort_flag);
+    tc_pdl_wait();
     const uint32_t lut0 = smem_u32(lut) + (uint32_t)(cg * cols) * 256u;
     first += set * step;
     step *= sets;
@@ -779,6 +797,7 @@ __device__ __forceinline__ void tc_setup(TcShared* sh, int stages, uint32_t tmem
         for (int s = 0; s < stages; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         for (int a = 0; a < TC_MAX_ACC; a++) { mbar_init(smem_u32(&sh->acc_full[a]), 1); mbar_init(smem_u32(&sh->acc_empty[a]), epi_active); }
         mbar_init(smem_u32(&sh->w_full), 1);
+        mbar_init(smem_u32(&sh->lut_full), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -28,8 +28,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int lane = threadIdx.x & 31;
     const int kblocks = p.taps * p.cin_blocks;
 
-    tc_load_tables(tab, p);
-    tc_load_lut(lut, p, (int)(blockIdx.x % p.tiles_n) * BN, BN);
     tc_setup(sh, p.stages, TMEM_COLS, warp, p.epi_wps);
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
@@ -160,7 +158,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             }
         }
     } else {
-        tc_pdl_wait();
         tc_epilogue_role<BN, CONTRACT, OUT_F32, EPI, (KC == 64 && EPI != EPI_RUNTIME && !OUT_F32)>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
                                                 blockIdx.x, gridDim.x, p.total_tiles, 1, 0, 0u);
     }

@@ -43,12 +43,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const int m_tiles = p.tiles_w * p.tiles_h * p.tiles_b;
     const int total = p.tiles_n * ((m_tiles + 1) >> 1);  // pair tiles
 
-    tc_load_tables(tab, p);
-    tc_load_lut(lut, p, (int)(pair_id % p.tiles_n) * BN, BN);
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         for (int a = 0; a < TC_MAX_ACC; a++) { mbar_init(smem_u32(&sh->acc_full[a]), 1); mbar_init(smem_u32(&sh->acc_empty[a]), 2 * p.epi_wps); }
         mbar_init(smem_u32(&sh->w_full), 1);
+        mbar_init(smem_u32(&sh->lut_full), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -62,7 +61,6 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     __syncthreads();
     cluster_sync_all();                                  // peer's barriers are initialised
     tc_fence_after();
-    tc_pdl_wait();
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
@@ -89,6 +87,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             const int tn = pair_id % p.tiles_n;
             TileWalk wk;
             walk_init(wk, p, (pair_id / p.tiles_n) * 2 + (int)rank, (n_pairs / p.tiles_n) * 2);
+            tc_pdl_wait();
             for (int tile = pair_id; tile < total && ok; tile += n_pairs, walk_next(wk, p)) {
                 const int tw = wk.tw, th = wk.th, tb = wk.tb;   // tb may be past the batch: TMA zero-fills
                 const int x0 = tw * p.TW * p.stride - p.pad;

@@ -17,10 +17,10 @@
 #define SC_BN 64
 #define SC_SLOTS (TC_NACC(SC_BN) / 2)          // tiles in flight: two accumulators each
 
-__device__ __forceinline__ void sc_load_tables(float* tab, const EpiTables& t, int Cout)
+__device__ __forceinline__ void sc_load_tables(float* tab, const EpiTables& t, int Cout, int tid)
 {
 #pragma unroll 1
-    for (int i = threadIdx.x; i < Cout; i += TC_THREADS) {
+    for (int i = tid; i < Cout; i += 512) {
         tab[0 * TC_MAX_COUT + i] = t.w_scale[i];
         tab[1 * TC_MAX_COUT + i] = t.bias[i];
         tab[2 * TC_MAX_COUT + i] = t.slope ? t.slope[i] : 0.0f;
@@ -57,14 +57,6 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int n_steps = kblocks / G;
     const int tn = blockIdx.x % p.tiles_n;
 
-    sc_load_tables(tab1, p.t, p.Cout);
-    sc_load_tables(tab2, q.t2, p.Cout);
-    if (q.lut_bytes) {
-        const int4* src = (const int4*)(q.t2.bn_lut + (size_t)tn * BN * 256);
-        int4* dst = (int4*)lut;
-#pragma unroll 1
-        for (int i = threadIdx.x; i < BN * 16; i += TC_THREADS) dst[i] = __ldg(src + i);
-    }
     tc_setup(sh, p.stages, TMEM_COLS, warp, p.epi_wps);
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
@@ -160,6 +152,15 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         }
     } else if (warp < TC_ISSUER2_WARP) {
         // Epilogue: 16 / wps sets of wps warps on alternate tiles; a warp = (TMEM lane quarter, column group).
+        // First the tables, while the first operands are on their way (as tc_epi_prologue).
+        if (threadIdx.x == 64 && q.lut_bytes) {
+            mbar_expect_tx(smem_u32(&sh->lut_full), BN * 256u);
+            bulk_load(smem_u32(lut), q.t2.bn_lut + (size_t)tn * BN * 256, BN * 256u, smem_u32(&sh->lut_full));
+        }
+        sc_load_tables(tab1, p.t, p.Cout, (int)threadIdx.x - 64);
+        sc_load_tables(tab2, q.t2, p.Cout, (int)threadIdx.x - 64);
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        bool ok = !q.lut_bytes || mbar_wait(smem_u32(&sh->lut_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
         tc_pdl_wait();
         const int wps = p.epi_wps;
         const int sets = TC_EPI_TOTAL_WARPS / wps;
@@ -178,7 +179,6 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const uint32_t lut0 = smem_u32(lut) + (uint32_t)(cg * cols) * 256u;
         // this set's tiles: set, set + sets, ... of the CTA's; tile slot and phase follow the CTA's tile count
         int local = set;
-        bool ok = true;
         TileWalk wk;
         walk_init(wk, p, (int)(blockIdx.x + set * gridDim.x) / p.tiles_n, (int)(gridDim.x * sets) / p.tiles_n);
         for (int tile = blockIdx.x + set * gridDim.x; tile < p.total_tiles && ok;

@@ -78,8 +78,6 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    tc_load_tables(tab, p);
-    tc_load_lut(lut, p, 0, BN);
     if (IN_U8) {
         // An 8-bit pixel has 256 values: normalise and quantise each once, with the arithmetic of the fp32
         // path ((p - 127.5) / 127.5 in fp32, then x * inv, lrintf, clamp), and let the producers look it up.
@@ -90,7 +88,6 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
         }
     }
     tc_setup(sh, p.stages, TMEM_COLS, warp, p.epi_wps);
-    tc_pdl_wait();
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
@@ -101,6 +98,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
             mbar_expect_tx(smem_u32(&sh->w_full), W_BYTES);
             tma_load_4d(smem_u32(s_w), &mapB, smem_u32(&sh->w_full), 0, 0, 0, 0);
         }
+        tc_pdl_wait();
         const float i0 = __ldg(inv3), i1 = __ldg(inv3 + 1), i2 = __ldg(inv3 + 2);
         uint32_t* patch = s_patch[me];
         bool ok = true;

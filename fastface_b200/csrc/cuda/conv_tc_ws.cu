@@ -39,10 +39,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    tc_load_tables(tab, p);
-    tc_load_lut(lut, p, 0 * BN, BN);
     tc_setup(sh, p.stages, TMEM_COLS, warp, p.epi_wps);
-    tc_pdl_wait();
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
@@ -53,6 +50,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             if (lane == 0) mbar_expect_tx(wbar, W_BYTES);
             __syncwarp();
             if (lane < 9) tma_load_4d(smem_u32(s_w + lane * W_TAP_BYTES), &mapB, wbar, lane * p.Cp, 0, 0, 0);
+            tc_pdl_wait();                               // the weights are no kernel's output: requested before the wait
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             TileWalk wk;

@@ -51,12 +51,11 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const int pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int total = p.total_tiles;                      // pair tiles: (images / 2) x tiles per image
 
-    tc_load_tables(tab, p);
-    tc_load_lut(lut, p, 0, BN);
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         for (int a = 0; a < TC_MAX_ACC; a++) { mbar_init(smem_u32(&sh->acc_full[a]), 1); mbar_init(smem_u32(&sh->acc_empty[a]), 2 * p.epi_wps); }
         mbar_init(smem_u32(&sh->w_full), 1);
+        mbar_init(smem_u32(&sh->lut_full), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -164,7 +163,6 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             }
         }
     } else {
-        tc_pdl_wait();
         const uint32_t leader_acc_empty = map_to_cta(smem_u32(&sh->acc_empty[0]), 0);
         tc_epilogue_role<BN, CONTRACT, false, EPI>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
                                                    pair_id, n_pairs, total, 2, (int)rank, leader_acc_empty);
