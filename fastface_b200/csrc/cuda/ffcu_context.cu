@@ -2,6 +2,7 @@
 // launch list, submit / wait, dump points and the resident-input timing loop.
 
 #include "ffcu_internal.cuh"
+#include "cos_sim.cuh"
 #include <math.h>
 
 #include <stdarg.h>
@@ -86,6 +87,7 @@ struct ffcu_ctx {
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
+    CosWorkspace cos;            // similarity matrices (cos_sim.cu): has its own stream, is made by the first one
 };
 
 extern "C" int ffcu_device_count(void)
@@ -185,6 +187,7 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     }
     cudaFree(c->d_err); cudaFree(c->d_fc_scratch); cudaFree(c->d_fc_tc_scratch);
     if (c->h_err) cudaFreeHost(c->h_err);
+    c->cos.release();
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->s_in) cudaStreamDestroy(c->s_in);
     if (c->s_out) cudaStreamDestroy(c->s_out);
@@ -651,6 +654,12 @@ extern "C" int ffcu_wait(ffcu_ctx* c)
         return 1000 + e;
     }
     return 0;
+}
+
+extern "C" int ffcu_ctx_cos_sim_matrix(ffcu_ctx* c, const float* a, int n, const float* b, int m, float* out)
+{
+    if (!c) { ffcu_set_error("ffcu_ctx_cos_sim_matrix: NULL context"); return -1; }
+    return c->cos.call(c->device, a, n, b, m, out);
 }
 
 extern "C" int ffcu_trace(ffcu_ctx* c, const float* host_in, int n, float* host_out,

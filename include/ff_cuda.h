@@ -177,6 +177,9 @@ int ffcu_fc_small_noalloc(const int8_t* act, const int8_t* w, const float* w_sca
 /* Cosine-similarity matrix out[n][m] of host embeddings a[n][512], b[m][512] with the float64
  * accumulation of the reference's Go wrapper (go/fastface/fastface.go:157-168), bit for bit. */
 int ffcu_cos_sim_matrix(int device, const float* a, int n, const float* b, int m, float* out);
+/* The same on the context's device, with device buffers (at most 44 MB) that the context keeps from its first call to
+ * ffcu_destroy.  May be called from several threads at once, also beside ffcu_submit. */
+int ffcu_ctx_cos_sim_matrix(ffcu_ctx* c, const float* a, int n, const float* b, int m, float* out);
 
 /* Dense INT8 tensor-core throughput (TOP/s, 2 ops per MAC) measured with operands already in
  * shared memory: M=128, N=bn (64/128/256), all SMs busy, `iters` rounds of four K=32 MMAs.

@@ -1,0 +1,77 @@
+"""Similarity matrix at the edges of its tiles and slices: the bits of fastface_cos_sim for every pair looked at."""
+import threading
+
+import numpy as np
+import pytest
+
+import fastface_b200 as ff
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine(built_lib, model_root, ffw4):
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=2) as e:
+        yield e
+
+
+def check(got, a, b, rng, count=400):
+    n, m = len(a), len(b)
+    assert got.shape == (n, m)
+    edge_i = [i for i in (0, 15, 16, 63, 64, n - 65, n - 2, n - 1, 2047, 2048) if 0 <= i < n]
+    edge_j = [j for j in (0, 63, 64, 65, m - 66, m - 2, m - 1, 4095, 4096) if 0 <= j < m]
+    pairs = [(i, j) for i in edge_i for j in edge_j]
+    pairs += [(int(rng.integers(n)), int(rng.integers(m))) for _ in range(count)]
+    want = np.array([ff.FastFace.cos_sim(a[i], b[j]) for i, j in pairs], np.float32)
+    have = np.array([got[i, j] for i, j in pairs], np.float32)
+    same = (have.view(np.uint32) == want.view(np.uint32)) | (np.isnan(have) & np.isnan(want))
+    assert same.all(), [pairs[k] for k in np.flatnonzero(~same)[:5]]
+
+
+# 16- and 64-row blocks (32 | 33 rows, and 64-row blocks only where they fill half the SMs), ragged last tiles, one
+# slice and several of 2048 x 4096
+@pytest.mark.parametrize("n,m", [(1, 1), (1, 4097), (15, 65), (17, 64), (32, 4736), (33, 4737), (33, 100), (64, 4736), (65, 4800),
+                                 (1000, 333), (2049, 130), (70, 8193), (2049, 4097)])
+def test_matrix_edges(engine, n, m):
+    rng = np.random.default_rng(n * 7919 + m)
+    a = rng.standard_normal((n, 512), dtype=np.float32)
+    b = rng.standard_normal((m, 512), dtype=np.float32) * np.float32(7.0)
+    b[m // 2] = 0
+    a[n - 1] *= np.float32(1e-30)
+    check(engine.cos_sim_matrix(a, b), a, b, rng)
+
+
+def test_matrix_special_values(engine):
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal((20, 512), dtype=np.float32)
+    b = rng.standard_normal((70, 512), dtype=np.float32)
+    a[1, 5], a[2, 6], a[3, 7] = np.inf, -np.inf, np.nan
+    a[4] = np.float32(1e-45)            # denormal: the squared norm is representable in float64
+    a[5] = np.float32(3e38)
+    a[6] = np.float32(-0.0)
+    b[1, 5], b[2] = np.nan, 0
+    check(engine.cos_sim_matrix(a, b), a, b, rng, 1400)
+
+
+def test_matrix_from_several_threads(engine):
+    """Calls that overlap on one context (also beside an embedding call) each give their own matrix."""
+    rng = np.random.default_rng(4)
+    sets = [(rng.standard_normal((40 + 100 * k, 512), dtype=np.float32), rng.standard_normal((300 - 50 * k, 512), dtype=np.float32))
+            for k in range(4)]
+    want = [engine.cos_sim_matrix(a, b) for a, b in sets]
+    face = rng.uniform(-1, 1, ff.FACE_SHAPE).astype(np.float32)
+    emb = engine.embed(face)
+    bad = []
+
+    def work(k):
+        for _ in range(20):
+            if not np.array_equal(engine.cos_sim_matrix(*sets[k]).view(np.uint32), want[k].view(np.uint32)):
+                bad.append(k)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in ts]
+    for _ in range(20):
+        if not np.array_equal(engine.embed(face), emb):
+            bad.append("embed")
+    [t.join() for t in ts]
+    assert not bad
