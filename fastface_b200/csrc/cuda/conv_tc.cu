@@ -612,13 +612,14 @@ struct ChainPlan {
     ChainParams prm;
     int smem_bytes;
     int clusters;            // clusters the device holds at once
+    int bn;                  // output channels per CTA: 64 (eight CTAs per face) or 128 (four)
 };
 
 // layers[i]: device pointers of layer i (weights, tables, residual, outputs); all layers are 3x3 stride-1
 // pad-1 convolutions C -> C on an H x W map, layer i + 1 reading what layer i writes (its fused BN's
 // output where it has one).  d_in = the first layer's input (one face, NHWC).  NULL when the shape does
-// not fit the kernel (C / 64 column tiles x row tiles of 128 positions must be exactly eight CTAs).
-ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers)
+// not fit the kernel (C / bn column tiles x row tiles of 128 positions must be exactly a cluster's CTAs).
+ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers)
 {
     encode_tiled_fn enc = get_encode();
     if (!enc || n_layers < 2 || C % 128 != 0 || C > TC_MAX_COUT) return nullptr;
@@ -626,7 +627,7 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_i
     // left-hand slot, and the last tap of the last row reads one line past row H: one more (zero) row.
     int P = 1;
     while (P < W + 1) P <<= 1;
-    const int tiles_n = C / CHAIN_BN;
+    const int tiles_n = C / bn;
     const int tiles_m = (H * P + TC_TILE_M - 1) / TC_TILE_M;
     // rows a CTA holds: the padded rows its row tile's outputs read (first output row .. last + 2)
     int rows = 0;
@@ -637,23 +638,23 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_i
         if (ohi - olo + 3 > rows) rows = ohi - olo + 3;
     }
     rows += (P == W + 1 ? 1 : 0);
-    if (tiles_n * tiles_m != CHAIN_CLUSTER || P > 256 || P % 8 != 0 || rows > 256) return nullptr;
+    if (tiles_n * tiles_m != CHAIN_CLUSTER_OF(bn) || P > 256 || P % 8 != 0 || rows > 256) return nullptr;
     const int planes = C / 128;
     if (planes != 2 && planes != 4) return nullptr;       // the issue loops are built for 256 and 512 channels
     const int plane_bytes = P * rows * 128;
     if (plane_bytes % 1024 != 0) return nullptr;
-    const int fixed = 2 * planes * plane_bytes + CHAIN_BN * 256 + 5 * CHAIN_BN * 4 + 512 /* barriers */ + 1024 /* alignment */;
+    const int fixed = 2 * planes * plane_bytes + bn * 256 + 5 * bn * 4 + 512 /* barriers */ + 1024 /* alignment */;
     // Filter taps per stage of the weight ring (1, or 3 where two such stages fit and $FF_CHAIN_TPS=3 asks for it).
     int tps = 1;
     { const char* e = getenv("FF_CHAIN_TPS"); if (e && (atoi(e) == 1 || atoi(e) == 3) && planes == 2) tps = atoi(e); }
-    while (tps > 1 && (232448 - fixed) / (tps * planes * CHAIN_BN * 128) < 2) tps /= 3;
-    const int stage_bytes = tps * planes * CHAIN_BN * 128;
+    while (tps > 1 && (232448 - fixed) / (tps * planes * bn * 128) < 2) tps /= 3;
+    const int stage_bytes = bn == 128 ? bn * 128 : tps * planes * bn * 128;
     int stages = (232448 - fixed) / stage_bytes;
     if (stages > CHAIN_MAX_STAGES) stages = CHAIN_MAX_STAGES;
     stages &= ~1;                                         // two issuers on alternate stages: the ring must be even
     if (stages < 2) return nullptr;
-    const int clusters = tc_chain_clusters(fixed + stages * stage_bytes);
-    if (clusters < 1) return nullptr;                     // no room for a cluster of eight on this device
+    const int clusters = tc_chain_clusters(bn, fixed + stages * stage_bytes);
+    if (clusters < 1) return nullptr;                     // no room for a cluster on this device
     ChainPlan* p = new ChainPlan();
     p->d_layers = nullptr;
     {
@@ -673,7 +674,7 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_i
         cuuint64_t Ktot = (cuuint64_t)9 * C;
         cuuint64_t dims[4] = {Ktot, (cuuint64_t)C, 1, 1};
         cuuint64_t strides[3] = {Ktot, Ktot * C, Ktot * C};
-        cuuint32_t box[4] = {128, CHAIN_BN, 1, 1};
+        cuuint32_t box[4] = {128, (cuuint32_t)bn, 1, 1};
         cuuint32_t es[4] = {1, 1, 1, 1};
         CUresult r = enc(&h[i].mapB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d.w, dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -695,7 +696,7 @@ ChainPlan* ffcu_chain_plan(int H, int W, int C, int max_batch, const int8_t* d_i
     p->prm.planes = planes; p->prm.plane_bytes = plane_bytes; p->prm.win_rows = rows; p->prm.tiles_n = tiles_n; p->prm.stages = stages; p->prm.tps = tps;
     p->prm.err = nullptr;
     p->smem_bytes = fixed + stages * stage_bytes;
-    p->clusters = clusters;
+    p->clusters = clusters; p->bn = bn;
     return p;
 }
 
@@ -738,7 +739,7 @@ int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaS
         if (!d_ts) cudaMalloc(&d_ts, 64 * 4 * sizeof(unsigned long long));
         prm.ts = d_ts;
         if (++calls == 29 || calls == 30) {
-            int rc = tc_launch_chain(mode, faces, p->smem_bytes, s, p->mapA, prm);
+            int rc = tc_launch_chain(p->bn, mode, faces, p->smem_bytes, s, p->mapA, prm);
             cudaStreamSynchronize(s);
             unsigned long long h[256];
             cudaMemcpy(h, d_ts, sizeof h, cudaMemcpyDeviceToHost);
@@ -750,7 +751,7 @@ int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaS
         }
     }
 #endif
-    return tc_launch_chain(mode, faces, p->smem_bytes, s, p->mapA, prm);
+    return tc_launch_chain(p->bn, mode, faces, p->smem_bytes, s, p->mapA, prm);
 }
 
 // ---------------------------------------------------------------------------

@@ -871,14 +871,14 @@ struct FcTcParams {
 int tc_launch_fc(int mode, int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const FcTcParams& prm);
 
 // Layer chain (conv_tc_chain.cu)
-#define CHAIN_CLUSTER 8
-#define CHAIN_BN 64
+#define CHAIN_BN 64                       // output channels per CTA: 64, or 128 in the wide form
+#define CHAIN_CLUSTER_OF(BN) (512 / (BN))   // CTAs per face: two row tiles of 256 channels, or one of 512
 #define CHAIN_MAX_STAGES 8
 #define CHAIN_EPI_WARPS 16
 #define CHAIN_EPI_THREADS (32 * CHAIN_EPI_WARPS)
 
 struct ChainLayer {                       // one layer of the chain, in global memory (256 bytes, 128-byte aligned)
-    CUtensorMap mapB;                     // weights [Cout][9 * C] K-major, box {128, 64}
+    CUtensorMap mapB;                     // weights [Cout][9 * C] K-major, box {128, 64 or 128}
     const float* w_scale; const float* bias; const float* slope; const float* res_scale; const float* inv_out;
     const int8_t* lut;                    // fused BN byte table [Cout][256], or NULL
     const int8_t* res;                    // residual (NHWC int8), or NULL
@@ -894,8 +894,8 @@ struct ChainParams {
     int H, W, P, C;                       // feature map, pitch in lines, channels (in = out)
     int planes, plane_bytes;              // C / 128 planes of P * win_rows lines of 128 bytes
     int win_rows;                         // padded rows a CTA holds (the rows its row tile reads)
-    int tiles_n;                          // C / 64 column tiles; CHAIN_CLUSTER / tiles_n row tiles
-    int stages;                           // weight ring
+    int tiles_n;                          // C / 64 (wide form: / 128) column tiles
+    int stages;                           // weight ring (wide form: slots of one plane of one tap, two per step)
     int tps;                              // filter taps per stage (1 or 3), planes x 8 KB each
     long long wait_cycles;                // limit of every barrier wait (TC_WAIT_CYCLES unless a test shortened it)
     int drop_step;                        // >= 0: CTA 0's producer leaves out this ring step (ffcu_test_arm_chain_timeout; -1 otherwise)
@@ -906,8 +906,8 @@ struct ChainParams {
 #endif
 };
 
-int tc_launch_chain(int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
-int tc_chain_clusters(int smem);
+int tc_launch_chain(int bn, int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
+int tc_chain_clusters(int bn, int smem);
 
 // Flat-pitch weight-stationary pair kernel: activation buffer = guard + box of WSP_BOX_ROWS image rows
 #define WSP_GUARD_BYTES 1024

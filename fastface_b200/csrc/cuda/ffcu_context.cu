@@ -83,7 +83,7 @@ struct ffcu_ctx {
     int lean_max_batch = 1;
     bool lean_last = false;      // the previous submit took that path
     bool err_copied = false;     // ... and queued the error word's copy already
-    struct Chain { size_t first; int count; ChainPlan* plan; };
+    struct Chain { size_t first; int count; ChainPlan* plan[2]; };   // clusters of eight (64 channels per CTA), of four (128)
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
@@ -171,7 +171,7 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     if (c->s_in) cudaStreamSynchronize(c->s_in);
     if (c->s_out) cudaStreamSynchronize(c->s_out);
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-    for (auto& ch : c->chains) ffcu_chain_free(ch.plan);
+    for (auto& ch : c->chains) for (ChainPlan* q : ch.plan) ffcu_chain_free(q);
     for (auto& L : c->layers) {
         for (TcPlan* q : L.tc_bn) if (q) ffcu_tc_free(q);      // L.tc is one of them
         if (L.stem_tc) ffcu_stem_tc_free(L.stem_tc);
@@ -464,18 +464,22 @@ static void build_chains(ffcu_ctx* c)
                 desc[i].out2 = L.d.bn2_dst_buf >= 0 ? c->bufs[L.d.bn2_dst_buf] : nullptr;
             }
             const ffcu_layer& d0 = c->layers[k].d;
-            ChainPlan* plan = ffcu_chain_plan(d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
-            if (plan) c->chains.push_back({k, count, plan});
+            ffcu_ctx::Chain ch = {k, count, {nullptr, nullptr}};
+            ch.plan[0] = ffcu_chain_plan(64, d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
+            // the wide form serves calls beyond what clusters of eight hold
+            if (ch.plan[0] && c->max_batch > ffcu_chain_clusters(ch.plan[0]))
+                ch.plan[1] = ffcu_chain_plan(128, d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
+            if (ch.plan[0]) c->chains.push_back(ch);
         }
         k = e;
     }
 }
 
 // Largest call that takes the layer chains (each chain's own limit, the clusters the device holds at once, comes on
-// top: one cluster of eight CTAs works on one face, and a second wave of clusters doubles the stage's time).  Measured,
-// forward of 2 / 4 / 8 / 12 / 16 faces, chains against one launch per layer: 300 / 311 / 332 / 363 / 547 us against
-// 366 / 379 / 403 / 445 / 467 on a device that holds 15 clusters.  A context made for two or three faces keeps one
-// launch per layer beyond a single face, the launch count fastface_launches_per_forward has always given there.
+// top: one cluster works on one face, and a second wave of clusters doubles the stage's time).  Measured, forward of
+// 2 / 4 / 8 / 12 faces, chains against one launch per layer: 300 / 311 / 332 / 363 us against 366 / 379 / 403 / 445; the wide
+// form's figures stand in conv_tc_chain.cu.  A context made for two or three faces keeps one launch per layer beyond a
+// single face, the launch count fastface_launches_per_forward has always given there.
 static int chain_max_faces(const ffcu_ctx* c)
 {
     return c->max_batch >= 4 ? FFCU_CHAIN_MAX_FACES : 1;
@@ -490,12 +494,14 @@ static int launch_forward(ffcu_ctx* c, int n)
     for (size_t k = 0; k < c->layers.size(); k++) {
         if (chain_call && !c->no_chain) {
             while (next_chain < c->chains.size() && c->chains[next_chain].first < k) next_chain++;
-            if (next_chain < c->chains.size() && c->chains[next_chain].first == k &&
-                n <= ffcu_chain_clusters(c->chains[next_chain].plan)) {
-                const ffcu_ctx::Chain& ch = c->chains[next_chain];
-                if (ffcu_chain_launch(ch.plan, n, c->mode, c->d_err, c->stream) == 0) {
+            const ChainPlan* plan = nullptr;                // the narrowest clusters the device holds n of at once
+            if (next_chain < c->chains.size() && c->chains[next_chain].first == k)
+                for (const ChainPlan* q : c->chains[next_chain].plan)
+                    if (!plan && q && n <= ffcu_chain_clusters(q)) plan = q;
+            if (plan) {
+                if (ffcu_chain_launch(plan, n, c->mode, c->d_err, c->stream) == 0) {
                     launches++;
-                    k += (size_t)ch.count - 1;
+                    k += (size_t)c->chains[next_chain].count - 1;
                     continue;
                 }
                 // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...):

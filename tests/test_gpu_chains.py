@@ -10,16 +10,16 @@ from oracle import ffo
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2, 4, 15, 16, 17])
+@pytest.mark.parametrize("n", [2, 4, 15, 16, 17, 24, 32, 33, 34, 35, 36, 37, 38])
 def test_small_batch_layer_chains(built_lib, model_root, ffw4, oracle, monkeypatch, n):
-    """One cluster per face, for as many faces as the device holds clusters (15-18, by its GPC sizes): eager, captured
-    and replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
+    """One cluster per face, for as many faces as the device holds clusters (of eight CTAs: 15-18, of four: 32-37, by
+    its GPC sizes; beyond that one launch per layer): eager, captured and replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
     faces = synth.faces(n, seed=500 + n)
     sample = sorted({0, n // 2, n - 1})
     got = {}
     for flag in ("1", "0"):
         monkeypatch.setenv("FF_CHAIN", flag)
-        with ff.FastFace(ffw4, cwd=model_root, max_batch=20) as e:
+        with ff.FastFace(ffw4, cwd=model_root, max_batch=40) as e:
             for mode in (ffo.CONTRACT, ffo.STRICT):
                 e.set_epilogue_mode(mode)
                 for rep in range(3):
