@@ -20,7 +20,7 @@ OBJ = os.path.join(PKG, "csrc", "_obj")
 LIB = os.path.join(PKG, "libfastface_b200.so")
 CLI = os.path.join(PKG, "fastface_int8_b200")     # reference-compatible command-line driver
 
-HOST_SRCS = ["csrc/host/ff_model.c", "csrc/host/ff_plan.c", "csrc/host/fastface_api.c"]
+HOST_SRCS = ["csrc/host/ff_model.c", "csrc/host/ff_plan.c", "csrc/host/ff_copy.c", "csrc/host/fastface_api.c"]
 CUDA_SRCS = ["csrc/cuda/ffcu_context.cu", "csrc/cuda/kernels_simt.cu", "csrc/cuda/conv_tc.cu",
              "csrc/cuda/conv_tc_generic.cu", "csrc/cuda/conv_tc_ws.cu", "csrc/cuda/conv_tc_pair.cu", "csrc/cuda/conv_tc_wsp.cu", "csrc/cuda/conv_tc_chain.cu", "csrc/cuda/conv_tc_sc.cu", "csrc/cuda/conv_tc_fc.cu", "csrc/cuda/conv_tc_stem.cu", "csrc/cuda/peak_probe.cu", "csrc/cuda/cos_sim.cu", "csrc/cuda/fc_small_noalloc.cu", "csrc/cuda/winograd_f23.cu"]
 

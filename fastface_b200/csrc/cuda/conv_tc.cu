@@ -351,10 +351,11 @@ int ffcu_fc_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t,
 }
 
 int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, const int8_t* res,
-                   int32_t* acc_out, void* out, int8_t* out_bn2, int* d_err, cudaStream_t s)
+                   int32_t* acc_out, void* out, int8_t* out_bn2, int* d_err, cudaStream_t s, int b0)
 {
     TcPlan* p = const_cast<TcPlan*>(cp);
-    if (batch < 1 || batch > p->max_batch) { ffcu_set_error("tc launch: batch out of range"); return -1; }
+    if (batch < 1 || b0 < 0 || batch > p->max_batch - b0) { ffcu_set_error("tc launch: batch out of range"); return -1; }
+    if (b0 && (p->pair || p->wsp || p->out_f32)) { ffcu_set_error("tc launch: this kernel starts at face 0"); return -1; }
     const ffcu_layer& d = p->d;
 #ifdef FF_TC_TIMING
     static int dbg = -1;
@@ -376,7 +377,7 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
         TcParams prm = {};
         prm.t = t; prm.res = res; prm.acc_out = acc_out; prm.out = out; prm.err = d_err;
         prm.out2 = (out_bn2 && t.bn_in) ? out_bn2 : nullptr;
-        prm.batch = batch; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
+        prm.batch = batch; prm.b0 = b0; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
         prm.taps = 9; prm.Kw = 3; prm.Cp = 64; prm.cin_blocks = 1; prm.stride = 1; prm.pad = 1;
         prm.TW = WS_TW; prm.TH = WS_TH; prm.TB = 1;
         prm.tiles_w = d.Wo / WS_TW; prm.tiles_h = (d.Ho + WS_TH - 1) / WS_TH; prm.tiles_b = batch; prm.tiles_n = 1;
@@ -394,7 +395,7 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
         TcParams prm = {};
         prm.t = t; prm.res = res; prm.acc_out = acc_out; prm.out = out; prm.err = d_err;
         prm.out2 = (out_bn2 && t.bn_in) ? out_bn2 : nullptr;
-        prm.batch = batch; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
+        prm.batch = batch; prm.b0 = b0; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
         prm.taps = 9; prm.Kw = 3; prm.Cp = 128; prm.cin_blocks = 1; prm.stride = 1; prm.pad = 1;
         prm.TW = TC_TILE_M; prm.TH = 1; prm.TB = 1;        // not used for the mapping: flat_P is set
         prm.flat_P = p->wsp_P;
@@ -426,7 +427,7 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
     TcParams prm = {};
     prm.t = t; prm.res = res; prm.acc_out = acc_out; prm.out = out; prm.err = d_err;
     prm.out2 = (out_bn2 && t.bn_in) ? out_bn2 : nullptr;
-    prm.batch = batch; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
+    prm.batch = batch; prm.b0 = b0; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
     prm.taps = d.Kh * d.Kw; prm.Kw = d.Kw; prm.Cp = d.Cin_pad; prm.cin_blocks = d.Cin_pad / p->KC;
     prm.stride = d.stride; prm.pad = d.pad;
     prm.TW = TW; prm.TH = TH; prm.TB = TB;
@@ -551,11 +552,11 @@ void ffcu_sc_free(ScPlan* sp)
 // t1 / t2: the main path's and the shortcut's tables; out_main: where the main path's int8 output goes when another
 // layer reads it (write_main), out_sc / out2_sc: the block's output and its fused BN output (or NULL).
 int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, const EpiTables& t2, int8_t* out_main,
-                   int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s)
+                   int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s, int b0)
 {
     ScPlan* sp = const_cast<ScPlan*>(csp);
     TcPlan* p = sp->main;
-    if (batch < 1 || batch > p->max_batch) { ffcu_set_error("shortcut-fused launch: batch out of range"); return -1; }
+    if (batch < 1 || b0 < 0 || batch > p->max_batch - b0) { ffcu_set_error("shortcut-fused launch: batch out of range"); return -1; }
     const ffcu_layer& d = p->d;
     int TW, TH, TB;
     pick_geometry(d.Wo, d.Ho, batch, &TW, &TH, &TB);
@@ -581,7 +582,7 @@ int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, 
     }
     TcParams prm = {};
     prm.t = t1; prm.res = nullptr; prm.acc_out = nullptr; prm.out = out_main; prm.out2 = nullptr; prm.err = d_err;
-    prm.batch = batch; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
+    prm.batch = batch; prm.b0 = b0; prm.Ho = d.Ho; prm.Wo = d.Wo; prm.Cout = d.Cout;
     prm.taps = 9; prm.Kw = 3; prm.Cp = d.Cin_pad; prm.cin_blocks = d.Cin_pad / p->KC;
     prm.stride = 2; prm.pad = 1;
     prm.TW = TW; prm.TH = TH; prm.TB = TB;

@@ -337,6 +337,7 @@ struct TcParams {
     int8_t* out2;            // fused BN second output (NULL: none)
     int* err;
     int batch, Ho, Wo, Cout;
+    int b0;                  // first face in the activation map (outputs, residual: the pointers are that face's already)
     int taps, Kw, cin_blocks, Cp;
     int stride, pad;
     int TW, TH, TB;

@@ -80,7 +80,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 const int tw = wk.tw, th = wk.th, tb = wk.tb;   // tb may be past the batch: TMA zero-fills
                 const int x0 = tw * p.TW * p.stride - p.pad;
                 const int y0 = th * p.TH * p.stride - p.pad;
-                const int c3 = is_a ? tb * p.TB : 0;
+                const int c3 = is_a ? p.b0 + tb * p.TB : 0;
                 int c0 = c0_first, kw = kw_first, kh = kh_first;
 #pragma unroll 1
                 for (int it = 0; it < n_steps; it++) {

@@ -56,7 +56,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             TileWalk wk;
             walk_init(wk, p, blockIdx.x, gridDim.x);
             for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x, walk_next(wk, p)) {
-                const int tw = wk.tw, th = wk.th, b = wk.tb;
+                const int tw = wk.tw, th = wk.th, b = p.b0 + wk.tb;
                 ok = mbar_wait(smem_u32(&sh->empty[stage]), phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
                 if (!ok) break;
                 const uint32_t bar = smem_u32(&sh->full[stage]);

@@ -3,14 +3,29 @@
 
 #include "ffcu_internal.cuh"
 #include "cos_sim.cuh"
+#include "../host/ff_copy.h"
 #include <math.h>
 
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <algorithm>
 #include <map>
 #include <vector>
+
+#define OUT_HEAD 64            // bytes in front of an output slot: its error word
+#define STAGE_SLOTS 4          // page-locked ring the input of a pageable call goes through
+#define STAGE_FACES 16         // faces (fp32) per ring slot
+#define STAGE_OUT_FACES 4096   // most faces whose output goes through page-locked memory
+
+// A step of at least this many faces that finds the device idle runs its first layers in chunks while the rest of its input is
+// on its way (submit_impl); below it a call is one stream of copy, forward, copy.  Half a step under 128 faces, 64
+// from there on: smaller chunks fill the SMs worse (these layers take 2.6 us a face at 256 faces, 2.85 at 64, 3.3 at 32) and
+// larger ones leave more of the copy in front (2.8 us a face of fp32).  Calls before -> after, staging included: 256 faces of page-
+// locked fp32 2713 -> 2319 us, 64 pageable 1440 -> 1245, 100 page-locked 8-bit 1190 -> 1167, 1024 of them 8140 -> 7960.
+#define CHUNK_MIN_FACES 40
+#define CHUNK_FACES 64
 
 static thread_local char g_cu_err[512];
 
@@ -56,8 +71,20 @@ struct ffcu_ctx {
     cudaEvent_t ev_in_ready[2] = {}, ev_compute_done[2] = {}, ev_out_copied[2] = {};
     unsigned long long seq = 0;
     int* d_fc_scratch = nullptr; // small-batch FC: 64 ticket counters + int32 [16][512] split-K accumulator (kept zero between calls)
-    int* d_err = nullptr;        // device error word
-    int* h_err = nullptr;        // pinned mirror
+    int* d_err = nullptr;        // device error word of the current slot: in front of its output, so that one copy brings both
+    char* out_mem[2] = {};       // allocation of out_slot[k]: OUT_HEAD bytes, then the embeddings
+    // Page-locked staging.  An input in pageable memory is copied into a ring by several threads (ff_copy.c) and goes
+    // on from there: the driver's own staging is one thread, and for an output it blocks the caller until the forward is done.
+    ff_copy_pool* pool = nullptr;
+    char* stage_in = nullptr;
+    size_t stage_slot_bytes = 0;
+    cudaEvent_t ev_stage[STAGE_SLOTS] = {};
+    unsigned long long stage_seq = 0;
+    char* stage_out[2] = {};     // [OUT_HEAD: error word | embeddings of min(max_batch, STAGE_OUT_FACES) faces]
+    bool err_read[2] = {true, true};                 // the slot's error word is in (or on its way to) stage_out
+    struct Pending { float* dst; size_t bytes; } pending[2] = {};   // output that waits in stage_out for its caller's memory
+    bool idle = true;            // nothing submitted since the last wait
+    int head_end[2] = {};        // layers [0, head_end) a step may run in chunks: fp32 / 8-bit input
     cudaStream_t stream = nullptr;       // compute
     cudaStream_t s_in = nullptr, s_out = nullptr;
     std::vector<DevLayer> layers;
@@ -82,7 +109,6 @@ struct ffcu_ctx {
     // the next call's copy-in with this call's kernels is worth more than the hops it costs from a few faces up).
     int lean_max_batch = 1;
     bool lean_last = false;      // the previous submit took that path
-    bool err_copied = false;     // ... and queued the error word's copy already
     struct Chain { size_t first; int count; ChainPlan* plan[2]; };   // clusters of eight (64 channels per CTA), of four (128)
     std::vector<Chain> chains;
     bool chains_built = false;
@@ -125,15 +151,15 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
     for (int i = 0; i < n_bufs && ok; i++) ok = cudaMalloc(&c->bufs[i], act) == cudaSuccess;
     for (int k = 0; k < 2; k++) {
         ok = ok && cudaMalloc(&c->in_slot[k], (size_t)max_batch * 37632 * sizeof(float)) == cudaSuccess;
-        ok = ok && cudaMalloc(&c->out_slot[k], (size_t)max_batch * 512 * sizeof(float)) == cudaSuccess;
+        ok = ok && cudaMalloc(&c->out_mem[k], OUT_HEAD + (size_t)max_batch * 512 * sizeof(float)) == cudaSuccess;
+        if (ok) { c->out_slot[k] = (float*)(c->out_mem[k] + OUT_HEAD); cudaMemset(c->out_mem[k], 0, OUT_HEAD); }
         ok = ok && cudaEventCreateWithFlags(&c->ev_in_ready[k], cudaEventDisableTiming) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&c->ev_compute_done[k], cudaEventDisableTiming) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&c->ev_out_copied[k], cudaEventDisableTiming) == cudaSuccess;
     }
-    c->d_in = c->in_slot[0]; c->d_out = c->out_slot[0];
+    c->d_in = c->in_slot[0]; c->d_out = c->out_slot[0]; c->d_err = (int*)c->out_mem[0];
     ok = ok && cudaStreamCreateWithFlags(&c->s_in, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&c->s_out, cudaStreamNonBlocking) == cudaSuccess;
-    ok = ok && cudaMalloc(&c->d_err, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMalloc(&c->d_fc_scratch, (FFCU_FC_SMALL_TICKETS + FFCU_FC_SMALL_MAX_BATCH * 512) * sizeof(int)) == cudaSuccess;
     if (ok) cudaMemset(c->d_fc_scratch, 0, (FFCU_FC_SMALL_TICKETS + FFCU_FC_SMALL_MAX_BATCH * 512) * sizeof(int));
     c->fc_tc_rows = (max_batch + 127) / 128 * 128;
@@ -142,9 +168,16 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
         ok = ok && cudaMalloc(&c->d_fc_tc_scratch, nb) == cudaSuccess;
         if (ok) cudaMemset(c->d_fc_tc_scratch, 0, nb);
     }
-    ok = ok && cudaHostAlloc(&c->h_err, sizeof(int), cudaHostAllocDefault) == cudaSuccess;
+    for (int k = 0; k < 2 && ok; k++) {
+        const size_t nb = OUT_HEAD + (size_t)std::min(max_batch, STAGE_OUT_FACES) * 512 * sizeof(float);
+        ok = cudaHostAlloc(&c->stage_out[k], nb, cudaHostAllocDefault) == cudaSuccess;
+        if (ok) *(int*)c->stage_out[k] = 0;
+    }
+    c->stage_slot_bytes = (size_t)std::min(max_batch, STAGE_FACES) * 37632 * sizeof(float);
+    ok = ok && cudaHostAlloc(&c->stage_in, STAGE_SLOTS * c->stage_slot_bytes, cudaHostAllocDefault) == cudaSuccess;
+    for (int k = 0; k < STAGE_SLOTS && ok; k++) ok = cudaEventCreateWithFlags(&c->ev_stage[k], cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && (c->pool = ff_copy_pool_create(3)) != nullptr;
     ok = ok && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess;
-    if (ok) { cudaMemset(c->d_err, 0, sizeof(int)); *c->h_err = 0; }
     const char* impl = getenv("FF_CONV_IMPL");
     c->force_simt = (impl && strcmp(impl, "simt") == 0) ? 1 : 0;
     { const char* e = getenv("FF_FC_SMALL"); c->no_fc_small = (e && e[0] == '0') ? 1 : 0; }
@@ -180,13 +213,16 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     }
     for (int i = 0; i < FFCU_MAX_BUFS; i++) cudaFree(c->bufs[i]);
     for (int k = 0; k < 2; k++) {
-        cudaFree(c->in_slot[k]); cudaFree(c->out_slot[k]);
+        cudaFree(c->in_slot[k]); cudaFree(c->out_mem[k]);
+        if (c->stage_out[k]) cudaFreeHost(c->stage_out[k]);
         if (c->ev_in_ready[k]) cudaEventDestroy(c->ev_in_ready[k]);
         if (c->ev_compute_done[k]) cudaEventDestroy(c->ev_compute_done[k]);
         if (c->ev_out_copied[k]) cudaEventDestroy(c->ev_out_copied[k]);
     }
-    cudaFree(c->d_err); cudaFree(c->d_fc_scratch); cudaFree(c->d_fc_tc_scratch);
-    if (c->h_err) cudaFreeHost(c->h_err);
+    cudaFree(c->d_fc_scratch); cudaFree(c->d_fc_tc_scratch);
+    for (cudaEvent_t ev : c->ev_stage) if (ev) cudaEventDestroy(ev);
+    if (c->stage_in) cudaFreeHost(c->stage_in);
+    ff_copy_pool_destroy(c->pool);
     c->cos.release();
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->s_in) cudaStreamDestroy(c->s_in);
@@ -292,6 +328,38 @@ extern "C" int ffcu_add_layer(ffcu_ctx* c, const ffcu_layer* l)
     return (int)c->layers.size() - 1;
 }
 
+static size_t out_bytes_per_face(const ffcu_layer& d) { return (size_t)d.Ho * d.Wo * d.Cout; }
+
+// The layers a step may run chunk by chunk (submit_impl), each chunk through all of them before the next one starts:
+// the stem alone for 8-bit input (its time is about its input's on PCIe), all leading layers with 64 input
+// channels for fp32 (four times the bytes).  A buffer holds tensors of different bytes per face, so face f of one tensor may
+// lie where a lower face of another does: a head is only taken when no layer of it writes a buffer at fewer bytes
+// per face than the tensor that the rest of the network finds there (then chunk j writes behind all that chunks < j left).
+static void find_heads(ffcu_ctx* c)
+{
+    c->head_end[0] = c->head_end[1] = 0;
+    const size_t nl = c->layers.size();
+    if (nl < 3 || !c->layers[1].fused_stem || !c->layers[1].stem_tc) return;
+    size_t end = 2;
+    while (end < nl && c->layers[end].d.kind == FFCU_CONV && c->layers[end].tc && c->layers[end].d.Cin_pad == 64) end++;
+    for (; end > 2; end--) {
+        if (end < nl && c->layers[end - 1].sc) continue;      // a fused pair stays together
+        std::vector<size_t> left((size_t)c->n_bufs, 0);       // bytes per face of the last tensor the head writes there
+        bool ok = true;
+        for (size_t k = end - 1; k >= 1 && ok; k--) {
+            const ffcu_layer& d = c->layers[k].d;
+            for (int b : {d.dst_buf, d.bn2_dst_buf}) {
+                if (b < 0) continue;
+                if (!left[b]) left[b] = out_bytes_per_face(d);
+                else if (out_bytes_per_face(d) < left[b]) ok = false;
+            }
+        }
+        if (ok) break;
+    }
+    c->head_end[0] = (int)end;
+    c->head_end[1] = 2;
+}
+
 extern "C" int ffcu_finalize(ffcu_ctx* c)
 {
     if (!c) return -1;
@@ -353,6 +421,7 @@ extern "C" int ffcu_finalize(ffcu_ctx* c)
     }
     c->launches = 0;
     for (auto& L : c->layers) if (!L.skip) c->launches++;
+    find_heads(c);
     c->finalized = true;
     return 0;
 }
@@ -387,25 +456,27 @@ static TcPlan* tc_plan_for(ffcu_ctx* c, DevLayer& L, int n)
 
 // Launch layer k for n faces.  acc_dbg (optional) receives the conv's int32 accumulators;
 // unfused = dump-point mode: the stem runs as separate quantise + conv launches.
-static int launch_layer(ffcu_ctx* c, size_t k, int n, int32_t* acc_dbg, bool unfused = false)
+// b0: the launch's first face (layers of a head only).
+static int launch_layer(ffcu_ctx* c, size_t k, int n, int32_t* acc_dbg, bool unfused = false, int b0 = 0)
 {
     DevLayer& L = c->layers[k];
     const ffcu_layer& d = L.d;
     cudaStream_t s = c->stream;
-    int8_t* out2 = d.bn2_dst_buf >= 0 ? c->bufs[d.bn2_dst_buf] : nullptr;
+    const size_t off = (size_t)b0 * out_bytes_per_face(d);
+    int8_t* out2 = d.bn2_dst_buf >= 0 ? c->bufs[d.bn2_dst_buf] + off : nullptr;
     switch (d.kind) {
     case FFCU_QUANT:
         if (L.skip && !unfused) return 0;
         if (c->in_u8) { ffcu_set_error("8-bit pixel input needs the fused stem (FF_FUSE_STEM=0 or a dump-point run is in effect)"); return -1; }
         return ffcu_launch_quant(c->d_in, n * d.H * d.W, L.tab[4], c->bufs[d.dst_buf], s);
     case FFCU_CONV: {
-        const int8_t* res = d.res_buf >= 0 ? c->bufs[d.res_buf] : nullptr;
+        const int8_t* res = d.res_buf >= 0 ? c->bufs[d.res_buf] + off : nullptr;
         if (L.fused_stem && !unfused && L.stem_tc)
-            return ffcu_stem_fused_launch(L.stem_tc, c->d_in, c->in_u8 ? 1 : 0, c->layers[0].tab[4], n, c->mode, L.epi,
-                                          c->bufs[d.dst_buf], out2, c->d_err, s);
+            return ffcu_stem_fused_launch(L.stem_tc, (const char*)c->d_in + (size_t)b0 * 37632 * (c->in_u8 ? 1 : 4), c->in_u8 ? 1 : 0,
+                                          c->layers[0].tab[4], n, c->mode, L.epi, c->bufs[d.dst_buf] + off, out2, c->d_err, s);
         if (L.fused_stem && !unfused)
             return ffcu_launch_stem(c->d_in, c->in_u8 ? 1 : 0, c->layers[0].tab[4], L.w, L.epi, n, c->mode, c->bufs[d.dst_buf], out2, nullptr, s);
-        if (L.tc) return ffcu_tc_launch(tc_plan_for(c, L, n), n, c->mode, L.epi, res, acc_dbg, c->bufs[d.dst_buf], out2, c->d_err, s);
+        if (L.tc) return ffcu_tc_launch(tc_plan_for(c, L, n), n, c->mode, L.epi, res, acc_dbg, c->bufs[d.dst_buf] + off, out2, c->d_err, s, b0);
         return ffcu_launch_conv_simt(d, n, c->mode, c->bufs[d.src_buf], L.w, L.epi, res, acc_dbg, c->bufs[d.dst_buf], out2, s);
     }
     case FFCU_BN:
@@ -485,13 +556,14 @@ static int chain_max_faces(const ffcu_ctx* c)
     return c->max_batch >= 4 ? FFCU_CHAIN_MAX_FACES : 1;
 }
 
-static int launch_forward(ffcu_ctx* c, int n)
+// Layers [k0, k1) for faces b0 .. b0 + n - 1 (b0 > 0 within a head only); c->launches = the launches made.
+static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
 {
     int launches = 0;
     const bool chain_call = n <= chain_max_faces(c);
     if (chain_call && !c->chains_built) build_chains(c);
     size_t next_chain = 0;
-    for (size_t k = 0; k < c->layers.size(); k++) {
+    for (size_t k = k0; k < k1; k++) {
         if (chain_call && !c->no_chain) {
             while (next_chain < c->chains.size() && c->chains[next_chain].first < k) next_chain++;
             const ChainPlan* plan = nullptr;                // the narrowest clusters the device holds n of at once
@@ -516,16 +588,17 @@ static int launch_forward(ffcu_ctx* c, int n)
             if (M.sc && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64) {
                 // stride-2 conv + the block's shortcut, one launch
                 DevLayer& S = c->layers[k + 1];
-                int8_t* out2 = S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] : nullptr;
-                int rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf], M.sc_write_main,
-                                        c->bufs[S.d.dst_buf], out2, c->d_err, c->stream);
+                const size_t off = (size_t)b0 * out_bytes_per_face(S.d);
+                int8_t* out2 = S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] + off : nullptr;
+                int rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf] + off, M.sc_write_main,
+                                        c->bufs[S.d.dst_buf] + off, out2, c->d_err, c->stream, b0);
                 if (rc != 0) return rc;
                 launches++;
                 k++;
                 continue;
             }
         }
-        int rc = launch_layer(c, k, n, nullptr);
+        int rc = launch_layer(c, k, n, nullptr, false, b0);
         if (rc != 0) return rc;
         const DevLayer& L = c->layers[k];
         if (!L.skip) launches++;
@@ -534,12 +607,14 @@ static int launch_forward(ffcu_ctx* c, int n)
     return 0;
 }
 
-// Forward for n faces on the compute stream: replay of a captured graph for small batches
+static int launch_forward(ffcu_ctx* c, int n, int k0 = 0) { return launch_range(c, n, (size_t)k0, c->layers.size(), 0); }
+
+// Forward for n faces on the compute stream, from layer k0 on (a head's end, or 0): replay of a captured graph
 // (after one eager run of that shape, which also sets the kernels' one-time attributes).
-static int run_forward(ffcu_ctx* c, int n, int slot)
+static int run_forward(ffcu_ctx* c, int n, int slot, int k0 = 0)
 {
-    if (n > c->graph_max_batch) return launch_forward(c, n);
-    const long long key = ((long long)n << 8) | ((long long)c->mode << 4) | (c->in_u8 ? 2 : 0) | slot;
+    if (n > c->graph_max_batch) return launch_forward(c, n, k0);
+    const long long key = ((long long)n << 16) | ((long long)k0 << 8) | ((long long)c->mode << 4) | (c->in_u8 ? 2 : 0) | slot;
     auto it = c->graphs.find(key);
     if (it != c->graphs.end()) {
         FFCU_CHECK(cudaGraphLaunch(it->second, c->stream));
@@ -548,31 +623,81 @@ static int run_forward(ffcu_ctx* c, int n, int slot)
     }
     auto seen = c->graph_launches.find(key);
     if (seen == c->graph_launches.end()) {          // first time: eager
-        int rc = launch_forward(c, n);
+        int rc = launch_forward(c, n, k0);
         if (rc == 0) c->graph_launches[key] = c->launches;
         return rc;
     }
-    if (c->graphs.size() >= 64) return launch_forward(c, n);   // a serving loop with many distinct batch sizes: stay eager beyond 64 graphs
+    if (c->graphs.size() >= 64) return launch_forward(c, n, k0);   // a serving loop with many distinct batch sizes: stay eager beyond 64 graphs
     cudaGraph_t graph = nullptr;
     FFCU_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = launch_forward(c, n);
+    int rc = launch_forward(c, n, k0);
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc != 0 || e != cudaSuccess || !graph) {
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
         c->graph_max_batch = 0;                     // capture not possible here: stay eager
-        return rc != 0 ? rc : launch_forward(c, n);
+        return rc != 0 ? rc : launch_forward(c, n, k0);
     }
     cudaGraphExec_t exec = nullptr;
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess || !exec) { cudaGetLastError(); c->graph_max_batch = 0; return launch_forward(c, n); }
+    if (e != cudaSuccess || !exec) { cudaGetLastError(); c->graph_max_batch = 0; return launch_forward(c, n, k0); }
     c->graphs[key] = exec;
     FFCU_CHECK(cudaGraphLaunch(exec, c->stream));
     return 0;
 }
 
-static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, bool u8, int n, float* host_out)
+// Memory that CUDA knows nothing of, first byte and last: what the driver would copy from or to by a staging of its own.
+static bool is_pageable(const void* p, size_t bytes)
+{
+    for (const char* q : {(const char*)p, (const char*)p + bytes - 1}) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (a.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
+
+// Host -> device on stream s; a pageable source goes through the ring (and has been read when this returns).
+static int copy_in(ffcu_ctx* c, void* dst, const void* src, size_t bytes, bool staged, cudaStream_t s)
+{
+    if (!staged) { FFCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s)); return 0; }
+    for (size_t o = 0; o < bytes; o += c->stage_slot_bytes, c->stage_seq++) {
+        const size_t nb = std::min(c->stage_slot_bytes, bytes - o);
+        const int k = (int)(c->stage_seq % STAGE_SLOTS);
+        char* ring = c->stage_in + (size_t)k * c->stage_slot_bytes;
+        if (c->stage_seq >= STAGE_SLOTS) FFCU_CHECK(cudaEventSynchronize(c->ev_stage[k]));      // the slot's last copy has left it
+        ff_copy(c->pool, ring, (const char*)src + o, nb);
+        FFCU_CHECK(cudaMemcpyAsync((char*)dst + o, ring, nb, cudaMemcpyHostToDevice, s));
+        FFCU_CHECK(cudaEventRecord(c->ev_stage[k], s));
+    }
+    return 0;
+}
+
+// The slot's embeddings and error word -> host, on stream s behind the forward.
+static int copy_out(ffcu_ctx* c, int slot, int n, float* host_out, cudaStream_t s)
+{
+    const size_t nb = (size_t)n * 512 * sizeof(float);
+    if (n <= STAGE_OUT_FACES && is_pageable(host_out, nb)) {
+        FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], OUT_HEAD + nb, cudaMemcpyDeviceToHost, s));
+        c->pending[slot] = {host_out, nb};
+    } else {
+        FFCU_CHECK(cudaMemcpyAsync(host_out, c->out_slot[slot], nb, cudaMemcpyDeviceToHost, s));
+        FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
+    c->err_read[slot] = true;
+    return 0;
+}
+
+// Hands a finished copy's output on to its caller's memory.
+static void deliver(ffcu_ctx* c, int slot)
+{
+    if (!c->pending[slot].dst) return;
+    ff_copy(c->pool, c->pending[slot].dst, c->stage_out[slot] + OUT_HEAD, c->pending[slot].bytes);
+    c->pending[slot].dst = nullptr;
+}
+
+static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, bool u8, int n, float* host_out, bool single)
 {
     if (!c || !c->finalized || !host_in || !host_out || n < 1 || n > c->max_batch) {
         ffcu_set_error("ffcu_submit: bad arguments");
@@ -581,47 +706,74 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
     FFCU_CHECK(cudaSetDevice(c->device));
     const int slot = (int)(c->seq & 1);
     const bool reused = c->seq >= 2;
-    if (n <= c->lean_max_batch) {
-        // Latency path (a handful of faces): copy-in, forward and copy-out in order on the compute stream.  The three-
-        // stream pipeline below buys overlap a small batch has no use for and costs it two cross-stream hops and a
-        // dozen driver calls per face.
+    const bool staged = is_pageable(host_in, (size_t)n * bytes_per_face);
+    const bool was_idle = c->idle;
+    c->idle = false;
+    if (c->pending[slot].dst) {                       // the output two steps ago still sits in the slot's staging
+        if (c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->stream));
+        else              FFCU_CHECK(cudaEventSynchronize(c->ev_out_copied[slot]));
+        deliver(c, slot);
+    }
+    c->d_in = c->in_slot[slot]; c->d_out = c->out_slot[slot]; c->d_err = (int*)c->out_mem[slot];
+    if (n <= c->lean_max_batch || (single && c->lean_max_batch > 0 && n < CHUNK_MIN_FACES)) {
+        // Latency path (a handful of faces, or a call that is one small step): copy-in, forward and copy-out in order on
+        // the compute stream.  The three-stream pipeline below buys overlap such a call has no use for and costs it two
+        // cross-stream hops and a dozen driver calls.
         if (!c->lean_last) {                          // the pipeline's copy streams may still hold the slots
             FFCU_CHECK(cudaStreamSynchronize(c->s_in));
             FFCU_CHECK(cudaStreamSynchronize(c->s_out));
+            for (int k = 0; k < 2; k++) deliver(c, k);
             c->lean_last = true;
         }
-        FFCU_CHECK(cudaMemcpyAsync(c->in_slot[slot], host_in, (size_t)n * bytes_per_face, cudaMemcpyHostToDevice, c->stream));
-        c->d_in = c->in_slot[slot]; c->d_out = c->out_slot[slot];
-        c->in_u8 = u8;
-        int rc = run_forward(c, n, slot);
-        c->in_u8 = false;
+        int rc = copy_in(c, c->in_slot[slot], host_in, (size_t)n * bytes_per_face, staged, c->stream);
         if (rc != 0) return rc;
-        FFCU_CHECK(cudaMemcpyAsync(host_out, c->out_slot[slot], (size_t)n * 512 * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-        FFCU_CHECK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        c->err_copied = true;
+        c->in_u8 = u8;
+        rc = run_forward(c, n, slot);
+        c->in_u8 = false;
+        if (rc == 0) rc = copy_out(c, slot, n, host_out, c->stream);
+        if (rc != 0) return rc;
         c->seq++;
         return 0;
     }
     if (c->lean_last) {                               // back to the pipeline: the compute stream owns the slots until it drains
         FFCU_CHECK(cudaStreamSynchronize(c->stream));
+        for (int k = 0; k < 2; k++) deliver(c, k);
         c->lean_last = false;
     }
     // copy-in stream: the slot is free once the forward that last read it has finished
     if (reused) FFCU_CHECK(cudaStreamWaitEvent(c->s_in, c->ev_compute_done[slot], 0));
-    FFCU_CHECK(cudaMemcpyAsync(c->in_slot[slot], host_in, (size_t)n * bytes_per_face, cudaMemcpyHostToDevice, c->s_in));
-    FFCU_CHECK(cudaEventRecord(c->ev_in_ready[slot], c->s_in));
-    // compute stream: needs the input, and the output slot drained by the copy-out of two steps ago
-    FFCU_CHECK(cudaStreamWaitEvent(c->stream, c->ev_in_ready[slot], 0));
+    int rc = 0, head = 0, head_launches = 0;
+    if (was_idle && n >= CHUNK_MIN_FACES) head = c->head_end[u8 ? 1 : 0];
+    // A step that finds the device idle has nothing to hide its copy behind but its own layers: the first ones run
+    // chunk by chunk as the input arrives.
+    const int chunk = !head ? n : n >= 2 * CHUNK_FACES ? CHUNK_FACES : (n + 1) / 2;
+    for (int f = 0; f < n; f += chunk) {
+        const int cnt = std::min(chunk, n - f);
+        rc = copy_in(c, (char*)c->in_slot[slot] + (size_t)f * bytes_per_face, (const char*)host_in + (size_t)f * bytes_per_face,
+                     (size_t)cnt * bytes_per_face, staged, c->s_in);
+        if (rc != 0) return rc;
+        FFCU_CHECK(cudaEventRecord(c->ev_in_ready[slot], c->s_in));
+        FFCU_CHECK(cudaStreamWaitEvent(c->stream, c->ev_in_ready[slot], 0));
+        if (head) {
+            c->in_u8 = u8;
+            rc = launch_range(c, cnt, 0, (size_t)head, f);
+            c->in_u8 = false;
+            if (rc != 0) return rc;
+            head_launches = c->launches;
+        }
+    }
+    // compute stream: needs the output slot drained by the copy-out of two steps ago
     if (reused) FFCU_CHECK(cudaStreamWaitEvent(c->stream, c->ev_out_copied[slot], 0));
-    c->d_in = c->in_slot[slot]; c->d_out = c->out_slot[slot];
     c->in_u8 = u8;
-    int rc = run_forward(c, n, slot);
+    rc = run_forward(c, n, slot, head);
     c->in_u8 = false;
     if (rc != 0) return rc;
+    c->launches += head_launches;
     FFCU_CHECK(cudaEventRecord(c->ev_compute_done[slot], c->stream));
     // copy-out stream
     FFCU_CHECK(cudaStreamWaitEvent(c->s_out, c->ev_compute_done[slot], 0));
-    FFCU_CHECK(cudaMemcpyAsync(host_out, c->out_slot[slot], (size_t)n * 512 * sizeof(float), cudaMemcpyDeviceToHost, c->s_out));
+    rc = copy_out(c, slot, n, host_out, c->s_out);
+    if (rc != 0) return rc;
     FFCU_CHECK(cudaEventRecord(c->ev_out_copied[slot], c->s_out));
     c->seq++;
     return 0;
@@ -629,37 +781,66 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
 
 extern "C" int ffcu_submit(ffcu_ctx* c, const float* host_in, int n, float* host_out)
 {
-    return submit_impl(c, host_in, 37632 * sizeof(float), false, n, host_out);
+    return submit_impl(c, host_in, 37632 * sizeof(float), false, n, host_out, false);
 }
 
 extern "C" int ffcu_submit_u8(ffcu_ctx* c, const uint8_t* host_pixels, int n, float* host_out)
 {
-    return submit_impl(c, host_pixels, 37632, true, n, host_out);
+    return submit_impl(c, host_pixels, 37632, true, n, host_out, false);
+}
+
+extern "C" int ffcu_run(ffcu_ctx* c, const float* host_in, const uint8_t* host_pixels, int n, float* host_out)
+{
+    if (!c || (!host_in && !host_pixels) || !host_out || n < 1) { ffcu_set_error("ffcu_run: bad arguments"); return -1; }
+    const bool u8 = host_pixels != nullptr;
+    const size_t bytes = 37632 * (u8 ? 1 : sizeof(float));
+    const char* in = u8 ? (const char*)host_pixels : (const char*)host_in;
+    int rc = 0;
+    for (int done = 0; done < n && rc == 0; ) {
+        const int step = std::min(n - done, c->max_batch);
+        rc = submit_impl(c, in + (size_t)done * bytes, bytes, u8, step, host_out + (size_t)done * 512, n <= c->max_batch);
+        done += step;
+    }
+    const int wrc = ffcu_wait(c);
+    return rc != 0 ? rc : wrc;
+}
+
+static int wait_impl(ffcu_ctx* c)
+{
+    FFCU_CHECK(cudaSetDevice(c->device));
+    for (int k = 0; k < 2; k++)
+        if (!c->err_read[k]) FFCU_CHECK(cudaMemcpyAsync(c->stage_out[k], c->out_mem[k], sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_in));
+    FFCU_CHECK(cudaStreamSynchronize(c->stream));
+    if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_out));
+    c->idle = true;
+    int err = 0;
+    for (int k = 0; k < 2; k++) {
+        c->err_read[k] = true;
+        deliver(c, k);
+        if (err == 0) err = *(int*)c->stage_out[k];
+    }
+    if (err != 0) {
+        ffcu_set_error("device reported error word %d (a bounded wait inside a kernel ran out)", err);
+        for (int k = 0; k < 2; k++) {
+            *(int*)c->stage_out[k] = 0;
+            cudaMemsetAsync(c->out_mem[k], 0, sizeof(int), c->stream);
+        }
+        // a launch that gave up may have left partial sums or tickets behind
+        cudaMemsetAsync(c->d_fc_scratch, 0, (FFCU_FC_SMALL_TICKETS + FFCU_FC_SMALL_MAX_BATCH * 512) * sizeof(int), c->stream);
+        cudaMemsetAsync(c->d_fc_tc_scratch, 0, ((size_t)FFCU_FC_TC_TICKETS + (size_t)c->fc_tc_rows * 512) * sizeof(int), c->stream);
+        return 1000 + err;
+    }
+    return 0;
 }
 
 extern "C" int ffcu_wait(ffcu_ctx* c)
 {
     if (!c) return -1;
-    FFCU_CHECK(cudaSetDevice(c->device));
-    if (c->lean_last && c->err_copied) {
-        FFCU_CHECK(cudaStreamSynchronize(c->stream));    // the error word's copy was queued behind the forward
-    } else {
-        FFCU_CHECK(cudaStreamSynchronize(c->s_in));
-        FFCU_CHECK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        FFCU_CHECK(cudaStreamSynchronize(c->stream));
-        FFCU_CHECK(cudaStreamSynchronize(c->s_out));
-    }
-    c->err_copied = false;
-    if (*c->h_err != 0) {
-        ffcu_set_error("device reported error word %d (a bounded wait inside a kernel ran out)", *c->h_err);
-        int e = *c->h_err;
-        cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-        // a launch that gave up may have left partial sums or tickets behind
-        cudaMemsetAsync(c->d_fc_scratch, 0, (FFCU_FC_SMALL_TICKETS + FFCU_FC_SMALL_MAX_BATCH * 512) * sizeof(int), c->stream);
-        cudaMemsetAsync(c->d_fc_tc_scratch, 0, ((size_t)FFCU_FC_TC_TICKETS + (size_t)c->fc_tc_rows * 512) * sizeof(int), c->stream);
-        return 1000 + e;
-    }
-    return 0;
+    const int rc = wait_impl(c);
+    // whatever happened: once the wait has returned, the callers' buffers are theirs again
+    for (auto& q : c->pending) q.dst = nullptr;
+    return rc;
 }
 
 extern "C" int ffcu_ctx_cos_sim_matrix(ffcu_ctx* c, const float* a, int n, const float* b, int m, float* out)
@@ -684,6 +865,7 @@ extern "C" int ffcu_trace(ffcu_ctx* c, const float* host_in, int n, float* host_
     }
     for (size_t k = 0; k < c->layers.size() && rc == 0; k++) {
         const ffcu_layer& d = c->layers[k].d;
+        c->err_read[c->d_err == (int*)c->out_mem[1]] = false;
         rc = launch_layer(c, k, n, d.kind == FFCU_CONV ? d_acc : nullptr, true);
         if (rc != 0) break;
         rc = ffcu_wait(c);
@@ -726,7 +908,8 @@ extern "C" int ffcu_bench_resident(ffcu_ctx* c, const float* host_in, int n, int
 {
     if (!c || !c->finalized || !host_in || !ms || n < 1 || n > c->max_batch || iters < 1) return -1;
     FFCU_CHECK(cudaSetDevice(c->device));
-    c->d_in = c->in_slot[0]; c->d_out = c->out_slot[0];
+    c->d_in = c->in_slot[0]; c->d_out = c->out_slot[0]; c->d_err = (int*)c->out_mem[0];
+    c->err_read[0] = false;
     FFCU_CHECK(cudaMemcpyAsync(c->d_in, host_in, (size_t)n * 37632 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     cudaEvent_t e0, e1;
     FFCU_CHECK(cudaEventCreate(&e0));
@@ -760,6 +943,7 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     if (cap < nl) { ffcu_set_error("ffcu_bench_layers: ms[] too small"); return -1; }
     FFCU_CHECK(cudaSetDevice(c->device));
     FFCU_CHECK(cudaMemcpyAsync(c->d_in, host_in, (size_t)n * 37632 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    c->err_read[c->d_err == (int*)c->out_mem[1]] = false;
     int rc = launch_forward(c, n);
     if (rc != 0) return rc;
     std::vector<cudaEvent_t> ev(2 * nl);

@@ -201,7 +201,7 @@ ScPlan* ffcu_sc_plan(const ffcu_layer& main, const ffcu_layer& sc, int max_batch
                      const int8_t* d_in_sc, const int8_t* d_w_sc, int device);
 void    ffcu_sc_free(ScPlan* sp);
 int     ffcu_sc_launch(const ScPlan* sp, int batch, int mode, const EpiTables& t1, const EpiTables& t2, int8_t* out_main,
-                       int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s);
+                       int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s, int b0 = 0);
 // Layer chain (small batches, one cluster of eight or four CTAs per face): consecutive 3x3 stride-1 C -> C convolutions of one feature-map size in one launch.
 #define FFCU_CHAIN_MAX_FACES 37     // 148 SMs hold at most 18 clusters of eight and 37 of four, fewer where GPCs are smaller
 struct ChainPlan;
@@ -228,4 +228,6 @@ int ffcu_stem_fused_launch(const StemTcPlan* p, const void* in_any, int in_u8, c
 TcPlan* ffcu_tc_plan(const ffcu_layer& L, int max_batch, const int8_t* d_in, const int8_t* d_w, int device, int bn);
 void    ffcu_tc_free(TcPlan* p);
 int     ffcu_tc_launch(const TcPlan* p, int batch, int mode, const EpiTables& t, const int8_t* res,
-                       int32_t* acc_out, void* out, int8_t* out_bn2, int* d_err, cudaStream_t s);
+                       int32_t* acc_out, void* out, int8_t* out_bn2, int* d_err, cudaStream_t s, int b0 = 0);
+// b0 (here and in ffcu_sc_launch): the launch's first face in the input tensor; output and residual pointers are that
+// face's.  Layers with 64 input channels only (the ones a call may run in chunks while its input arrives).

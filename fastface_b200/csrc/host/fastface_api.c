@@ -147,9 +147,9 @@ void fastface_destroy(FastFace* ff)
     free(ff);
 }
 
-/* one device's share of a batch, in steps of max_batch */
+/* one device's share of a batch */
 typedef struct {
-    ffcu_ctx* ctx; const float* in; float* out; int n; int max_batch; int rc;
+    ffcu_ctx* ctx; const float* in; float* out; int n; int rc;
     const uint8_t* in_u8;      /* non-NULL: 8-bit pixel input instead of `in` */
     char err[256];             /* the CUDA side's message, copied on the thread that ran the job */
 } dev_job;
@@ -157,17 +157,7 @@ typedef struct {
 static void* dev_job_run(void* arg)
 {
     dev_job* j = (dev_job*)arg;
-    j->rc = 0;
-    for (int done = 0; done < j->n; ) {
-        int step = j->n - done < j->max_batch ? j->n - done : j->max_batch;
-        int rc = j->in_u8
-            ? ffcu_submit_u8(j->ctx, j->in_u8 + (size_t)done * FASTFACE_INPUT_N, step, j->out + (size_t)done * FASTFACE_OUTPUT_N)
-            : ffcu_submit(j->ctx, j->in + (size_t)done * FASTFACE_INPUT_N, step, j->out + (size_t)done * FASTFACE_OUTPUT_N);
-        if (rc != 0) { j->rc = rc; break; }
-        done += step;
-    }
-    int rc = ffcu_wait(j->ctx);
-    if (j->rc == 0) j->rc = rc;
+    j->rc = ffcu_run(j->ctx, j->in, j->in_u8, j->n, j->out);
     /* the CUDA side keeps its last message per thread: take it here, where it was set */
     j->err[0] = 0;
     if (j->rc != 0) snprintf(j->err, sizeof j->err, "%s", ffcu_last_error());
@@ -209,7 +199,7 @@ static int embed_batch_any(FastFace* ff, const float* input_hwc, const uint8_t* 
     int used = fastface_shard_plan(n, ff->n_dev, starts, counts);
     for (int d = 0; d < used; d++)
         jobs[d] = (dev_job){ ff->dev[d], input_hwc ? input_hwc + (size_t)starts[d] * FASTFACE_INPUT_N : NULL,
-                             out_emb + (size_t)starts[d] * FASTFACE_OUTPUT_N, counts[d], ff->max_batch, 0,
+                             out_emb + (size_t)starts[d] * FASTFACE_OUTPUT_N, counts[d], 0,
                              pixels_hwc ? pixels_hwc + (size_t)starts[d] * FASTFACE_INPUT_N : NULL, {0} };
     if (used == 1) {
         dev_job_run(&jobs[0]);

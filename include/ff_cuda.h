@@ -94,6 +94,9 @@ int ffcu_submit(ffcu_ctx* c, const float* host_in, int n, float* host_out);
  * cross PCIe.  Needs the fused stem (the default). */
 int ffcu_submit_u8(ffcu_ctx* c, const uint8_t* host_pixels, int n, float* host_out);
 int ffcu_wait(ffcu_ctx* c);
+/* A whole call: n faces (any number; fp32 from host_in, or 8-bit pixels where host_pixels is not NULL) in steps of
+ * max_batch, then ffcu_wait. */
+int ffcu_run(ffcu_ctx* c, const float* host_in, const uint8_t* host_pixels, int n, float* host_out);
 
 /* Same forward with dump points; fn is called on the host after each layer. */
 typedef void (*ffcu_trace_fn)(void* user, int op_index, int kind,
