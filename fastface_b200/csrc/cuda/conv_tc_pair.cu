@@ -87,31 +87,52 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             const int tn = pair_id % p.tiles_n;
             TileWalk wk;
             walk_init(wk, p, (pair_id / p.tiles_n) * 2 + (int)rank, (n_pairs / p.tiles_n) * 2);
+            // this lane's first block of a tile: kb = g
+            int c0_first = g * KC, kw_first = 0, kh_first = 0;
+            while (c0_first >= p.Cp) { c0_first -= p.Cp; if (++kw_first == p.Kw) { kw_first = 0; kh_first++; } }
+            // The weights are no kernel's output: the first tile's first steps' (as many as the ring holds) are requested
+            // before the programmatic-dependency wait.  Each slot's byte count is armed here for both operands.  256-column
+            // tiles only: forward of 48 / 64 / 100 faces 718 / 778 / 1068 -> 710 / 770 / 1048 us; 128-column tiles, whose launches
+            // leave hardly an SM free, lose by it (34 / 40 faces 588 / 648 -> 594 / 655).
+            int pre = 0;
+            if (BN == 256 && pair_id < total && !TC_DBG(p, 1)) {
+                pre = n_steps < p.stages ? n_steps : p.stages;
+#pragma unroll 1
+                for (int it = 0; it < pre; it++) {
+                    if (rank == 0 && lane == 0) mbar_expect_tx(full0 + it * 8, 2 * G * SUB_BYTES);
+                    __syncwarp();
+                    if (issuer && !is_a) tma2_load_4d(smem0 + it * stage_bytes, map, full0_leader + it * 8, (it * G + g) * KC, tn * BN + (int)rank * (BN / 2), 0, 0);
+                }
+            }
             tc_pdl_wait();
             for (int tile = pair_id; tile < total && ok; tile += n_pairs, walk_next(wk, p)) {
                 const int tw = wk.tw, th = wk.th, tb = wk.tb;   // tb may be past the batch: TMA zero-fills
                 const int x0 = tw * p.TW * p.stride - p.pad;
                 const int y0 = th * p.TH * p.stride - p.pad;
                 const int c3 = is_a ? tb * p.TB : 0;
-                // this lane's first block: kb = g
-                int c0 = g * KC, kw = 0, kh = 0;
-                while (c0 >= p.Cp) { c0 -= p.Cp; if (++kw == p.Kw) { kw = 0; kh++; } }
+                int c0 = c0_first, kw = kw_first, kh = kh_first;
 #pragma unroll 1
                 for (int it = 0; it < n_steps; it++) {
-                    ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
-                    if (!ok) break;
+                    const bool first_fill = it < pre;          // slot is fresh, armed, and its weight box is on its way
+                    if (!first_fill) {
+                        ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
+                        if (!ok) break;
+                    }
                     if (TC_DBG(p, 1)) { if (rank == 0 && lane == 0) mbar_arrive(full0 + stage * 8); }
                     else {
-                        if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * G * SUB_BYTES);
-                        __syncwarp();                           // the byte count is armed before any copy can land
+                        if (!first_fill) {
+                            if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * G * SUB_BYTES);
+                            __syncwarp();                       // the byte count is armed before any copy can land
+                        }
                         const int tapk = (kh * p.Kw + kw) * p.Cp + c0;
-                        if (issuer) tma2_load_4d(smem0 + stage * stage_bytes, map, full0_leader + stage * 8,
+                        if (issuer && (is_a || !first_fill)) tma2_load_4d(smem0 + stage * stage_bytes, map, full0_leader + stage * 8,
                                     is_a ? c0 : tapk, is_a ? x0 + kw : tn * BN + (int)rank * (BN / 2), is_a ? y0 + kh : 0, c3);
                     }
                     c0 += G * KC;
                     while (c0 >= p.Cp) { c0 -= p.Cp; if (++kw == p.Kw) { kw = 0; kh++; } }
                     if (++stage == p.stages) { stage = 0; phase ^= 1; }
                 }
+                pre = 0;
             }
         }
     } else if (warp == 1) {
