@@ -286,6 +286,15 @@ static int tc_epi_wps(int bn, int tiles_per_cta)
     return tiles_per_cta <= 1 ? 16 : 8;
 }
 
+bool tc_const_args(const TcParams& prm, int bn, int epi, TcConst* out)
+{
+    const float* h = prm.t.host;
+    if (!h || bn != 64 || prm.Cout != 64 || prm.epi_wps != 4) return false;
+    const int row[4] = {0, 1, epi == EPI_RES_BN ? 3 : 2, 4};
+    for (int t = 0; t < 4; t++) memcpy(out->v[t], h + row[t] * 64, sizeof out->v[t]);
+    return true;
+}
+
 static int g_test_fc_drop_step = -1;
 static long long g_test_fc_wait = 0;
 

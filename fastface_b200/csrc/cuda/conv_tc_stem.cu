@@ -54,10 +54,10 @@ __device__ __forceinline__ void stem_load_patch(const void* in_any, int b, int y
     }
 }
 
-template <bool CONTRACT, int EPI, bool IN_U8>
+template <bool CONTRACT, int EPI, bool IN_U8, bool CT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, const void* __restrict__ in_any,
-                 const float* __restrict__ inv3)
+                 const float* __restrict__ inv3, const __grid_constant__ TcConstArg<CT> ct)
 {
     tc_pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -185,17 +185,17 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
             umma_commit_w(leader, smem_u32(&sh->acc_full[a]));
         }
     } else {
-        tc_epilogue_role<BN, CONTRACT, false, EPI, (EPI != EPI_RUNTIME)>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
-                                                   blockIdx.x, gridDim.x, p.total_tiles, 1, 0, 0u);
+        tc_epilogue_role<BN, CONTRACT, false, EPI, (EPI != EPI_RUNTIME), CT>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
+                                                   blockIdx.x, gridDim.x, p.total_tiles, 1, 0, 0u, ct);
     }
     tc_teardown(abort_flag, tmem_base, TMEM_COLS, warp);
 }
 
-template <bool CONTRACT, int EPI, bool IN_U8>
-static int launch_stem(int grid, int smem, cudaStream_t s, const CUtensorMap& mapB, const TcParams& prm, const void* in_any,
-                       const float* inv3)
+template <bool CONTRACT, int EPI, bool IN_U8, bool CT>
+static int launch_stem_c(int grid, int smem, cudaStream_t s, const CUtensorMap& mapB, const TcParams& prm, const void* in_any,
+                         const float* inv3, const TcConstArg<CT>& ct)
 {
-    auto kern = conv_stem_kernel<CONTRACT, EPI, IN_U8>;
+    auto kern = conv_stem_kernel<CONTRACT, EPI, IN_U8, CT>;
     static int smem_set[64] = {};      // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
     FFCU_CHECK(cudaGetDevice(&dev));
@@ -203,7 +203,20 @@ static int launch_stem(int grid, int smem, cudaStream_t s, const CUtensorMap& ma
         FFCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         smem_set[dev & 63] = smem;
     }
-    return tc_launch_ex(kern, grid, smem, s, 1, mapB, prm, in_any, inv3);
+    return tc_launch_ex(kern, grid, smem, s, 1, mapB, prm, in_any, inv3, ct);
+}
+
+template <bool CONTRACT, int EPI, bool IN_U8>
+static int launch_stem(int grid, int smem, cudaStream_t s, const CUtensorMap& mapB, const TcParams& prm, const void* in_any,
+                       const float* inv3)
+{
+    if constexpr (EPI == EPI_SLOPE_BN) {
+        // From 30 tiles per CTA on (45 faces): below, the launch is shorter but its unrolled code, fetched cold in every
+        // forward, costs as much (forward of 17 / 24 / 33 faces 411.4 / 444.2 / 485.2 -> 413.2 / 446.0 / 487.2 us; 48: 706 -> 702).
+        TcConst ct;
+        if (prm.total_tiles / grid >= 30 && tc_const_args(prm, 64, EPI, &ct)) return launch_stem_c<CONTRACT, EPI, IN_U8, true>(grid, smem, s, mapB, prm, in_any, inv3, ct);
+    }
+    return launch_stem_c<CONTRACT, EPI, IN_U8, false>(grid, smem, s, mapB, prm, in_any, inv3, TcNoConst{});
 }
 
 int tc_launch_stem(int mode, int epi, int in_u8, int grid, int smem, cudaStream_t s, const CUtensorMap& mapB,

@@ -15,9 +15,9 @@
 //     180 rows of 64 B.
 // ---------------------------------------------------------------------------
 
-template <int BN, bool CONTRACT, int EPI>
+template <int BN, bool CONTRACT, int EPI, bool CT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const TcParams p)
+conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const TcParams p, const __grid_constant__ TcConstArg<CT> ct)
 {
     tc_pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -125,18 +125,19 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             }
         }
     } else {
-        tc_epilogue_role<BN, CONTRACT, false, EPI, (EPI != EPI_RUNTIME)>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
-                                             blockIdx.x, gridDim.x, p.total_tiles, 1, 0, 0u);
+        tc_epilogue_role<BN, CONTRACT, false, EPI, (EPI != EPI_RUNTIME), CT>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
+                                             blockIdx.x, gridDim.x, p.total_tiles, 1, 0, 0u, ct);
     }
     tc_teardown(abort_flag, tmem_base, TMEM_COLS, warp);
 }
 
 
 
-template <int BN, bool CONTRACT, int EPI>
-static int launch_w(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
+template <int BN, bool CONTRACT, int EPI, bool CT>
+static int launch_wc(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm,
+                     const TcConstArg<CT>& ct)
 {
-    auto kern = conv_ws_kernel<BN, CONTRACT, EPI>;
+    auto kern = conv_ws_kernel<BN, CONTRACT, EPI, CT>;
     static int smem_set[64] = {};      // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
     FFCU_CHECK(cudaGetDevice(&dev));
@@ -144,7 +145,17 @@ static int launch_w(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA,
         FFCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         smem_set[dev & 63] = smem;
     }
-    return tc_launch_ex(kern, grid, smem, s, 1, mapA, mapB, prm);
+    return tc_launch_ex(kern, grid, smem, s, 1, mapA, mapB, prm, ct);
+}
+
+template <int BN, bool CONTRACT, int EPI>
+static int launch_w(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
+{
+    if constexpr (BN == 64 && EPI == EPI_RES_BN) {
+        TcConst ct;
+        if (tc_const_args(prm, BN, EPI, &ct)) return launch_wc<BN, CONTRACT, EPI, true>(grid, smem, s, mapA, mapB, prm, ct);
+    }
+    return launch_wc<BN, CONTRACT, EPI, false>(grid, smem, s, mapA, mapB, prm, TcNoConst{});
 }
 
 template <int BN, bool CONTRACT>

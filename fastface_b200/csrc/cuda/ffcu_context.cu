@@ -44,6 +44,7 @@ struct DevLayer {
     int8_t* w = nullptr;
     float* tab[12] = {};   // w_scale,bias,slope,res_scale,inv_out | in_scale,bn_scale,bn_offset | bn2 in,scale,offset,inv
     EpiTables epi{};
+    std::vector<float> host_tab;   // what epi.host points to
     TcPlan* tc = nullptr;  // non-NULL: tensor-core implicit GEMM takes this layer (plan with the widest column tile)
     TcPlan* tc_bn[3] = {}; // plans for column tiles of 64 / 128 / 256 channels, made when a call first needs them
     int8_t* bn_lut = nullptr;  // device copy of the fused BN's table
@@ -280,6 +281,18 @@ static void free_layer_memory(DevLayer& L)
     cudaFree(L.wk32); L.wk32 = nullptr;
 }
 
+// EpiTables::host of a layer (empty: none)
+static std::vector<float> host_tables(const ffcu_layer* l)
+{
+    std::vector<float> v;
+    if (l->kind != FFCU_CONV || l->Cout != 64) return v;
+    v.assign(5 * 64, 0.0f);
+    const float* src[5] = {l->w_scale, l->bias, l->slope, l->res_scale, l->inv_out};
+    for (int t = 0; t < 5; t++)
+        if (src[t]) memcpy(&v[t * 64], src[t], 64 * sizeof(float));
+    return v;
+}
+
 extern "C" int ffcu_add_layer(ffcu_ctx* c, const ffcu_layer* l)
 {
     if (!c || !l || c->finalized) { ffcu_set_error("ffcu_add_layer: bad state"); return -1; }
@@ -316,6 +329,8 @@ extern "C" int ffcu_add_layer(ffcu_ctx* c, const ffcu_layer* l)
         if (cudaMemcpy(L.bn_lut, lut.data(), lut.size(), cudaMemcpyHostToDevice) != cudaSuccess) return fail("BN table upload failed");
     }
     L.epi.bn_lut = L.bn_lut;
+    L.host_tab = host_tables(l);
+    L.epi.host = L.host_tab.empty() ? nullptr : L.host_tab.data();
     L.epi.no_overflow = epilogue_cannot_overflow(l) ? 1 : 0;
     L.epi.acc22 = accumulator_fits_22_bits(l) ? 1 : 0;
     L.d.bn2_lut = nullptr;
@@ -324,7 +339,7 @@ extern "C" int ffcu_add_layer(ffcu_ctx* c, const ffcu_layer* l)
     L.d.w_scale = L.d.bias = L.d.slope = L.d.res_scale = L.d.inv_out = nullptr;
     L.d.in_scale = L.d.bn_scale = L.d.bn_offset = nullptr;
     if (cudaGetLastError() != cudaSuccess) return fail("upload failed");
-    c->layers.push_back(L);
+    c->layers.push_back(std::move(L));       // (moving the vector leaves epi.host valid)
     return (int)c->layers.size() - 1;
 }
 
@@ -991,6 +1006,7 @@ static int conv_once_impl(int device, const ffcu_layer* l, int batch, int mode, 
     float* tab[9] = {};
     cudaStream_t s = nullptr;
     TcPlan* plan = nullptr;
+    const std::vector<float> htab = host_tables(l);
     const bool bn2 = out_bn2 && l->bn2_in_scale && l->bn2_scale && l->bn2_offset && l->bn2_inv_out;
     int rc = 0;
     // one exit: everything allocated so far is released whatever step failed
@@ -1036,6 +1052,7 @@ static int conv_once_impl(int device, const ffcu_layer* l, int batch, int mode, 
         EpiTables t{tab[0], tab[1], tab[2], tab[3], tab[4], tab[5], tab[6], tab[7], tab[8], d_lut};
         t.no_overflow = epilogue_cannot_overflow(l) ? 1 : 0;
         t.acc22 = accumulator_fits_22_bits(l) ? 1 : 0;
+        t.host = htab.empty() ? nullptr : htab.data();
         if (impl == 0) {
             plan = ffcu_tc_plan(*l, batch, d_in, d_w, device, ffcu_tc_pick_bn(*l, batch, device));
             if (!plan) { ffcu_set_error("layer shape is not covered by the tensor-core kernel"); rc = -2; }
@@ -1056,6 +1073,7 @@ static int conv_once_impl(int device, const ffcu_layer* l, int batch, int mode, 
         EpiTables t{tab[0], tab[1], tab[2], tab[3], tab[4], tab[5], tab[6], tab[7], tab[8], d_lut};
         t.no_overflow = epilogue_cannot_overflow(l) ? 1 : 0;
         t.acc22 = accumulator_fits_22_bits(l) ? 1 : 0;
+        t.host = htab.empty() ? nullptr : htab.data();
         if (rc == 0) ONCE_TRY(cudaEventRecord(e0, s));
         for (int it = 0; it < iters && rc == 0; it++)
             rc = impl == 0 ? ffcu_tc_launch(plan, batch, mode, t, d_res, d_acc, d_out, d_out2, d_err, s)
