@@ -286,12 +286,12 @@ static int tc_epi_wps(int bn, int tiles_per_cta)
     return tiles_per_cta <= 1 ? 16 : 8;
 }
 
-bool tc_const_args(const TcParams& prm, int bn, int epi, TcConst* out)
+bool tc_const_args(const TcParams& prm, int bn, int epi, float* out)
 {
     const float* h = prm.t.host;
-    if (!h || bn != 64 || prm.Cout != 64 || prm.epi_wps != 4) return false;
+    if (!h || (bn != 64 && bn != 128) || prm.Cout != bn || prm.epi_wps != bn / 16) return false;
     const int row[4] = {0, 1, epi == EPI_RES_BN ? 3 : 2, 4};
-    for (int t = 0; t < 4; t++) memcpy(out->v[t], h + row[t] * 64, sizeof out->v[t]);
+    for (int t = 0; t < 4; t++) memcpy(out + t * bn, h + row[t] * bn, bn * sizeof(float));
     return true;
 }
 

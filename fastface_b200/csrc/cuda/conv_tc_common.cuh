@@ -506,21 +506,22 @@ __device__ __forceinline__ uint32_t tc_lut_byte(uint32_t w, uint32_t lut_base)
     return r;
 }
 
-// The per-channel constants of a 64-channel layer as kernel parameters, for launches whose epilogue warps walk all 64
-// columns (four warps per set): the column loop is unrolled, so every constant is an operand from the constant bank
-// instead of a shared-memory read.  Taken where a fused BN's byte look-ups load the same path: the stem's load / store
+// The per-channel constants of a 64- or 128-channel layer as kernel parameters, for launches whose epilogue warps walk 64
+// columns each (four warps per set, or eight): the column loop is unrolled, with 128 channels once per half, so every
+// constant is an operand from the constant bank instead of a shared-memory read.  Taken where a fused BN's byte look-ups load the same path: the stem's load / store
 // data path was 81 % busy, a third of it these reads (154 -> 143 us at 256 faces), the 56x56 residual + BN layers' 63 % (60 ->
 // 51 us).  The PReLU variants have no look-ups and are 3 % slower with the unrolled loop (112x112: 123.5 -> 127.6 us).
-struct TcConst { float v[4][64]; };       // w_scale, bias, slope (stem) or residual scale, inv_out
+template <int N>
+struct TcConst { float v[4][N]; };       // w_scale, bias, slope (stem) or residual scale, inv_out
 struct TcNoConst {};
-template <bool CT>
-using TcConstArg = typename std::conditional<CT, TcConst, TcNoConst>::type;
+template <bool CT, int N = 64>
+using TcConstArg = typename std::conditional<CT, TcConst<N>, TcNoConst>::type;
 
 // Sixteen columns of one accumulator row: v[16] int32 at channels cb .. cb + 15 -> four packed
 // int8 words (and four more for the fused BN's output).  CI = 0 / 1: first or second chunk of the
 // pair whose 32 table rows start at shared-memory address lut_pr.
-template <bool CONTRACT, int EPI, bool CHECK, int CI, bool ACC22 = false, bool CT = false>
-__device__ __forceinline__ void tc_epilogue16(const TcParams& p, const float* tab, const TcConstArg<CT>& ct, uint32_t lut_pr,
+template <bool CONTRACT, int EPI, bool CHECK, int CI, bool ACC22 = false, bool CT = false, int CN = 64>
+__device__ __forceinline__ void tc_epilogue16(const TcParams& p, const float* tab, const TcConstArg<CT, CN>& ct, uint32_t lut_pr,
                                               const int (&v)[16], const int* rw, int cb,
                                               bool rt_res, bool rt_slope, bool rt_bn2, int (&ow)[4], int (&ow2)[4])
 {
@@ -687,14 +688,14 @@ template <int BN, bool CONTRACT, bool OUT_F32, int EPI, bool ACC22 = false, bool
 __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, uint8_t* lut, TcShared* sh,
                                                  uint32_t tmem_base, volatile int* abort_flag, int warp, int lane,
                                                  int first, int step, int total, int m_mul, int m_off,
-                                                 uint32_t remote_acc_empty /* 0: local barrier */, const TcConstArg<CT>& ct = {})
+                                                 uint32_t remote_acc_empty /* 0: local barrier */, const TcConstArg<CT, BN>& ct = {})
 {
-    static_assert(!CT || (BN == 64 && (EPI == EPI_RES_BN || EPI == EPI_SLOPE_BN)), "constants as parameters: 64-column launches with a fused BN");
+    static_assert(!CT || (BN <= 128 && (EPI == EPI_RES_BN || EPI == EPI_SLOPE_BN)), "constants as parameters: launches with a fused BN");
     if (warp >= TC_ISSUER2_WARP) return;                  // not an epilogue warp
-    const int wps = CT ? 4 : p.epi_wps;
+    const int wps = CT ? BN / 16 : p.epi_wps;
     const int sets = TC_EPI_TOTAL_WARPS / wps;
     const int cols = BN / (wps >> 2);                     // columns this warp covers
-    constexpr int PAIR_UNROLL = CT ? BN / 32 : 1;
+    constexpr int PAIR_UNROLL = CT ? 2 : 1;
     const int n_pairs = cols >> 5;                        // pairs of 16-column chunks
     const int q = warp & 3;
     const int set = (warp - 2) / wps;                     // which of the CTA's tiles this warp takes
@@ -711,12 +712,14 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
     const bool dump = (EPI == EPI_RUNTIME) && p.acc_out != nullptr;
     int local = set;
     const int tn = first % p.tiles_n;
-    const int c0 = CT ? 0 : tn * BN + cg * cols;          // first channel of this warp's range
+    const int c0_rt = tn * BN + cg * cols;                // first channel of this warp's range
     bool ok = tc_epi_prologue(tab, lut, p, sh, tn * BN, BN, abort_flag);
     tc_pdl_wait();
     const uint32_t lut0 = smem_u32(lut) + (uint32_t)(cg * cols) * 256u;
     first += set * step;
     step *= sets;
+    auto walk_tiles = [&](auto c0c) {
+    const int c0 = CT ? decltype(c0c)::value : c0_rt;
     TileWalk wk;
     walk_init(wk, p, (first / p.tiles_n) * m_mul + m_off, (step / p.tiles_n) * m_mul);
     for (int tile = first; tile < total && ok; tile += step, local += sets, walk_next(wk, p)) {
@@ -769,8 +772,8 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
                     st_global_32B(p.acc_out + o + 8, d1);
                 }
                 if (OUT_F32) tc_fc16<CONTRACT>(p, tab, v0, cb, o);
-                else if (check) tc_epilogue16<CONTRACT, EPI, true, 0, false, CT>(p, tab, ct, lut_pr, v0, rw, cb, has_res, has_slope, has_bn2, w0, w0b);
-                else            tc_epilogue16<CONTRACT, EPI, false, 0, ACC22, CT>(p, tab, ct, lut_pr, v0, rw, cb, has_res, has_slope, has_bn2, w0, w0b);
+                else if (check) tc_epilogue16<CONTRACT, EPI, true, 0, false, CT, BN>(p, tab, ct, lut_pr, v0, rw, cb, has_res, has_slope, has_bn2, w0, w0b);
+                else            tc_epilogue16<CONTRACT, EPI, false, 0, ACC22, CT, BN>(p, tab, ct, lut_pr, v0, rw, cb, has_res, has_slope, has_bn2, w0, w0b);
             }
             tmem_ld_wait(v1);
             if (more) tmem_ld16_issue(taddr + (uint32_t)(pr * 32 + 32), v0);  // lands while v1 is computed
@@ -783,8 +786,8 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
                 }
                 if (OUT_F32) tc_fc16<CONTRACT>(p, tab, v1, cb + 16, o + 16);
                 else {
-                    if (check) tc_epilogue16<CONTRACT, EPI, true, 1, false, CT>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
-                    else       tc_epilogue16<CONTRACT, EPI, false, 1, ACC22, CT>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
+                    if (check) tc_epilogue16<CONTRACT, EPI, true, 1, false, CT, BN>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
+                    else       tc_epilogue16<CONTRACT, EPI, false, 1, ACC22, CT, BN>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
                     if (!TC_DBG(p, 4)) {
                         const int w8[8] = {w0[0], w0[1], w0[2], w0[3], w1[0], w1[1], w1[2], w1[3]};
                         st_global_32B((int8_t*)p.out + o, w8);
@@ -808,6 +811,9 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
             else mbar_arrive_relaxed(smem_u32(&sh->acc_empty[a]));
         }
     }
+    };
+    if (CT && BN == 128 && cg) walk_tiles(std::integral_constant<int, 64>{});
+    else walk_tiles(std::integral_constant<int, 0>{});
 }
 
 __device__ __forceinline__ void tc_setup(TcShared* sh, int stages, uint32_t tmem_cols, int warp, int epi_active)
@@ -856,7 +862,7 @@ int tc_launch_generic(int bn, int kc, int mode, int epi, bool f32, int grid, int
 int tc_launch_ws(int bn, int mode, int epi, int grid, int smem, cudaStream_t s,
                  const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm);
 // The launch's constants for the variants that take them as parameters; false: this launch keeps the shared-memory tables.
-bool tc_const_args(const TcParams& prm, int bn, int epi, TcConst* out);
+bool tc_const_args(const TcParams& prm, int bn, int epi, float* out /* [4][bn] */);
 int tc_launch_pair(int bn, int mode, int epi, bool f32, int grid, int smem, cudaStream_t s,
                    const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm);
 int tc_launch_stem(int mode, int epi, int in_u8, int grid, int smem, cudaStream_t s, const CUtensorMap& mapB,

@@ -152,8 +152,8 @@ template <int BN, bool CONTRACT, int EPI>
 static int launch_w(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
 {
     if constexpr (BN == 64 && EPI == EPI_RES_BN) {
-        TcConst ct;
-        if (tc_const_args(prm, BN, EPI, &ct)) return launch_wc<BN, CONTRACT, EPI, true>(grid, smem, s, mapA, mapB, prm, ct);
+        TcConst<64> ct;
+        if (tc_const_args(prm, BN, EPI, &ct.v[0][0])) return launch_wc<BN, CONTRACT, EPI, true>(grid, smem, s, mapA, mapB, prm, ct);
     }
     return launch_wc<BN, CONTRACT, EPI, false>(grid, smem, s, mapA, mapB, prm, TcNoConst{});
 }

@@ -23,9 +23,10 @@
 // Warp roles, barriers, bounded waits and teardown as in the per-tap pair kernel; two issuer
 // warps (leader CTA) take alternate tiles as in the 64-channel weight-stationary kernel.
 // ---------------------------------------------------------------------------
-template <bool CONTRACT, int EPI>
+template <bool CONTRACT, int EPI, bool CT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const TcParams p)
+conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const TcParams p,
+                const __grid_constant__ TcConstArg<CT, 128> ct)
 {
     tc_pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -164,8 +165,8 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         }
     } else {
         const uint32_t leader_acc_empty = map_to_cta(smem_u32(&sh->acc_empty[0]), 0);
-        tc_epilogue_role<BN, CONTRACT, false, EPI>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
-                                                   pair_id, n_pairs, total, 2, (int)rank, leader_acc_empty);
+        tc_epilogue_role<BN, CONTRACT, false, EPI, false, CT>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,
+                                                   pair_id, n_pairs, total, 2, (int)rank, leader_acc_empty, ct);
     }
 
     // ---- teardown: neither CTA may leave while its partner can still read its smem / TMEM ----
@@ -183,10 +184,11 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     }
 }
 
-template <bool CONTRACT, int EPI>
-static int launch_wsp(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
+template <bool CONTRACT, int EPI, bool CT>
+static int launch_wsp_c(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm,
+                        const TcConstArg<CT, 128>& ct)
 {
-    auto kern = conv_wsp_kernel<CONTRACT, EPI>;
+    auto kern = conv_wsp_kernel<CONTRACT, EPI, CT>;
     static int smem_set[64] = {};      // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
     FFCU_CHECK(cudaGetDevice(&dev));
@@ -194,7 +196,19 @@ static int launch_wsp(int grid, int smem, cudaStream_t s, const CUtensorMap& map
         FFCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         smem_set[dev & 63] = smem;
     }
-    return tc_launch_ex(kern, grid, smem, s, 2, mapA, mapB, prm);
+    return tc_launch_ex(kern, grid, smem, s, 2, mapA, mapB, prm, ct);
+}
+
+template <bool CONTRACT, int EPI>
+static int launch_wsp(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& prm)
+{
+    if constexpr (EPI == EPI_RES_BN) {
+        // Constants as parameters where a pair sees two tiles or more (43 faces): 14.3 -> 13.0 us at 64 faces, 44 -> 39 at 256;
+        // at 17 faces the longer code costs more than it saves (8.1 -> 8.7 us).
+        TcConst<128> ct;
+        if (prm.total_tiles / (grid / 2) >= 2 && tc_const_args(prm, 128, EPI, &ct.v[0][0])) return launch_wsp_c<CONTRACT, EPI, true>(grid, smem, s, mapA, mapB, prm, ct);
+    }
+    return launch_wsp_c<CONTRACT, EPI, false>(grid, smem, s, mapA, mapB, prm, TcNoConst{});
 }
 
 template <bool CONTRACT>

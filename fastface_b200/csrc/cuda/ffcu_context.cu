@@ -285,11 +285,12 @@ static void free_layer_memory(DevLayer& L)
 static std::vector<float> host_tables(const ffcu_layer* l)
 {
     std::vector<float> v;
-    if (l->kind != FFCU_CONV || l->Cout != 64) return v;
-    v.assign(5 * 64, 0.0f);
+    if (l->kind != FFCU_CONV || (l->Cout != 64 && l->Cout != 128)) return v;
+    const size_t C = (size_t)l->Cout;
+    v.assign(5 * C, 0.0f);
     const float* src[5] = {l->w_scale, l->bias, l->slope, l->res_scale, l->inv_out};
     for (int t = 0; t < 5; t++)
-        if (src[t]) memcpy(&v[t * 64], src[t], 64 * sizeof(float));
+        if (src[t]) memcpy(&v[t * C], src[t], C * sizeof(float));
     return v;
 }
 

@@ -52,7 +52,7 @@ struct EpiTables {
     // the kernels may then convert the accumulator to float with one integer add and one float add instead
     // of the conversion unit (the 64-input-channel layers and the stem are bound by that unit).
     int acc22;
-    const float* host = nullptr;     // 64-channel convolutions: w_scale, bias, slope, res_scale, inv_out [5][64] on the host
+    const float* host = nullptr;     // convolutions with 64 or 128 output channels: w_scale, bias, slope, res_scale, inv_out [5][Cout] on the host
 };
 
 // ---------------------------------------------------------------------------
