@@ -91,7 +91,9 @@ static bool encode_A(const TcPlan* p, TcGeom* g)
 // weight stream instead of one SM reading all of it.  $FF_TC_BN: 64 / 128 / 256 pins the tile
 // where it divides Cout; "wide" keeps the widest tile at any batch.  The tile is halved while the launch would
 // fill less than 1 / fill_div of the SMs: half (the default, $FF_TC_BN_FILL) measured best at batch 16-128, where
-// a wider tile on half the SMs beats twice the CTAs each streaming the same activations again; the fused
+// a wider tile on half the SMs beats twice the CTAs each streaming the same activations again (tiles counted with their
+// padding: forward of 40 / 41 / 44 / 47 / 90 faces 645 / 767 / 783 / 791 / 903 -> 630 / 667 / 690 / 698 / 877 us against counting
+// pixels); the fused
 // stride-2 + shortcut launch (64 columns only) asks with fill_div = 1, the rule it was measured with.
 int ffcu_tc_pick_bn(const ffcu_layer& L, int batch, int device, int fill_div)
 {
@@ -107,9 +109,17 @@ int ffcu_tc_pick_bn(const ffcu_layer& L, int batch, int device, int fill_div)
     if (!n_sm && cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n_sm = 148;
     static int fill_env = -1;
     if (fill_env < 0) { const char* e = getenv("FF_TC_BN_FILL"); fill_env = (e && atoi(e) >= 1 && atoi(e) <= 4) ? atoi(e) : 2; }
-    if (fill_div < 1) fill_div = fill_env;
+    const bool own_rule = fill_div < 1;
+    if (own_rule) fill_div = fill_env;
     const long long rows = (L.kind == FFCU_FC) ? (long long)batch : (long long)batch * L.Ho * L.Wo;
-    const long long m_tiles = (rows + TC_TILE_M - 1) / TC_TILE_M;
+    long long m_tiles = (rows + TC_TILE_M - 1) / TC_TILE_M;
+    if (L.kind == FFCU_CONV && own_rule) {
+        // the tiles the launch will have, padding of the map and the batch to the tile included: counted without it, 41-47
+        // faces' 14x14 layers were halved into two waves of tiles
+        int TW, TH, TB;
+        pick_geometry(L.Wo, L.Ho, batch, &TW, &TH, &TB);
+        m_tiles = (long long)((L.Wo + TW - 1) / TW) * ((L.Ho + TH - 1) / TH) * ((batch + TB - 1) / TB);
+    }
     while (bn > 64 && L.Cout % (bn / 2) == 0 && m_tiles * (L.Cout / bn) * fill_div < n_sm) bn /= 2;
     return bn;
 }
