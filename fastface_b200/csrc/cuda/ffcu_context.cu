@@ -15,15 +15,15 @@
 #include <vector>
 
 #define OUT_HEAD 64            // bytes in front of an output slot: its error word
-#define STAGE_SLOTS 4          // page-locked ring the input of a pageable call goes through
-#define STAGE_FACES 16         // faces (fp32) per ring slot
+#define STAGE_SLOTS 8          // page-locked ring the input of a pageable call goes through
+#define STAGE_FACES 8          // faces (fp32) per ring slot
 #define STAGE_OUT_FACES 4096   // most faces whose output goes through page-locked memory
 
 // A step of at least this many faces that finds the device idle runs its first layers in chunks while the rest of its input is
 // on its way (submit_impl); below it a call is one stream of copy, forward, copy.  Half a step under 128 faces, 64
 // from there on: smaller chunks fill the SMs worse (these layers take 2.6 us a face at 256 faces, 2.85 at 64, 3.3 at 32) and
 // larger ones leave more of the copy in front (2.8 us a face of fp32).  Calls before -> after, staging included: 256 faces of page-
-// locked fp32 2713 -> 2319 us, 64 pageable 1440 -> 1245, 100 page-locked 8-bit 1190 -> 1167, 1024 of them 8140 -> 7960.
+// locked fp32 2713 -> 2319 us, 64 pageable 1440 -> 1110, 100 page-locked 8-bit 1190 -> 1167, 1024 of them 8140 -> 7960.
 #define CHUNK_MIN_FACES 40
 #define CHUNK_FACES 64
 
@@ -683,7 +683,7 @@ static int copy_in(ffcu_ctx* c, void* dst, const void* src, size_t bytes, bool s
         const int k = (int)(c->stage_seq % STAGE_SLOTS);
         char* ring = c->stage_in + (size_t)k * c->stage_slot_bytes;
         if (c->stage_seq >= STAGE_SLOTS) FFCU_CHECK(cudaEventSynchronize(c->ev_stage[k]));      // the slot's last copy has left it
-        ff_copy(c->pool, ring, (const char*)src + o, nb);
+        ff_copy(c->pool, ring, (const char*)src + o, nb, 1);
         FFCU_CHECK(cudaMemcpyAsync((char*)dst + o, ring, nb, cudaMemcpyHostToDevice, s));
         FFCU_CHECK(cudaEventRecord(c->ev_stage[k], s));
     }
@@ -709,7 +709,7 @@ static int copy_out(ffcu_ctx* c, int slot, int n, float* host_out, cudaStream_t 
 static void deliver(ffcu_ctx* c, int slot)
 {
     if (!c->pending[slot].dst) return;
-    ff_copy(c->pool, c->pending[slot].dst, c->stage_out[slot] + OUT_HEAD, c->pending[slot].bytes);
+    ff_copy(c->pool, c->pending[slot].dst, c->stage_out[slot] + OUT_HEAD, c->pending[slot].bytes, 0);
     c->pending[slot].dst = nullptr;
 }
 

@@ -4,6 +4,10 @@
  * staging of a pageable copy is one thread (12 GB/s at 150 MB).  The job is cut into pieces that whoever is awake
  * claims under a mutex, the caller included: helpers that are slow to wake cost nothing, they find less to do.
  * A helper looks for the next job for some 50 us before it sleeps, which spans the gap between two chunks of a call.
+ *
+ * A copy whose destination a device reads next uses streaming stores: lines left dirty in the caches of several cores
+ * slow the copy engine's reads down (2.56 MB, copied by one thread and sent: 259-309 us with plain stores, 199-231 with
+ * streaming ones; the driver's own staging 242).
  */
 #define _GNU_SOURCE
 #include "ff_copy.h"
@@ -15,6 +19,9 @@
 #include <stdlib.h>
 #include <string.h>
 #include <time.h>
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
 
 #define FF_COPY_MAX_HELPERS 3
 #define FF_COPY_PIECE ((size_t)128 << 10)
@@ -29,6 +36,7 @@ struct ff_copy_pool {
     size_t bytes, next;      /* next: first byte nobody has claimed */
     _Atomic size_t open;     /* bytes nobody has claimed, readable without the mutex */
     _Atomic size_t left;     /* bytes not copied yet */
+    int streaming;           /* of the job */
     int wanted, started, stop, sleeping;
     pthread_t th[FF_COPY_MAX_HELPERS];
 };
@@ -47,6 +55,27 @@ static long long now_ns(void)
     return (long long)t.tv_sec * 1000000000ll + t.tv_nsec;
 }
 
+static void copy_streaming(char* d, const char* s, size_t n)
+{
+#if defined(__SSE2__)
+    const size_t head = (64 - ((size_t)d & 63)) & 63;
+    if (n >= 256) {
+        memcpy(d, s, head);
+        d += head; s += head; n -= head;
+        for (; n >= 64; d += 64, s += 64, n -= 64) {
+            const __m128i a = _mm_loadu_si128((const __m128i*)s), b = _mm_loadu_si128((const __m128i*)(s + 16));
+            const __m128i c = _mm_loadu_si128((const __m128i*)(s + 32)), e = _mm_loadu_si128((const __m128i*)(s + 48));
+            _mm_stream_si128((__m128i*)d, a);
+            _mm_stream_si128((__m128i*)(d + 16), b);
+            _mm_stream_si128((__m128i*)(d + 32), c);
+            _mm_stream_si128((__m128i*)(d + 48), e);
+        }
+        _mm_sfence();                /* streaming stores are not ordered by the release that follows */
+    }
+#endif
+    memcpy(d, s, n);
+}
+
 /* claims and copies one piece; 0 when there is none.  Called with the mutex held, returns with it held. */
 static int copy_piece(ff_copy_pool* p)
 {
@@ -55,10 +84,12 @@ static int copy_piece(ff_copy_pool* p)
     const size_t n = p->bytes - o < FF_COPY_PIECE ? p->bytes - o : FF_COPY_PIECE;
     char* d = p->dst + o;
     const char* s = p->src + o;
+    const int streaming = p->streaming;
     p->next = o + n;
     atomic_store_explicit(&p->open, p->bytes - p->next, memory_order_relaxed);
     pthread_mutex_unlock(&p->mu);
-    memcpy(d, s, n);
+    if (streaming) copy_streaming(d, s, n);
+    else memcpy(d, s, n);
     atomic_fetch_sub_explicit(&p->left, n, memory_order_release);
     pthread_mutex_lock(&p->mu);
     return 1;
@@ -126,15 +157,16 @@ void ff_copy_pool_destroy(ff_copy_pool* p)
     free(p);
 }
 
-void ff_copy(ff_copy_pool* p, void* dst, const void* src, size_t bytes)
+void ff_copy(ff_copy_pool* p, void* dst, const void* src, size_t bytes, int streaming)
 {
     if (!p || p->wanted == 0 || bytes < FF_COPY_MIN_SHARED) {
-        memcpy(dst, src, bytes);
+        if (streaming) copy_streaming((char*)dst, (const char*)src, bytes);
+        else memcpy(dst, src, bytes);
         return;
     }
     if (p->started < p->wanted) start_helpers(p);
     pthread_mutex_lock(&p->mu);
-    p->dst = (char*)dst; p->src = (const char*)src; p->bytes = bytes; p->next = 0;
+    p->dst = (char*)dst; p->src = (const char*)src; p->bytes = bytes; p->next = 0; p->streaming = streaming;
     atomic_store_explicit(&p->left, bytes, memory_order_relaxed);
     atomic_store_explicit(&p->open, bytes, memory_order_relaxed);
     if (p->sleeping) pthread_cond_broadcast(&p->wake);

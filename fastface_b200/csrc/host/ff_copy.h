@@ -16,8 +16,9 @@ ff_copy_pool* ff_copy_pool_create(int helpers);
 void ff_copy_pool_destroy(ff_copy_pool* p);
 
 /* memcpy(dst, src, bytes), shared with the pool's threads from 512 KB up; returns when every byte is in place.  One
- * caller at a time per pool.  p may be NULL (plain memcpy). */
-void ff_copy(ff_copy_pool* p, void* dst, const void* src, size_t bytes);
+ * caller at a time per pool.  p may be NULL (the caller alone).  streaming: the destination is not read by a CPU next
+ * (stores that bypass the caches). */
+void ff_copy(ff_copy_pool* p, void* dst, const void* src, size_t bytes, int streaming);
 
 #ifdef __cplusplus
 }

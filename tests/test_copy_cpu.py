@@ -17,11 +17,11 @@ def lib(built_lib):
     L.ff_copy_pool_destroy.restype = None
     L.ff_copy_pool_destroy.argtypes = [C.c_void_p]
     L.ff_copy.restype = None
-    L.ff_copy.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t]
+    L.ff_copy.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
     return L
 
 
-SIZES = [1, 4095, (512 << 10) - 1, 512 << 10, (512 << 10) + 1, (640 << 10) - 3, 1 << 20, 2408448, 5_000_001]
+SIZES = [1, 63, 255, 256, 257, 319, 4095, (512 << 10) - 1, 512 << 10, (512 << 10) + 1, (640 << 10) - 3, 1 << 20, 2408448, 5_000_001]
 
 
 def copies(lib, pool, seed, rounds):
@@ -31,7 +31,7 @@ def copies(lib, pool, seed, rounds):
             so, do = int(rng.integers(0, 70)), int(rng.integers(0, 70))
             src = rng.integers(0, 256, n + 200, dtype=np.uint8)
             dst = np.full(n + 200, 0xA5, np.uint8)
-            lib.ff_copy(pool, dst.ctypes.data + do, src.ctypes.data + so, n)
+            lib.ff_copy(pool, dst.ctypes.data + do, src.ctypes.data + so, n, int(rng.integers(0, 2)))
             assert np.array_equal(dst[do:do + n], src[so:so + n])
             assert np.all(dst[:do] == 0xA5) and np.all(dst[do + n:] == 0xA5)
 
