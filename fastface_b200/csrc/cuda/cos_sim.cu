@@ -6,90 +6,141 @@
 // float32 x float32 product is exact in float64 (48 bits), so one fused multiply-add per step rounds exactly where
 // "dot += x * y" does: the kernel reproduces the host function bit for bit.
 //
-// Bound: float64 FMA (64 per cycle and SM) from a few hundred rows up, copies below and around it.  A block of 256
-// threads computes 16 * RM x 64 outputs, RM x 4 per thread, from operands converted to float64 once per block and
-// staged CS_KC dimensions at a time; its first threads carry the norms of the block's rows along (one FMA per
-// dimension each), so every norm is computed once per block and not once per pair.
-// 1024 x 1024 from and to pageable host arrays: 3060 -> 620 us a call (three allocations and frees a call, norms summed
-// per pair and separate multiplies and adds before); what is left is the copies.
+// Bound: a pair's sum is a chain of 512 dependent float64 FMAs, about 10 us however small the matrix, and from a few
+// hundred blocks on the float64 rate.  Everything else is arranged around that chain: the operands of the next CS_KC
+// dimensions are fetched into registers while the current ones are used, converted to float64 once per block and stored into the
+// other of two shared buffers (one barrier per chunk), and the norms have warps of their own, one row a thread, so that
+// their chains run beside the pairs'.  Rows lie KC + 2 doubles apart: 16-byte reads of two dimensions at eight
+// consecutive rows touch every bank once, and a warp's 4 x 8 lanes read 4 rows of `a` and 8 of `b` for each 32 sums.
+//
+// Kernel times, us, one output a thread and no prefetch | 16 x 64 or 64 x 64 outputs a block, norms in front of each chunk's
+// sums | this kernel: 1 x 100 24.7 | 61.6 | 12.5, 24 x 300 26.8 | 61.6 | 12.4, 64 x 1000 32.9 | 61.6 | 20.7, 1 x 10000 59 | 98 | 45,
+// 128 x 1000 51.4 | 61.6 | 22.6, 256 x 1000 82 | 72 | 37, 1024 x 1000 287 | 119 | 95, 1024 x 10000 2656 | 884 | 779.  Calls (pageable arrays, copies included): 1 x 100 90 | 115 | 57,
+// 16 x 300 120 | 137 | 78, 128 x 300 146 | 156 | 108, 256 x 1000 1613 | 359 | 295, 1024 x 1000 2643 | 643 | 617.
 #include "ffcu_internal.cuh"
 #include "cos_sim.cuh"
 
 #include <algorithm>
-#include <new>
 
 #define CS_DIM 512
-#define CS_KC 16
-#define CS_TJ 64
 
-// Rows of a tile lie CS_PAD doubles apart per dimension: [k][row], so a thread's 4 rows are 32 contiguous bytes.
-template <int RM>
-__global__ void __launch_bounds__(256) cos_sim_matrix_kernel(const float* __restrict__ a, int n, const float* __restrict__ b, int m,
-                                                             float* __restrict__ out, size_t pitch)
+// WR x WC warps of 4 x 8 lanes, RM x RN pairs per thread (rows 4 apart, columns 8 apart), KC dimensions at a time.
+template <int WR, int WC, int RM, int RN, int KC>
+struct CosTile {
+    static constexpr int TI = WR * 4 * RM, TJ = WC * 8 * RN, ROWS = TI + TJ;
+    static constexpr int PAIR_THREADS = 32 * WR * WC;
+    static constexpr int THREADS = PAIR_THREADS + (ROWS + 31) / 32 * 32;       // then one thread per row for the norms
+    static constexpr int VECS = KC / 4, FETCH = (ROWS * VECS + THREADS - 1) / THREADS;
+};
+
+template <int WR, int WC, int RM, int RN, int KC>
+__global__ void __launch_bounds__(CosTile<WR, WC, RM, RN, KC>::THREADS)
+cos_sim_matrix_kernel(const float* __restrict__ a, int n, const float* __restrict__ b, int m, float* __restrict__ out, size_t pitch)
 {
-    constexpr int TI = 16 * RM;
-    __shared__ alignas(16) double sa[CS_KC][TI + 2], sb[CS_KC][CS_TJ + 2];
-    __shared__ double na[TI], nb[CS_TJ];                   // square roots of the squared norms
-    const int t = threadIdx.x, tx = t % 16, ty = t / 16;
-    const int i0 = blockIdx.y * TI, j0 = blockIdx.x * CS_TJ;
-    double acc[RM][4] = {};
+    using T = CosTile<WR, WC, RM, RN, KC>;
+    __shared__ alignas(16) double s[2][T::ROWS][KC + 2];   // rows of a, then rows of b
+    __shared__ double root[T::ROWS];                       // square roots of the squared norms
+    const int t = threadIdx.x, warp = t / 32, lane = t % 32;
+    const int i0 = blockIdx.y * T::TI, j0 = blockIdx.x * T::TJ;
+    float4 v[T::FETCH];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < T::FETCH; u++) {
+            const int e = t + u * T::THREADS, r = e / T::VECS, c = e % T::VECS * 4;
+            v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (r < T::ROWS) {
+                const bool is_a = r < T::TI;
+                const int row = is_a ? i0 + r : j0 + r - T::TI;
+                if (row < (is_a ? n : m)) v[u] = __ldg((const float4*)((is_a ? a : b) + (size_t)row * CS_DIM + k0 + c));
+            }
+        }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < T::FETCH; u++) {
+            const int e = t + u * T::THREADS, r = e / T::VECS, c = e % T::VECS * 4;
+            if (r < T::ROWS) {
+                double2* d = (double2*)&s[buf][r][c];
+                d[0] = make_double2((double)v[u].x, (double)v[u].y);
+                d[1] = make_double2((double)v[u].z, (double)v[u].w);
+            }
+        }
+    };
+    const int ri = warp / WC * 4 * RM + lane / 8, cj = warp % WC * 8 * RN + lane % 8;      // of this thread's first pair
+    const int norm_row = t - T::PAIR_THREADS;
+    double acc[RM][RN] = {};
     double nrm = 0.0;
-    for (int k0 = 0; k0 < CS_DIM; k0 += CS_KC) {
-        for (int e = t; e < (TI + CS_TJ) * (CS_KC / 4); e += 256) {
-            const int r = e / (CS_KC / 4), c = e % (CS_KC / 4) * 4;
-            const bool is_a = r < TI;
-            const int row = is_a ? i0 + r : j0 + r - TI;
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (row < (is_a ? n : m)) v = __ldg((const float4*)((is_a ? a : b) + (size_t)row * CS_DIM + k0 + c));
-            double* d = is_a ? &sa[c][r] : &sb[c][r - TI];
-            const int ld = is_a ? TI + 2 : CS_TJ + 2;
-            d[0] = (double)v.x; d[ld] = (double)v.y; d[2 * ld] = (double)v.z; d[3 * ld] = (double)v.w;
+    fetch(0);
+    put(0);
+    for (int k0 = 0; k0 < CS_DIM; k0 += KC) {
+        const int buf = k0 / KC & 1;
+        const bool more = k0 + KC < CS_DIM;
+        __syncthreads();                                   // this chunk is in place, the other buffer free
+        if (more) fetch(k0 + KC);
+        if (norm_row < 0) {
+#pragma unroll
+            for (int k = 0; k < KC; k += 2) {
+                double2 x[RM], y[RN];
+#pragma unroll
+                for (int r = 0; r < RM; r++) x[r] = *(const double2*)&s[buf][ri + 4 * r][k];
+#pragma unroll
+                for (int c = 0; c < RN; c++) y[c] = *(const double2*)&s[buf][T::TI + cj + 8 * c][k];
+#pragma unroll
+                for (int r = 0; r < RM; r++)
+#pragma unroll
+                    for (int c = 0; c < RN; c++) {
+                        acc[r][c] = __fma_rn(x[r].x, y[c].x, acc[r][c]);
+                        acc[r][c] = __fma_rn(x[r].y, y[c].y, acc[r][c]);
+                    }
+            }
+        } else if (norm_row < T::ROWS) {
+#pragma unroll
+            for (int k = 0; k < KC; k += 2) {
+                const double2 x = *(const double2*)&s[buf][norm_row][k];
+                nrm = __fma_rn(x.x, x.x, nrm);
+                nrm = __fma_rn(x.y, x.y, nrm);
+            }
         }
-        __syncthreads();
-        if (t < TI + CS_TJ) {
-            const double* p = t < TI ? &sa[0][t] : &sb[0][t - TI];
-            const int ld = t < TI ? TI + 2 : CS_TJ + 2;
-#pragma unroll
-            for (int k = 0; k < CS_KC; k++) nrm = __fma_rn(p[k * ld], p[k * ld], nrm);
-        }
-#pragma unroll
-        for (int k = 0; k < CS_KC; k++) {
-            double x[RM], y[4];
-#pragma unroll
-            for (int r = 0; r < RM; r++) x[r] = sa[k][ty * RM + r];
-#pragma unroll
-            for (int c = 0; c < 4; c++) y[c] = sb[k][tx * 4 + c];
-#pragma unroll
-            for (int r = 0; r < RM; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) acc[r][c] = __fma_rn(x[r], y[c], acc[r][c]);
-        }
-        __syncthreads();
+        if (more) put(buf ^ 1);
     }
-    if (t < TI + CS_TJ) (t < TI ? na[t] : nb[t - TI]) = __dsqrt_rn(nrm);
+    if (norm_row >= 0 && norm_row < T::ROWS) root[norm_row] = __dsqrt_rn(nrm);
     __syncthreads();
+    if (norm_row >= 0) return;
 #pragma unroll
     for (int r = 0; r < RM; r++) {
-        const int i = i0 + ty * RM + r;
-        const double ra = na[ty * RM + r];
+        const int i = i0 + ri + 4 * r;
+        const double ra = root[ri + 4 * r];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int j = j0 + tx * 4 + c;
-            const double rb = nb[tx * 4 + c];
+        for (int c = 0; c < RN; c++) {
+            const int j = j0 + cj + 8 * c;
+            const double rb = root[T::TI + cj + 8 * c];
             // the square root of a squared norm is 0 exactly where the squared norm is
-            const float v = (ra != 0.0 && rb != 0.0) ? (float)__ddiv_rn(acc[r][c], __dmul_rn(ra, rb)) : 0.0f;
-            if (i < n && j < m) out[(size_t)i * pitch + j] = v;
+            const float q = (ra != 0.0 && rb != 0.0) ? (float)__ddiv_rn(acc[r][c], __dmul_rn(ra, rb)) : 0.0f;
+            if (i < n && j < m) out[(size_t)i * pitch + j] = q;
         }
     }
 }
 
-static void launch_matrix(const float* a, int n, const float* b, int m, float* out, size_t pitch, cudaStream_t s)
+template <int WR, int WC, int RM, int RN, int KC>
+static void launch_tile(const float* a, int n, const float* b, int m, float* out, size_t pitch, cudaStream_t s)
 {
-    // Rows per block: 64 when that fills half the SMs' worth of blocks, else 16 (a handful of queries against a gallery
-    // would spend the FMAs on rows that are not there).
-    const int gx = (m + CS_TJ - 1) / CS_TJ;
-    if (n > 32 && gx * ((n + 63) / 64) >= 74) cos_sim_matrix_kernel<4><<<dim3(gx, (n + 63) / 64), 256, 0, s>>>(a, n, b, m, out, pitch);
-    else cos_sim_matrix_kernel<1><<<dim3(gx, (n + 15) / 16), 256, 0, s>>>(a, n, b, m, out, pitch);
+    using T = CosTile<WR, WC, RM, RN, KC>;
+    cos_sim_matrix_kernel<WR, WC, RM, RN, KC><<<dim3((m + T::TJ - 1) / T::TJ, (n + T::TI - 1) / T::TI), T::THREADS, 0, s>>>(a, n, b, m, out, pitch);
+}
+
+// Tiles of 16 x 16, 32 x 32 or 64 x 64 outputs: a larger one reads less shared memory per FMA and takes longer by itself.  A
+// launch's time is close to fixed + wave x ceil(blocks / SMs) for each of them, with the constants below (us, fitted to
+// 1 .. 1024 x 100 .. 10000: within 6 % of every time measured), and the least of the three is taken.
+static void launch_matrix(const float* a, int n, const float* b, int m, float* out, size_t pitch, int n_sm, cudaStream_t s)
+{
+    auto estimate = [&](int tile, double fixed, double wave) {
+        const long long blocks = (long long)((n + tile - 1) / tile) * ((m + tile - 1) / tile);
+        return fixed + wave * (double)((blocks + n_sm - 1) / n_sm);
+    };
+    const double t16 = estimate(16, 4.0, 8.2), t32 = estimate(32, 6.0, 15.7), t64 = estimate(64, 1.0, 46.0);
+    if (t16 <= t32 && t16 <= t64) launch_tile<4, 2, 1, 1, 64>(a, n, b, m, out, pitch, s);
+    else if (t32 <= t64)          launch_tile<4, 2, 2, 2, 32>(a, n, b, m, out, pitch, s);
+    else                          launch_tile<4, 2, 4, 4, 16>(a, n, b, m, out, pitch, s);
 }
 
 // One call works in slices of at most CS_MAX_N x CS_MAX_M pairs, so the workspace a context keeps is bounded
@@ -114,7 +165,7 @@ static bool grow(float** p, size_t* cap, size_t need)
     return true;
 }
 
-int CosWorkspace::run(const float* ha, int n, const float* hb, int m, float* hout)
+int CosWorkspace::run(int device, const float* ha, int n, const float* hb, int m, float* hout)
 {
     const int sn = std::min(n, CS_MAX_N), sm = std::min(m, CS_MAX_M);
     if ((!stream && cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) ||
@@ -123,6 +174,8 @@ int CosWorkspace::run(const float* ha, int n, const float* hb, int m, float* hou
         cudaGetLastError();
         return -2;
     }
+    int n_sm = 0;
+    if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n_sm < 1) n_sm = 148;
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < n && e == cudaSuccess; i += sn) {
         const int cn = std::min(sn, n - i);
@@ -131,7 +184,7 @@ int CosWorkspace::run(const float* ha, int n, const float* hb, int m, float* hou
             const int cm = std::min(sm, m - j);
             e = cudaMemcpyAsync(b, hb + (size_t)j * CS_DIM, (size_t)cm * CS_DIM * 4, cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) break;
-            launch_matrix(a, cn, b, cm, out, (size_t)cm, stream);
+            launch_matrix(a, cn, b, cm, out, (size_t)cm, n_sm, stream);
             e = cudaGetLastError();
             if (e == cudaSuccess)
                 e = cm == m ? cudaMemcpyAsync(hout + (size_t)i * m, out, (size_t)cn * m * 4, cudaMemcpyDeviceToHost, stream)
@@ -151,7 +204,7 @@ extern "C" int ffcu_cos_sim_matrix(int device, const float* a, int n, const floa
     if (!a || !b || !out || n < 1 || m < 1) { ffcu_set_error("ffcu_cos_sim_matrix: bad arguments"); return -1; }
     FFCU_CHECK(cudaSetDevice(device));
     CosWorkspace w;
-    const int rc = w.run(a, n, b, m, out);
+    const int rc = w.run(device, a, n, b, m, out);
     w.release();
     return rc;
 }
@@ -164,7 +217,7 @@ int CosWorkspace::call(int device, const float* ha, int n, const float* hb, int 
     if (!mu.try_lock()) return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
     int rc = cudaSetDevice(device) == cudaSuccess ? 0 : -100;
     if (rc) { ffcu_set_error("cudaSetDevice(%d) failed", device); cudaGetLastError(); }
-    else rc = run(ha, n, hb, m, hout);
+    else rc = run(device, ha, n, hb, m, hout);
     mu.unlock();
     return rc;
 }

@@ -9,6 +9,6 @@ struct CosWorkspace {
     size_t cap_a = 0, cap_b = 0, cap_out = 0;        // floats
     cudaStream_t stream = nullptr;
     int call(int device, const float* ha, int n, const float* hb, int m, float* hout);
-    int run(const float* ha, int n, const float* hb, int m, float* hout);
+    int run(int device, const float* ha, int n, const float* hb, int m, float* hout);
     void release();
 };

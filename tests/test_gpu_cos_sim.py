@@ -41,6 +41,26 @@ def test_matrix_edges(engine, n, m):
     check(engine.cos_sim_matrix(a, b), a, b, rng)
 
 
+# each tile (16, 32 and 64 rows and columns a block) at its edges, one row or column more or less than whole tiles included;
+# 148 SMs change tile between 128 x 500 and 128 x 1000, between 256 x 1000 and 512 x 1000, and at few rows by columns
+@pytest.mark.parametrize("n,m", [(1, 15), (16, 16), (17, 17), (15, 2369), (1, 10001), (16, 9999), (128, 500), (128, 1000), (95, 1023),
+                                 (97, 1025), (256, 1000), (512, 1000), (511, 1023), (513, 1025), (1024, 300), (64, 10000)])
+def test_matrix_tiles(engine, n, m):
+    rng = np.random.default_rng(n * 104729 + m)
+    a = rng.standard_normal((n, 512), dtype=np.float32)
+    b = rng.standard_normal((m, 512), dtype=np.float32)
+    a[n // 2] = 0
+    b[0] = np.float32(1e-30) * b[0]
+    got = engine.cos_sim_matrix(a, b)
+    check(got, a, b, rng)
+    # every output: two float64 evaluations of a sum of 512 terms differ by at most 1024 * 2^-53 of the norms' product
+    # (Cauchy-Schwarz), far below the half unit of the float32 result (2^-25 for |value| <= 1)
+    x, y = a.astype(np.float64), b.astype(np.float64)
+    nx, ny = np.sqrt((x * x).sum(1)), np.sqrt((y * y).sum(1))
+    want = np.divide(x @ y.T, np.outer(nx, ny), out=np.zeros((n, m)), where=np.outer(nx, ny) != 0)
+    assert np.abs(got - want).max() <= 2.0 ** -25 + 1e-12
+
+
 def test_matrix_special_values(engine):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((20, 512), dtype=np.float32)
