@@ -20,6 +20,7 @@
 #include "ffcu_internal.cuh"
 #include "cos_sim.cuh"
 
+#include <stdint.h>
 #include <algorithm>
 
 #define CS_DIM 512
@@ -148,6 +149,15 @@ static void launch_matrix(const float* a, int n, const float* b, int m, float* o
 #define CS_MAX_N 2048
 #define CS_MAX_M 4096
 
+static bool beyond_one_slice(int n, int m) { return n > CS_MAX_N || m > CS_MAX_M; }
+
+// A result that takes the place of an input: every row has to be read before the first result is written.
+static bool written_over(const float* out, int n, int m, const float* in, int rows)
+{
+    const uintptr_t o = (uintptr_t)out, i = (uintptr_t)in;
+    return o < i + (size_t)rows * CS_DIM * sizeof(float) && i < o + (size_t)n * m * sizeof(float);
+}
+
 void CosWorkspace::release()
 {
     cudaFree(a); cudaFree(b); cudaFree(out);
@@ -167,7 +177,8 @@ static bool grow(float** p, size_t* cap, size_t need)
 
 int CosWorkspace::run(int device, const float* ha, int n, const float* hb, int m, float* hout)
 {
-    const int sn = std::min(n, CS_MAX_N), sm = std::min(m, CS_MAX_M);
+    const bool whole = written_over(hout, n, m, ha, n) || written_over(hout, n, m, hb, m);
+    const int sn = whole ? n : std::min(n, CS_MAX_N), sm = whole ? m : std::min(m, CS_MAX_M);
     if ((!stream && cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) ||
         !grow(&a, &cap_a, (size_t)sn * CS_DIM) || !grow(&b, &cap_b, (size_t)sm * CS_DIM) || !grow(&out, &cap_out, (size_t)sn * sm)) {
         ffcu_set_error("ffcu_cos_sim_matrix: device allocation failed");
@@ -210,10 +221,12 @@ extern "C" int ffcu_cos_sim_matrix(int device, const float* a, int n, const floa
 }
 
 // The same through a workspace that its owner keeps.  Calls from several threads each go through: one takes the
-// workspace, the others make their own for the call.
+// workspace, the others make their own for the call; so does a call that cannot go in slices, which the bound is for.
 int CosWorkspace::call(int device, const float* ha, int n, const float* hb, int m, float* hout)
 {
     if (!ha || !hb || !hout || n < 1 || m < 1) { ffcu_set_error("ffcu_cos_sim_matrix: bad arguments"); return -1; }
+    if (beyond_one_slice(n, m) && (written_over(hout, n, m, ha, n) || written_over(hout, n, m, hb, m)))
+        return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
     if (!mu.try_lock()) return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
     int rc = cudaSetDevice(device) == cudaSuccess ? 0 : -100;
     if (rc) { ffcu_set_error("cudaSetDevice(%d) failed", device); cudaGetLastError(); }

@@ -95,3 +95,18 @@ def test_matrix_from_several_threads(engine):
             bad.append("embed")
     [t.join() for t in ts]
     assert not bad
+
+
+@pytest.mark.parametrize("n,m,over", [(500, 5000, "b"), (2500, 520, "a"), (300, 600, "b")])
+def test_matrix_written_over_an_input(engine, n, m, over):
+    """A result that takes the place of an input, also where the matrix goes in slices: the inputs are read first."""
+    rng = np.random.default_rng(n + m)
+    a = rng.standard_normal((n, 512), dtype=np.float32)
+    b = rng.standard_normal((m, 512), dtype=np.float32)
+    want = engine.cos_sim_matrix(a, b)
+    src = a if over == "a" else b
+    shared = np.empty(max(n * m, src.size), np.float32)
+    shared[:src.size] = src.reshape(-1)
+    pa, pb = (shared, b) if over == "a" else (a, shared)
+    assert engine.lib.fastface_cos_sim_matrix(engine.h, pa.ctypes.data, n, pb.ctypes.data, m, shared.ctypes.data) == 0
+    assert np.array_equal(shared[:n * m].reshape(n, m), want)
