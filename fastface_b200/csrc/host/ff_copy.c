@@ -19,6 +19,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <time.h>
+#include <unistd.h>
 #if defined(__SSE2__)
 #include <emmintrin.h>
 #endif
@@ -39,6 +40,7 @@ struct ff_copy_pool {
     int streaming;           /* of the job */
     int wanted, started, stop, sleeping;
     pthread_t th[FF_COPY_MAX_HELPERS];
+    pid_t owner;             /* a process forked from the owner has no helpers, and the locks as the fork found them */
 };
 
 static void relax(void)
@@ -126,6 +128,7 @@ ff_copy_pool* ff_copy_pool_create(int helpers)
     if (helpers > FF_COPY_MAX_HELPERS) helpers = FF_COPY_MAX_HELPERS;
     if (helpers > cpus / 3) helpers = cpus / 3;
     p->wanted = helpers < 0 ? 0 : helpers;
+    p->owner = getpid();
     if (pthread_mutex_init(&p->mu, NULL) != 0) { free(p); return NULL; }
     if (pthread_cond_init(&p->wake, NULL) != 0) { pthread_mutex_destroy(&p->mu); free(p); return NULL; }
     return p;
@@ -147,6 +150,7 @@ static void start_helpers(ff_copy_pool* p)
 void ff_copy_pool_destroy(ff_copy_pool* p)
 {
     if (!p) return;
+    if (p->owner != getpid()) return;            /* left as it is: the condition's sleepers would be waited for for good */
     pthread_mutex_lock(&p->mu);
     p->stop = 1;
     pthread_cond_broadcast(&p->wake);
@@ -159,7 +163,7 @@ void ff_copy_pool_destroy(ff_copy_pool* p)
 
 void ff_copy(ff_copy_pool* p, void* dst, const void* src, size_t bytes, int streaming)
 {
-    if (!p || p->wanted == 0 || bytes < FF_COPY_MIN_SHARED) {
+    if (!p || p->wanted == 0 || bytes < FF_COPY_MIN_SHARED || p->owner != getpid()) {
         if (streaming) copy_streaming((char*)dst, (const char*)src, bytes);
         else memcpy(dst, src, bytes);
         return;

@@ -11,7 +11,8 @@ extern "C" {
 typedef struct ff_copy_pool ff_copy_pool;
 
 /* Helper threads for ff_copy: as many as asked for, but never more than a third of the CPUs the process may run on and
- * at most 3.  The threads start with the first copy that is worth sharing.  NULL when out of memory. */
+ * at most 3.  The threads start with the first copy that is worth sharing.  NULL when out of memory.  In a process forked
+ * from the one that made the pool, ff_copy copies without helpers and ff_copy_pool_destroy does nothing. */
 ff_copy_pool* ff_copy_pool_create(int helpers);
 void ff_copy_pool_destroy(ff_copy_pool* p);
 

@@ -1,6 +1,10 @@
 """The shared copy (csrc/host/ff_copy.c): every byte, at sizes around its piece and its sharing threshold, at odd
 addresses, with pools of several owners at work."""
 import ctypes as C
+import os
+import signal
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -65,3 +69,42 @@ def test_pools_of_several_threads(lib):
     [t.start() for t in ts]
     [t.join(timeout=120) for t in ts]
     assert not bad and not any(t.is_alive() for t in ts)
+
+
+FORKED = """
+import ctypes as C, os, sys, time
+L = C.CDLL(sys.argv[1])
+L.ff_copy_pool_create.restype = C.c_void_p
+L.ff_copy_pool_create.argtypes = [C.c_int]
+L.ff_copy_pool_destroy.argtypes = [C.c_void_p]
+L.ff_copy.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+n = 4 << 20
+src, dst, again = C.create_string_buffer(os.urandom(n), n), C.create_string_buffer(n), C.create_string_buffer(n)
+pool = L.ff_copy_pool_create(3)
+L.ff_copy(pool, dst, src, n, 0)
+time.sleep(0.05)                       # the helpers sleep by now
+bad = 0
+for first_copies in (0, 1):
+    pid = os.fork()
+    if pid == 0:
+        if first_copies:
+            L.ff_copy(pool, again, src, n, 1)
+        L.ff_copy_pool_destroy(pool)
+        os._exit(0 if again.raw == src.raw or not first_copies else 1)
+    bad |= os.waitpid(pid, 0)[1]
+L.ff_copy(pool, again, src, n, 0)      # the parent's pool is as it was
+L.ff_copy_pool_destroy(pool)
+sys.exit(0 if bad == 0 and dst.raw == src.raw and again.raw == src.raw else 1)
+"""
+
+
+def test_forked_process_copies_and_destroys(lib):
+    """A child forked after the helpers have started has none of them: it must neither wait for them nor for the
+    locks they left (a program that forks workers and lets them drop the object they inherited)."""
+    p = subprocess.Popen([sys.executable, "-W", "ignore", "-c", FORKED, ff.LIB_PATH], start_new_session=True)
+    try:
+        assert p.wait(timeout=20) == 0
+    finally:
+        if p.poll() is None:
+            os.killpg(p.pid, signal.SIGKILL)           # parent and the child that hangs
+            p.wait()
