@@ -76,13 +76,17 @@ struct ffcu_ctx {
     char* out_mem[2] = {};       // allocation of out_slot[k]: OUT_HEAD bytes, then the embeddings
     // Page-locked staging.  An input in pageable memory is copied into a ring by several threads (ff_copy.c) and goes
     // on from there: the driver's own staging is one thread, and for an output it blocks the caller until the forward is done.
+    // Made with the context (a first call that made it would take 6-12 ms longer); NULL where the host has no memory to
+    // lock: the driver's staging serves then.
     ff_copy_pool* pool = nullptr;
     char* stage_in = nullptr;
     size_t stage_slot_bytes = 0;
     cudaEvent_t ev_stage[STAGE_SLOTS] = {};
     unsigned long long stage_seq = 0;
     char* stage_out[2] = {};     // [OUT_HEAD: error word | embeddings of min(max_batch, STAGE_OUT_FACES) faces]
-    bool err_read[2] = {true, true};                 // the slot's error word is in (or on its way to) stage_out
+    int* h_err = nullptr;        // page-locked, [2]: the slots' error words where their outputs are not staged
+    int* err_at[2] = {};         // where the slot's error word arrives: h_err or the front of stage_out
+    bool err_read[2] = {true, true};                 // it is there or on its way
     struct Pending { float* dst; size_t bytes; } pending[2] = {};   // output that waits in stage_out for its caller's memory
     bool idle = true;            // nothing submitted since the last wait
     int head_end[2] = {};        // layers [0, head_end) a step may run in chunks: fp32 / 8-bit input
@@ -134,6 +138,30 @@ static float* upload_f32(const float* src, int n)
     return d;
 }
 
+static int g_test_deny_staging = 0;
+
+// The next `count` page-locked staging allocations of the process fail (for the test of a host that has none to give).
+extern "C" void ffcu_test_deny_staging(int count) { g_test_deny_staging = count; }
+
+static char* stage_alloc(size_t bytes)
+{
+    void* p = nullptr;
+    if (g_test_deny_staging > 0) { g_test_deny_staging--; return nullptr; }
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    memset(p, 0, OUT_HEAD);
+    return (char*)p;
+}
+
+// The staging, as far as the host gives it.
+static void make_staging(ffcu_ctx* c)
+{
+    const size_t out_bytes = OUT_HEAD + (size_t)std::min(c->max_batch, STAGE_OUT_FACES) * 512 * sizeof(float);
+    c->stage_slot_bytes = (size_t)std::min(c->max_batch, STAGE_FACES) * 37632 * sizeof(float);
+    c->stage_in = stage_alloc(STAGE_SLOTS * c->stage_slot_bytes);
+    for (int k = 0; k < 2; k++) c->stage_out[k] = stage_alloc(out_bytes);
+    c->pool = ff_copy_pool_create(3);                 // NULL: the caller's thread copies alone
+}
+
 extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t bytes_per_face)
 {
     if (n_bufs < 1 || n_bufs > FFCU_MAX_BUFS || max_batch < 1) { ffcu_set_error("bad ffcu_create arguments"); return nullptr; }
@@ -169,15 +197,10 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
         ok = ok && cudaMalloc(&c->d_fc_tc_scratch, nb) == cudaSuccess;
         if (ok) cudaMemset(c->d_fc_tc_scratch, 0, nb);
     }
-    for (int k = 0; k < 2 && ok; k++) {
-        const size_t nb = OUT_HEAD + (size_t)std::min(max_batch, STAGE_OUT_FACES) * 512 * sizeof(float);
-        ok = cudaHostAlloc(&c->stage_out[k], nb, cudaHostAllocDefault) == cudaSuccess;
-        if (ok) *(int*)c->stage_out[k] = 0;
-    }
-    c->stage_slot_bytes = (size_t)std::min(max_batch, STAGE_FACES) * 37632 * sizeof(float);
-    ok = ok && cudaHostAlloc(&c->stage_in, STAGE_SLOTS * c->stage_slot_bytes, cudaHostAllocDefault) == cudaSuccess;
+    ok = ok && cudaHostAlloc(&c->h_err, 2 * sizeof(int), cudaHostAllocDefault) == cudaSuccess;
+    for (int k = 0; k < 2 && ok; k++) { c->h_err[k] = 0; c->err_at[k] = &c->h_err[k]; }
+    if (ok) make_staging(c);
     for (int k = 0; k < STAGE_SLOTS && ok; k++) ok = cudaEventCreateWithFlags(&c->ev_stage[k], cudaEventDisableTiming) == cudaSuccess;
-    ok = ok && (c->pool = ff_copy_pool_create(3)) != nullptr;
     ok = ok && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess;
     const char* impl = getenv("FF_CONV_IMPL");
     c->force_simt = (impl && strcmp(impl, "simt") == 0) ? 1 : 0;
@@ -223,6 +246,7 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     cudaFree(c->d_fc_scratch); cudaFree(c->d_fc_tc_scratch);
     for (cudaEvent_t ev : c->ev_stage) if (ev) cudaEventDestroy(ev);
     if (c->stage_in) cudaFreeHost(c->stage_in);
+    if (c->h_err) cudaFreeHost(c->h_err);
     ff_copy_pool_destroy(c->pool);
     c->cos.release();
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -694,12 +718,14 @@ static int copy_in(ffcu_ctx* c, void* dst, const void* src, size_t bytes, bool s
 static int copy_out(ffcu_ctx* c, int slot, int n, float* host_out, cudaStream_t s)
 {
     const size_t nb = (size_t)n * 512 * sizeof(float);
-    if (n <= STAGE_OUT_FACES && is_pageable(host_out, nb)) {
+    if (n <= STAGE_OUT_FACES && c->stage_out[slot] && is_pageable(host_out, nb)) {
         FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], OUT_HEAD + nb, cudaMemcpyDeviceToHost, s));
         c->pending[slot] = {host_out, nb};
+        c->err_at[slot] = (int*)c->stage_out[slot];
     } else {
         FFCU_CHECK(cudaMemcpyAsync(host_out, c->out_slot[slot], nb, cudaMemcpyDeviceToHost, s));
-        FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], sizeof(int), cudaMemcpyDeviceToHost, s));
+        FFCU_CHECK(cudaMemcpyAsync(&c->h_err[slot], c->out_mem[slot], sizeof(int), cudaMemcpyDeviceToHost, s));
+        c->err_at[slot] = &c->h_err[slot];
     }
     c->err_read[slot] = true;
     return 0;
@@ -722,7 +748,7 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
     FFCU_CHECK(cudaSetDevice(c->device));
     const int slot = (int)(c->seq & 1);
     const bool reused = c->seq >= 2;
-    const bool staged = is_pageable(host_in, (size_t)n * bytes_per_face);
+    const bool staged = c->stage_in && is_pageable(host_in, (size_t)n * bytes_per_face);
     const bool was_idle = c->idle;
     c->idle = false;
     if (c->pending[slot].dst) {                       // the output two steps ago still sits in the slot's staging
@@ -825,7 +851,10 @@ static int wait_impl(ffcu_ctx* c)
 {
     FFCU_CHECK(cudaSetDevice(c->device));
     for (int k = 0; k < 2; k++)
-        if (!c->err_read[k]) FFCU_CHECK(cudaMemcpyAsync(c->stage_out[k], c->out_mem[k], sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        if (!c->err_read[k]) {
+            FFCU_CHECK(cudaMemcpyAsync(&c->h_err[k], c->out_mem[k], sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            c->err_at[k] = &c->h_err[k];
+        }
     if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_in));
     FFCU_CHECK(cudaStreamSynchronize(c->stream));
     if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_out));
@@ -834,12 +863,12 @@ static int wait_impl(ffcu_ctx* c)
     for (int k = 0; k < 2; k++) {
         c->err_read[k] = true;
         deliver(c, k);
-        if (err == 0) err = *(int*)c->stage_out[k];
+        if (err == 0) err = *c->err_at[k];
     }
     if (err != 0) {
         ffcu_set_error("device reported error word %d (a bounded wait inside a kernel ran out)", err);
         for (int k = 0; k < 2; k++) {
-            *(int*)c->stage_out[k] = 0;
+            *c->err_at[k] = 0;
             cudaMemsetAsync(c->out_mem[k], 0, sizeof(int), c->stream);
         }
         // a launch that gave up may have left partial sums or tickets behind

@@ -1,5 +1,7 @@
 """Input and output paths of a call: pageable and page-locked memory, one stream or the pipeline, first layers in
 chunks.  Every face must come out with the bytes a batch-8 call gives it."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -83,3 +85,28 @@ def test_launches_of_every_chunk_are_counted(data, model_root, ffw4):
                 e.embed_batch(f32[:n])
                 extra = e.launches_per_forward - whole
                 assert extra == 0 if chunks == 1 else extra >= 2 * (chunks - 1), n
+
+
+@pytest.mark.parametrize("denied", [1, 2, 3], ids=["no-ring", "one-output-slot", "nothing"])
+def test_hosts_without_memory_to_lock(data, model_root, ffw4, denied):
+    """Page-locked staging is not needed: where the host has none to give, the context is made all the same and
+    pageable calls go through the driver's own staging."""
+    px, f32, want = data
+    want = want[ff.EPILOGUE_CONTRACT]
+    lib = ff.load_library()
+    lib.ffcu_test_deny_staging.restype = None
+    lib.ffcu_test_deny_staging.argtypes = [C.c_int]
+    lib.ffcu_test_deny_staging(denied)                 # the ring, then the two output slots
+    try:
+        e = ff.FastFace(ffw4, cwd=model_root, max_batch=130)
+    finally:
+        lib.ffcu_test_deny_staging(0)
+    with e:
+        for rep in range(3):
+            for n in (1, 39, 40, 129, 300):
+                o = (11 * n + rep) % (N - n + 1)
+                for src, run in ((f32, e.embed_into), (px, e.embed_into_u8)):
+                    for pin_in in (False, True):
+                        out = np.full((n, 512), 9, np.float32)
+                        run(pinned(src[o:o + n]) if pin_in else src[o:o + n], out)
+                        assert np.array_equal(out, want[o:o + n]), (rep, n)
