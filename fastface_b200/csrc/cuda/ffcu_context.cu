@@ -219,14 +219,16 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
 }
 
 static void free_layer_memory(DevLayer& L);
+static void deliver(ffcu_ctx* c, int slot);
 
 extern "C" void ffcu_destroy(ffcu_ctx* c)
 {
     if (!c) return;
     cudaSetDevice(c->device);
-    if (c->stream) cudaStreamSynchronize(c->stream);
-    if (c->s_in) cudaStreamSynchronize(c->s_in);
-    if (c->s_out) cudaStreamSynchronize(c->s_out);
+    bool done = true;
+    for (cudaStream_t s : {c->stream, c->s_in, c->s_out})
+        if (s && cudaStreamSynchronize(s) != cudaSuccess) done = false;
+    for (int k = 0; k < 2 && done; k++) deliver(c, k);    // outputs nobody has waited for
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
     for (auto& ch : c->chains) for (ChainPlan* q : ch.plan) ffcu_chain_free(q);
     for (auto& L : c->layers) {
