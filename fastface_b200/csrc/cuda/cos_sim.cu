@@ -123,25 +123,29 @@ cos_sim_matrix_kernel(const float* __restrict__ a, int n, const float* __restric
 }
 
 template <int WR, int WC, int RM, int RN, int KC>
-static void launch_tile(const float* a, int n, const float* b, int m, float* out, size_t pitch, cudaStream_t s)
+static cudaError_t launch_tile(const float* a, int n, const float* b, int m, float* out, size_t pitch, cudaStream_t s)
 {
     using T = CosTile<WR, WC, RM, RN, KC>;
-    cos_sim_matrix_kernel<WR, WC, RM, RN, KC><<<dim3((m + T::TJ - 1) / T::TJ, (n + T::TI - 1) / T::TI), T::THREADS, 0, s>>>(a, n, b, m, out, pitch);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((m + T::TJ - 1) / T::TJ, (n + T::TI - 1) / T::TI);
+    cfg.blockDim = dim3(T::THREADS);
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, cos_sim_matrix_kernel<WR, WC, RM, RN, KC>, a, n, b, m, out, pitch);
 }
 
 // Tiles of 16 x 16, 32 x 32 or 64 x 64 outputs: a larger one reads less shared memory per FMA and takes longer by itself.  A
 // launch's time is close to fixed + wave x ceil(blocks / SMs) for each of them, with the constants below (us, fitted to
 // 1 .. 1024 x 100 .. 10000: within 6 % of every time measured), and the least of the three is taken.
-static void launch_matrix(const float* a, int n, const float* b, int m, float* out, size_t pitch, int n_sm, cudaStream_t s)
+static cudaError_t launch_matrix(const float* a, int n, const float* b, int m, float* out, size_t pitch, int n_sm, cudaStream_t s)
 {
     auto estimate = [&](int tile, double fixed, double wave) {
         const long long blocks = (long long)((n + tile - 1) / tile) * ((m + tile - 1) / tile);
         return fixed + wave * (double)((blocks + n_sm - 1) / n_sm);
     };
     const double t16 = estimate(16, 4.0, 8.2), t32 = estimate(32, 6.0, 15.7), t64 = estimate(64, 1.0, 46.0);
-    if (t16 <= t32 && t16 <= t64) launch_tile<4, 2, 1, 1, 64>(a, n, b, m, out, pitch, s);
-    else if (t32 <= t64)          launch_tile<4, 2, 2, 2, 32>(a, n, b, m, out, pitch, s);
-    else                          launch_tile<4, 2, 4, 4, 16>(a, n, b, m, out, pitch, s);
+    if (t16 <= t32 && t16 <= t64) return launch_tile<4, 2, 1, 1, 64>(a, n, b, m, out, pitch, s);
+    if (t32 <= t64) return launch_tile<4, 2, 2, 2, 32>(a, n, b, m, out, pitch, s);
+    return launch_tile<4, 2, 4, 4, 16>(a, n, b, m, out, pitch, s);
 }
 
 // One call works in slices of at most CS_MAX_N x CS_MAX_M pairs, so the workspace a context keeps is bounded
@@ -195,8 +199,8 @@ int CosWorkspace::run(int device, const float* ha, int n, const float* hb, int m
             const int cm = std::min(sm, m - j);
             e = cudaMemcpyAsync(b, hb + (size_t)j * CS_DIM, (size_t)cm * CS_DIM * 4, cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) break;
-            launch_matrix(a, cn, b, cm, out, (size_t)cm, n_sm, stream);
-            e = cudaGetLastError();
+            // (the launch's own result: the thread's last error may be one that the caller has left there)
+            e = launch_matrix(a, cn, b, cm, out, (size_t)cm, n_sm, stream);
             if (e == cudaSuccess)
                 e = cm == m ? cudaMemcpyAsync(hout + (size_t)i * m, out, (size_t)cn * m * 4, cudaMemcpyDeviceToHost, stream)
                             : cudaMemcpy2DAsync(hout + (size_t)i * m + j, (size_t)m * 4, out, (size_t)cm * 4, (size_t)cm * 4, cn,

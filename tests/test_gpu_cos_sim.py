@@ -1,4 +1,5 @@
 """Similarity matrix at the edges of its tiles and slices: the bits of fastface_cos_sim for every pair looked at."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -110,3 +111,15 @@ def test_matrix_written_over_an_input(engine, n, m, over):
     pa, pb = (shared, b) if over == "a" else (a, shared)
     assert engine.lib.fastface_cos_sim_matrix(engine.h, pa.ctypes.data, n, pb.ctypes.data, m, shared.ctypes.data) == 0
     assert np.array_equal(shared[:n * m].reshape(n, m), want)
+
+
+def test_matrix_after_an_error_of_the_callers(engine):
+    """The CUDA runtime is the process's: an error that other code has left behind on this thread is none of the call's."""
+    rng = np.random.default_rng(9)
+    a, b = rng.standard_normal((5, 512), dtype=np.float32), rng.standard_normal((9, 512), dtype=np.float32)
+    want = engine.cos_sim_matrix(a, b)
+    rt = C.CDLL("libcudart.so.12")
+    p = C.c_void_p()
+    assert rt.cudaMalloc(C.byref(p), C.c_size_t(1 << 60)) == 2         # more than any device has: out of memory
+    assert np.array_equal(engine.cos_sim_matrix(a, b), want)
+    rt.cudaGetLastError()
