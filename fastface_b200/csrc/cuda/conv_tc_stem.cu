@@ -211,8 +211,9 @@ static int launch_stem(int grid, int smem, cudaStream_t s, const CUtensorMap& ma
                        const float* inv3)
 {
     if constexpr (EPI == EPI_SLOPE_BN) {
-        // From 30 tiles per CTA on (45 faces): below, the launch is shorter but its unrolled code, fetched cold in every
-        // forward, costs as much (forward of 17 / 24 / 33 faces 411.4 / 444.2 / 485.2 -> 413.2 / 446.0 / 487.2 us; 48: 706 -> 702).
+        // From 30 tiles per CTA on (46 faces in the launch; a chunk of a larger call counts by itself): below, the launch is shorter but
+        // its unrolled code, fetched cold in every forward, costs as much (forward of 17 / 24 / 33 faces in one launch 411.4 / 444.2 /
+        // 485.2 -> 413.2 / 446.0 / 487.2 us; 48: 706 -> 702).
         TcConst<64> ct;
         if (prm.total_tiles / grid >= 30 && tc_const_args(prm, 64, EPI, &ct.v[0][0])) return launch_stem_c<CONTRACT, EPI, IN_U8, true>(grid, smem, s, mapB, prm, in_any, inv3, ct);
     }

@@ -1,5 +1,7 @@
-"""Launches whose per-channel constants are kernel parameters (stem from 30 tiles per CTA, 56x56 residual + BN layers from 8):
-the faces on both sides of each line, with a ragged last tile wave, give the bytes of batch-8 calls."""
+"""Launches whose per-channel constants are kernel parameters: both sides of each line, with ragged last tile waves, give
+the bytes of batch-8 calls.  On 148 SMs: the stem from 46 faces per launch (30 tiles of 98 a face for every CTA), the 56x56
+residual + BN layers from 43 (8 tiles of 28 a face), the 28x28 ones from 43 per call (two tiles per CTA pair).  A call below
+128 faces runs the stem, and for fp32 the 56x56 layers too, in two chunks of (n + 1) / 2 and n / 2 faces."""
 import numpy as np
 import pytest
 
@@ -7,7 +9,9 @@ import fastface_b200 as ff
 from fastface_b200 import synth
 
 pytestmark = pytest.mark.gpu
-SIZES = (42, 43, 45, 46, 47, 90)
+# 8-bit: stem 45 + 45 | 46 + 45 | 46 + 46 faces at 90 | 91 | 92; 56x56 and 28x28 at 42 | 43.  fp32: the same for the stem;
+# 56x56 42 + 42 | 43 + 42 | 43 + 43 at 84 | 85 | 86.  128: chunks of 64
+SIZES = (42, 43, 45, 47, 84, 85, 86, 90, 91, 92, 128)
 
 
 @pytest.mark.parametrize("mode", [ff.EPILOGUE_CONTRACT, ff.EPILOGUE_STRICT], ids=["contract", "strict"])
