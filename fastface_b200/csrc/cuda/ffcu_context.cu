@@ -4,6 +4,7 @@
 #include "ffcu_internal.cuh"
 #include "cos_sim.cuh"
 #include "../host/ff_copy.h"
+#include "../host/ff_plan.h"
 #include <math.h>
 
 #include <stdarg.h>
@@ -374,9 +375,7 @@ static size_t out_bytes_per_face(const ffcu_layer& d) { return (size_t)d.Ho * d.
 
 // The layers a step may run chunk by chunk (submit_impl), each chunk through all of them before the next one starts:
 // the stem alone for 8-bit input (its time is about its input's on PCIe), all leading layers with 64 input
-// channels for fp32 (four times the bytes).  A buffer holds tensors of different bytes per face, so face f of one tensor may
-// lie where a lower face of another does: a head is only taken when no layer of it writes a buffer at fewer bytes
-// per face than the tensor that the rest of the network finds there (then chunk j writes behind all that chunks < j left).
+// channels for fp32 (four times the bytes) as far as the buffers allow (ff_plan_head_end).
 static void find_heads(ffcu_ctx* c)
 {
     c->head_end[0] = c->head_end[1] = 0;
@@ -384,21 +383,10 @@ static void find_heads(ffcu_ctx* c)
     if (nl < 3 || !c->layers[1].fused_stem || !c->layers[1].stem_tc) return;
     size_t end = 2;
     while (end < nl && c->layers[end].d.kind == FFCU_CONV && c->layers[end].tc && c->layers[end].d.Cin_pad == 64) end++;
-    for (; end > 2; end--) {
-        if (end < nl && c->layers[end - 1].sc) continue;      // a fused pair stays together
-        std::vector<size_t> left((size_t)c->n_bufs, 0);       // bytes per face of the last tensor the head writes there
-        bool ok = true;
-        for (size_t k = end - 1; k >= 1 && ok; k--) {
-            const ffcu_layer& d = c->layers[k].d;
-            for (int b : {d.dst_buf, d.bn2_dst_buf}) {
-                if (b < 0) continue;
-                if (!left[b]) left[b] = out_bytes_per_face(d);
-                else if (out_bytes_per_face(d) < left[b]) ok = false;
-            }
-        }
-        if (ok) break;
-    }
-    c->head_end[0] = (int)end;
+    std::vector<ffcu_layer> d;
+    std::vector<unsigned char> with_next;
+    for (const DevLayer& L : c->layers) { d.push_back(L.d); with_next.push_back(L.sc ? 1 : 0); }
+    c->head_end[0] = ff_plan_head_end(d.data(), (int)nl, (int)end, with_next.data());
     c->head_end[1] = 2;
 }
 

@@ -337,3 +337,23 @@ void ff_plan_free(ff_plan* p)
     free(p->pool); free(p->layers);
     memset(p, 0, sizeof *p);
 }
+
+int ff_plan_head_end(const ffcu_layer* l, int n, int end, const unsigned char* with_next)
+{
+    for (; end > 2; end--) {
+        if (end < n && with_next[end - 1]) continue;
+        size_t left[FF_MAX_BUFS] = {0};                 /* bytes per face of the last tensor the head writes there */
+        int ok = 1;
+        for (int k = end - 1; k >= 1 && ok; k--) {
+            const size_t bytes = (size_t)l[k].Ho * (size_t)l[k].Wo * (size_t)l[k].Cout;
+            const int dst[2] = { l[k].dst_buf, l[k].bn2_dst_buf };
+            for (int i = 0; i < 2; i++) {
+                if (dst[i] < 0 || dst[i] >= FF_MAX_BUFS) continue;
+                if (!left[dst[i]]) left[dst[i]] = bytes;
+                else if (bytes < left[dst[i]]) ok = 0;
+            }
+        }
+        if (ok) break;
+    }
+    return end;
+}

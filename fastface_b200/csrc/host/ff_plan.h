@@ -5,6 +5,10 @@
 #include "ff_model.h"
 #include "ff_cuda.h"
 
+#ifdef __cplusplus
+extern "C" {
+#endif
+
 typedef struct {
     int n_layers;
     ffcu_layer* layers;      /* arrays inside are owned by the plan (see pool) */
@@ -21,4 +25,15 @@ typedef struct {
 int  ff_plan_build(ff_plan* p, const ff_model* m);
 void ff_plan_free(ff_plan* p);
 
+/* The layers [0, return value) of l[0 .. n) that may run chunk by chunk, each chunk of faces through all of them before the
+ * next one starts; at most `end`, at least 2 (the input's quantisation and the stem).  Tensors are laid out face after face
+ * from their buffer's start, and a buffer holds tensors of different bytes per face, so face f of one may lie where
+ * a lower face of another does: a head is only taken where no layer of it writes a buffer at fewer bytes per face than
+ * the tensor that the rest of the network finds there (then chunk j writes behind all that chunks < j left).  with_next[k] != 0:
+ * layers k and k + 1 go out as one launch and stay on one side. */
+int  ff_plan_head_end(const ffcu_layer* l, int n, int end, const unsigned char* with_next);
+
+#ifdef __cplusplus
+}
+#endif
 #endif
