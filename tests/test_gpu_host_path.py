@@ -71,22 +71,6 @@ def test_unaligned_and_interleaved_calls(data, model_root, ffw4):
             assert np.array_equal(out, want[o:o + n]), (n, o)
 
 
-def test_launches_of_every_chunk_are_counted(data, model_root, ffw4):
-    """A step whose first layers run in chunks reports what it launched: the stem once per chunk for 8-bit input, the
-    stem and the layers behind it once per chunk for fp32; eager, captured and replayed."""
-    px, f32, _ = data
-    with ff.FastFace(ffw4, cwd=model_root, max_batch=N) as e:
-        for n, chunks in ((39, 1), (40, 2), (127, 2), (128, 2), (129, 3), (256, 4)):
-            e.bench_resident(f32[:n], iters=1)
-            whole = e.launches_per_forward
-            for _ in range(3):
-                e.embed_batch_u8(px[:n])
-                assert e.launches_per_forward == whole + chunks - 1, n
-                e.embed_batch(f32[:n])
-                extra = e.launches_per_forward - whole
-                assert extra == 0 if chunks == 1 else extra >= 2 * (chunks - 1), n
-
-
 @pytest.mark.parametrize("denied", [1, 2, 3], ids=["no-ring", "one-output-slot", "nothing"])
 def test_hosts_without_memory_to_lock(data, model_root, ffw4, denied):
     """Page-locked staging is not needed: where the host has none to give, the context is made all the same and
