@@ -791,7 +791,7 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
             rc = launch_range(c, cnt, 0, (size_t)head, f);
             c->in_u8 = false;
             if (rc != 0) return rc;
-            head_launches = c->launches;
+            if (f == 0) head_launches = c->launches;        // counted once, at the full chunks' size
         }
     }
     // compute stream: needs the output slot drained by the copy-out of two steps ago

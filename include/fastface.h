@@ -115,7 +115,9 @@ int fastface_layer_count(const FastFace* ff);
 int fastface_layer_desc(const FastFace* ff, int k, int* desc12);
 int fastface_bench_layers(FastFace* ff, const float* input_hwc, int n, int iters, float* ms, int cap);
 
-/* Number of kernel launches the last embed/bench call issued per forward pass. */
+/* Number of kernel launches a forward pass of the last embed/bench call consists of: what every face goes through.  A step of
+ * 40 faces or more that finds the device idle runs its first layers in chunks; their launches count once here, not once per
+ * chunk. */
 int fastface_launches_per_forward(const FastFace* ff);
 
 /* Text of the last error on the calling thread ("" if none). */

@@ -107,6 +107,7 @@ int ffcu_trace(ffcu_ctx* c, const float* host_in, int n, float* host_out,
 /* iters forwards over n faces already on the device; CUDA-event milliseconds. */
 int ffcu_bench_resident(ffcu_ctx* c, const float* host_in, int n, int iters, float* ms);
 
+/* Launches that every face of the last call went through (layers run in chunks count once). */
 int ffcu_launches_per_forward(const ffcu_ctx* c);
 
 /* Per-layer timing: after one full forward over n resident faces, each layer is

@@ -94,3 +94,18 @@ def test_hosts_without_memory_to_lock(data, model_root, ffw4, denied):
                         out = np.full((n, 512), 9, np.float32)
                         run(pinned(src[o:o + n]) if pin_in else src[o:o + n], out)
                         assert np.array_equal(out, want[o:o + n]), (rep, n)
+
+
+def test_launch_count_does_not_depend_on_chunks(data, model_root, ffw4):
+    """The reported launches are those a face goes through: the same resident, in one piece and in chunks, a last chunk
+    of a single face included (129)."""
+    px, f32, _ = data
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=N) as e:
+        for n in (39, 40, 127, 128, 129, 256):
+            e.bench_resident(f32[:n], iters=1)
+            whole = e.launches_per_forward
+            for _ in range(3):
+                e.embed_batch_u8(px[:n])
+                assert e.launches_per_forward == whole, n
+                e.embed_batch(f32[:n])
+                assert e.launches_per_forward == whole, n
