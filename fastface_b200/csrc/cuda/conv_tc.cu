@@ -637,7 +637,8 @@ struct ChainPlan {
 
 // layers[i]: device pointers of layer i (weights, tables, residual, outputs); all layers are 3x3 stride-1
 // pad-1 convolutions C -> C on an H x W map, layer i + 1 reading what layer i writes (its fused BN's
-// output where it has one).  d_in = the first layer's input (one face, NHWC).  NULL when the shape does
+// output where it has one).  d_in = the first layer's input (max_batch faces, NHWC; a launch of n faces reads the first n).
+// bn = output channels per CTA (64: clusters of eight, 128: of four).  NULL when the shape does
 // not fit the kernel (C / bn column tiles x row tiles of 128 positions must be exactly a cluster's CTAs).
 ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers)
 {

@@ -670,12 +670,13 @@ __device__ __forceinline__ void walk_next(TileWalk& w, const TcParams& p)
 }
 
 // Epilogue warps: sixteen (warps 2..17), organised as 16 / wps sets of wps warps (TcParams::epi_wps,
-// 4 or 8).  Set s takes the CTA's tiles s, s + sets, ...; within a set, warp e covers the TMEM lane
+// 4, 8 or 16).  Set s takes the CTA's tiles s, s + sets, ...; within a set, warp e covers the TMEM lane
 // quarter its index gives it (hardware: warp w reads lanes [32*(w%4), +32)) and column group e / 4 of
 // wps / 4.  With four warps per set each warp walks all columns of its 32 rows, so the per-tile
 // bookkeeping (tile walk, addresses, two barrier operations) is spread over twice the elements: the
 // choice for narrow tiles at large batch.  Eight warps per set halve a tile's latency: the choice
-// when a CTA sees only a few tiles.  The sets never exceed the accumulator ring.
+// when a CTA sees only a few tiles.  All sixteen share a 256-column tile that is its CTA's only one.  The sets
+// never exceed the accumulator ring.
 #define TC_EPI_TOTAL_WARPS 16
 
 // Epilogue role shared by all kernels.  A warp walks its column range in pairs of 16-column chunks:

@@ -25,6 +25,8 @@
 // from there on: smaller chunks fill the SMs worse (these layers take 2.6 us a face at 256 faces, 2.85 at 64, 3.3 at 32) and
 // larger ones leave more of the copy in front (2.8 us a face of fp32).  Calls before -> after, staging included: 256 faces of page-
 // locked fp32 2713 -> 2319 us, 64 pageable 1440 -> 1110, 100 page-locked 8-bit 1190 -> 1167, 1024 of them 8140 -> 7960.
+// At the line, one stream -> chunks: 40 / 48 / 56 / 63 faces of page-locked fp32 775 / 863 / 913 / 957 -> 756 / 837 / 880 / 919 us,
+// of page-locked 8-bit pixels 689 / 769 / 801 / 830 -> 692 / 759 / 797 / 823, pageable fp32 835 / 931 / 992 / 1038 -> 824 / 903 / 956 / 990.
 #define CHUNK_MIN_FACES 40
 #define CHUNK_FACES 64
 
@@ -110,15 +112,16 @@ struct ffcu_ctx {
     std::map<long long, int> graph_launches;
     // Small batches: runs of same-shape 3x3 stride-1 convolutions (the 14x14 and 7x7 stages) go out as one
     // launch each (conv_tc_chain.cu).  Found on the first such forward; FF_CHAIN=0 disables.
-    // Calls of at most lean_max_batch faces run copy-in, forward and copy-out on the compute stream alone
-    // (FF_LEAN_MAX_BATCH, default 1: the single-face call; 0 = always the three-stream pipeline, whose overlap of
-    // the next call's copy-in with this call's kernels is worth more than the hops it costs from a few faces up).
-    int lean_max_batch = 1;
-    bool lean_last = false;      // the previous submit took that path
     struct Chain { size_t first; int count; ChainPlan* plan[2]; };   // clusters of eight (64 channels per CTA), of four (128)
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
+    // A whole call that is one step of fewer than CHUNK_MIN_FACES faces, and any submit of at most lean_max_batch
+    // (FF_LEAN_MAX_BATCH, default 1), runs copy-in, forward and copy-out on the compute stream alone: it has nothing to overlap and
+    // is spared the pipeline's two cross-stream hops.  Other submits go through the three-stream pipeline, where the next step's
+    // copy-in overlaps this one's kernels.  FF_LEAN_MAX_BATCH=0: the pipeline for all.
+    int lean_max_batch = 1;
+    bool lean_last = false;      // the previous submit took the compute stream alone
     CosWorkspace cos;            // similarity matrices (cos_sim.cu): has its own stream, is made by the first one
 };
 
