@@ -214,7 +214,6 @@ template <bool CONTRACT, int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
 {
-    tc_pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int CLUSTER = CHAIN_CLUSTER_OF(BN);
@@ -400,6 +399,11 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             // All epilogue warps are past the previous layer (its table reads included).  The two barriers
             // are executed by every warp in every iteration, whatever its ok flag: none may be left waiting.
             chain_bar_sync_epi();
+            // The next kernel may come up now, a layer ahead, and not from the start: its CTAs wait on the SMs this launch leaves
+            // free, and those of the kernels behind it too, so that for the 150 us of a chain no other context's kernel found an
+            // SM.  Four threads with a context each, 1 / 4 / 8 faces a call: 4.5 / 16.9 / 29.4 -> 10.7 / 32.2 / 41.2 thousand faces/s; one
+            // thread 3.01 / 11.60 / 20.97 -> 3.03 / 11.53 / 20.98.
+            if (L == p.n_layers - 1 && warp == 2) tc_pdl_trigger();
             const ChainLayer* cl = p.layers + L;
             const int8_t* lutp = cl->lut;
             int8_t* out2 = cl->out2;

@@ -602,7 +602,7 @@ __device__ __forceinline__ void tc_fc16(const TcParams& p, const float* tab, con
 
 // Programmatic dependent launch.  Each tensor-core kernel is launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization.  tc_pdl_trigger, the kernel's first
-// statement, lets the NEXT kernel of the stream become resident at once (on SMs this one leaves
+// statement (a layer chain's at its last layer), lets the NEXT kernel of the stream become resident at once (on SMs this one leaves
 // free: always the case at small batch, where a launch is 8-16 CTAs), so that its launch latency
 // and set-up (barriers, TMEM, the per-channel tables, which no kernel writes) are hidden several
 // kernels deep.  tc_pdl_wait blocks until the PREVIOUS kernel has completed and its stores are

@@ -1,6 +1,8 @@
 """Layer-chain launches (runs of same-shape convolutions in one launch) beyond a single face: same bytes as one
 launch per layer, and as the oracle."""
 import ctypes as C
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -55,3 +57,38 @@ def test_bounded_waits_run_out_with_several_clusters(built_lib, model_root, ffw4
         for _ in range(4):
             assert np.array_equal(e.embed_batch(faces), want)
         assert e.launches_per_forward < 30
+
+
+def test_contexts_share_the_device(built_lib, model_root, ffw4):
+    """A chain keeps eight SMs per face for 150 us; the kernels queued behind it must not keep the others waiting with them.
+    Four threads with a context each get 3.5 times one thread's single-face rate on an idle box, and got 1.5 times with a
+    successor launched at the chain's start."""
+    face = synth.faces(1, seed=8)[0]
+    engines = [ff.FastFace(ffw4, cwd=model_root, max_batch=1) for _ in range(4)]
+    want = [e.embed(face) for e in engines for _ in range(4)][0]
+
+    def rate(k):
+        counts, start = [0] * k, threading.Barrier(k + 1)
+
+        def work(i):
+            start.wait()
+            while time.perf_counter() < until:
+                got = engines[i].embed(face)
+                counts[i] += 1
+            assert np.array_equal(got, want)
+
+        ts = [threading.Thread(target=work, args=(i,)) for i in range(k)]
+        until = time.perf_counter() + 0.3
+        [t.start() for t in ts]
+        start.wait()
+        [t.join() for t in ts]
+        return sum(counts)
+
+    ratios = []
+    for _ in range(5):                                     # the best of five: other work on the host only slows it down
+        one = rate(1)
+        ratios.append(rate(4) / one)
+        if ratios[-1] >= 2.2:
+            break
+    [e.close() for e in engines]
+    assert max(ratios) >= 2.2, ratios
