@@ -6,8 +6,9 @@
 // float32 x float32 product is exact in float64 (48 bits), so one fused multiply-add per step rounds exactly where
 // "dot += x * y" does: the kernel reproduces the host function bit for bit.
 //
-// Bound: a pair's sum is a chain of 512 dependent float64 FMAs, about 10 us however small the matrix, and from a few
-// hundred blocks on the float64 rate.  Everything else is arranged around that chain: the operands of the next CS_KC
+// Bound: latency.  A pair's sum is a chain of 512 dependent float64 FMAs, with its shared-memory reads about 10 us however
+// small the matrix; with many blocks the shared-memory data path is two thirds busy and the float64 pipe 44 % (64 x 64 outputs a
+// block, 1024 x 1000).  Everything else is arranged around that chain: the operands of the next CS_KC
 // dimensions are fetched into registers while the current ones are used, converted to float64 once per block and stored into the
 // other of two shared buffers (one barrier per chunk), and the norms have warps of their own, one row a thread, so that
 // their chains run beside the pairs'.  Rows lie KC + 2 doubles apart: 16-byte reads of two dimensions at eight
