@@ -750,6 +750,7 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
         deliver(c, slot);
     }
     c->d_in = c->in_slot[slot]; c->d_out = c->out_slot[slot]; c->d_err = (int*)c->out_mem[slot];
+    c->err_read[slot] = false;                        // until copy_out: a submit that fails on the way leaves it to the wait
     if (n <= c->lean_max_batch || (single && c->lean_max_batch > 0 && n < CHUNK_MIN_FACES)) {
         // Latency path (a handful of faces, or a call that is one small step): copy-in, forward and copy-out in order on
         // the compute stream.  The three-stream pipeline below buys overlap such a call has no use for and costs it two
