@@ -87,8 +87,8 @@ struct ffcu_ctx {
     cudaEvent_t ev_stage[STAGE_SLOTS] = {};
     unsigned long long stage_seq = 0;
     char* stage_out[2] = {};     // [OUT_HEAD: error word | embeddings of min(max_batch, STAGE_OUT_FACES) faces]
-    int* h_err = nullptr;        // page-locked, [2]: the slots' error words where their outputs are not staged
-    int* err_at[2] = {};         // where the slot's error word arrives: h_err or the front of stage_out
+    int* h_err = nullptr;        // page-locked, [2]: the error words of slots that have no staging
+    int* err_at[2] = {};         // where the slot's error word arrives: the front of stage_out, or h_err
     bool err_read[2] = {true, true};                 // it is there or on its way
     struct Pending { float* dst; size_t bytes; } pending[2] = {};   // output that waits in stage_out for its caller's memory
     bool idle = true;            // nothing submitted since the last wait
@@ -162,7 +162,7 @@ static void make_staging(ffcu_ctx* c)
     const size_t out_bytes = OUT_HEAD + (size_t)std::min(c->max_batch, STAGE_OUT_FACES) * 512 * sizeof(float);
     c->stage_slot_bytes = (size_t)std::min(c->max_batch, STAGE_FACES) * 37632 * sizeof(float);
     c->stage_in = stage_alloc(STAGE_SLOTS * c->stage_slot_bytes);
-    for (int k = 0; k < 2; k++) c->stage_out[k] = stage_alloc(out_bytes);
+    for (int k = 0; k < 2; k++) c->err_at[k] = (int*)(c->stage_out[k] = stage_alloc(out_bytes));
     c->pool = ff_copy_pool_create(3);                 // NULL: the caller's thread copies alone
 }
 
@@ -201,9 +201,10 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
         ok = ok && cudaMalloc(&c->d_fc_tc_scratch, nb) == cudaSuccess;
         if (ok) cudaMemset(c->d_fc_tc_scratch, 0, nb);
     }
-    ok = ok && cudaHostAlloc(&c->h_err, 2 * sizeof(int), cudaHostAllocDefault) == cudaSuccess;
-    for (int k = 0; k < 2 && ok; k++) { c->h_err[k] = 0; c->err_at[k] = &c->h_err[k]; }
     if (ok) make_staging(c);
+    if (ok && !(c->stage_out[0] && c->stage_out[1])) ok = cudaHostAlloc(&c->h_err, 2 * sizeof(int), cudaHostAllocDefault) == cudaSuccess;
+    for (int k = 0; k < 2 && ok; k++)
+        if (!c->err_at[k]) { c->h_err[k] = 0; c->err_at[k] = &c->h_err[k]; }
     for (int k = 0; k < STAGE_SLOTS && ok; k++) ok = cudaEventCreateWithFlags(&c->ev_stage[k], cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess;
     const char* impl = getenv("FF_CONV_IMPL");
@@ -714,11 +715,9 @@ static int copy_out(ffcu_ctx* c, int slot, int n, float* host_out, cudaStream_t 
     if (n <= STAGE_OUT_FACES && c->stage_out[slot] && is_pageable(host_out, nb)) {
         FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], OUT_HEAD + nb, cudaMemcpyDeviceToHost, s));
         c->pending[slot] = {host_out, nb};
-        c->err_at[slot] = (int*)c->stage_out[slot];
     } else {
         FFCU_CHECK(cudaMemcpyAsync(host_out, c->out_slot[slot], nb, cudaMemcpyDeviceToHost, s));
-        FFCU_CHECK(cudaMemcpyAsync(&c->h_err[slot], c->out_mem[slot], sizeof(int), cudaMemcpyDeviceToHost, s));
-        c->err_at[slot] = &c->h_err[slot];
+        FFCU_CHECK(cudaMemcpyAsync(c->err_at[slot], c->out_mem[slot], sizeof(int), cudaMemcpyDeviceToHost, s));
     }
     c->err_read[slot] = true;
     return 0;
@@ -845,10 +844,7 @@ static int wait_impl(ffcu_ctx* c)
 {
     FFCU_CHECK(cudaSetDevice(c->device));
     for (int k = 0; k < 2; k++)
-        if (!c->err_read[k]) {
-            FFCU_CHECK(cudaMemcpyAsync(&c->h_err[k], c->out_mem[k], sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            c->err_at[k] = &c->h_err[k];
-        }
+        if (!c->err_read[k]) FFCU_CHECK(cudaMemcpyAsync(c->err_at[k], c->out_mem[k], sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_in));
     FFCU_CHECK(cudaStreamSynchronize(c->stream));
     if (!c->lean_last) FFCU_CHECK(cudaStreamSynchronize(c->s_out));
