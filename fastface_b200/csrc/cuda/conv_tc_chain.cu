@@ -50,16 +50,15 @@ __device__ __forceinline__ void chain_bar_sync_epi()
     asm volatile("bar.sync 1, %0;" ::"n"(CHAIN_EPI_THREADS) : "memory");
 }
 
-// Two MMA issuers (warps 1 and 18; each warp loops and waits together, lane 0 issues).  One thread issues an
-// N = 64 MMA about every 70 cycles and pays a few hundred more per pipeline stage, which is slower than the
-// tensor core retires them (51 cycles): the issuers take alternate stages of the weight ring, each
+// Two MMA issuers.  One thread that also waits for a pipeline stage every few MMAs issues them more slowly than the
+// tensor core retires N = 64 ones (48 cycles): the issuers take alternate stages of the weight ring, each
 // accumulating into its own 64 TMEM columns; the epilogue adds the two (integer adds commute).  The ring is
 // even, so a slot is always the same issuer's (a parity wait cannot tell "this fill" from "two fills ago",
 // and with an odd ring the fill in between would be the other issuer's to consume).  PLANES (C / 128) and
 // TPS (filter taps per stage) are compile-time so that a stage's MMAs are one straight-line block, and the
 // ring / layer bookkeeping is carried forward by additions only.
 template <int PLANES, int TPS>
-__device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainShared* sh, int me, int lane, uint32_t rank,
+__device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainShared* sh, int me, uint32_t rank,
                                                   uint32_t tmem_base, uint32_t s_a_addr, uint32_t s_b_addr,
                                                   int tile_line0, uint32_t in_bytes)
 {
@@ -71,7 +70,6 @@ __device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainSha
     volatile int* abort_flag = &sh->abort_flag;
     const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
     const int stages = p.stages, n_layers = p.n_layers;
-    const uint32_t leader = (lane == 0) ? 1u : 0u;
     const uint32_t d_tmem = tmem_base + (uint32_t)(me * CHAIN_BN);
     const uint64_t db_base = smem_desc<128>(s_b_addr);
     const uint32_t a_buf_bytes = (uint32_t)(PLANES * p.plane_bytes);
@@ -91,7 +89,7 @@ __device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainSha
             const int buf = L & 1;
             // arm the barrier of the buffer the peers fill during this layer (bytes that land before this
             // only drive the count negative for a moment: the phase cannot complete before this arrival)
-            if (me == 0 && L + 1 < n_layers && lane == 0) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
+            if (me == 0 && L + 1 < n_layers) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
             if (L == 0) ok = mbar_wait(smem_u32(&sh->a0_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
             else {
                 ok = mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) >> 1) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
@@ -101,7 +99,7 @@ __device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainSha
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_after();
 #ifdef FF_TC_TIMING
-            if (p.ts && rank == 0 && lane == 0 && me == 0) p.ts[4 * L + 0] = globaltimer_ns();      // input complete
+            if (p.ts && rank == 0 && me == 0) p.ts[4 * L + 0] = globaltimer_ns();      // input complete
 #endif
             da_layer = smem_desc<128>(s_a_addr + (uint32_t)buf * a_buf_bytes + (uint32_t)(tile_line0 * 128));
             first = 0;
@@ -127,18 +125,18 @@ __device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainSha
                 for (int pl = 0; pl < PLANES; pl++)
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        umma_i8_w(leader, d_tmem, da0 + (uint64_t)(g * 8 + 2 * k) + (uint64_t)pl * dplane,
+                        umma_i8(d_tmem, da0 + (uint64_t)(g * 8 + 2 * k) + (uint64_t)pl * dplane,
                                   db0 + (uint64_t)(((g * PLANES + pl) * B_BLOCK >> 4) + 2 * k), IDESC,
                                   (g | pl | k) ? 1u : first);
             first = 1;
         }
-        umma_commit_w(leader, empty0 + stage * 8);
+        umma_commit(empty0 + stage * 8);
         stage = ns; phase = np;
         st += 2;
         if (st >= S) {                                      // that was this issuer's last stage of the layer
-            umma_commit_w(leader, smem_u32(&sh->acc_full));
+            umma_commit(smem_u32(&sh->acc_full));
 #ifdef FF_TC_TIMING
-            if (p.ts && rank == 0 && lane == 0 && st - 2 == S - 1) p.ts[4 * L + 1] = globaltimer_ns();   // last MMA issued
+            if (p.ts && rank == 0 && st - 2 == S - 1) p.ts[4 * L + 1] = globaltimer_ns();   // last MMA issued
 #endif
             st -= S; L++; new_layer = true;
         }
@@ -149,7 +147,7 @@ __device__ __forceinline__ void chain_issuer_role(const ChainParams& p, ChainSha
 // 16 KB, slot 2 * d + i holding plane 2 * pp + i of the pair, and issuer i takes its slot of every step.  Four
 // N = 128 MMAs per slot (64 cycles each at the tensor rate), so the two issuers have 512 cycles per step.
 template <int PLANES>
-__device__ __forceinline__ void chain_issuer_wide(const ChainParams& p, ChainShared* sh, int me, int lane, uint32_t tmem_base,
+__device__ __forceinline__ void chain_issuer_wide(const ChainParams& p, ChainShared* sh, int me, uint32_t tmem_base,
                                                   uint32_t s_a_addr, uint32_t s_b_addr, int tile_line0, uint32_t in_bytes)
 {
     constexpr int BN = 128;
@@ -159,7 +157,6 @@ __device__ __forceinline__ void chain_issuer_wide(const ChainParams& p, ChainSha
     volatile int* abort_flag = &sh->abort_flag;
     const uint32_t full0 = smem_u32(&sh->full[me]), empty0 = smem_u32(&sh->empty[me]);
     const int steps_in_ring = p.stages >> 1;
-    const uint32_t leader = (lane == 0) ? 1u : 0u;
     const uint32_t d_tmem = tmem_base + (uint32_t)(me * BN);
     const uint64_t db_base = smem_desc<128>(s_b_addr + (uint32_t)(me * SLOT));
     const uint64_t dplane = (uint64_t)(p.plane_bytes >> 4);
@@ -171,7 +168,7 @@ __device__ __forceinline__ void chain_issuer_wide(const ChainParams& p, ChainSha
 #pragma unroll 1
     for (int L = 0; L < p.n_layers && ok; L++) {
         const int buf = L & 1;
-        if (me == 0 && L + 1 < p.n_layers && lane == 0) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
+        if (me == 0 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
         if (L == 0) ok = mbar_wait(smem_u32(&sh->a0_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
         else {
             ok = mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) >> 1) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
@@ -199,13 +196,13 @@ __device__ __forceinline__ void chain_issuer_wide(const ChainParams& p, ChainSha
                 const uint64_t db0 = db_base + (uint64_t)((uint32_t)(d * 2 * SLOT) >> 4);
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    umma_i8_w(leader, d_tmem, da0 + (uint64_t)(2 * k), db0 + (uint64_t)(2 * k), IDESC, k ? 1u : first);
+                    umma_i8(d_tmem, da0 + (uint64_t)(2 * k), db0 + (uint64_t)(2 * k), IDESC, k ? 1u : first);
                 first = 1;
-                umma_commit_w(leader, empty0 + d * 16);
+                umma_commit(empty0 + d * 16);
                 d = nd; phase = np;
             }
         }
-        if (ok) umma_commit_w(leader, smem_u32(&sh->acc_full));
+        if (ok) umma_commit(smem_u32(&sh->acc_full));
     }
 }
 
@@ -254,7 +251,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -267,7 +264,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
     volatile int* abort_flag = &sh->abort_flag;
     const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
 
-    if (warp == 0 && WIDE) {
+    if (warp == TC_PRODUCER_WARP && WIDE) {
         // Weight producer of the wide form: a step is one plane pair of one tap, two slots (lane i: plane 2 * pp + i).
         const int pp_n = p.planes >> 1;
         const int steps_in_ring = p.stages >> 1;
@@ -301,7 +298,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             if (++d == steps_in_ring) { d = 0; phase ^= 1; }
             if (++pp == pp_n) { pp = 0; if (++tap == 9) { tap = 0; L++; } }
         }
-    } else if (warp == 0) {
+    } else if (warp == TC_PRODUCER_WARP) {
         // Weight producer.  One stage = p.tps filter taps of this CTA's 64 output channels (planes boxes of
         // 8 KB each); the ring runs ahead across layers.  The first layer's activations are requested once the
         // ring is full of weights: they are the only thing that depends on the previous kernel.
@@ -357,24 +354,25 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             tap += G;
             if (tap == 9) { tap = 0; L++; }
         }
-    } else if (warp == 1 || warp == TC_ISSUER2_WARP) {
-        const int me = (warp == 1) ? 0 : 1;
+    } else if (warp == TC_ISSUER_WARP || warp == TC_ISSUER2_WARP) {
+        const int me = (warp == TC_ISSUER_WARP) ? 0 : 1;
         const int tile_line0 = tile_m * TC_TILE_M - base_line(tile_m);
         const int my_lo = rows_lo(tile_m) < 0 ? 0 : rows_lo(tile_m);
         const int my_hi = rows_hi(tile_m) > p.H - 1 ? p.H - 1 : rows_hi(tile_m);
         const uint32_t in_bytes = (uint32_t)((my_hi - my_lo + 1) * p.W * p.C);
-        if (WIDE) {
-            if (p.planes == 2) chain_issuer_wide<2>(p, sh, me, lane, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
-            else               chain_issuer_wide<4>(p, sh, me, lane, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
-        } else if (p.planes == 2 && p.tps == 3) chain_issuer_role<2, 3>(p, sh, me, lane, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
-        else if (p.planes == 2)               chain_issuer_role<2, 1>(p, sh, me, lane, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
-        else                                  chain_issuer_role<4, 1>(p, sh, me, lane, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
+        if (!tc_elect_one()) {
+        } else if (WIDE) {
+            if (p.planes == 2) chain_issuer_wide<2>(p, sh, me, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
+            else               chain_issuer_wide<4>(p, sh, me, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
+        } else if (p.planes == 2 && p.tps == 3) chain_issuer_role<2, 3>(p, sh, me, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
+        else if (p.planes == 2)               chain_issuer_role<2, 1>(p, sh, me, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
+        else                                  chain_issuer_role<4, 1>(p, sh, me, rank, tmem_base, smem_u32(s_a), smem_u32(s_b), tile_line0, in_bytes);
     } else {
         // Epilogue: sixteen warps on the CTA's one tile, warp = (TMEM lane quarter, group of BN / 4 channels), walked in
         // chunks of sixteen.
         constexpr int CHUNKS = BN / 64;
         const int q = warp & 3;
-        const int cg = (warp - 2) >> 2;
+        const int cg = warp >> 2;
         const int qpos = tile_m * TC_TILE_M + q * 32 + lane;      // position r * P + c of this thread's output
         const int r = qpos / p.P, c = qpos - r * p.P;
         const bool valid = (c < p.W) && (r < p.H);
@@ -390,7 +388,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             const int t = rk / p.tiles_n;
             if (valid && r >= rows_lo(t) && r <= rows_hi(t)) dest_mask |= 1u << rk;
         }
-        const int et = threadIdx.x - 64;                           // 0 .. 511 among the epilogue threads
+        const int et = threadIdx.x;                           // 0 .. 511 among the epilogue threads
         int lut_layer = -1;                                        // layer whose table s_lut holds
         bool ok = true;
         tc_pdl_wait();
@@ -403,7 +401,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             // free, and those of the kernels behind it too, so that for the 150 us of a chain no other context's kernel found an
             // SM.  Four threads with a context each, 1 / 4 / 8 faces a call: 4.5 / 16.9 / 29.4 -> 10.7 / 32.2 / 41.2 thousand faces/s; one
             // thread 3.01 / 11.60 / 20.97 -> 3.03 / 11.53 / 20.98.
-            if (L == p.n_layers - 1 && warp == 2) tc_pdl_trigger();
+            if (L == p.n_layers - 1 && warp == 0) tc_pdl_trigger();
             const ChainLayer* cl = p.layers + L;
             const int8_t* lutp = cl->lut;
             int8_t* out2 = cl->out2;
@@ -452,7 +450,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             if (!ok) continue;
             tc_fence_after();
 #ifdef FF_TC_TIMING
-            if (p.ts && rank == 0 && warp == 2 && lane == 0) p.ts[4 * L + 2] = globaltimer_ns();   // accumulator complete
+            if (p.ts && rank == 0 && warp == 0 && lane == 0) p.ts[4 * L + 2] = globaltimer_ns();   // accumulator complete
 #endif
             int owa[CHUNKS][4], ow2a[CHUNKS][4];
 #pragma unroll
@@ -512,7 +510,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
             __syncwarp();
             if (lane == 0) mbar_arrive_relaxed(smem_u32(&sh->acc_empty));
 #ifdef FF_TC_TIMING
-            if (p.ts && rank == 0 && warp == 2 && lane == 0) p.ts[4 * L + 3] = globaltimer_ns();   // results sent
+            if (p.ts && rank == 0 && warp == 0 && lane == 0) p.ts[4 * L + 3] = globaltimer_ns();   // results sent
 #endif
             if (valid) {
 #pragma unroll
@@ -532,7 +530,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
     }
     __syncthreads();
     cluster_sync_all();
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }

@@ -16,10 +16,9 @@
 // * tcgen05.mma kind::i8, M=128 per CTA (cta_group::1) or M=256 per CTA pair
 //   (cta_group::2), N=BN, K=32 per instruction; a ring of 512/BN accumulators in
 //   TMEM so the epilogue of one tile overlaps the MMAs of the next ones.
-// * Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer (+TMEM alloc),
-//   warps 2..17 = epilogue, two sets of eight (tcgen05.ld -> exact fp32 chain ->
-//   int8 NHWC stores), warp 18 = second MMA issuer in the kernels whose tiles are
-//   a handful of MMAs (weight-stationary and stem kernels).
+// * Warp roles: warps 0..15 = epilogue (tcgen05.ld -> exact fp32 chain -> int8 NHWC stores),
+//   warp 16 = TMA producer, warp 17 = second MMA issuer in the kernels whose tiles are
+//   a handful of MMAs (second producer in the stem), warp 18 = MMA issuer (+TMEM alloc).
 // * Every wait is bounded; on expiry the kernel records an error word, drains
 //   and frees its TMEM, and returns.  The CTA-pair kernel is a cluster of two;
 //   no TMA load is multicast.
@@ -145,19 +144,12 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// Warp-uniform issue: every lane executes the surrounding code (so the descriptor arithmetic is
-// uniform across the warp and needs no per-lane-to-uniform register moves), `leader` is
-// non-zero in the one lane whose instruction takes effect.
-__device__ __forceinline__ void umma_i8_w(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+// True in one lane of a converged warp, always the same one.
+__device__ __forceinline__ bool tc_elect_one()
 {
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-}
-__device__ __forceinline__ void umma_commit_w(uint32_t leader, uint32_t bar)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(leader) : "memory");
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r) :: "memory");
+    return r != 0;
 }
 // arrives on the mbarrier once every MMA issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint32_t bar)
@@ -220,18 +212,6 @@ __device__ __forceinline__ void umma2_i8(uint32_t d_tmem, uint64_t a_desc, uint6
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma2_i8_w(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-}
-__device__ __forceinline__ void umma2_commit_both_w(uint32_t leader, uint32_t bar)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-                 ::"r"(bar), "h"((uint16_t)3), "r"(leader) : "memory");
 }
 // arrives, once the pair's MMAs issued so far are complete, on the mbarrier at this offset in BOTH CTAs
 __device__ __forceinline__ void umma2_commit_both(uint32_t bar)
@@ -378,9 +358,16 @@ enum { EPI_RUNTIME = 0, EPI_PLAIN = 1, EPI_SLOPE = 2, EPI_RES_BN = 3, EPI_RES = 
 // epilogue warps and back, so the issuer must be able to run several tiles ahead.
 #define TC_MAX_ACC 8
 #define TC_NACC(BN) (512 / (BN) > TC_MAX_ACC ? TC_MAX_ACC : 512 / (BN))
-// Warp 0: TMA producer, warp 1: MMA issuer, warps 2 .. 17: epilogue, warp 18: second MMA issuer
-// (weight-stationary and stem kernels, idle elsewhere).
-#define TC_ISSUER2_WARP 18
+// Warps 0 .. 15: epilogue, 16: TMA producer, 17: second MMA issuer (weight-stationary kernels, chains; the stem's second
+// producer; idle elsewhere), 18: MMA issuer.  The issuer shares its scheduler with four epilogue warps, and the scheduler
+// prefers the highest-numbered warp that is ready: with sixteen warps of independent FMAs beside it, one M = 256, N = 224
+// MMA was issued every 365 cycles by warp 1 and every 158 by warp 18 (110 alone, the tensor rate).  An issuer's loop
+// runs in one elected lane: predicated on the lane in a converged warp, an MMA took several times the instructions
+// (1 730 cycles in the same place).  Both together: forward of 1 / 8 / 64 / 100 / 256 / 1024 faces 292.9 / 321.2 / 756.7 / 1032 /
+// 2010 / 7250 -> 274.5 / 308.6 / 739 / 994 / 1943 / 7000 us.
+#define TC_PRODUCER_WARP 16
+#define TC_ISSUER2_WARP 17
+#define TC_ISSUER_WARP 18
 #define TC_THREADS (32 * 19)
 
 struct TcShared {                 // lives after the stage ring and the tables
@@ -428,7 +415,7 @@ __device__ __forceinline__ void tc_load_tables(float* tab, const TcParams& p, in
 __device__ __forceinline__ bool tc_epi_prologue(float* tab, uint8_t* lut, const TcParams& p, TcShared* sh, int c0, int bn,
                                                 volatile int* abort_flag)
 {
-    const int tid = (int)threadIdx.x - 64;                // epilogue warps are 2 .. 17
+    const int tid = (int)threadIdx.x;                     // epilogue warps are 0 .. 15
     const bool has_lut = p.out2 && p.lut_bytes;
     if (tid == 0 && has_lut) {
         mbar_expect_tx(smem_u32(&sh->lut_full), (uint32_t)bn * 256u);
@@ -669,7 +656,7 @@ __device__ __forceinline__ void walk_next(TileWalk& w, const TcParams& p)
     w.tb += w.db + c;
 }
 
-// Epilogue warps: sixteen (warps 2..17), organised as 16 / wps sets of wps warps (TcParams::epi_wps,
+// Epilogue warps: sixteen (warps 0..15), organised as 16 / wps sets of wps warps (TcParams::epi_wps,
 // 4, 8 or 16).  Set s takes the CTA's tiles s, s + sets, ...; within a set, warp e covers the TMEM lane
 // quarter its index gives it (hardware: warp w reads lanes [32*(w%4), +32)) and column group e / 4 of
 // wps / 4.  With four warps per set each warp walks all columns of its 32 rows, so the per-tile
@@ -692,15 +679,15 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
                                                  uint32_t remote_acc_empty /* 0: local barrier */, const TcConstArg<CT, BN>& ct = {})
 {
     static_assert(!CT || (BN <= 128 && (EPI == EPI_RES_BN || EPI == EPI_SLOPE_BN)), "constants as parameters: launches with a fused BN");
-    if (warp >= TC_ISSUER2_WARP) return;                  // not an epilogue warp
+    if (warp >= TC_EPI_TOTAL_WARPS) return;
     const int wps = CT ? BN / 16 : p.epi_wps;
     const int sets = TC_EPI_TOTAL_WARPS / wps;
     const int cols = BN / (wps >> 2);                     // columns this warp covers
     constexpr int PAIR_UNROLL = CT ? 2 : 1;
     const int n_pairs = cols >> 5;                        // pairs of 16-column chunks
     const int q = warp & 3;
-    const int set = (warp - 2) / wps;                     // which of the CTA's tiles this warp takes
-    const int cg = ((warp - 2) % wps) >> 2;               // column group of this warp
+    const int set = warp / wps;                           // which of the CTA's tiles this warp takes
+    const int cg = (warp % wps) >> 2;                     // column group of this warp
     const int row = q * 32 + lane;
     const int iw = row % p.TW;
     const int ih = (row / p.TW) % p.TH;
@@ -828,7 +815,7 @@ __device__ __forceinline__ void tc_setup(TcShared* sh, int stages, uint32_t tmem
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -849,7 +836,7 @@ __device__ __forceinline__ void tc_teardown(volatile int* abort_flag, uint32_t t
         for (int i = 0; i < 1000; i++) __nanosleep(1000);
     }
     __syncthreads();
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }

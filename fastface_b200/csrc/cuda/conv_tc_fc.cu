@@ -45,7 +45,7 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
     const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
     const int stage_bytes = G * FCT_SUB_BYTES;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         // TMA producer: lane 2g fetches the activation box of the stage's K block g, lane 2g + 1 its weight box.
         // The weights do not depend on the previous kernel: the weight boxes of the first ring-full of steps are
         // requested before the programmatic-dependency wait.
@@ -81,13 +81,12 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
             }
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-    } else if (warp == 1) {
-        // MMA issuer: the warp loops and waits together, lane 0 issues
+    } else if (warp == TC_ISSUER_WARP) {
+        if (tc_elect_one()) {
         int stage = 0; uint32_t phase = 0;
         bool ok = true;
         const uint64_t da0 = smem_desc<FCT_KC>(smem_u32(smem));
         const uint64_t db0 = smem_desc<FCT_KC>(smem_u32(smem) + FCT_A_BYTES);
-        const uint32_t leader = (lane == 0) ? 1u : 0u;
 #pragma unroll 1
         for (int it = 0; it < n_steps; it++) {
             ok = mbar_wait(full0 + stage * 8, phase, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
@@ -98,13 +97,14 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
             for (int g = 0; g < G; g++, soff += (uint32_t)(FCT_SUB_BYTES >> 4)) {
 #pragma unroll
                 for (int k = 0; k < FCT_KC / 32; k++)
-                    umma_i8_w(leader, tmem_base, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
+                    umma_i8(tmem_base, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
             }
-            umma_commit_w(leader, empty0 + stage * 8);
+            umma_commit(empty0 + stage * 8);
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_w(leader, smem_u32(&sh->acc_full[0]));
-    } else if (warp < 6) {
+        if (ok) umma_commit(smem_u32(&sh->acc_full[0]));
+        }
+    } else if (warp < 4) {
         // Epilogue: four warps, one TMEM lane quarter (32 faces) each, all 64 columns.  A TMEM load gives a lane one
         // face's columns; global memory wants a warp on consecutive columns of ONE face (a face's row of sums is 2 KB
         // from the next: 32 lanes on 32 faces would be 32 sectors per instruction).  So the warp turns its 32 x 64
@@ -115,7 +115,7 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
         const int b0 = tm * TC_TILE_M + q * 32;              // first face of this warp's quarter
         const int rows = p.batch - b0 < 32 ? p.batch - b0 : 32;      // faces of the quarter that exist (may be <= 0)
         const int n0 = tn * FCT_BN;
-        int* stg = (int*)smem + (warp - 2) * (32 * 65);
+        int* stg = (int*)smem + warp * (32 * 65);
         const float ws0 = __ldg(p.w_scale + n0 + lane), ws1 = __ldg(p.w_scale + n0 + 32 + lane);
         const float bi0 = __ldg(p.bias + n0 + lane), bi1 = __ldg(p.bias + n0 + 32 + lane);
         bool ok = mbar_wait(smem_u32(&sh->acc_full[0]), 0, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
@@ -149,7 +149,7 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
             // every epilogue thread's additions are out (or the CTA has given up) before the ticket is taken
             __threadfence();
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (warp == 2 && lane == 0)
+            if (warp == 0 && lane == 0)
                 s_last = (!*abort_flag && atomicAdd(p.tickets + tm * p.tiles_n + tn, 1) == p.splits - 1) ? 1 : 0;
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (s_last) {
@@ -173,7 +173,7 @@ fc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
                         p.out[o + 32] = ffcu_fc_fp<CONTRACT>(d1[k], ws1, bi1);
                     }
                 }
-                if (warp == 2 && lane == 0) p.tickets[tm * p.tiles_n + tn] = 0;
+                if (warp == 0 && lane == 0) p.tickets[tm * p.tiles_n + tn] = 0;
             }
         }
     }

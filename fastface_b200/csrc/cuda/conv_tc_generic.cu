@@ -32,7 +32,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         const int G = p.group;
         {
             // TMA producer.  The whole warp runs the loop (lanes stay converged; a lone lane
@@ -109,11 +109,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 pre = 0;
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == TC_ISSUER_WARP) {
         const int G = p.group;
         const int n_steps = kblocks / G;
-        {
-            // MMA issuer: the warp loops and waits together, lane 0 issues
+        if (tc_elect_one()) {
             int stage = 0; uint32_t phase = 0;
             int local = 0;
             bool ok = true;
@@ -121,7 +120,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
             const uint64_t da0 = smem_desc<KC>(smem_u32(smem));
             const uint64_t db0 = smem_desc<KC>(smem_u32(smem) + A_BYTES);
-            const uint32_t leader = (lane == 0) ? 1u : 0u;
             uint32_t ready = 0;                          // answer of the early test for the upcoming stage
             for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x, local++) {
                 const int a = local % TC_NACC(BN);
@@ -148,13 +146,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         for (int g = 0; g < G; g++, soff += (uint32_t)(SUB_BYTES >> 4)) {
 #pragma unroll
                             for (int k = 0; k < KC / 32; k++)
-                                umma_i8_w(leader, d_tmem, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
+                                umma_i8(d_tmem, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
                         }
-                        umma_commit_w(leader, empty0 + stage * 8);   // frees the stage once these MMAs have read it
+                        umma_commit(empty0 + stage * 8);   // frees the stage once these MMAs have read it
                     }
                     stage = ns; phase = np;
                 }
-                if (ok) umma_commit_w(leader, smem_u32(&sh->acc_full[a]));
+                if (ok) umma_commit(smem_u32(&sh->acc_full[a]));
             }
         }
     } else {

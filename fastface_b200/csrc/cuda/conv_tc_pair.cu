@@ -52,7 +52,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -64,7 +64,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         const int G = p.group;
         {
             // TMA producer.  The whole warp runs the loop (lanes stay converged); lanes
@@ -135,11 +135,10 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 pre = 0;
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == TC_ISSUER_WARP) {
         const int G = p.group;
         const int n_steps = kblocks / G;
-        if (rank == 0) {
-            // MMA issuer (leader CTA): the warp loops and waits together, lane 0 issues
+        if (rank == 0 && tc_elect_one()) {                // the leader CTA's issuer
             int stage = 0; uint32_t phase = 0;
             int local = 0;
             bool ok = true;
@@ -147,7 +146,6 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
             const uint64_t da0 = smem_desc<KC>(smem_u32(smem));
             const uint64_t db0 = smem_desc<KC>(smem_u32(smem) + A_BYTES);
-            const uint32_t leader = (lane == 0) ? 1u : 0u;
             uint32_t ready = 0;                          // answer of the early test for the upcoming stage
             for (int tile = pair_id; tile < total && ok; tile += n_pairs, local++) {
                 const int a = local % TC_NACC(BN);
@@ -174,13 +172,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                         for (int g = 0; g < G; g++, soff += (uint32_t)(SUB_BYTES >> 4)) {
 #pragma unroll
                             for (int k = 0; k < KC / 32; k++)
-                                umma2_i8_w(leader, d_tmem, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
+                                umma2_i8(d_tmem, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC, (it | g | k) ? 1u : 0u);
                         }
-                        umma2_commit_both_w(leader, empty0 + stage * 8);   // frees the stage once these MMAs have read it
+                        umma2_commit_both(empty0 + stage * 8);   // frees the stage once these MMAs have read it
                     }
                     stage = ns; phase = np;
                 }
-                if (ok) umma2_commit_both_w(leader, smem_u32(&sh->acc_full[a]));
+                if (ok) umma2_commit_both(smem_u32(&sh->acc_full[a]));
             }
         }
     } else {
@@ -198,7 +196,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     }
     __syncthreads();
     cluster_sync_all();
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }

@@ -63,7 +63,7 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
     const int stage_bytes = G * SUB_BYTES;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         // TMA producer: per tile the main path's K loop (lane 2g: activation box of block g, lane 2g+1: its weight
         // box, G blocks per stage), then ONE stage with the shortcut's kb_sc blocks from its own tensor maps.
         int stage = 0; uint32_t phase = 0;
@@ -109,14 +109,13 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (++stage == p.stages) { stage = 0; phase ^= 1; }
             }
         }
-    } else if (warp == 1) {
-        // MMA issuer: the warp loops and waits together, lane 0 issues
+    } else if (warp == TC_ISSUER_WARP) {
+        if (tc_elect_one()) {
         int stage = 0; uint32_t phase = 0;
         int ts = 0; uint32_t tphase = 0;                    // tile slot (two accumulators) and its phase
         bool ok = true;
         const uint64_t da0 = smem_desc<KC>(smem_u32(smem));
         const uint64_t db0 = smem_desc<KC>(smem_u32(smem) + A_BYTES);
-        const uint32_t leader = (lane == 0) ? 1u : 0u;
         uint32_t ready = 0;
         for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
             ok = mbar_wait(smem_u32(&sh->acc_empty[ts]), tphase ^ 1, abort_flag, p.err, FFCU_ERR_TMEM_TIMEOUT);
@@ -141,24 +140,25 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 for (int g = 0; g < nb; g++, soff += (uint32_t)(SUB_BYTES >> 4)) {
 #pragma unroll
                     for (int k = 0; k < KC / 32; k++)
-                        umma_i8_w(leader, d, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC,
+                        umma_i8(d, da0 + (uint64_t)(soff + 2 * k), db0 + (uint64_t)(soff + 2 * k), IDESC,
                                   ((it < n_steps ? it : 0) | g | k) ? 1u : 0u);
                 }
-                umma_commit_w(leader, empty0 + stage * 8);
+                umma_commit(empty0 + stage * 8);
                 stage = ns; phase = np;
             }
-            if (ok) umma_commit_w(leader, smem_u32(&sh->acc_full[ts]));
+            if (ok) umma_commit(smem_u32(&sh->acc_full[ts]));
             if (++ts == SC_SLOTS) { ts = 0; tphase ^= 1; }
         }
-    } else if (warp < TC_ISSUER2_WARP) {
+        }
+    } else if (warp < TC_EPI_TOTAL_WARPS) {
         // Epilogue: 16 / wps sets of wps warps on alternate tiles; a warp = (TMEM lane quarter, column group).
         // First the tables, while the first operands are on their way (as tc_epi_prologue).
-        if (threadIdx.x == 64 && q.lut_bytes) {
+        if (threadIdx.x == 0 && q.lut_bytes) {
             mbar_expect_tx(smem_u32(&sh->lut_full), BN * 256u);
             bulk_load(smem_u32(lut), q.t2.bn_lut + (size_t)tn * BN * 256, BN * 256u, smem_u32(&sh->lut_full));
         }
-        sc_load_tables(tab1, p.t, p.Cout, (int)threadIdx.x - 64);
-        sc_load_tables(tab2, q.t2, p.Cout, (int)threadIdx.x - 64);
+        sc_load_tables(tab1, p.t, p.Cout, (int)threadIdx.x);
+        sc_load_tables(tab2, q.t2, p.Cout, (int)threadIdx.x);
         asm volatile("bar.sync 1, 512;" ::: "memory");
         bool ok = !q.lut_bytes || mbar_wait(smem_u32(&sh->lut_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
         tc_pdl_wait();
@@ -167,8 +167,8 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int cols = BN / (wps >> 2);
         const int n_chunks = cols >> 4;
         const int qd = warp & 3;
-        const int set = (warp - 2) / wps;
-        const int cg = ((warp - 2) % wps) >> 2;
+        const int set = warp / wps;
+        const int cg = (warp % wps) >> 2;
         const int row = qd * 32 + lane;
         const int iw = row % p.TW;
         const int ih = (row / p.TW) % p.TH;

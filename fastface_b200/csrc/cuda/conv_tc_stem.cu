@@ -18,7 +18,7 @@
 //     16-byte halves exchanged when bit 2 of r is set), so the K-major operand descriptor is the usual
 //     one.  A proxy fence makes the stores visible to the tensor core before the stage's barrier is
 //     arrived on;
-//   * warp 1 issues ONE tcgen05.mma (128 x 64 x 32) per tile; sixteen epilogue warps as everywhere.
+//   * the issuer warp issues ONE tcgen05.mma (128 x 64 x 32) per tile; sixteen epilogue warps as everywhere.
 // The two producers take alternate tiles (the stage ring is even), and each has its next tile's
 // patch loads in flight while it packs the current one.
 // Traffic per face: 150 528 B (or 37 632 B) read, 2 x 802 816 B written; nothing in between.
@@ -91,9 +91,9 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
-    if (warp == 0 || warp == TC_ISSUER2_WARP) {
+    if (warp == TC_PRODUCER_WARP || warp == TC_ISSUER2_WARP) {
         // ---- producers: quantise + pack, alternate tiles ----
-        const int me = (warp == 0) ? 0 : 1;
+        const int me = (warp == TC_PRODUCER_WARP) ? 0 : 1;
         if (me == 0 && lane == 0) {                              // the 2 KB weight matrix, once
             mbar_expect_tx(smem_u32(&sh->w_full), W_BYTES);
             tma_load_4d(smem_u32(s_w), &mapB, smem_u32(&sh->w_full), 0, 0, 0, 0);
@@ -163,11 +163,11 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh->full[stage]));
         }
-    } else if (warp == 1) {
+    } else if (warp == TC_ISSUER_WARP) {
+        if (tc_elect_one()) {
         bool ok = mbar_wait(smem_u32(&sh->w_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
         tc_fence_after();
         const uint64_t dw = smem_desc_sw32(smem_u32(s_w));
-        const uint32_t leader = (lane == 0) ? 1u : 0u;
         for (int tile = blockIdx.x, local = 0; tile < p.total_tiles && ok; tile += gridDim.x, local++) {
             const int stage = local % p.stages;
             const uint32_t phase = (uint32_t)(local / p.stages) & 1;
@@ -180,9 +180,10 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
             const uint64_t da = smem_desc_sw32(smem_u32(s_a + (size_t)stage * STEM_A_BYTES));
-            if (!TC_DBG(p, 2)) umma_i8_w(leader, d_tmem, da, dw, IDESC, 0u);
-            umma_commit_w(leader, smem_u32(&sh->empty[stage]));
-            umma_commit_w(leader, smem_u32(&sh->acc_full[a]));
+            if (!TC_DBG(p, 2)) umma_i8(d_tmem, da, dw, IDESC, 0u);
+            umma_commit(smem_u32(&sh->empty[stage]));
+            umma_commit(smem_u32(&sh->acc_full[a]));
+        }
         }
     } else {
         tc_epilogue_role<BN, CONTRACT, false, EPI, (EPI != EPI_RUNTIME), CT>(p, tab, lut, sh, tmem_base, abort_flag, warp, lane,

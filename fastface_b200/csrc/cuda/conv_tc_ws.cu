@@ -43,7 +43,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         {
             // the warp loops and waits together (lanes stay converged); lanes 0..8 fetch one weight tap each, lane 0 the boxes
             const uint32_t wbar = smem_u32(&sh->w_full);
@@ -70,17 +70,16 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (++stage == p.stages) { stage = 0; phase ^= 1; }
             }
         }
-    } else if (warp == 1 || warp == TC_ISSUER2_WARP) {
-        {
+    } else if (warp == TC_ISSUER_WARP || warp == TC_ISSUER2_WARP) {
+        if (tc_elect_one()) {
             // Two MMA issuers take alternate tiles: a tile is 18 short MMAs (128 x BN x 32), and one
             // thread cannot issue them as fast as the tensor pipe retires them.  Each issuer derives
             // its ring positions from the tile's index, so the two never touch the same stage or
-            // accumulator.  The warp loops and waits together, lane 0 issues.
-            const int me = (warp == 1) ? 0 : 1;
+            // accumulator.
+            const int me = (warp == TC_ISSUER_WARP) ? 0 : 1;
             bool ok = mbar_wait(smem_u32(&sh->w_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
             tc_fence_after();
             const uint64_t dw = smem_desc<KC>(smem_u32(s_w));
-            const uint32_t leader = (lane == 0) ? 1u : 0u;
             uint32_t ready_a = 0, ready_f = 0;           // answers of the early tests for this issuer's next tile
             // ring positions carried forward by additions (both rings are even: +2 keeps this issuer on its own slots)
             const int stages = p.stages;
@@ -116,10 +115,10 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         const uint64_t db = dw + (uint64_t)(((kh * 3 + kw) * W_TAP_BYTES) >> 4);
 #pragma unroll
                         for (int k = 0; k < 2; k++)
-                            umma_i8_w(leader, d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kw | kh | k) ? 1u : 0u);
+                            umma_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kw | kh | k) ? 1u : 0u);
                     }
-                umma_commit_w(leader, smem_u32(&sh->empty[stage]));
-                umma_commit_w(leader, smem_u32(&sh->acc_full[a]));
+                umma_commit(smem_u32(&sh->empty[stage]));
+                umma_commit(smem_u32(&sh->acc_full[a]));
                 }
                 stage = ns; phase = np; a = na; aphase = nap;
             }

@@ -61,7 +61,7 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -73,7 +73,7 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
 
-    if (warp == 0) {
+    if (warp == TC_PRODUCER_WARP) {
         // TMA producer (both CTAs).  The weights do not depend on the previous kernel: they are
         // requested before the programmatic-dependency wait, the activations after it.
         const uint32_t wbar_leader = map_to_cta(smem_u32(&sh->w_full), 0);
@@ -104,16 +104,15 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-    } else if (warp == 1 || warp == TC_ISSUER2_WARP) {
+    } else if (warp == TC_ISSUER_WARP || warp == TC_ISSUER2_WARP) {
         tc_pdl_wait();
-        if (rank == 0) {
+        if (rank == 0 && tc_elect_one()) {
             // Two MMA issuers (leader CTA) take alternate tiles; each derives its ring positions from
-            // the tile's index.  The warp loops and waits together, lane 0 issues.
-            const int me = (warp == 1) ? 0 : 1;
+            // the tile's index.
+            const int me = (warp == TC_ISSUER_WARP) ? 0 : 1;
             bool ok = mbar_wait_cluster(smem_u32(&sh->w_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
             tc_fence_after();
             const uint64_t dw = smem_desc<KC>(smem_u32(s_w));
-            const uint32_t leader = (lane == 0) ? 1u : 0u;
             uint32_t ready_a = 0, ready_f = 0;
             TileWalk wk;
             walk_init(wk, p, (pair_id + me * n_pairs) * 2, n_pairs * 4);
@@ -156,11 +155,11 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                             const uint64_t db = dw + (uint64_t)(((kh * 3 + kw) * W_TAP_BYTES) >> 4);
 #pragma unroll
                             for (int k = 0; k < KC / 32; k++)
-                                umma2_i8_w(leader, d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kh | kw | k) ? 1u : 0u);
+                                umma2_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kh | kw | k) ? 1u : 0u);
                         }
                 }
-                umma2_commit_both_w(leader, smem_u32(&sh->empty[stage]));
-                umma2_commit_both_w(leader, smem_u32(&sh->acc_full[a]));
+                umma2_commit_both(smem_u32(&sh->empty[stage]));
+                umma2_commit_both(smem_u32(&sh->acc_full[a]));
             }
         }
     } else {
@@ -178,7 +177,7 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     }
     __syncthreads();
     cluster_sync_all();
-    if (warp == 1) {
+    if (warp == TC_ISSUER_WARP) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
