@@ -13,8 +13,7 @@ not redistributable).  Rank 0 prints ONE JSON line.
   e2e   : faces/s through the public C API: ONE fastface_embed_batch call over K*B faces
           in pinned HOST memory, which the library runs as K steps of B; every step's H2D copy
           of its fp32 faces and D2H copy of its embeddings is inside the timed region.
-  roofline : the dominant kernel (CTA-pair tensor-core implicit GEMM on the 14x14 256->256
-          layers): algorithmic int8 ops of one launch / mean CUDA-event time of its launches,
+  roofline : the dominant kernel (the 14x14 stage, 26 3x3 256->256 layers in one launch): algorithmic int8 ops of its launch / its CUDA-event time,
           against 2 x the measured dense bf16 BURST rate (the kernel is timed in short
           bursts; int8 runs at twice the bf16 rate), with the sustained-rate, probe and nominal
           fractions beside it.  roofline_stem is the HBM-bound counterpart for the stem.
@@ -42,11 +41,7 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 METRIC = "faces/sec (IR-ResNet50 INT8, 112x112)"
-# dram__bytes_read + dram__bytes_write of ONE launch of the dominant kernel at batch 1024 (residual + fused-BN
-# variant: input, residual, two outputs, weights) from the ncu capture summarised in the file named here; a
-# constant, valid while that kernel's memory behaviour is unchanged (algorithmic bytes: 206.1 MB)
-DOMINANT_TRAFFIC_BYTES = 166.3e6
-DOMINANT_TRAFFIC_SOURCE = "constant from profiles/tensor_core_conv_kernels_single_layer_ncu_full.md, case 1 (ncu capture, not measured in this run)"
+DOMINANT_TRAFFIC_SOURCE = "not captured at this batch; 31 MB read at 148 faces (profiles/face_stage_ncu.md): weights once, activations in and out once"
 # stem (one launch): 150 528 B fp32 face in + 2 x 802 816 B int8 out (conv output and its fused BN)
 STEM_BYTES_PER_FACE = 150528 + 2 * 802816
 GOP_PER_FACE = 12.619          # 6.3093 GMAC: 53 convs + FC, real K, no padding
@@ -435,8 +430,7 @@ def run_own_arm(args, rank, local_rank, world):
         # denominator; a seconds-long region would take the sustained one
         timed_s = ms * 1e-3
         peak = peak_burst if timed_s < 1.0 else peak_sustained
-        # dominant kernel: the CTA-pair tensor-core kernel on the 14x14 256->256 3x3 layers
-        # (26 launches of one shape per forward, the largest share of the launch list)
+        # dominant kernel: the 14x14 stage, 26 3x3 256->256 layers in one launch (its time comes shared equally among them)
         dom = [(l, t) for l, t in tc if (l["Cin"], l["Cout"], l["Kh"], l["stride"], l["H"]) == (256, 256, 3, 1, 14)]
         if not dom:
             dom = tc
@@ -449,13 +443,14 @@ def run_own_arm(args, rank, local_rank, world):
                 "frac_of_2x_bf16_burst": round(achieved / peak_burst, 4),
                 "frac_of_2x_bf16_sustained": round(achieved / peak_sustained, 4),
                 "frac_of_nominal_4500_tops": round(achieved / 4500.0, 4),
-                "traffic": DOMINANT_TRAFFIC_BYTES if B == 1024 else None,
+                "traffic": None,
                 "traffic_source": DOMINANT_TRAFFIC_SOURCE,
-                "kernel": "conv_tc2_kernel<256> (tcgen05 kind::i8 cta_group::2 implicit GEMM), 3x3 256->256 on 14x14",
-                "launches_per_forward": len(dom), "ops_per_launch": dom_ops, "ms_per_launch": round(dom_ms, 4),
+                "kernel": "conv_face_kernel (tcgen05 kind::i8 cta_group::2, activations resident), 3x3 256->256 on 14x14",
+                "launches_per_forward": 1, "layers_per_launch": len(dom), "ops_per_launch": dom_ops * len(dom),
+                "ms_per_launch": round(dom_ms * len(dom), 4),
                 "i8_mma_probe_tops": probe, "frac_of_probe": round(achieved / probe, 4) if probe else None,
-                "note": f"achieved = algorithmic int8 ops of one launch / mean CUDA-event duration of its {len(dom)} launches "
-                        f"(timed in bursts of 3 launches per layer); frac = achieved / peak with peak = 2 x bf16 "
+                "note": f"achieved = algorithmic int8 ops of the stage's {len(dom)} layers / CUDA-event duration of its launch "
+                        f"(a burst of 3 launches); frac = achieved / peak with peak = 2 x bf16 "
                         f"{'burst' if peak == peak_burst else 'sustained'} of {peaks['source']} MEASURED_PEAKS (int8 runs at twice "
                         f"the bf16 rate; the driver measures no int8 figure); i8_mma_probe_tops = kind::i8 MMAs on "
                         f"shared-memory operands with no loads, measured in this run"}

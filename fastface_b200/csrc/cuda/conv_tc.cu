@@ -740,9 +740,10 @@ extern "C" void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles
     g_test_chain_wait = wait_cycles;
 }
 
-int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s)
+int ffcu_chain_launch(const ChainPlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
 {
     ChainParams prm = p->prm;
+    prm.face0 = face0;
     prm.err = d_err;
     prm.wait_cycles = TC_WAIT_CYCLES; prm.drop_step = -1;
     if (g_test_chain_drop_step >= 0) {                    // armed for this one launch
@@ -773,6 +774,91 @@ int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaS
     }
 #endif
     return tc_launch_chain(p->bn, mode, faces, p->smem_bytes, s, p->mapA, prm);
+}
+
+// ---------------------------------------------------------------------------
+// 14x14 stage, a CTA pair per face (conv_tc_face.cu)
+// ---------------------------------------------------------------------------
+struct FacePlan {
+    CUtensorMap mapA;
+    FaceLayer* d_layers;
+    char* d_tables;          // every layer's constants and byte table
+    int8_t* d_kept;
+    int n_layers, pairs;
+};
+
+// layers[i]: device pointers of layer i; host[i]: its constants on the host ([4][256]: w_scale, bias, slope or residual scale,
+// inv_out) and its fused BN's table ([256][256], PReLU layers none).  d_in = the first layer's input.  NULL: not on this device.
+FacePlan* ffcu_face_plan(int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers)
+{
+    encode_tiled_fn enc = get_encode();
+    const int pairs = tc_face_pairs();
+    if (!enc || pairs < 1 || n_layers < 1) return nullptr;
+    const size_t tab = FACE_C * sizeof(float4), lut = (size_t)FACE_C * 256;
+    std::vector<char> t((size_t)n_layers * (tab + lut), 0);
+    std::vector<FaceLayer> h((size_t)n_layers);
+    memset(h.data(), 0, h.size() * sizeof(FaceLayer));
+    FacePlan* p = new FacePlan();
+    p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->n_layers = n_layers; p->pairs = pairs;
+    bool ok = cudaMalloc(&p->d_layers, h.size() * sizeof(FaceLayer)) == cudaSuccess && cudaMalloc(&p->d_tables, t.size()) == cudaSuccess &&
+              cudaMalloc(&p->d_kept, (size_t)pairs * 2 * FACE_KEPT_BYTES) == cudaSuccess;
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    {
+        cuuint64_t dims[4] = {FACE_C, 14, 14, (cuuint64_t)max_batch};
+        cuuint64_t strides[3] = {FACE_C, FACE_C * 14, FACE_C * 196};
+        cuuint32_t box[4] = {128, 16, 9, 1};
+        ok = ok && enc(&p->mapA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    for (int i = 0; i < n_layers && ok; i++) {
+        const FaceLayerDesc& d = layers[i];
+        const cuuint64_t K = 9 * FACE_C;
+        cuuint64_t dims[4] = {K, FACE_C, 1, 1};
+        cuuint64_t strides[3] = {K, K * FACE_C, K * FACE_C};
+        cuuint32_t box[4] = {128, 128, 1, 1};
+        ok = enc(&h[i].mapB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        const size_t o = (size_t)i * (tab + lut);
+        float* ft = (float*)&t[o];
+        for (int c = 0; c < FACE_C; c++)
+            for (int k = 0; k < 4; k++) ft[4 * c + k] = d.tab[k * FACE_C + c];
+        h[i].tab = (const float4*)(p->d_tables + o);
+        if (d.lut) {
+            // entry q of channel 128 * r + 32 * quarter + lane -> word 128 * (q / 4) + 32 * quarter + lane of CTA r's half, byte q % 4
+            char* lt = &t[o + tab];
+            for (int c = 0; c < FACE_C; c++)
+                for (int q = 0; q < 256; q++)
+                    lt[(c / 128) * 32768 + (q >> 2) * 512 + (c % 128) * 4 + (q & 3)] = (char)d.lut[c * 256 + q];
+            h[i].lut = (const uint8_t*)(p->d_tables + o + tab);
+        }
+        h[i].res = d.res; h[i].out = d.out; h[i].out2 = d.out2;
+    }
+    ok = ok && cudaMemcpy(p->d_layers, h.data(), h.size() * sizeof(FaceLayer), cudaMemcpyHostToDevice) == cudaSuccess &&
+         cudaMemcpy(p->d_tables, t.data(), t.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+    if (!ok) { ffcu_face_free(p); cudaGetLastError(); return nullptr; }
+    return p;
+}
+
+void ffcu_face_free(FacePlan* p)
+{
+    if (!p) return;
+    cudaFree(p->d_layers); cudaFree(p->d_tables); cudaFree(p->d_kept);
+    delete p;
+}
+
+int ffcu_face_pairs(const FacePlan* p) { return p->pairs; }
+
+int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+{
+    FaceParams prm = {};
+    prm.layers = p->d_layers; prm.kept = p->d_kept; prm.n_layers = p->n_layers; prm.face0 = face0; prm.faces = faces; prm.err = d_err;
+    prm.wait_cycles = TC_WAIT_CYCLES; prm.drop_step = -1;
+    if (g_test_chain_drop_step >= 0) {                    // armed for this one launch
+        prm.drop_step = g_test_chain_drop_step;
+        if (g_test_chain_wait > 0) prm.wait_cycles = g_test_chain_wait;
+        g_test_chain_drop_step = -1; g_test_chain_wait = 0;
+    }
+    return tc_launch_face(mode, faces < p->pairs ? faces : p->pairs, s, p->mapA, prm);
 }
 
 // ---------------------------------------------------------------------------

@@ -906,6 +906,7 @@ static_assert(sizeof(ChainLayer) == 256, "ChainLayer layout");
 struct ChainParams {
     const ChainLayer* layers;
     int n_layers;
+    int face0;                            // first face
     int H, W, P, C;                       // feature map, pitch in lines, channels (in = out)
     int planes, plane_bytes;              // C / 128 planes of P * win_rows lines of 128 bytes
     int win_rows;                         // padded rows a CTA holds (the rows its row tile reads)
@@ -923,6 +924,31 @@ struct ChainParams {
 
 int tc_launch_chain(int bn, int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
 int tc_chain_clusters(int bn, int smem);
+
+// 14x14 stage, a CTA pair per face (conv_tc_face.cu)
+#define FACE_C FFCU_FACE_C
+#define FACE_KEPT_BYTES (28 * 8 * FACE_C)   // half rows of eight positions, as the epilogue's threads hold them
+#define FACE_STAGES 5                     // weight ring, 16 KB per CTA and stage
+struct FaceLayer {                        // one layer, in global memory
+    CUtensorMap mapB;                     // weights [256][9 * 256] K-major, box {128, 128}
+    const float4* tab;                    // per channel: w_scale, bias, PReLU slope or residual scale, inv_out
+    const uint8_t* lut;                   // fused BN byte table as the kernel's look-ups want it [2][32 KB], or NULL (a PReLU layer)
+    const int8_t* res;                    // residual that another kernel left (NHWC); NULL: the result of the residual layer before
+    int8_t* out; int8_t* out2;            // last layer: NHWC result and its fused BN
+    uint8_t pad_[256 - 128 - 5 * 8];
+};
+static_assert(sizeof(FaceLayer) == 256, "FaceLayer layout");
+struct FaceParams {
+    const FaceLayer* layers;
+    int8_t* kept;                         // a residual layer's result until the next one, FACE_KEPT_BYTES per pair and slot
+    int n_layers, face0, faces;           // faces face0 .. face0 + faces - 1
+    long long wait_cycles;                // limit of every barrier wait
+    int drop_step;                        // >= 0: each pair's CTA 0 leaves out this ring step (timeout test); -1 otherwise
+    int* err;
+};
+int tc_face_smem_bytes();
+int tc_face_pairs();
+int tc_launch_face(int mode, int pairs, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
 
 // Flat-pitch weight-stationary pair kernel: activation buffer = guard + box of WSP_BOX_ROWS image rows
 #define WSP_GUARD_BYTES 1024

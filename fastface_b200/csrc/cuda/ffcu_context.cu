@@ -30,6 +30,11 @@
 #define CHUNK_MIN_FACES 40
 #define CHUNK_FACES 64
 
+// Smallest call whose 14x14 stage goes out with a CTA pair per face where no chain takes it (chains come first, being 1.5 %
+// quicker at 16-33 faces): from 34 faces on it is quicker than one launch per layer at every size measured, 34 ... 1024 by
+// 2-25 %.  Below 16, where only a device without room for the chains' clusters gets, not measured: one launch per layer as before.
+#define FACE_MIN_FACES 16
+
 static thread_local char g_cu_err[512];
 
 void ffcu_set_error(const char* fmt, ...)
@@ -116,6 +121,11 @@ struct ffcu_ctx {
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
+    // Calls beyond the layer chains' reach: the 14x14 stage as one launch with a CTA pair per face (conv_tc_face.cu); FF_FACE=0
+    // disables.
+    FacePlan* face = nullptr;
+    size_t face_first = 0;
+    int face_count = 0;
     // A whole call that is one step of fewer than CHUNK_MIN_FACES faces, and any submit of at most lean_max_batch
     // (FF_LEAN_MAX_BATCH, default 1), runs copy-in, forward and copy-out on the compute stream alone: it has nothing to overlap and
     // is spared the pipeline's two cross-stream hops.  Other submits go through the three-stream pipeline, where the next step's
@@ -236,6 +246,7 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     for (int k = 0; k < 2 && done; k++) deliver(c, k);    // outputs nobody has waited for
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
     for (auto& ch : c->chains) for (ChainPlan* q : ch.plan) ffcu_chain_free(q);
+    ffcu_face_free(c->face);
     for (auto& L : c->layers) {
         for (TcPlan* q : L.tc_bn) if (q) ffcu_tc_free(q);      // L.tc is one of them
         if (L.stem_tc) ffcu_stem_tc_free(L.stem_tc);
@@ -394,6 +405,69 @@ static void find_heads(ffcu_ctx* c)
     c->head_end[1] = 2;
 }
 
+// A layer the chain kernel can take: tensor-core 3x3 stride-1 pad-1 convolution C -> C (C = 256 or 512)
+// with the no-overflow proof, its fused BN (if any) as a byte table.
+static bool chain_eligible(const ffcu_ctx* c, const DevLayer& L)
+{
+    const ffcu_layer& d = L.d;
+    return d.kind == FFCU_CONV && L.tc && !L.skip && !L.fused_stem && !c->force_simt && d.Kh == 3 && d.Kw == 3 &&
+           d.stride == 1 && d.pad == 1 && d.Cin_pad == d.Cout && d.Cin == d.Cout && d.Cout % 128 == 0 && d.H == d.W &&
+           d.Ho == d.H && d.Wo == d.W && L.epi.no_overflow && (d.bn2_dst_buf < 0 || L.bn_lut != nullptr);
+}
+
+// End of the run of layers from k on that the chain kernels can take: one shape, each reading what the one before it wrote.
+static size_t chain_end(const ffcu_ctx* c, size_t k)
+{
+    if (!chain_eligible(c, c->layers[k])) return k;
+    size_t e = k + 1;
+    for (; e < c->layers.size() && chain_eligible(c, c->layers[e]) && c->layers[e].d.H == c->layers[k].d.H &&
+           c->layers[e].d.Cout == c->layers[k].d.Cout; e++) {
+        const ffcu_layer& prev = c->layers[e - 1].d;
+        if (c->layers[e].d.src_buf != (prev.bn2_dst_buf >= 0 ? prev.bn2_dst_buf : prev.dst_buf)) break;
+    }
+    return e;
+}
+
+// The 14x14 stage as one launch (conv_tc_face.cu), which leaves only the last layer's tensors in memory (ff_plan_stage).
+static void build_face(ffcu_ctx* c)
+{
+    const char* e = getenv("FF_FACE");
+    if (c->no_chain || (e && e[0] == '0')) return;
+    std::vector<ffcu_layer> d;
+    for (size_t k = 0; k < c->layers.size(); k++) d.push_back(c->layers[k].d);
+    for (size_t k = 0; k < d.size(); ) {
+        const size_t end = chain_end(c, k);
+        if (end < k + 2 || d[k].H != 14 || d[k].Cout != FFCU_FACE_C) { k = end > k ? end : k + 1; continue; }
+        const int n = (int)(end - k);
+        std::vector<int> from((size_t)n);
+        if (!ff_plan_stage(d.data(), (int)d.size(), (int)k, n, from.data())) return;
+        std::vector<FaceLayerDesc> desc((size_t)n);
+        std::vector<std::vector<float>> tab((size_t)n, std::vector<float>(4 * FFCU_FACE_C));
+        std::vector<std::vector<int8_t>> lut((size_t)n);
+        for (int i = 0; i < n; i++) {
+            const DevLayer& L = c->layers[k + i];
+            const bool res = L.d.res_buf >= 0 && L.epi.res_scale, slope = L.epi.slope != nullptr, bn = L.d.bn2_dst_buf >= 0;
+            if (!(slope && !res && !bn) && !(res && bn && !slope)) return;
+            if (i == n - 1 && !bn) return;
+            const float* src[4] = {L.epi.w_scale, L.epi.bias, slope ? L.epi.slope : L.epi.res_scale, L.epi.inv_out};
+            for (int t = 0; t < 4; t++)
+                if (cudaMemcpy(&tab[i][(size_t)t * FFCU_FACE_C], src[t], FFCU_FACE_C * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return; }
+            if (bn) {
+                lut[i].resize(FFCU_FACE_C * 256);
+                if (cudaMemcpy(lut[i].data(), L.bn_lut, lut[i].size(), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return; }
+            }
+            FaceLayerDesc& f = desc[i];
+            f = {};
+            f.w = L.w; f.tab = tab[i].data(); f.lut = bn ? lut[i].data() : nullptr;
+            f.res = res && from[i] < 0 ? c->bufs[L.d.res_buf] : nullptr;
+            f.out = c->bufs[L.d.dst_buf]; f.out2 = bn ? c->bufs[L.d.bn2_dst_buf] : nullptr;
+        }
+        c->face = ffcu_face_plan(c->max_batch, c->bufs[d[k].src_buf], desc.data(), n);
+        c->face_first = k; c->face_count = n;
+        return;
+    }
+}
+
 extern "C" int ffcu_finalize(ffcu_ctx* c)
 {
     if (!c) return -1;
@@ -456,6 +530,7 @@ extern "C" int ffcu_finalize(ffcu_ctx* c)
     c->launches = 0;
     for (auto& L : c->layers) if (!L.skip) c->launches++;
     find_heads(c);
+    build_face(c);
     c->finalized = true;
     return 0;
 }
@@ -533,31 +608,14 @@ static int launch_layer(ffcu_ctx* c, size_t k, int n, int32_t* acc_dbg, bool unf
     return -1;
 }
 
-// A layer the chain kernel can take: tensor-core 3x3 stride-1 pad-1 convolution C -> C (C = 256 or 512)
-// with the no-overflow proof, its fused BN (if any) as a byte table.
-static bool chain_eligible(const ffcu_ctx* c, const DevLayer& L)
-{
-    const ffcu_layer& d = L.d;
-    return d.kind == FFCU_CONV && L.tc && !L.skip && !L.fused_stem && !c->force_simt && d.Kh == 3 && d.Kw == 3 &&
-           d.stride == 1 && d.pad == 1 && d.Cin_pad == d.Cout && d.Cin == d.Cout && d.Cout % 128 == 0 && d.H == d.W &&
-           d.Ho == d.H && d.Wo == d.W && L.epi.no_overflow && (d.bn2_dst_buf < 0 || L.bn_lut != nullptr);
-}
-
 static void build_chains(ffcu_ctx* c)
 {
     c->chains_built = true;
     if (c->no_chain) return;
     size_t k = 0;
     while (k < c->layers.size()) {
-        if (!chain_eligible(c, c->layers[k])) { k++; continue; }
-        size_t e = k + 1;
-        while (e < c->layers.size() && chain_eligible(c, c->layers[e]) && c->layers[e].d.H == c->layers[k].d.H &&
-               c->layers[e].d.Cout == c->layers[k].d.Cout) {
-            const ffcu_layer& prev = c->layers[e - 1].d;
-            const int feeds = prev.bn2_dst_buf >= 0 ? prev.bn2_dst_buf : prev.dst_buf;
-            if (c->layers[e].d.src_buf != feeds) break;
-            e++;
-        }
+        const size_t e = chain_end(c, k);
+        if (e == k) { k++; continue; }
         const int count = (int)(e - k);
         if (count >= 2) {
             std::vector<ChainLayerDesc> desc((size_t)count);
@@ -590,24 +648,54 @@ static int chain_max_faces(const ffcu_ctx* c)
     return c->max_batch >= 4 ? FFCU_CHAIN_MAX_FACES : 1;
 }
 
+// The chain that starts at layer k, in the narrowest clusters of which the device holds n at once; NULL: none.
+static const ffcu_ctx::Chain* chain_at(const ffcu_ctx* c, size_t k, int n, const ChainPlan** plan)
+{
+    *plan = nullptr;
+    for (const ffcu_ctx::Chain& ch : c->chains)
+        if (ch.first == k)
+            for (const ChainPlan* q : ch.plan)
+                if (!*plan && q && n <= ffcu_chain_clusters(q)) { *plan = q; return &ch; }
+    return nullptr;
+}
+
+// The 14x14 stage's launches for n faces: a pair takes two faces at a time through the stage, so whole rounds of two per pair go
+// out as one launch, and what is left over in chains where the device holds a cluster for each, which is quicker than a round
+// with one face per pair (149 / 160 / 300 faces: 1199 / 1245 / 2170 -> 1174 / 1196 / 2110 us).
+static int launch_face_stage(ffcu_ctx* c, int n, int* launches)
+{
+    int left = n % (2 * ffcu_face_pairs(c->face));
+    const ChainPlan* plan = nullptr;
+    if (left < n && left <= FFCU_CHAIN_MAX_FACES && !c->no_chain) {
+        if (!c->chains_built) build_chains(c);
+        const ffcu_ctx::Chain* ch = chain_at(c, c->face_first, left, &plan);
+        if (ch && ch->count != c->face_count) plan = nullptr;
+    }
+    if (!plan) left = 0;
+    int rc = ffcu_face_launch(c->face, 0, n - left, c->mode, c->d_err, c->stream);
+    (*launches)++;
+    if (rc != 0 || !left) return rc;
+    (*launches)++;
+    if (ffcu_chain_launch(plan, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
+    cudaGetLastError();                                    // refused, as below
+    c->no_chain = 1;
+    return ffcu_face_launch(c->face, n - left, left, c->mode, c->d_err, c->stream);
+}
+
 // Layers [k0, k1) for faces b0 .. b0 + n - 1 (b0 > 0 within a head only); c->launches = the launches made.
 static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
 {
     int launches = 0;
     const bool chain_call = n <= chain_max_faces(c);
     if (chain_call && !c->chains_built) build_chains(c);
-    size_t next_chain = 0;
     for (size_t k = k0; k < k1; k++) {
         if (chain_call && !c->no_chain) {
-            while (next_chain < c->chains.size() && c->chains[next_chain].first < k) next_chain++;
-            const ChainPlan* plan = nullptr;                // the narrowest clusters the device holds n of at once
-            if (next_chain < c->chains.size() && c->chains[next_chain].first == k)
-                for (const ChainPlan* q : c->chains[next_chain].plan)
-                    if (!plan && q && n <= ffcu_chain_clusters(q)) plan = q;
-            if (plan) {
-                if (ffcu_chain_launch(plan, n, c->mode, c->d_err, c->stream) == 0) {
+            const ChainPlan* plan = nullptr;
+            const ffcu_ctx::Chain* ch = chain_at(c, k, n, &plan);
+            if (ch) {
+                if (ffcu_chain_launch(plan, 0, n, c->mode, c->d_err, c->stream) == 0) {
                     launches++;
-                    k += (size_t)c->chains[next_chain].count - 1;
+                    k += (size_t)ch->count - 1;
                     continue;
                 }
                 // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...):
@@ -616,6 +704,12 @@ static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
                 cudaGetLastError();
                 c->no_chain = 1;
             }
+        }
+        if (c->face && k == c->face_first && n >= FACE_MIN_FACES && k + (size_t)c->face_count <= k1) {
+            const int rc = launch_face_stage(c, n, &launches);
+            if (rc != 0) return rc;
+            k += (size_t)c->face_count - 1;
+            continue;
         }
         {
             DevLayer& M = c->layers[k];
@@ -983,8 +1077,18 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     if (rc != 0) return rc;
     std::vector<cudaEvent_t> ev(2 * nl);
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
+    // the 14x14 stage as the forward runs it: the time of its one or two launches, shared equally among its layers
+    const bool face = c->face && n >= FACE_MIN_FACES && n > chain_max_faces(c);
+    const int f0 = (int)c->face_first, f1 = f0 + c->face_count;
     for (int k = 0; k < nl && rc == 0; k++) {
         DevLayer& M = c->layers[k];
+        if (face && k >= f0 && k < f1) {
+            int launched = 0;
+            FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
+            if (k == f0) for (int it = 0; it < iters && rc == 0; it++) rc = launch_face_stage(c, n, &launched);
+            FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
+            continue;
+        }
         // a stride-2 conv that shares its launch with the block's shortcut at this batch is timed as the forward runs
         // it: the pair's one launch under the conv, nothing under the shortcut
         const bool pair = M.sc && k + 1 < nl && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64;
@@ -1006,6 +1110,7 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     int wrc = ffcu_wait(c);
     if (rc == 0) rc = wrc;
     for (int k = 0; k < nl && rc == 0; k++) FFCU_CHECK(cudaEventElapsedTime(&ms[k], ev[2 * k], ev[2 * k + 1]));
+    if (face && rc == 0) for (int k = f1 - 1; k >= f0; k--) ms[k] = ms[f0] / (float)c->face_count;
     for (auto& e : ev) cudaEventDestroy(e);
     return rc == 0 ? nl : rc;
 }

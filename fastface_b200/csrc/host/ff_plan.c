@@ -357,3 +357,30 @@ int ff_plan_head_end(const ffcu_layer* l, int n, int end, const unsigned char* w
     }
     return end;
 }
+
+int ff_plan_stage(const ffcu_layer* l, int n, int first, int count, int* from)
+{
+    int in[FF_MAX_BUFS];                                /* what a buffer holds: layer i's result, -1 a tensor from outside, -2 a fused BN's output */
+    int kept = -1;                                      /* the last layer with a residual */
+    for (int b = 0; b < FF_MAX_BUFS; b++) in[b] = -1;
+    for (int i = 0; i < count; i++) {
+        const ffcu_layer* d = &l[first + i];
+        from[i] = -1;
+        if (d->res_buf >= 0) {
+            from[i] = in[d->res_buf];
+            if (from[i] == -2 || (from[i] >= 0 && from[i] != kept)) return 0;
+            kept = i;
+        }
+        in[d->dst_buf] = i;
+        if (d->bn2_dst_buf >= 0) in[d->bn2_dst_buf] = -2;
+    }
+    const ffcu_layer* e = &l[first + count - 1];
+    in[e->dst_buf] = -1;
+    if (e->bn2_dst_buf >= 0) in[e->bn2_dst_buf] = -1;
+    for (int k = first + count; k < n; k++) {
+        if ((l[k].src_buf >= 0 && in[l[k].src_buf] != -1) || (l[k].res_buf >= 0 && in[l[k].res_buf] != -1)) return 0;
+        if (l[k].dst_buf >= 0) in[l[k].dst_buf] = -1;
+        if (l[k].bn2_dst_buf >= 0) in[l[k].bn2_dst_buf] = -1;
+    }
+    return 1;
+}

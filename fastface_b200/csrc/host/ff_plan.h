@@ -33,6 +33,12 @@ void ff_plan_free(ff_plan* p);
  * layers k and k + 1 go out as one launch and stay on one side. */
 int  ff_plan_head_end(const ffcu_layer* l, int n, int end, const unsigned char* with_next);
 
+/* May layers [first, first + count) of l[0 .. n) run face by face with only the last one's tensors in their buffers, and each
+ * residual taken from outside or from the layer with a residual before it, whose result is kept until then?  Not where a layer
+ * behind them reads another tensor of theirs.  from[i]: the layer, counted from `first`, whose result layer i adds; -1: a tensor
+ * that was in its buffer before, or none.  1 / 0. */
+int  ff_plan_stage(const ffcu_layer* l, int n, int first, int count, int* from);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,55 @@
+"""The 14x14 stage as one launch with a CTA pair per face: same bytes as one launch per layer, and as the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import fastface_b200 as ff
+from fastface_b200 import synth
+from oracle import ffo
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [34, 73, 74, 75, 147, 148, 149, 163, 164, 182, 190, 222, 223, 296, 297])
+def test_stage_in_one_launch(built_lib, model_root, ffw4, oracle, monkeypatch, n):
+    """One and two faces per pair, a round more, and what is left of a round in chains (74 pairs on a B200): eager, captured and
+    replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
+    faces = synth.faces(n, seed=700 + n)
+    sample = sorted({0, n // 2, n - 1})
+    got, launches = {}, {}
+    for flag in ("1", "0"):
+        monkeypatch.setenv("FF_FACE", flag)
+        with ff.FastFace(ffw4, cwd=model_root, max_batch=297) as e:
+            for mode in (ffo.CONTRACT, ffo.STRICT):
+                e.set_epilogue_mode(mode)
+                for rep in range(3 if flag == "1" else 1):
+                    got[flag, mode, rep] = e.embed_batch(faces)
+            launches[flag] = e.launches_per_forward
+    assert launches["0"] - launches["1"] in (24, 25), launches
+    for mode in (ffo.CONTRACT, ffo.STRICT):
+        for rep in range(3):
+            bad = np.flatnonzero((got["1", mode, rep] != got["0", mode, 0]).any(axis=1))
+            assert bad.size == 0, f"mode {mode} rep {rep}: faces {bad[:16].tolist()}"
+        assert np.array_equal(got["1", mode, 0][sample], oracle.forward(faces[sample], mode))
+
+
+@pytest.mark.parametrize("n", [40, 80], ids=["one-face-a-pair", "two-faces-a-pair"])
+def test_bounded_waits_run_out(built_lib, model_root, ffw4, oracle, n):
+    """The timeout path, without faulting anything: the hook makes the first CTA of every pair leave out one step of its weights
+    and limits every wait of that launch to two million cycles.  All must give up, meet at their pair's barrier and return; the
+    call reports 1000 + the error word, and the same context then serves the same faces bit-exactly."""
+    lib = ff.load_library()
+    lib.ffcu_test_arm_chain_timeout.restype = None
+    lib.ffcu_test_arm_chain_timeout.argtypes = [C.c_int, C.c_longlong]
+    faces = synth.faces(n, seed=78)
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=80) as e:
+        want = e.embed_batch(faces)
+    assert np.array_equal(want[:2], oracle.forward(faces[:2], ffo.CONTRACT))
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=80) as e:
+        lib.ffcu_test_arm_chain_timeout(25, 2_000_000)          # second layer, or the second face's first
+        with pytest.raises(RuntimeError) as ei:
+            e.embed_batch(faces)
+        assert "rc=1001" in str(ei.value) or "rc=1004" in str(ei.value), str(ei.value)
+        for _ in range(4):
+            assert np.array_equal(e.embed_batch(faces), want)
