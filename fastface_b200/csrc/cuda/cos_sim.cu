@@ -16,12 +16,13 @@
 //
 // Kernel times, us, one output a thread and no prefetch | 16 x 64 or 64 x 64 outputs a block, norms in front of each chunk's
 // sums | this kernel: 1 x 100 24.7 | 61.6 | 12.5, 24 x 300 26.8 | 61.6 | 12.4, 64 x 1000 32.9 | 61.6 | 20.7, 1 x 10000 59 | 98 | 45,
-// 128 x 1000 51.4 | 61.6 | 22.6, 256 x 1000 82 | 72 | 37, 1024 x 1000 287 | 119 | 95, 1024 x 10000 2656 | 884 | 779.  Calls (pageable arrays, copies included): 1 x 100 90 | 115 | 57,
-// 16 x 300 120 | 137 | 78, 128 x 300 146 | 156 | 108, 256 x 1000 1613 | 359 | 295, 1024 x 1000 2643 | 643 | 617.
+// 128 x 1000 51.4 | 61.6 | 22.6, 256 x 1000 82 | 72 | 37, 1024 x 1000 287 | 119 | 95, 1024 x 10000 2656 | 884 | 779.
 #include "ffcu_internal.cuh"
 #include "cos_sim.cuh"
+#include "../host/ff_copy.h"
 
 #include <stdint.h>
+#include <string.h>
 #include <algorithm>
 
 #define CS_DIM 512
@@ -149,12 +150,13 @@ static cudaError_t launch_matrix(const float* a, int n, const float* b, int m, f
     return launch_tile<4, 2, 4, 4, 16>(a, n, b, m, out, pitch, s);
 }
 
-// One call works in slices of at most CS_MAX_N x CS_MAX_M pairs, so the workspace a context keeps is bounded
-// (4 + 8 + 32 MB) whatever the matrix.
+// One call works in slices of at most CS_MAX_N rows of `a` and CS_MAX_M of `b`, and a launch gives at most CS_MAX_OUT results,
+// so the workspace a context keeps is bounded (4 + 32 + 2 x 10 MB on the device, 8 MB page-locked) whatever the matrix.
 #define CS_MAX_N 2048
-#define CS_MAX_M 4096
+#define CS_MAX_M 16384
+#define CS_MAX_OUT ((size_t)10 << 18)
 
-static bool beyond_one_slice(int n, int m) { return n > CS_MAX_N || m > CS_MAX_M; }
+static bool beyond_one_slice(int n, int m) { return n > CS_MAX_N || m > CS_MAX_M || (size_t)n * m > CS_MAX_OUT; }
 
 // A result that takes the place of an input: every row has to be read before the first result is written.
 static bool written_over(const float* out, int n, int m, const float* in, int rows)
@@ -166,8 +168,14 @@ static bool written_over(const float* out, int n, int m, const float* in, int ro
 void CosWorkspace::release()
 {
     cudaFree(a); cudaFree(b); cudaFree(out);
-    if (stream) cudaStreamDestroy(stream);
-    a = b = out = nullptr; cap_a = cap_b = cap_out = 0; stream = nullptr;
+    for (cudaStream_t* s : {&stream, &s_in, &s_out}) { if (*s) cudaStreamDestroy(*s); *s = nullptr; }
+    for (int k = 0; k < CS_PIECES; k++) for (cudaEvent_t* e : {&ev_in[k], &ev_out[k]}) { if (*e) cudaEventDestroy(*e); *e = nullptr; }
+    for (cudaEvent_t* e : {&ev_uploaded, &ev_done[0], &ev_done[1]}) { if (*e) cudaEventDestroy(*e); *e = nullptr; }
+    if (pin_in) cudaFreeHost(pin_in);
+    if (pin_out) cudaFreeHost(pin_out);
+    ff_copy_pool_destroy(pool);
+    pin_in = pin_out = nullptr; pool = nullptr; tried = false; pieces_in = 0;
+    a = b = out = nullptr; cap_a = cap_b = cap_out = 0;
 }
 
 static bool grow(float** p, size_t* cap, size_t need)
@@ -180,18 +188,26 @@ static bool grow(float** p, size_t* cap, size_t need)
     return true;
 }
 
+static int device_sms(int device)
+{
+    int n_sm = 0;
+    if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n_sm < 1) n_sm = 148;
+    return n_sm;
+}
+
+// The plain way: a workspace of the call's own, or a result that takes the place of an input.
 int CosWorkspace::run(int device, const float* ha, int n, const float* hb, int m, float* hout)
 {
     const bool whole = written_over(hout, n, m, ha, n) || written_over(hout, n, m, hb, m);
-    const int sn = whole ? n : std::min(n, CS_MAX_N), sm = whole ? m : std::min(m, CS_MAX_M);
+    const int sn = whole ? n : std::min(n, CS_MAX_N);
+    const int sm = whole ? m : (int)std::min<size_t>(std::min(m, CS_MAX_M), std::max<size_t>(CS_MAX_OUT / sn, 64));
     if ((!stream && cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) ||
         !grow(&a, &cap_a, (size_t)sn * CS_DIM) || !grow(&b, &cap_b, (size_t)sm * CS_DIM) || !grow(&out, &cap_out, (size_t)sn * sm)) {
         ffcu_set_error("ffcu_cos_sim_matrix: device allocation failed");
         cudaGetLastError();
         return -2;
     }
-    int n_sm = 0;
-    if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n_sm < 1) n_sm = 148;
+    const int n_sm = device_sms(device);
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < n && e == cudaSuccess; i += sn) {
         const int cn = std::min(sn, n - i);
@@ -214,6 +230,167 @@ int CosWorkspace::run(int device, const float* ha, int n, const float* hb, int m
     return 0;
 }
 
+// ---------------------------------------------------------------------------
+// A kept workspace: copies shared by several threads through page-locked pieces, one way beside the other and beside the
+// kernels.  The driver's own staging of pageable memory is one thread (12 GB/s) and blocks the caller: of the 647 us of a
+// 1024 x 1024 call the kernel was 95.  Pageable calls, driver's staging -> this, us: 1 x 100 56 -> 53, 16 x 300 79 -> 63, 1 x 1000
+// 169 -> 108, 64 x 1000 207 -> 138, 1 x 10000 1220 -> 560, 128 x 10000 1622 -> 798, 1024 x 1000 597 -> 338, 1024 x 10000 9697 -> 4819
+// (the caller's untouched pages); 1 ... 1024 x 100 ... 10000, 54 sizes: none slower.
+// ---------------------------------------------------------------------------
+bool CosWorkspace::pipeline_ready()
+{
+    if (tried) return pin_out != nullptr;
+    tried = true;
+    bool ok = true;
+    for (cudaStream_t* s : {&stream, &s_in, &s_out}) if (!*s) ok = ok && cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) == cudaSuccess;
+    for (int k = 0; k < CS_PIECES; k++)
+        for (cudaEvent_t* e : {&ev_in[k], &ev_out[k]}) ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+    for (cudaEvent_t* e : {&ev_uploaded, &ev_done[0], &ev_done[1]}) ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && (pin_in = ffcu_stage_alloc(CS_PIECES * CS_PIECE)) && (pin_out = ffcu_stage_alloc(CS_PIECES * CS_PIECE));
+    if (!ok) {
+        cudaGetLastError();
+        if (pin_in) cudaFreeHost(pin_in);
+        if (pin_out) cudaFreeHost(pin_out);
+        pin_in = pin_out = nullptr;
+        return false;
+    }
+    pool = ff_copy_pool_create(3);                    // NULL: the caller's thread copies alone
+    return true;
+}
+
+// Host -> device on s_in; a pageable source has been read when this returns.
+cudaError_t CosWorkspace::upload(float* dst, const float* src, size_t bytes, bool staged)
+{
+    if (!staged) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s_in);
+    cudaError_t e = cudaSuccess;
+    for (size_t o = 0; o < bytes && e == cudaSuccess; o += CS_PIECE, pieces_in++) {
+        const size_t nb = std::min(CS_PIECE, bytes - o);
+        const unsigned k = pieces_in % CS_PIECES;
+        if (pieces_in >= CS_PIECES) e = cudaEventSynchronize(ev_in[k]);        // the slot's last copy has left it
+        if (e != cudaSuccess) break;
+        ff_copy(pool, pin_in + k * CS_PIECE, (const char*)src + o, nb, 1);
+        e = cudaMemcpyAsync((char*)dst + o, pin_in + k * CS_PIECE, nb, cudaMemcpyHostToDevice, s_in);
+        if (e == cudaSuccess) e = cudaEventRecord(ev_in[k], s_in);
+    }
+    return e;
+}
+
+// rows x cols results at src, complete with event `done`, -> host rows `pitch` floats apart, by way of s_out.
+cudaError_t CosWorkspace::deliver(float* hout, size_t pitch, const float* src, int rows, int cols, bool staged, cudaEvent_t done)
+{
+    cudaError_t e = cudaStreamWaitEvent(s_out, done, 0);
+    if (e != cudaSuccess) return e;
+    if (!staged)
+        return (size_t)cols == pitch ? cudaMemcpyAsync(hout, src, (size_t)rows * cols * 4, cudaMemcpyDeviceToHost, s_out)
+                                     : cudaMemcpy2DAsync(hout, pitch * 4, src, (size_t)cols * 4, (size_t)cols * 4, rows, cudaMemcpyDeviceToHost, s_out);
+    const size_t total = (size_t)rows * cols * 4, n = (total + CS_PIECE - 1) / CS_PIECE;
+    auto fetch = [&](size_t p) {
+        const size_t nb = std::min(CS_PIECE, total - p * CS_PIECE);
+        cudaError_t r = cudaMemcpyAsync(pin_out + p % CS_PIECES * CS_PIECE, (const char*)src + p * CS_PIECE, nb, cudaMemcpyDeviceToHost, s_out);
+        return r == cudaSuccess ? cudaEventRecord(ev_out[p % CS_PIECES], s_out) : r;
+    };
+    for (size_t p = 0; p < std::min<size_t>(n, CS_PIECES) && e == cudaSuccess; p++) e = fetch(p);
+    for (size_t p = 0; p < n && e == cudaSuccess; p++) {
+        e = cudaEventSynchronize(ev_out[p % CS_PIECES]);
+        if (e != cudaSuccess) break;
+        const size_t o = p * CS_PIECE, nb = std::min(CS_PIECE, total - o), line = (size_t)cols * 4;
+        const char* from = pin_out + p % CS_PIECES * CS_PIECE;
+        if ((size_t)cols == pitch) ff_copy(pool, (char*)hout + o, from, nb, 0);
+        else
+            for (size_t x = o; x < o + nb; ) {                                  // the rows of a column slice, a piece's first and last in parts
+                const size_t row = x / line, at = x % line, part = std::min(line - at, o + nb - x);
+                memcpy((char*)(hout + row * pitch) + at, from + (x - o), part);
+                x += part;
+            }
+        if (p + CS_PIECES < n) e = fetch(p + CS_PIECES);
+    }
+    return e;
+}
+
+// Rows of a launch for m columns: whole 64-row tiles that fill the SMs (at least 85 % of the launch's last wave), as few as
+// that takes, so that the results of one launch are on their way while the next one runs; at most CS_MAX_OUT results.
+static int launch_rows(int m, int n_sm)
+{
+    const int tiles = (m + 63) / 64;
+    const int most = (int)std::max<size_t>(CS_MAX_OUT / ((size_t)64 * m), 1);
+    int best = 1;
+    double best_fill = 0.0;
+    for (int k = 1; k <= most && best_fill < 0.85; k++) {
+        const long long blocks = (long long)k * tiles, waves = (blocks + n_sm - 1) / n_sm;
+        const double fill = (double)blocks / (double)(waves * n_sm);
+        if (fill > best_fill) { best = k; best_fill = fill; }
+    }
+    return 64 * best;
+}
+
+int CosWorkspace::run_pipeline(int n_sm, const float* ha, int n, const float* hb, int m, float* hout, bool in_a, bool in_b, bool out_staged)
+{
+    const size_t in_bytes = (size_t)(n + m) * CS_DIM * 4, out_bytes = (size_t)n * m * 4;
+    if (in_a && in_b && out_staged && in_bytes <= CS_PIECE && out_bytes <= CS_PIECE) {
+        // a small matrix: both inputs in one copy, everything in order on one stream (1 x 100 / 1 x 300: 63 / 77 -> 53 / 60 us)
+        if (!grow(&b, &cap_b, (size_t)(n + m) * CS_DIM) || !grow(&out, &cap_out, (size_t)n * m)) {
+            ffcu_set_error("ffcu_cos_sim_matrix: device allocation failed");
+            cudaGetLastError();
+            return -2;
+        }
+        ff_copy(pool, pin_in, hb, (size_t)m * CS_DIM * 4, 1);
+        ff_copy(pool, pin_in + (size_t)m * CS_DIM * 4, ha, (size_t)n * CS_DIM * 4, 1);
+        cudaError_t e = cudaMemcpyAsync(b, pin_in, in_bytes, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = launch_matrix(b + (size_t)m * CS_DIM, n, b, m, out, (size_t)m, n_sm, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pin_out, out, out_bytes, cudaMemcpyDeviceToHost, stream);
+        const cudaError_t e2 = cudaStreamSynchronize(stream);
+        if (e == cudaSuccess) e = e2;
+        if (e != cudaSuccess) { ffcu_set_error("ffcu_cos_sim_matrix: %s", cudaGetErrorString(e)); return -100; }
+        ff_copy(pool, hout, pin_out, out_bytes, 0);
+        return 0;
+    }
+    const int sn = std::min(n, CS_MAX_N), sm = std::min(m, CS_MAX_M);
+    const int step = std::min(sn, launch_rows(sm, n_sm));
+    const size_t slot = (size_t)step * sm;
+    cudaError_t e = cudaSuccess;
+    int rc = 0;
+    if (!grow(&a, &cap_a, (size_t)sn * CS_DIM) || !grow(&b, &cap_b, (size_t)sm * CS_DIM) ||
+        !grow(&out, &cap_out, slot * (step < n || sm < m ? 2 : 1))) {
+        ffcu_set_error("ffcu_cos_sim_matrix: device allocation failed");
+        cudaGetLastError();
+        return -2;
+    }
+    struct { float* to; const float* from; int rows, cols; } last = {nullptr, nullptr, 0, 0};      // launched, not delivered
+    int k = 0;                                        // launches so far
+    auto flush = [&]() {
+        if (e == cudaSuccess && last.to) e = deliver(last.to, (size_t)m, last.from, last.rows, last.cols, out_staged, ev_done[(k - 1) & 1]);
+        last.to = nullptr;
+    };
+    for (int i0 = 0; i0 < n && e == cudaSuccess; i0 += sn) {
+        const int cn = std::min(sn, n - i0);
+        for (int j = 0; j < m && e == cudaSuccess; j += sm) {
+            const int cm = std::min(sm, m - j);
+            if (k) e = cudaStreamWaitEvent(s_in, ev_done[(k - 1) & 1], 0);      // what the earlier launches read is replaced
+            if (e == cudaSuccess) e = upload(b, hb + (size_t)j * CS_DIM, (size_t)cm * CS_DIM * 4, in_b);
+            for (int i = 0; i < cn && e == cudaSuccess; i += step) {
+                const int rows = std::min(step, cn - i);
+                if (j == 0) e = upload(a + (size_t)i * CS_DIM, ha + (size_t)(i0 + i) * CS_DIM, (size_t)rows * CS_DIM * 4, in_a);
+                if (e == cudaSuccess) e = cudaEventRecord(ev_uploaded, s_in);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ev_uploaded, 0);
+                float* to = out + (size_t)(k & 1) * slot;
+                if (e == cudaSuccess && !out_staged && k >= 2) e = cudaStreamSynchronize(s_out);    // the slot's copy has left it (a staged one has been waited for)
+                if (e == cudaSuccess) e = launch_matrix(a + (size_t)i * CS_DIM, rows, b, cm, to, (size_t)cm, n_sm, stream);
+                if (e == cudaSuccess) e = cudaEventRecord(ev_done[k & 1], stream);
+                flush();                              // the launch before, while this one runs
+                last = {hout + (size_t)(i0 + i) * m + j, to, rows, cm};
+                k++;
+            }
+        }
+    }
+    flush();
+    for (cudaStream_t s : {s_in, stream, s_out}) {
+        const cudaError_t e2 = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = e2;
+    }
+    if (e != cudaSuccess) { ffcu_set_error("ffcu_cos_sim_matrix: %s", cudaGetErrorString(e)); rc = -100; }
+    return rc;
+}
+
 // a: host [n][512], b: host [m][512], out: host [n][m].  Returns 0 or a negative code.
 extern "C" int ffcu_cos_sim_matrix(int device, const float* a, int n, const float* b, int m, float* out)
 {
@@ -230,12 +407,14 @@ extern "C" int ffcu_cos_sim_matrix(int device, const float* a, int n, const floa
 int CosWorkspace::call(int device, const float* ha, int n, const float* hb, int m, float* hout)
 {
     if (!ha || !hb || !hout || n < 1 || m < 1) { ffcu_set_error("ffcu_cos_sim_matrix: bad arguments"); return -1; }
-    if (beyond_one_slice(n, m) && (written_over(hout, n, m, ha, n) || written_over(hout, n, m, hb, m)))
-        return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
+    const bool over = written_over(hout, n, m, ha, n) || written_over(hout, n, m, hb, m);
+    if (beyond_one_slice(n, m) && over) return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
     if (!mu.try_lock()) return ffcu_cos_sim_matrix(device, ha, n, hb, m, hout);
     int rc = cudaSetDevice(device) == cudaSuccess ? 0 : -100;
     if (rc) { ffcu_set_error("cudaSetDevice(%d) failed", device); cudaGetLastError(); }
-    else rc = run(device, ha, n, hb, m, hout);
+    else if (over || !pipeline_ready()) rc = run(device, ha, n, hb, m, hout);
+    else rc = run_pipeline(device_sms(device), ha, n, hb, m, hout, ffcu_is_pageable(ha, (size_t)n * CS_DIM * 4),
+                           ffcu_is_pageable(hb, (size_t)m * CS_DIM * 4), ffcu_is_pageable(hout, (size_t)n * m * 4));
     mu.unlock();
     return rc;
 }

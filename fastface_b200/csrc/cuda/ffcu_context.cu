@@ -157,12 +157,12 @@ static int g_test_deny_staging = 0;
 // The next `count` page-locked staging allocations of the process fail (for the test of a host that has none to give).
 extern "C" void ffcu_test_deny_staging(int count) { g_test_deny_staging = count; }
 
-static char* stage_alloc(size_t bytes)
+char* ffcu_stage_alloc(size_t bytes)
 {
     void* p = nullptr;
     if (g_test_deny_staging > 0) { g_test_deny_staging--; return nullptr; }
     if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    memset(p, 0, OUT_HEAD);
+    memset(p, 0, std::min(bytes, (size_t)OUT_HEAD));
     return (char*)p;
 }
 
@@ -171,8 +171,8 @@ static void make_staging(ffcu_ctx* c)
 {
     const size_t out_bytes = OUT_HEAD + (size_t)std::min(c->max_batch, STAGE_OUT_FACES) * 512 * sizeof(float);
     c->stage_slot_bytes = (size_t)std::min(c->max_batch, STAGE_FACES) * 37632 * sizeof(float);
-    c->stage_in = stage_alloc(STAGE_SLOTS * c->stage_slot_bytes);
-    for (int k = 0; k < 2; k++) c->err_at[k] = (int*)(c->stage_out[k] = stage_alloc(out_bytes));
+    c->stage_in = ffcu_stage_alloc(STAGE_SLOTS * c->stage_slot_bytes);
+    for (int k = 0; k < 2; k++) c->err_at[k] = (int*)(c->stage_out[k] = ffcu_stage_alloc(out_bytes));
     c->pool = ff_copy_pool_create(3);                 // NULL: the caller's thread copies alone
 }
 
@@ -776,7 +776,7 @@ static int run_forward(ffcu_ctx* c, int n, int slot, int k0 = 0)
 }
 
 // Memory that CUDA knows nothing of, first byte and last: what the driver would copy from or to by a staging of its own.
-static bool is_pageable(const void* p, size_t bytes)
+bool ffcu_is_pageable(const void* p, size_t bytes)
 {
     for (const char* q : {(const char*)p, (const char*)p + bytes - 1}) {
         cudaPointerAttributes a;
@@ -806,7 +806,7 @@ static int copy_in(ffcu_ctx* c, void* dst, const void* src, size_t bytes, bool s
 static int copy_out(ffcu_ctx* c, int slot, int n, float* host_out, cudaStream_t s)
 {
     const size_t nb = (size_t)n * 512 * sizeof(float);
-    if (n <= STAGE_OUT_FACES && c->stage_out[slot] && is_pageable(host_out, nb)) {
+    if (n <= STAGE_OUT_FACES && c->stage_out[slot] && ffcu_is_pageable(host_out, nb)) {
         FFCU_CHECK(cudaMemcpyAsync(c->stage_out[slot], c->out_mem[slot], OUT_HEAD + nb, cudaMemcpyDeviceToHost, s));
         c->pending[slot] = {host_out, nb};
     } else {
@@ -834,7 +834,7 @@ static int submit_impl(ffcu_ctx* c, const void* host_in, size_t bytes_per_face, 
     FFCU_CHECK(cudaSetDevice(c->device));
     const int slot = (int)(c->seq & 1);
     const bool reused = c->seq >= 2;
-    const bool staged = c->stage_in && is_pageable(host_in, (size_t)n * bytes_per_face);
+    const bool staged = c->stage_in && ffcu_is_pageable(host_in, (size_t)n * bytes_per_face);
     const bool was_idle = c->idle;
     c->idle = false;
     if (c->pending[slot].dst) {                       // the output two steps ago still sits in the slot's staging

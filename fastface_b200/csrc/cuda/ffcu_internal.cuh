@@ -21,6 +21,10 @@ enum {
 };
 
 void ffcu_set_error(const char* fmt, ...);
+// Page-locked staging memory; NULL where the host has none to give.
+char* ffcu_stage_alloc(size_t bytes);
+// Memory that CUDA knows nothing of, first byte and last.
+bool ffcu_is_pageable(const void* p, size_t bytes);
 
 #define FFCU_CHECK(expr)                                                                    \
     do {                                                                                    \

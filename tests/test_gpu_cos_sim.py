@@ -123,3 +123,28 @@ def test_matrix_after_an_error_of_the_callers(engine):
     assert rt.cudaMalloc(C.byref(p), C.c_size_t(1 << 60)) == 2         # more than any device has: out of memory
     assert np.array_equal(engine.cos_sim_matrix(a, b), want)
     rt.cudaGetLastError()
+
+
+# both sides of the lines of a call's path: inputs of a megabyte (512 rows), results of a megabyte, launches of whole waves
+# (1024 columns: 512 rows), the launch's largest result, the widest gallery kept at once
+@pytest.mark.parametrize("n,m", [(12, 500), (13, 500), (255, 257), (512, 512), (513, 511), (1024, 1024), (1500, 1024), (1, 16385), (160, 16384), (161, 16390)])
+def test_matrix_paths(engine, n, m):
+    """Pageable and page-locked arrays, in every combination, give the same matrix; two calls, so that buffers are used again."""
+    import torch
+    rng = np.random.default_rng(n * 31 + m)
+    a = rng.standard_normal((n, 512), dtype=np.float32)
+    b = rng.standard_normal((m, 512), dtype=np.float32)
+    b[m // 3] = 0
+
+    def locked(x):
+        t = torch.empty(x.shape, dtype=torch.float32, pin_memory=True).numpy()
+        t[...] = x
+        return t
+
+    want = engine.cos_sim_matrix(a, b)
+    check(want, a, b, rng, 200)
+    la, lb = locked(a), locked(b)
+    for pa, pb, lo in ((a, b, False), (la, b, False), (a, lb, True), (la, lb, True), (a, b, True)):
+        out = locked(np.zeros((n, m), np.float32)) if lo else np.zeros((n, m), np.float32)
+        assert engine.lib.fastface_cos_sim_matrix(engine.h, pa.ctypes.data, n, pb.ctypes.data, m, out.ctypes.data) == 0
+        assert np.array_equal(out, want)
