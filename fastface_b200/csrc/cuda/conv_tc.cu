@@ -1,6 +1,7 @@
 // conv_tc.cu -- host side of the tensor-core convolution: per-layer kernel choice, tile
 // geometry, TMA descriptors, launch.  The kernels live in conv_tc_{generic,ws,pair,k32}.cu.
 #include "conv_tc_common.cuh"
+#include <algorithm>
 #include <vector>
 
 // ---------------------------------------------------------------------------
@@ -740,10 +741,9 @@ extern "C" void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles
     g_test_chain_wait = wait_cycles;
 }
 
-int ffcu_chain_launch(const ChainPlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s)
 {
     ChainParams prm = p->prm;
-    prm.face0 = face0;
     prm.err = d_err;
     prm.wait_cycles = TC_WAIT_CYCLES; prm.drop_step = -1;
     if (g_test_chain_drop_step >= 0) {                    // armed for this one launch
@@ -780,11 +780,12 @@ int ffcu_chain_launch(const ChainPlan* p, int face0, int faces, int mode, int* d
 // 14x14 stage, a CTA pair per face (conv_tc_face.cu)
 // ---------------------------------------------------------------------------
 struct FacePlan {
-    CUtensorMap mapA;
+    CUtensorMap mapA, mapA4;      // boxes of nine rows (a pair, two row tiles), of six (four row tiles)
     FaceLayer* d_layers;
     char* d_tables;          // every layer's constants and byte table
     int8_t* d_kept;
     int n_layers, pairs;
+    int clusters4, clusters2;     // clusters of eight and of four the device holds at once (conv_tc_stage.cu)
 };
 
 // layers[i]: device pointers of layer i; host[i]: its constants on the host ([4][256]: w_scale, bias, slope or residual scale,
@@ -800,15 +801,18 @@ FacePlan* ffcu_face_plan(int max_batch, const int8_t* d_in, const FaceLayerDesc*
     memset(h.data(), 0, h.size() * sizeof(FaceLayer));
     FacePlan* p = new FacePlan();
     p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->n_layers = n_layers; p->pairs = pairs;
+    p->clusters4 = std::min(tc_stage_clusters(4), 2 * pairs); p->clusters2 = std::min(tc_stage_clusters(2), 2 * pairs);     // (d_kept)
     bool ok = cudaMalloc(&p->d_layers, h.size() * sizeof(FaceLayer)) == cudaSuccess && cudaMalloc(&p->d_tables, t.size()) == cudaSuccess &&
               cudaMalloc(&p->d_kept, (size_t)pairs * 2 * FACE_KEPT_BYTES) == cudaSuccess;
     cuuint32_t es[4] = {1, 1, 1, 1};
     {
         cuuint64_t dims[4] = {FACE_C, 14, 14, (cuuint64_t)max_batch};
         cuuint64_t strides[3] = {FACE_C, FACE_C * 14, FACE_C * 196};
-        cuuint32_t box[4] = {128, 16, 9, 1};
-        ok = ok && enc(&p->mapA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        for (CUtensorMap* m : {&p->mapA, &p->mapA4}) {
+            cuuint32_t box[4] = {128, 16, m == &p->mapA ? 9u : 6u, 1};
+            ok = ok && enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        }
     }
     for (int i = 0; i < n_layers && ok; i++) {
         const FaceLayerDesc& d = layers[i];
@@ -848,7 +852,7 @@ void ffcu_face_free(FacePlan* p)
 
 int ffcu_face_pairs(const FacePlan* p) { return p->pairs; }
 
-int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+static FaceParams face_params(const FacePlan* p, int face0, int faces, int* d_err)
 {
     FaceParams prm = {};
     prm.layers = p->d_layers; prm.kept = p->d_kept; prm.n_layers = p->n_layers; prm.face0 = face0; prm.faces = faces; prm.err = d_err;
@@ -858,7 +862,19 @@ int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_e
         if (g_test_chain_wait > 0) prm.wait_cycles = g_test_chain_wait;
         g_test_chain_drop_step = -1; g_test_chain_wait = 0;
     }
-    return tc_launch_face(mode, faces < p->pairs ? faces : p->pairs, s, p->mapA, prm);
+    return prm;
+}
+
+int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+{
+    return tc_launch_face(mode, faces < p->pairs ? faces : p->pairs, s, p->mapA, face_params(p, face0, faces, d_err));
+}
+
+int ffcu_stage_row_tiles(const FacePlan* p, int faces) { return faces <= p->clusters4 ? 4 : faces <= p->clusters2 ? 2 : 0; }
+
+int ffcu_stage_launch(const FacePlan* p, int row_tiles, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+{
+    return tc_launch_stage(row_tiles, mode, faces, s, row_tiles == 4 ? p->mapA4 : p->mapA, face_params(p, face0, faces, d_err));
 }
 
 // ---------------------------------------------------------------------------

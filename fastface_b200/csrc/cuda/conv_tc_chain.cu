@@ -221,7 +221,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap mapA, const ChainParams p)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
-    const int face = p.face0 + (int)blockIdx.x / CLUSTER; // one cluster per face
+    const int face = (int)blockIdx.x / CLUSTER;           // one cluster per face
     const int tile_m = (int)rank / p.tiles_n;
     const int tile_n = (int)rank % p.tiles_n;
     const int a_buf_bytes = p.planes * p.plane_bytes;

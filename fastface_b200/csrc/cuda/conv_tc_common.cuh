@@ -906,7 +906,6 @@ static_assert(sizeof(ChainLayer) == 256, "ChainLayer layout");
 struct ChainParams {
     const ChainLayer* layers;
     int n_layers;
-    int face0;                            // first face
     int H, W, P, C;                       // feature map, pitch in lines, channels (in = out)
     int planes, plane_bytes;              // C / 128 planes of P * win_rows lines of 128 bytes
     int win_rows;                         // padded rows a CTA holds (the rows its row tile reads)
@@ -940,7 +939,7 @@ struct FaceLayer {                        // one layer, in global memory
 static_assert(sizeof(FaceLayer) == 256, "FaceLayer layout");
 struct FaceParams {
     const FaceLayer* layers;
-    int8_t* kept;                         // a residual layer's result until the next one, FACE_KEPT_BYTES per pair and slot
+    int8_t* kept;                         // a residual layer's result until the next one, FACE_KEPT_BYTES per pair and slot, or per cluster
     int n_layers, face0, faces;           // faces face0 .. face0 + faces - 1
     long long wait_cycles;                // limit of every barrier wait
     int drop_step;                        // >= 0: each pair's CTA 0 leaves out this ring step (timeout test); -1 otherwise
@@ -949,6 +948,9 @@ struct FaceParams {
 int tc_face_smem_bytes();
 int tc_face_pairs();
 int tc_launch_face(int mode, int pairs, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
+// The same stage for a handful of faces, a cluster of two CTAs per row tile and face (conv_tc_stage.cu): four row tiles or two
+int tc_launch_stage(int row_tiles, int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
+int tc_stage_clusters(int row_tiles);
 
 // Flat-pitch weight-stationary pair kernel: activation buffer = guard + box of WSP_BOX_ROWS image rows
 #define WSP_GUARD_BYTES 1024

@@ -17,13 +17,13 @@
 // 8.1), latency with one: 13-15 thousand cycles, of which the MMAs 8.9, the epilogue 3.1 (PReLU) or 4.6 (residual + BN; the
 // half-rate integer pipe and the look-ups), the exchange 1.5.  Forward of 34 / 64 / 74 / 75 / 100 / 148 / 256 / 512 / 1024 faces, one
 // launch per layer -> this: 560 / 744 / 771 / 776 / 1002 / 1240 / 1925 / 3500 / 6800 -> 491 / 613 / 636 / 698 / 805 / 1007 / 1750 / 3150 /
-// 6420 us.  Up to the 33 faces or so the wide layer chains hold, those are 1.5 % quicker (17 faces: 416 against 421).
+// 6420 us.  Up to the 33 faces or so that the device holds clusters of four for, those are quicker (conv_tc_stage.cu).
 // Tried and not kept: one warp that sends all staging buffers (its five copies one after another: +14 us at 64 faces), one remote
 // arrival per CTA behind local ones (+9 us), the epilogue as a loop over rows or pairs of rows (loads' latency, spills: +20-30 us).
 //
 // Replaces, per layer, what conv_tc2_kernel does (reference kernels/conv2d_nhwc.c:179-220, kernels/int8_epilogue.c:25-112,
 // :253-318); same arithmetic, same bytes.
-#include "conv_tc_common.cuh"
+#include "conv_tc_face.cuh"
 
 namespace {
 
@@ -31,7 +31,7 @@ constexpr int STEP_BYTES = 128 * 128;                        // one tap of one p
 constexpr int PLANE_BYTES = 9 * 16 * 128;
 constexpr int ACT_BYTES = 2 * PLANE_BYTES;
 constexpr int STG_BYTES = 8 * 16 * 128;                      // the eight rows the other CTA reads
-constexpr int LUT_BYTES = 128 * 256;
+constexpr int LUT_BYTES = FACE_LUT_BYTES;
 constexpr int STEPS = 18;                                    // per layer: nine taps of two planes
 constexpr int OFF_STG = 2 * ACT_BYTES;
 constexpr int OFF_LUT = OFF_STG + 2 * STG_BYTES;
@@ -51,12 +51,6 @@ struct FaceShared {
     int abort_flag;
 };
 
-__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 __device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, int (&v)[8])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -67,67 +61,6 @@ __device__ __forceinline__ void tmem_ld_wait8(int (&v)[8])
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]) :: "memory");
-}
-
-// What a thread's stores need: ad[k] = its byte's shared-memory address in a line of swizzle phase k of the row that is
-// written (lines of 128 B: column c lies c + 1 lines further on, in phase (c + 1) & 7), or, in the last layer, the NHWC pixel.
-struct FaceDst {
-    uint32_t ad[8];
-    int8_t* g;
-};
-
-// NV (four, or two at a row's end) positions c0 .. of one channel: accumulators v, constants k (w_scale, bias, PReLU slope or
-// residual scale, inv_out) -> int8.  rw: the residual's bytes in, the requantised ones out.  What the next layer reads (the
-// fused BN of it, where the layer has one) is stored byte by byte: a warp's 32 channels are 32 consecutive bytes of a line.
-// lut_lo, lut_hi: this channel's share of a table address, in every byte; entry q of channel 32 * quarter + lane lies at
-// (q >> 2) * 512 + quarter * 128 + lane * 4 + (q & 3) of the table, so 32 lanes never meet in a bank.
-template <bool CONTRACT, bool RESBN, int NV>
-__device__ __forceinline__ uint32_t face_quad(const int* v, uint32_t rw, const float4& k)
-{
-    int q[4] = {0, 0, 0, 0};
-    const uint32_t rx = rw ^ 0x80808080u;
-    TcUnroll<NV>::run([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        const float f = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(v[i]), k.x, k.y, RESBN, RESBN ? ffcu_byte2f<i>(rx) : 0.0f, k.z, !RESBN, k.z);
-        q[i] = ffcu_requant_nosat<false>(f, k.w);
-    });
-    return (uint32_t)ffcu_pack4(q[0], q[1], q[2], q[3]);
-}
-template <bool CONTRACT, bool RESBN, bool LAST, int C0, int C1, int ROW>
-__device__ __forceinline__ void face_cols(const int* v, uint32_t* rw, const float4& k, const uint8_t* lut, uint32_t lut_lo,
-                                          uint32_t lut_hi, const FaceDst& d)
-{
-    constexpr int N = C1 - C0, WORDS = (N + 3) / 4;
-    TcUnroll<WORDS>::run([&](auto gc) {
-        constexpr int g = decltype(gc)::value;
-        rw[g] = face_quad<CONTRACT, RESBN, (N - 4 * g < 4 ? N - 4 * g : 4)>(v + 4 * g, rw[g], k);
-    });
-    uint32_t b[N];
-    TcUnroll<N>::run([&](auto ic) {
-        constexpr int i = decltype(ic)::value, m = i & 3;
-        const uint32_t w = rw[i / 4];
-        if constexpr (RESBN) {
-            const uint32_t lo = (w & 0x03030303u) | lut_lo, hi = ((w >> 1) & 0x7e7e7e7eu) | lut_hi;
-            uint32_t off;            // byte 0: lo, byte 1: hi, above it hi's sign (zero)
-            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(off) : "r"(hi), "r"(lo), "n"(((m | 8) << 12) | ((m | 8) << 8) | (m << 4) | (4 + m)));
-            b[i] = lut[off];
-        } else b[i] = w >> (8 * m);
-    });
-    TcUnroll<N>::run([&](auto ic) {
-        constexpr int i = decltype(ic)::value, c = C0 + i;
-        if constexpr (LAST) d.g[(ROW * 14 + c) * FACE_C] = (int8_t)b[i];
-        else asm volatile("st.shared.u8 [%0 + %1], %2;" ::"r"(d.ad[(c + 1) & 7]), "n"(ROW * 2048 + (c + 1) * 128), "r"(b[i]));
-    });
-}
-template <bool CONTRACT, bool RESBN, bool LAST, int ROW>
-__device__ __forceinline__ void face_half_a(const int* v, uint32_t* rw, const float4& k, const uint8_t* lut, uint32_t lo, uint32_t hi, const FaceDst& d)
-{
-    face_cols<CONTRACT, RESBN, LAST, 0, 8, ROW>(v, rw, k, lut, lo, hi, d);
-}
-template <bool CONTRACT, bool RESBN, bool LAST, int ROW>
-__device__ __forceinline__ void face_half_b(const int* v, uint32_t* rw, const float4& k, const uint8_t* lut, uint32_t lo, uint32_t hi, const FaceDst& d)
-{
-    face_cols<CONTRACT, RESBN, LAST, 8, 14, ROW>(v, rw, k, lut, lo, hi, d);
 }
 
 // One thread of the epilogue: its channel and its warp's share of the rows.  Warps are (TMEM lane quarter q, group g); a
@@ -212,9 +145,7 @@ __device__ __forceinline__ void face_epilogue(uint8_t* smem, FaceShared* sh, con
         asm volatile("bar.sync %0, 128;" ::"r"(2 + e.g) : "memory");
         if (ok) {
             if (e.q == 0 && e.lane == 0)
-                asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(map_to_cta(s_act + (uint32_t)(e.rank * 2048 + e.g * 4096), e.peer)), "r"(s_stg), "r"(4096),
-                               "r"(map_to_cta(smem_u32(&sh->rx[slot]), e.peer)) : "memory");
+                bulk_send(map_to_cta(s_act + (uint32_t)(e.rank * 2048 + e.g * 4096), e.peer), s_stg, 4096, map_to_cta(smem_u32(&sh->rx[slot]), e.peer));
             if (e.g == (e.rank ? 3 : 0)) {
                 // rows 6 and 7 are read by both CTAs
                 const uint32_t t = (uint32_t)((e.q * 32 + e.lane) * 16), dst = s_act + (e.rank ? 0u : 7u * 2048u) + t;
@@ -471,7 +402,7 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                 }
 #pragma unroll 1
                 for (int s = 0; s < slots && ok; s++) {
-                    ok = mbar_wait(smem_u32(&sh->acc_full[s]), (acc_par >> s) & 1, abort_flag, p.err, FFCU_ERR_MMA_TIMEOUT, p.wait_cycles);
+                    ok = mbar_wait(smem_u32(&sh->acc_full[s]), (acc_par >> s) & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
                     acc_par ^= 1u << s;
                     const int j = 2 * (i + 1) + s;
                     if (ok && L + 1 == p.n_layers && j < nf) load_face(s, j);

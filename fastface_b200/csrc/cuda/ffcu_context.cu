@@ -30,11 +30,6 @@
 #define CHUNK_MIN_FACES 40
 #define CHUNK_FACES 64
 
-// Smallest call whose 14x14 stage goes out with a CTA pair per face where no chain takes it (chains come first, being 1.5 %
-// quicker at 16-33 faces): from 34 faces on it is quicker than one launch per layer at every size measured, 34 ... 1024 by
-// 2-25 %.  Below 16, where only a device without room for the chains' clusters gets, not measured: one launch per layer as before.
-#define FACE_MIN_FACES 16
-
 static thread_local char g_cu_err[512];
 
 void ffcu_set_error(const char* fmt, ...)
@@ -121,10 +116,10 @@ struct ffcu_ctx {
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
-    // Calls beyond the layer chains' reach: the 14x14 stage as one launch with a CTA pair per face (conv_tc_face.cu); FF_FACE=0
-    // disables.
+    // The 14x14 stage as one launch, a cluster (conv_tc_stage.cu) or a CTA pair (conv_tc_face.cu) per face; FF_FACE=0 disables.
     FacePlan* face = nullptr;
     size_t face_first = 0;
+    int no_clusters = 0;         // a cluster launch of it was refused
     int face_count = 0;
     // A whole call that is one step of fewer than CHUNK_MIN_FACES faces, and any submit of at most lean_max_batch
     // (FF_LEAN_MAX_BATCH, default 1), runs copy-in, forward and copy-out on the compute stream alone: it has nothing to overlap and
@@ -659,26 +654,28 @@ static const ffcu_ctx::Chain* chain_at(const ffcu_ctx* c, size_t k, int n, const
     return nullptr;
 }
 
-// The 14x14 stage's launches for n faces: a pair takes two faces at a time through the stage, so whole rounds of two per pair go
-// out as one launch, and what is left over in chains where the device holds a cluster for each, which is quicker than a round
-// with one face per pair (149 / 160 / 300 faces: 1199 / 1245 / 2170 -> 1174 / 1196 / 2110 us).
+// (A context made for two or three faces keeps one launch per layer beyond a single face: chain_max_faces.)
+static bool face_takes(const ffcu_ctx* c, int n) { return c->face && (n == 1 || c->max_batch >= 4); }
+
+// The 14x14 stage's launches for n faces.  A few faces: a cluster each, while the device holds one for each.  More: a pair takes
+// two faces at a time through the stage, so whole rounds of two per pair go out as one launch, and what is left over in
+// clusters where it can, which is quicker than a round with one face per pair (149 / 160 / 300 faces: 1199 / 1245 / 2170 ->
+// 1174 / 1196 / 2110 us).
 static int launch_face_stage(ffcu_ctx* c, int n, int* launches)
 {
     int left = n % (2 * ffcu_face_pairs(c->face));
-    const ChainPlan* plan = nullptr;
-    if (left < n && left <= FFCU_CHAIN_MAX_FACES && !c->no_chain) {
-        if (!c->chains_built) build_chains(c);
-        const ffcu_ctx::Chain* ch = chain_at(c, c->face_first, left, &plan);
-        if (ch && ch->count != c->face_count) plan = nullptr;
+    const int tiles = c->no_clusters ? 0 : ffcu_stage_row_tiles(c->face, left);
+    if (!tiles) left = 0;
+    if (left < n) {
+        const int rc = ffcu_face_launch(c->face, 0, n - left, c->mode, c->d_err, c->stream);
+        (*launches)++;
+        if (rc != 0 || !left) return rc;
     }
-    if (!plan) left = 0;
-    int rc = ffcu_face_launch(c->face, 0, n - left, c->mode, c->d_err, c->stream);
     (*launches)++;
-    if (rc != 0 || !left) return rc;
-    (*launches)++;
-    if (ffcu_chain_launch(plan, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
-    cudaGetLastError();                                    // refused, as below
-    c->no_chain = 1;
+    if (ffcu_stage_launch(c->face, tiles, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
+    // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...): no more in this context
+    cudaGetLastError();
+    c->no_clusters = 1;
     return ffcu_face_launch(c->face, n - left, left, c->mode, c->d_err, c->stream);
 }
 
@@ -689,11 +686,17 @@ static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
     const bool chain_call = n <= chain_max_faces(c);
     if (chain_call && !c->chains_built) build_chains(c);
     for (size_t k = k0; k < k1; k++) {
+        if (face_takes(c, n) && k == c->face_first && k + (size_t)c->face_count <= k1) {
+            const int rc = launch_face_stage(c, n, &launches);
+            if (rc != 0) return rc;
+            k += (size_t)c->face_count - 1;
+            continue;
+        }
         if (chain_call && !c->no_chain) {
             const ChainPlan* plan = nullptr;
             const ffcu_ctx::Chain* ch = chain_at(c, k, n, &plan);
             if (ch) {
-                if (ffcu_chain_launch(plan, 0, n, c->mode, c->d_err, c->stream) == 0) {
+                if (ffcu_chain_launch(plan, n, c->mode, c->d_err, c->stream) == 0) {
                     launches++;
                     k += (size_t)ch->count - 1;
                     continue;
@@ -704,12 +707,6 @@ static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
                 cudaGetLastError();
                 c->no_chain = 1;
             }
-        }
-        if (c->face && k == c->face_first && n >= FACE_MIN_FACES && k + (size_t)c->face_count <= k1) {
-            const int rc = launch_face_stage(c, n, &launches);
-            if (rc != 0) return rc;
-            k += (size_t)c->face_count - 1;
-            continue;
         }
         {
             DevLayer& M = c->layers[k];
@@ -1078,7 +1075,7 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     std::vector<cudaEvent_t> ev(2 * nl);
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
     // the 14x14 stage as the forward runs it: the time of its one or two launches, shared equally among its layers
-    const bool face = c->face && n >= FACE_MIN_FACES && n > chain_max_faces(c);
+    const bool face = face_takes(c, n) && n > chain_max_faces(c);
     const int f0 = (int)c->face_first, f1 = f0 + c->face_count;
     for (int k = 0; k < nl && rc == 0; k++) {
         DevLayer& M = c->layers[k];

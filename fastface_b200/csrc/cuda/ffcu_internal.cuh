@@ -214,7 +214,7 @@ struct ChainLayerDesc { const int8_t* w; EpiTables t; const int8_t* res; int8_t*
 ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers);
 int        ffcu_chain_clusters(const ChainPlan* p);
 void       ffcu_chain_free(ChainPlan* p);
-int        ffcu_chain_launch(const ChainPlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s);
+int        ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s);
 // 14x14 stage (a run of 3x3 stride-1 256 -> 256 convolutions: PReLU layers, and residual + fused BN ones), a CTA pair per face.
 #define FFCU_FACE_C 256
 struct FacePlan;
@@ -227,6 +227,9 @@ struct FaceLayerDesc {
 FacePlan* ffcu_face_plan(int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers);
 void      ffcu_face_free(FacePlan* p);
 int       ffcu_face_pairs(const FacePlan* p);                             // pairs the device holds at once
+// Row tiles of the form with a cluster of two CTAs per row tile and face that the device holds `faces` clusters of (4 or 2; 0: none).
+int       ffcu_stage_row_tiles(const FacePlan* p, int faces);
+int       ffcu_stage_launch(const FacePlan* p, int row_tiles, int face0, int faces, int mode, int* d_err, cudaStream_t s);
 int       ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s);
 struct TcPlan;   // opaque: tile shape, TMA descriptors, launch geometry for one layer
 int ffcu_stem_weight_k32(const int8_t* d_w, int8_t* d_wk, int Cout, cudaStream_t s);
