@@ -777,60 +777,67 @@ int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaS
 }
 
 // ---------------------------------------------------------------------------
-// 14x14 stage, a CTA pair per face (conv_tc_face.cu)
+// Stages taken face by face: a cluster per face (conv_tc_stage.cu), the 14x14 one also with a CTA pair per two (conv_tc_face.cu)
 // ---------------------------------------------------------------------------
 struct FacePlan {
-    CUtensorMap mapA, mapA4;      // boxes of nine rows (a pair, two row tiles), of six (four row tiles)
+    CUtensorMap mapA[2], map_pair;      // boxes of the first input
     FaceLayer* d_layers;
     char* d_tables;          // every layer's constants and byte table
     int8_t* d_kept;
-    int n_layers, pairs;
-    int clusters4, clusters2;     // clusters of eight and of four the device holds at once (conv_tc_stage.cu)
+    int H, n_layers;
+    int pairs;               // CTA pairs the device holds at once (14x14)
+    StageForm form[2];
 };
 
-// layers[i]: device pointers of layer i; host[i]: its constants on the host ([4][256]: w_scale, bias, slope or residual scale,
-// inv_out) and its fused BN's table ([256][256], PReLU layers none).  d_in = the first layer's input.  NULL: not on this device.
-FacePlan* ffcu_face_plan(int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers)
+// layers[i]: device pointers of layer i, and on the host its constants ([4][C]: w_scale, bias, slope or residual scale,
+// inv_out) and its fused BN's table ([C][256], PReLU layers none).  d_in = the first layer's input.  NULL: not on this device.
+FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers)
 {
     encode_tiled_fn enc = get_encode();
-    const int pairs = tc_face_pairs();
-    if (!enc || pairs < 1 || n_layers < 1) return nullptr;
-    const size_t tab = FACE_C * sizeof(float4), lut = (size_t)FACE_C * 256;
+    if (!enc || n_layers < 1 || !((C == 128 && H == 28) || (C == FACE_C && H == 14) || (C == 512 && H == 7))) return nullptr;
+    FacePlan* p = new FacePlan();
+    p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->H = H; p->n_layers = n_layers;
+    p->pairs = H == 14 ? tc_face_pairs() : 0;
+    size_t kept = (size_t)p->pairs * 2 * FACE_KEPT_BYTES;
+    for (int i = 0; i < 2; i++) {
+        p->form[i] = tc_stage_form(H, i);
+        kept = std::max(kept, (size_t)p->form[i].clusters * p->form[i].kept_bytes);
+    }
+    if (H == 14 ? p->pairs < 1 : kept == 0) { delete p; return nullptr; }
+    const size_t tab = (size_t)C * sizeof(float4), lut = (size_t)C * 256;
     std::vector<char> t((size_t)n_layers * (tab + lut), 0);
     std::vector<FaceLayer> h((size_t)n_layers);
     memset(h.data(), 0, h.size() * sizeof(FaceLayer));
-    FacePlan* p = new FacePlan();
-    p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->n_layers = n_layers; p->pairs = pairs;
-    p->clusters4 = std::min(tc_stage_clusters(4), 2 * pairs); p->clusters2 = std::min(tc_stage_clusters(2), 2 * pairs);     // (d_kept)
     bool ok = cudaMalloc(&p->d_layers, h.size() * sizeof(FaceLayer)) == cudaSuccess && cudaMalloc(&p->d_tables, t.size()) == cudaSuccess &&
-              cudaMalloc(&p->d_kept, (size_t)pairs * 2 * FACE_KEPT_BYTES) == cudaSuccess;
+              cudaMalloc(&p->d_kept, kept) == cudaSuccess;
     cuuint32_t es[4] = {1, 1, 1, 1};
     {
-        cuuint64_t dims[4] = {FACE_C, 14, 14, (cuuint64_t)max_batch};
-        cuuint64_t strides[3] = {FACE_C, FACE_C * 14, FACE_C * 196};
-        for (CUtensorMap* m : {&p->mapA, &p->mapA4}) {
-            cuuint32_t box[4] = {128, 16, m == &p->mapA ? 9u : 6u, 1};
-            ok = ok && enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)H, (cuuint64_t)H, (cuuint64_t)max_batch};
+        cuuint64_t strides[3] = {(cuuint64_t)C, (cuuint64_t)C * H, (cuuint64_t)C * H * H};
+        for (int i = 0; i < 3; i++) {
+            cuuint32_t box[4] = {128, i < 2 ? (cuuint32_t)p->form[i].pitch : 16u, i < 2 ? (cuuint32_t)p->form[i].win_rows : 9u, 1};
+            ok = ok && enc(i < 2 ? &p->mapA[i] : &p->map_pair, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
         }
     }
     for (int i = 0; i < n_layers && ok; i++) {
         const FaceLayerDesc& d = layers[i];
-        const cuuint64_t K = 9 * FACE_C;
-        cuuint64_t dims[4] = {K, FACE_C, 1, 1};
-        cuuint64_t strides[3] = {K, K * FACE_C, K * FACE_C};
+        const cuuint64_t K = 9 * (cuuint64_t)C;
+        cuuint64_t dims[4] = {K, (cuuint64_t)C, 1, 1};
+        cuuint64_t strides[3] = {K, K * C, K * C};
         cuuint32_t box[4] = {128, 128, 1, 1};
         ok = enc(&h[i].mapB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
         const size_t o = (size_t)i * (tab + lut);
         float* ft = (float*)&t[o];
-        for (int c = 0; c < FACE_C; c++)
-            for (int k = 0; k < 4; k++) ft[4 * c + k] = d.tab[k * FACE_C + c];
+        for (int c = 0; c < C; c++)
+            for (int k = 0; k < 4; k++) ft[4 * c + k] = d.tab[k * C + c];
         h[i].tab = (const float4*)(p->d_tables + o);
         if (d.lut) {
-            // entry q of channel 128 * r + 32 * quarter + lane -> word 128 * (q / 4) + 32 * quarter + lane of CTA r's half, byte q % 4
+            // entry q of channel 128 * r + 32 * quarter + lane -> word 128 * (q / 4) + 32 * quarter + lane of channel tile r's 32 KB, byte q % 4
             char* lt = &t[o + tab];
-            for (int c = 0; c < FACE_C; c++)
+            for (int c = 0; c < C; c++)
                 for (int q = 0; q < 256; q++)
                     lt[(c / 128) * 32768 + (q >> 2) * 512 + (c % 128) * 4 + (q & 3)] = (char)d.lut[c * 256 + q];
             h[i].lut = (const uint8_t*)(p->d_tables + o + tab);
@@ -867,14 +874,18 @@ static FaceParams face_params(const FacePlan* p, int face0, int faces, int* d_er
 
 int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s)
 {
-    return tc_launch_face(mode, faces < p->pairs ? faces : p->pairs, s, p->mapA, face_params(p, face0, faces, d_err));
+    return tc_launch_face(mode, faces < p->pairs ? faces : p->pairs, s, p->map_pair, face_params(p, face0, faces, d_err));
 }
 
-int ffcu_stage_row_tiles(const FacePlan* p, int faces) { return faces <= p->clusters4 ? 4 : faces <= p->clusters2 ? 2 : 0; }
-
-int ffcu_stage_launch(const FacePlan* p, int row_tiles, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+int ffcu_stage_form(const FacePlan* p, int faces)
 {
-    return tc_launch_stage(row_tiles, mode, faces, s, row_tiles == 4 ? p->mapA4 : p->mapA, face_params(p, face0, faces, d_err));
+    for (int i = 0; i < 2; i++) if (faces <= p->form[i].clusters) return i;
+    return -1;
+}
+
+int ffcu_stage_launch(const FacePlan* p, int form, int face0, int faces, int mode, int* d_err, cudaStream_t s)
+{
+    return tc_launch_stage(p->H, form, mode, faces, s, p->mapA[form], face_params(p, face0, faces, d_err));
 }
 
 // ---------------------------------------------------------------------------

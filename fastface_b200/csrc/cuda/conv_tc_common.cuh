@@ -929,9 +929,9 @@ int tc_chain_clusters(int bn, int smem);
 #define FACE_KEPT_BYTES (28 * 8 * FACE_C)   // half rows of eight positions, as the epilogue's threads hold them
 #define FACE_STAGES 5                     // weight ring, 16 KB per CTA and stage
 struct FaceLayer {                        // one layer, in global memory
-    CUtensorMap mapB;                     // weights [256][9 * 256] K-major, box {128, 128}
+    CUtensorMap mapB;                     // weights [C][9 * C] K-major, box {128, 128}
     const float4* tab;                    // per channel: w_scale, bias, PReLU slope or residual scale, inv_out
-    const uint8_t* lut;                   // fused BN byte table as the kernel's look-ups want it [2][32 KB], or NULL (a PReLU layer)
+    const uint8_t* lut;                   // fused BN byte table as the kernel's look-ups want it [C / 128][32 KB], or NULL (a PReLU layer)
     const int8_t* res;                    // residual that another kernel left (NHWC); NULL: the result of the residual layer before
     int8_t* out; int8_t* out2;            // last layer: NHWC result and its fused BN
     uint8_t pad_[256 - 128 - 5 * 8];
@@ -948,9 +948,10 @@ struct FaceParams {
 int tc_face_smem_bytes();
 int tc_face_pairs();
 int tc_launch_face(int mode, int pairs, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
-// The same stage for a handful of faces, a cluster of two CTAs per row tile and face (conv_tc_stage.cu): four row tiles or two
-int tc_launch_stage(int row_tiles, int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
-int tc_stage_clusters(int row_tiles);
+// Stages of 28x28, 14x14 and 7x7 maps for a handful of faces, a cluster per face, in two forms (conv_tc_stage.cu)
+struct StageForm { int win_rows, pitch, kept_bytes, clusters; };      // box of the first input; FaceParams::kept per cluster; clusters the device holds
+StageForm tc_stage_form(int H, int i);
+int tc_launch_stage(int H, int i, int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
 
 // Flat-pitch weight-stationary pair kernel: activation buffer = guard + box of WSP_BOX_ROWS image rows
 #define WSP_GUARD_BYTES 1024

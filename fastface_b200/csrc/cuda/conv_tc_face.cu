@@ -51,18 +51,6 @@ struct FaceShared {
     int abort_flag;
 };
 
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, int (&v)[8])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait8(int (&v)[8])
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]) :: "memory");
-}
-
 // One thread of the epilogue: its channel and its warp's share of the rows.  Warps are (TMEM lane quarter q, group g); a
 // group takes two of the eight rows the other CTA reads, first, and three half rows of the six that only this CTA reads.
 struct FaceEpi {

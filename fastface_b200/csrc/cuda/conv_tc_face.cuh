@@ -9,6 +9,17 @@ __device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_add
 {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, int (&v)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait8(int (&v)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]) :: "memory");
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Shared memory of this CTA -> a CTA of the cluster, counted on that CTA's barrier (all shared::cluster addresses but `from`).
@@ -42,7 +53,7 @@ __device__ __forceinline__ uint32_t face_quad(const int* v, uint32_t rw, const f
     });
     return (uint32_t)ffcu_pack4(q[0], q[1], q[2], q[3]);
 }
-template <bool CONTRACT, bool RESBN, bool LAST, int C0, int C1, int ROW>
+template <bool CONTRACT, bool RESBN, bool LAST, int C0, int C1, int ROW, int W = 14, int C = FACE_C, int PITCH = 16>
 __device__ __forceinline__ void face_cols(const int* v, uint32_t* rw, const float4& k, const uint8_t* lut, uint32_t lut_lo,
                                           uint32_t lut_hi, const FaceDst& d)
 {
@@ -64,8 +75,8 @@ __device__ __forceinline__ void face_cols(const int* v, uint32_t* rw, const floa
     });
     TcUnroll<N>::run([&](auto ic) {
         constexpr int i = decltype(ic)::value, c = C0 + i;
-        if constexpr (LAST) d.g[(ROW * 14 + c) * FACE_C] = (int8_t)b[i];
-        else asm volatile("st.shared.u8 [%0 + %1], %2;" ::"r"(d.ad[(c + 1) & 7]), "n"(ROW * 2048 + (c + 1) * 128), "r"(b[i]));
+        if constexpr (LAST) d.g[(ROW * W + c) * C] = (int8_t)b[i];
+        else asm volatile("st.shared.u8 [%0 + %1], %2;" ::"r"(d.ad[(c + 1) & 7]), "n"(ROW * PITCH * 128 + (c + 1) * 128), "r"(b[i]));
     });
 }
 template <bool CONTRACT, bool RESBN, bool LAST, int ROW>

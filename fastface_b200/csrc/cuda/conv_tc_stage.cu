@@ -1,18 +1,27 @@
-// conv_tc_stage.cu -- small batches: the 14x14 stage (a run of 3x3 stride-1 256 -> 256 convolutions) in ONE launch, a cluster of
-// eight or four CTAs per face, activations in shared memory.
+// conv_tc_stage.cu -- small batches: a stage (a run of 3x3 stride-1 C -> C convolutions) in ONE launch, a cluster of four to eight
+// CTAs per face, activations in shared memory: 128 channels on 28x28 maps, 256 on 14x14, 512 on 7x7.
 //
-// The operands as in conv_tc_face.cu (weights are the MMA's 128 rows, a row of the face 16 of its columns), but every CTA issues
-// its own MMAs: a cluster is 2 halves of the output channels x R tiles of the face's rows (R = 4: 4, 4, 3 and 3 rows, 64 columns;
-// R = 2: 7 rows, 112 columns).  A CTA holds, for both halves' channels, its rows and one above and below, in two buffers that
-// take turns.  Its epilogue writes its 128 channels of its rows into its own next buffer, bytewise, and sends the rows from there by
-// bulk copies: all of them to the CTA with the other channels of the same rows, the first and the last to both CTAs of the
-// neighbouring rows.
+// The operands as in conv_tc_face.cu (weights are the MMA's 128 rows, a row of the face 8, 16 or 32 of its columns), but every
+// CTA issues its own MMAs: a cluster is C / 128 tiles of the output channels x R tiles of the face's rows, in two forms:
+//
+//     maps        few faces                                  while the device holds that many clusters
+//     28x28       R = 7, 4 rows, 128 columns; 7 CTAs         R = 4, 7 rows, 224 columns; 4 CTAs
+//     14x14       R = 4, 4 / 3 rows, 64 columns; 8 CTAs      R = 2, 7 rows, 112 columns; 4 CTAs
+//     7x7         R = 2, 4 / 3 rows, 32 columns; 8 CTAs      R = 1, 7 rows, 64 columns; 4 CTAs
+//
+// A CTA holds, for all channels, its rows and one above and below, in two buffers that take turns.  Its epilogue writes its 128
+// channels of its rows into its own next buffer, bytewise, and sends the rows from there by bulk copies: all of them to the CTAs
+// with the other channels of the same rows, the first and the last to the CTAs of the neighbouring rows.
 //
 // Bound: latency.  What passes between shared memories goes at 20 B per cycle and CTA whatever instruction sends it (measured:
-// 8 KB to 1 / 2 / 4 / 8 CTAs of a cluster of eight 710 / 1110 / 1920 / 3550 cycles by 16-byte st.async, 810 / 1210 / 2005 / 3790 by bulk copies), so the split
-// is the one that sends least: 16 KB per CTA and layer instead of 36 KB for 2 row tiles x 4 channel tiles (conv_tc_chain.cu).
-// Forward of 1 / 4 / 8 / 15 faces, that chain -> clusters of eight: 273 / 287 / 309 / 349 -> 230 / 249 / 267 / 304 us; of 16 / 17 / 24 / 33
-// faces, its wide form -> clusters of four: 409 / 413 / 445 / 487 -> 357 / 361 / 396 / 435 us (14x14 layers 5.1 -> 3.5 and 7 -> 5 us).
+// 8 KB to 1 / 2 / 4 / 8 CTAs of a cluster of eight 710 / 1110 / 1920 / 3550 cycles by 16-byte st.async, 810 / 1210 / 2005 / 3790 by
+// bulk copies), so the split is the one that sends least: at 14x14 16 KB per CTA and layer instead of 36 KB for 2 row tiles x 4
+// channel tiles (conv_tc_chain.cu).
+// Forward of 1 / 4 / 8 / 15 faces, 14x14 stage by that chain -> clusters of eight: 273 / 287 / 309 / 349 -> 230 / 249 / 267 / 304 us; of
+// 16 / 17 / 24 / 33 faces, its wide form -> clusters of four: 409 / 413 / 445 / 487 -> 357 / 361 / 396 / 435 us (layers 5.1 -> 3.5 and 7 -> 5 us).
+// The 28x28 stage by one launch per layer and the 7x7 one by that chain (from 25 faces a launch per layer): forward of 1 / 8 / 15 /
+// 17 / 33 faces 231 / 264 / 302 / 357 / 430 us; with the 28x28 stage here 219 / 250 / 283 / 345 / 408, with the 7x7 one 225 / 262 / 298 / 347 /
+// 420, with both 214 / 248 / 279 / 335 / 397.  Their second forms at 1 / 8 / 15 faces: 28x28 223 / 255 / 287, 7x7 219 / 255 / 286.
 //
 // Replaces, per layer, what conv_tc_kernel does (reference kernels/conv2d_nhwc.c:179-220, kernels/int8_epilogue.c:25-112,
 // :253-318); same arithmetic, same bytes.
@@ -20,26 +29,38 @@
 
 namespace {
 
-template <int R>
+// C channels on an H x H map, R row tiles; a cluster has C / 128 x R CTAs (rank = row tile * C / 128 + channel tile).
+template <int C_, int H_, int R_>
 struct Stage {
-    static constexpr int ROWS = R == 4 ? 4 : 7;              // rows of a tile (R = 4: the last two have three)
+    static constexpr int C = C_, H = H_, R = R_;
+    static constexpr int CT = C / 128;                       // channel tiles = planes of 128 input channels
+    static constexpr int CLUSTER = CT * R;
+    static constexpr int PITCH = H == 28 ? 32 : H == 14 ? 16 : 8;        // lines of a row: a zero line before it, zero or unread ones behind
+    static constexpr int ROW_BYTES = PITCH * 128;
+    static constexpr int ROWS = (H + R - 1) / R;             // rows of a tile; where R does not divide H the last tiles have one less
+    static constexpr int WIN = ROWS + 2 + (PITCH == H + 1 ? 1 : 0);      // (a row's last tap may read the line behind it: the next row's zero line)
     static constexpr int PER_GROUP = (ROWS + 3) / 4;         // rows of an epilogue group of four warps
-    static constexpr int N = ROWS * 16;
-    static constexpr int PLANE_BYTES = (ROWS + 2) * 2048;
-    static constexpr int ACT_BYTES = 2 * PLANE_BYTES;
-    static constexpr int STEP_BYTES = 2 * 128 * 128;         // one filter tap: 128 output channels x 256 input channels
-    static constexpr int STAGES = R == 4 ? 4 : 3;
+    static constexpr int N = (ROWS * PITCH + 15) / 16 * 16;
+    static constexpr int PLANE_BYTES = WIN * ROW_BYTES;
+    static constexpr int ACT_BYTES = CT * PLANE_BYTES;
+    static constexpr int PL_STEP = CT < 2 ? CT : 2;          // a step of the weight ring: this many planes of one filter tap
+    static constexpr int STEPS = 9 * (CT / PL_STEP);
+    static constexpr int STEP_BYTES = PL_STEP * 128 * 128;
     static constexpr int OFF_LUT = 2 * ACT_BYTES;
     static constexpr int OFF_RING = OFF_LUT + FACE_LUT_BYTES;
+    static constexpr int FIT = (232448 - 512 - OFF_RING) / STEP_BYTES;
+    static constexpr int STAGES = FIT < 8 ? FIT : 8;
     static constexpr int OFF_SH = OFF_RING + STAGES * STEP_BYTES;
-    static constexpr uint32_t TMEM_COLS = R == 4 ? 64 : 128;
-    static_assert(OFF_RING % 1024 == 0 && ACT_BYTES % 1024 == 0, "swizzle atoms");
-    __device__ static int first_row(int t) { return R == 4 ? (t < 2 ? 4 * t : 8 + 3 * (t - 2)) : 7 * t; }
-    __device__ static int rows(int t) { return R == 4 ? (t < 2 ? 4 : 3) : 7; }
+    static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+    static constexpr int WORDS = (H + 3) / 4;                // a row of a channel in packed bytes
+    static constexpr int KEPT_BYTES = H * WORDS * C * 4;     // [row][word][channel]: a warp's 32 channels together
+    static_assert(STAGES >= 3 && OFF_RING % 1024 == 0 && ACT_BYTES % 1024 == 0 && N <= 256, "layout");
+    __device__ static int rows(int t) { return H / R + (t < H % R ? 1 : 0); }
+    __device__ static int first_row(int t) { return t * (H / R) + (t < H % R ? t : H % R); }
 };
 
 struct StageShared {
-    uint64_t full[4], empty[4];
+    uint64_t full[8], empty[8];
     uint64_t a0_full;             // the first input has landed, and the padding's zeros in both buffers
     uint64_t act_full[2];         // buffer b holds the next layer's input: own rows (sixteen warps), and the bytes that come
     uint64_t acc_full;
@@ -49,20 +70,19 @@ struct StageShared {
 };
 
 // One layer.  RESBN: residual and fused BN (else PReLU); LAST: results go to global memory as NHWC.
-template <bool CONTRACT, int R, bool RESBN, bool LAST>
+template <bool CONTRACT, typename S, bool RESBN, bool LAST>
 __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, const FaceLayer* cl, const float4& k, int L, int rank, int q, int g,
                                                int lane, uint32_t lut_lo, uint32_t lut_hi, int face, int8_t* kept, uint32_t tmem_base,
                                                uint32_t lut_parity, volatile int* abort_flag, const FaceParams& p, bool& ok)
 {
-    using S = Stage<R>;
-    constexpr int PG = S::PER_GROUP;
-    const int h = rank & 1, t = rank >> 1, ch = q * 32 + lane;
+    constexpr int PG = S::PER_GROUP, H = S::H, W4 = S::WORDS, CHUNKS = (H + 7) / 8;
+    const int h = rank % S::CT, t = rank / S::CT, ch = q * 32 + lane;
     const int n_rows = S::rows(t), r0 = S::first_row(t);
     const int mine = n_rows - g * PG < PG ? n_rows - g * PG : PG;          // rows of this warp's group: r0 + g * PG ..  (may be <= 0)
-    const size_t px0 = ((size_t)face * 196 + (size_t)(r0 + g * PG) * 14) * FACE_C + h * 128 + ch;
-    uint32_t rw[4 * PG];
+    const size_t px0 = ((size_t)face * (H * H) + (size_t)(r0 + g * PG) * H) * S::C + h * 128 + ch;
+    uint32_t rw[W4 * PG];
 #pragma unroll
-    for (int i = 0; i < 4 * PG; i++) rw[i] = 0;
+    for (int i = 0; i < W4 * PG; i++) rw[i] = 0;
     if (RESBN && ok) {
         const int8_t* res = cl->res;
 #pragma unroll
@@ -70,23 +90,25 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
             if (r >= mine) break;
             if (res) {
 #pragma unroll
-                for (int c = 0; c < 14; c++) {
+                for (int c = 0; c < H; c++) {
                     uint32_t b;
-                    asm volatile("ld.global.u8 %0, [%1];" : "=r"(b) : "l"(res + px0 + (size_t)(r * 14 + c) * FACE_C));
-                    rw[4 * r + c / 4] |= b << (8 * (c & 3));
+                    asm volatile("ld.global.u8 %0, [%1];" : "=r"(b) : "l"(res + px0 + (size_t)(r * H + c) * S::C));
+                    rw[W4 * r + c / 4] |= b << (8 * (c & 3));
                 }
-            } else
-                asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(rw[4 * r]), "=r"(rw[4 * r + 1]), "=r"(rw[4 * r + 2]), "=r"(rw[4 * r + 3])
-                             : "l"(kept + r * (FACE_C * 16)));
+            } else {
+#pragma unroll
+                for (int i = 0; i < W4; i++)
+                    asm volatile("ld.global.b32 %0, [%1];" : "=r"(rw[W4 * r + i]) : "l"(kept + ((size_t)r * W4 + i) * (S::C * 4)));
+            }
         }
     }
     if (RESBN && ok) ok = mbar_wait(smem_u32(&sh->lut_full), lut_parity, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
     if (ok) ok = mbar_wait(smem_u32(&sh->acc_full), (uint32_t)L & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
     tc_fence_after();
     const uint8_t* lut = smem + S::OFF_LUT;
-    const uint32_t taddr = tmem_base + (uint32_t)(g * PG * 16) + ((uint32_t)(q * 32) << 16);
+    const uint32_t taddr = tmem_base + (uint32_t)(g * PG * S::PITCH) + ((uint32_t)(q * 32) << 16);
     const uint32_t s_plane = smem_u32(smem) + (uint32_t)(((L + 1) & 1) * S::ACT_BYTES + h * S::PLANE_BYTES);
-    const uint32_t s_rows = s_plane + (uint32_t)((g * PG + 1) * 2048);     // the group's rows in the next input
+    const uint32_t s_rows = s_plane + (uint32_t)((g * PG + 1) * S::ROW_BYTES);     // the group's rows in the next input
     if (ok && mine > 0) {
         FaceDst d;
         if (LAST) d.g = cl->out2 + px0;
@@ -94,17 +116,20 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
 #pragma unroll
             for (int i = 0; i < 8; i++) d.ad[i] = (s_rows + (uint32_t)ch) ^ (uint32_t)(i << 4);
         }
-        int va[16], vb[16];
-        tmem_ld16_issue(taddr, va);
-        tmem_ld_wait(va);
-        if (PG == 2 && mine > 1) tmem_ld16_issue(taddr + 16, vb);
-        face_cols<CONTRACT, RESBN, LAST, 0, 8, 0>(va, rw, k, lut, lut_lo, lut_hi, d);
-        face_cols<CONTRACT, RESBN, LAST, 8, 14, 0>(va + 8, rw + 2, k, lut, lut_lo, lut_hi, d);
-        if (PG == 2 && mine > 1) {
-            tmem_ld_wait(vb);
-            face_cols<CONTRACT, RESBN, LAST, 0, 8, 1>(vb, rw + (PG == 2 ? 4 : 0), k, lut, lut_lo, lut_hi, d);
-            face_cols<CONTRACT, RESBN, LAST, 8, 14, 1>(vb + 8, rw + (PG == 2 ? 6 : 0), k, lut, lut_lo, lut_hi, d);
-        }
+        // eight columns at a time, the next ones landing meanwhile
+        int va[8], vb[8];
+        tmem_ld8_issue(taddr, va);
+        TcUnroll<PG * CHUNKS>::run([&](auto uc) {
+            constexpr int u = decltype(uc)::value, r = u / CHUNKS, j = u % CHUNKS, n = u + 1;
+            constexpr int c0 = 8 * j, c1 = c0 + 8 < H ? c0 + 8 : H;
+            int (&v)[8] = u % 2 ? vb : va;
+            int (&w)[8] = u % 2 ? va : vb;
+            if (r < mine) {
+                tmem_ld_wait8(v);
+                if (n < PG * CHUNKS && n / CHUNKS < mine) tmem_ld8_issue(taddr + (uint32_t)(n / CHUNKS * S::PITCH + n % CHUNKS * 8), w);
+                face_cols<CONTRACT, RESBN, LAST, c0, c1, r, H, S::C, S::PITCH>(v, rw + W4 * r + 2 * j, k, lut, lut_lo, lut_hi, d);
+            }
+        });
     }
     if (!LAST) {
         // Every warp comes here whatever its ok flag: none may be left waiting.  (What the warps have read of the accumulator
@@ -114,28 +139,34 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
         __syncwarp();
         if (lane == 0 && ok) mbar_arrive(smem_u32(&sh->act_full[(L + 1) & 1]));
         asm volatile("bar.sync %0, 128;" ::"r"(2 + g) : "memory");
-        if (ok && lane == 0 && mine > 0) {
+        if (ok && mine > 0) {
             const uint32_t bar = smem_u32(&sh->act_full[(L + 1) & 1]);
-            if (q == 0) bulk_send(map_to_cta(s_rows, (uint32_t)rank ^ 1u), s_rows, (uint32_t)(mine * 2048), map_to_cta(bar, (uint32_t)rank ^ 1u));
-            else if (q < 3) {
-                // the first row is the row below the tile above's, the last one the row above the tile below's
-                const uint32_t other = q == 1 ? 0u : 1u;
-                if (g == 0 && t > 0) {
-                    const uint32_t to = ((uint32_t)rank - 2u) ^ other;
-                    bulk_send(map_to_cta(s_plane + (uint32_t)((S::rows(t - 1) + 1) * 2048), to), s_rows, 2048, map_to_cta(bar, to));
+            const uint32_t tile0 = (uint32_t)(t * S::CT);                  // rank of this row tile's first CTA
+            if (q == 0) {
+                // all rows: to the CTAs with the tile's other channels
+                if (lane < S::CT - 1) {
+                    const uint32_t to = tile0 + (uint32_t)((h + 1 + lane) % S::CT);
+                    bulk_send(map_to_cta(s_rows, to), s_rows, (uint32_t)(mine * S::ROW_BYTES), map_to_cta(bar, to));
                 }
-                if (g == (n_rows - 1) / PG && t < R - 1) {
-                    const uint32_t to = ((uint32_t)rank + 2u) ^ other;
-                    bulk_send(map_to_cta(s_plane, to), s_plane + (uint32_t)(n_rows * 2048), 2048, map_to_cta(bar, to));
+            } else if (q == 1) {
+                // the first row is the row below the tile above's
+                if (g == 0 && t > 0 && lane < S::CT) {
+                    const uint32_t to = tile0 - (uint32_t)(S::CT - lane);
+                    bulk_send(map_to_cta(s_plane + (uint32_t)((S::rows(t - 1) + 1) * S::ROW_BYTES), to), s_rows, S::ROW_BYTES, map_to_cta(bar, to));
+                }
+            } else if (q == 2) {
+                // the last one the row above the tile below's
+                if (g == (n_rows - 1) / PG && t < S::R - 1 && lane < S::CT) {
+                    const uint32_t to = tile0 + (uint32_t)(S::CT + lane);
+                    bulk_send(map_to_cta(s_plane, to), s_plane + (uint32_t)(n_rows * S::ROW_BYTES), S::ROW_BYTES, map_to_cta(bar, to));
                 }
             }
         }
     }
     if (ok && RESBN && !LAST) {
 #pragma unroll
-        for (int r = 0; r < PG; r++)
-            if (r < mine)
-                asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(kept + r * (FACE_C * 16)), "r"(rw[4 * r]), "r"(rw[4 * r + 1]), "r"(rw[4 * r + 2]), "r"(rw[4 * r + 3]) : "memory");
+        for (int i = 0; i < PG * W4; i++)
+            if (i / W4 < mine) asm volatile("st.global.b32 [%0], %1;" ::"l"(kept + (size_t)i * (S::C * 4)), "r"(rw[i]) : "memory");
     }
     if (ok && LAST) {
         int8_t* out = cl->out + px0;
@@ -143,16 +174,15 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
         for (int r = 0; r < PG; r++)
             if (r < mine) {
 #pragma unroll
-                for (int c = 0; c < 14; c++) out[(r * 14 + c) * FACE_C] = (int8_t)(rw[4 * r + c / 4] >> (8 * (c & 3)));
+                for (int c = 0; c < H; c++) out[(r * H + c) * S::C] = (int8_t)(rw[W4 * r + c / 4] >> (8 * (c & 3)));
             }
     }
 }
 
-template <bool CONTRACT, int R>
+template <bool CONTRACT, typename S>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
 {
-    using S = Stage<R>;
     extern __shared__ __align__(1024) uint8_t smem[];
     StageShared* sh = (StageShared*)(smem + S::OFF_SH);
     if (smem_u32(smem) & 1023) {                              // the swizzle atoms' alignment, as the declaration asks for it
@@ -162,8 +192,8 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
-    const int cluster = (int)blockIdx.x / (2 * R), face = p.face0 + cluster;
-    const int h = rank & 1, t = rank >> 1;
+    const int cluster = (int)blockIdx.x / S::CLUSTER, face = p.face0 + cluster;
+    const int h = rank % S::CT, t = rank / S::CT;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
@@ -190,22 +220,23 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     const uint32_t s0 = smem_u32(smem);
 
     if (warp == TC_PRODUCER_WARP) {
-        // Weight producer: a step is one filter tap, two boxes (lane i: input channels 128 i ..)
+        // Weight producer: a step is one or two planes of a filter tap, a box each (lane i: input channels 128 i .. of the step's)
         int stage = 0, gs = 0; uint32_t phase = 0;
         bool ok = true;
 #pragma unroll 1
         for (int L = 0; L < p.n_layers && ok; L++) {
             const CUtensorMap* map = &p.layers[L].mapB;
-            if (lane < 2) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+            if (lane < S::PL_STEP) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
 #pragma unroll 1
-            for (int tap = 0; tap < 9; tap++, gs++) {
+            for (int st = 0; st < S::STEPS; st++, gs++) {
                 ok = mbar_wait(smem_u32(&sh->empty[stage]), phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, p.wait_cycles);
                 if (!ok) break;
                 if (lane == 0) mbar_expect_tx(smem_u32(&sh->full[stage]), S::STEP_BYTES);
                 __syncwarp();
                 // (drop_step: the timeout test's launch, CTA 0 leaves out this step)
-                if (lane < 2 && (gs != p.drop_step || rank != 0))
-                    tma_load_4d(s0 + S::OFF_RING + stage * S::STEP_BYTES + lane * (128 * 128), map, smem_u32(&sh->full[stage]), tap * FACE_C + lane * 128, h * 128, 0, 0);
+                if (lane < S::PL_STEP && (gs != p.drop_step || rank != 0))
+                    tma_load_4d(s0 + S::OFF_RING + stage * S::STEP_BYTES + lane * (128 * 128), map, smem_u32(&sh->full[stage]),
+                                (st * S::PL_STEP + lane) * 128, h * 128, 0, 0);
                 if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -215,7 +246,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
             const uint64_t da0 = smem_desc<128>(s0 + S::OFF_RING);
             // what this CTA receives of each layer: its rows' other channels, and the rows above and below
-            const uint32_t in_bytes = (uint32_t)(S::rows(t) * 2048 + (t > 0 ? 4096 : 0) + (t < R - 1 ? 4096 : 0));
+            const uint32_t in_bytes = (uint32_t)(S::ROW_BYTES * ((S::CT - 1) * S::rows(t) + S::CT * ((t > 0) + (t < S::R - 1))));
             int stage = 0; uint32_t phase = 0, ready = 0;
             bool ok = true;
 #pragma unroll 1
@@ -230,9 +261,11 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                 uint64_t db_row = smem_desc<128>(s0 + (uint32_t)(buf * S::ACT_BYTES));
                 uint32_t first = 0;
 #pragma unroll 1
-                for (int kh = 0; kh < 3 && ok; kh++, db_row += 2048 / 16) {
+                for (int kh = 0; kh < 3 && ok; kh++, db_row += S::ROW_BYTES / 16) {
 #pragma unroll
-                    for (int kw = 0; kw < 3; kw++) {
+                    for (int kp = 0; kp < 3 * (S::CT / S::PL_STEP); kp++) {      // (kw, planes of the step)
+                        constexpr int PS = S::CT / S::PL_STEP;
+                        const int kw = kp / PS, pl0 = kp % PS * S::PL_STEP;
                         if (!ready) {
                             ok = mbar_wait(full0 + stage * 8, phase, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
                             if (!ok) break;
@@ -243,11 +276,11 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                         tc_fence_after();
                         const uint64_t da = da0 + (uint64_t)((uint32_t)(stage * S::STEP_BYTES) >> 4);
 #pragma unroll
-                        for (int pl = 0; pl < 2; pl++)
+                        for (int pl = 0; pl < S::PL_STEP; pl++)
 #pragma unroll
                             for (int k = 0; k < 4; k++)
-                                umma_i8(tmem_base, da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k), db_row + (uint64_t)(((kw * 128 + pl * S::PLANE_BYTES) >> 4) + 2 * k),
-                                        IDESC, (kw | pl | k) ? 1u : first);
+                                umma_i8(tmem_base, da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k),
+                                        db_row + (uint64_t)(((kw * 128 + (pl0 + pl) * S::PLANE_BYTES) >> 4) + 2 * k), IDESC, (kp | pl | k) ? 1u : first);
                         first = 1;
                         umma_commit(empty0 + stage * 8);
                         stage = ns; phase = np;
@@ -262,8 +295,8 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             tc_pdl_wait();
             mbar_expect_tx(smem_u32(&sh->a0_full), 2 * S::ACT_BYTES);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                tma_load_4d(s0 + i * S::PLANE_BYTES, &mapA, smem_u32(&sh->a0_full), (i & 1) * 128, -1, S::first_row(t) - 1, face);
+            for (int i = 0; i < 2 * S::CT; i++)
+                tma_load_4d(s0 + i * S::PLANE_BYTES, &mapA, smem_u32(&sh->a0_full), i % S::CT * 128, -1, S::first_row(t) - 1, face);
             uint32_t lut_par = 0;
             bool ok = true;
 #pragma unroll 1
@@ -282,8 +315,8 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     } else {
         const int q = warp & 3, g = warp >> 2;
         const uint32_t lut_lo = (uint32_t)(lane * 4 + (q & 1) * 128) * 0x01010101u, lut_hi = (uint32_t)(q >> 1) * 0x01010101u;
-        // a result that the next residual layer adds lies as its thread left it: a row of a channel in 16 bytes
-        int8_t* kept = p.kept + (size_t)cluster * FACE_KEPT_BYTES + ((size_t)(S::first_row(t) + g * S::PER_GROUP) * FACE_C + h * 128 + q * 32 + lane) * 16;
+        // a result that the next residual layer adds lies as its thread left it
+        int8_t* kept = p.kept + (size_t)cluster * S::KEPT_BYTES + ((size_t)(S::first_row(t) + g * S::PER_GROUP) * S::WORDS * S::C + h * 128 + q * 32 + lane) * 4;
         uint32_t lut_par = 0;
         bool ok = true;
         tc_pdl_wait();
@@ -295,9 +328,9 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             const bool last = L + 1 == p.n_layers;
             // (the next kernel not before: its CTAs would keep other contexts' kernels off the SMs this launch leaves free)
             if (last && warp == 0) tc_pdl_trigger();
-            if (last)    stage_epilogue<CONTRACT, R, true, true>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else if (bn) stage_epilogue<CONTRACT, R, true, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else         stage_epilogue<CONTRACT, R, false, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
+            if (last)    stage_epilogue<CONTRACT, S, true, true>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
+            else if (bn) stage_epilogue<CONTRACT, S, true, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
+            else         stage_epilogue<CONTRACT, S, false, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
             if (bn) {
                 lut_par ^= 1;
                 __syncwarp();
@@ -320,53 +353,64 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     }
 }
 
-template <int R>
-constexpr int smem_bytes() { return Stage<R>::OFF_SH + (int)sizeof(StageShared); }
+template <typename S>
+constexpr int smem_bytes() { return S::OFF_SH + (int)sizeof(StageShared); }
 
-template <bool CONTRACT, int R>
+template <bool CONTRACT, typename S>
 int set_smem()
 {
     static int done[64] = {};             // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
     FFCU_CHECK(cudaGetDevice(&dev));
     if (!done[dev & 63]) {
-        FFCU_CHECK(cudaFuncSetAttribute(conv_stage_kernel<CONTRACT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<R>()));
+        FFCU_CHECK(cudaFuncSetAttribute(conv_stage_kernel<CONTRACT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<S>()));
         done[dev & 63] = 1;
     }
     return 0;
 }
 
-template <bool CONTRACT, int R>
-int launch_stage(int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm)
+template <typename S>
+int launch(int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm)
 {
-    const int rc = set_smem<CONTRACT, R>();
-    return rc != 0 ? rc : tc_launch_ex(conv_stage_kernel<CONTRACT, R>, 2 * R * faces, smem_bytes<R>(), s, 2 * R, mapA, prm);
+    const int rc = mode ? set_smem<true, S>() : set_smem<false, S>();
+    if (rc != 0) return rc;
+    return mode ? tc_launch_ex(conv_stage_kernel<true, S>, S::CLUSTER * faces, smem_bytes<S>(), s, S::CLUSTER, mapA, prm)
+                : tc_launch_ex(conv_stage_kernel<false, S>, S::CLUSTER * faces, smem_bytes<S>(), s, S::CLUSTER, mapA, prm);
 }
 
-template <int R>
-int stage_clusters()
+template <typename S>
+StageForm form()
 {
-    if (set_smem<true, R>() != 0 || set_smem<false, R>() != 0) { cudaGetLastError(); return 0; }
+    StageForm f = {S::WIN, S::PITCH, S::KEPT_BYTES, 0};
+    if (set_smem<true, S>() != 0 || set_smem<false, S>() != 0) { cudaGetLastError(); return f; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * R);
+    cfg.gridDim = dim3(S::CLUSTER);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = smem_bytes<R>();
+    cfg.dynamicSmemBytes = smem_bytes<S>();
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2 * R; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = S::CLUSTER; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, conv_stage_kernel<true, R>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return n;
+    if (cudaOccupancyMaxActiveClusters(&n, conv_stage_kernel<true, S>, &cfg) != cudaSuccess) { cudaGetLastError(); return f; }
+    f.clusters = n;
+    return f;
+}
+
+// calls fn with the form of the stage of H x H maps: 0, more and smaller tiles (few faces), or 1
+template <typename F>
+auto with_form(int H, int i, F&& fn)
+{
+    if (H == 28) return i == 0 ? fn(Stage<128, 28, 7>{}) : fn(Stage<128, 28, 4>{});
+    if (H == 7) return i == 0 ? fn(Stage<512, 7, 2>{}) : fn(Stage<512, 7, 1>{});
+    return i == 0 ? fn(Stage<256, 14, 4>{}) : fn(Stage<256, 14, 2>{});
 }
 
 }  // namespace
 
-int tc_launch_stage(int row_tiles, int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm)
-{
-    if (row_tiles == 4) return mode ? launch_stage<true, 4>(faces, s, mapA, prm) : launch_stage<false, 4>(faces, s, mapA, prm);
-    return mode ? launch_stage<true, 2>(faces, s, mapA, prm) : launch_stage<false, 2>(faces, s, mapA, prm);
-}
+StageForm tc_stage_form(int H, int i) { return with_form(H, i, [](auto s) { return form<decltype(s)>(); }); }
 
-// How many clusters (two CTAs per row tile) the device holds at once.
-int tc_stage_clusters(int row_tiles) { return row_tiles == 4 ? stage_clusters<4>() : stage_clusters<2>(); }
+int tc_launch_stage(int H, int i, int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm)
+{
+    return with_form(H, i, [&](auto st) { return launch<decltype(st)>(mode, faces, s, mapA, prm); });
+}

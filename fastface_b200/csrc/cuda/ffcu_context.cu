@@ -116,11 +116,11 @@ struct ffcu_ctx {
     std::vector<Chain> chains;
     bool chains_built = false;
     int no_chain = 0;
-    // The 14x14 stage as one launch, a cluster (conv_tc_stage.cu) or a CTA pair (conv_tc_face.cu) per face; FF_FACE=0 disables.
-    FacePlan* face = nullptr;
-    size_t face_first = 0;
-    int no_clusters = 0;         // a cluster launch of it was refused
-    int face_count = 0;
+    // The 28x28, 14x14 and 7x7 stages as one launch each, a cluster per face (conv_tc_stage.cu), beyond what the device holds
+    // clusters for a CTA pair per two faces of the 14x14 one (conv_tc_face.cu); FF_FACE=0 disables.
+    struct FaceRun { size_t first; int count, H; FacePlan* plan; };
+    std::vector<FaceRun> runs;
+    int no_clusters = 0;         // a cluster launch was refused
     // A whole call that is one step of fewer than CHUNK_MIN_FACES faces, and any submit of at most lean_max_batch
     // (FF_LEAN_MAX_BATCH, default 1), runs copy-in, forward and copy-out on the compute stream alone: it has nothing to overlap and
     // is spared the pipeline's two cross-stream hops.  Other submits go through the three-stream pipeline, where the next step's
@@ -241,7 +241,7 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
     for (int k = 0; k < 2 && done; k++) deliver(c, k);    // outputs nobody has waited for
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
     for (auto& ch : c->chains) for (ChainPlan* q : ch.plan) ffcu_chain_free(q);
-    ffcu_face_free(c->face);
+    for (auto& run : c->runs) ffcu_face_free(run.plan);
     for (auto& L : c->layers) {
         for (TcPlan* q : L.tc_bn) if (q) ffcu_tc_free(q);      // L.tc is one of them
         if (L.stem_tc) ffcu_stem_tc_free(L.stem_tc);
@@ -423,33 +423,34 @@ static size_t chain_end(const ffcu_ctx* c, size_t k)
     return e;
 }
 
-// The 14x14 stage as one launch (conv_tc_face.cu), which leaves only the last layer's tensors in memory (ff_plan_stage).
-static void build_face(ffcu_ctx* c)
+// The stages that go face by face, which leaves only their last layers' tensors in memory (ff_plan_stage).
+static void build_face_runs(ffcu_ctx* c)
 {
     const char* e = getenv("FF_FACE");
     if (c->no_chain || (e && e[0] == '0')) return;
     std::vector<ffcu_layer> d;
-    for (size_t k = 0; k < c->layers.size(); k++) d.push_back(c->layers[k].d);
-    for (size_t k = 0; k < d.size(); ) {
-        const size_t end = chain_end(c, k);
-        if (end < k + 2 || d[k].H != 14 || d[k].Cout != FFCU_FACE_C) { k = end > k ? end : k + 1; continue; }
+    for (const DevLayer& L : c->layers) d.push_back(L.d);
+    size_t end;
+    for (size_t k = 0; k < d.size(); k = end > k ? end : k + 1) {
+        end = chain_end(c, k);
+        if (end < k + 2) continue;
         const int n = (int)(end - k);
+        const size_t C = (size_t)d[k].Cout;
         std::vector<int> from((size_t)n);
-        if (!ff_plan_stage(d.data(), (int)d.size(), (int)k, n, from.data())) return;
+        if (!ff_plan_stage(d.data(), (int)d.size(), (int)k, n, from.data())) continue;
         std::vector<FaceLayerDesc> desc((size_t)n);
-        std::vector<std::vector<float>> tab((size_t)n, std::vector<float>(4 * FFCU_FACE_C));
+        std::vector<std::vector<float>> tab((size_t)n, std::vector<float>(4 * C));
         std::vector<std::vector<int8_t>> lut((size_t)n);
-        for (int i = 0; i < n; i++) {
+        bool ok = true;
+        for (int i = 0; i < n && ok; i++) {
             const DevLayer& L = c->layers[k + i];
             const bool res = L.d.res_buf >= 0 && L.epi.res_scale, slope = L.epi.slope != nullptr, bn = L.d.bn2_dst_buf >= 0;
-            if (!(slope && !res && !bn) && !(res && bn && !slope)) return;
-            if (i == n - 1 && !bn) return;
+            ok = ((slope && !res && !bn) || (res && bn && !slope)) && (bn || i < n - 1);
             const float* src[4] = {L.epi.w_scale, L.epi.bias, slope ? L.epi.slope : L.epi.res_scale, L.epi.inv_out};
-            for (int t = 0; t < 4; t++)
-                if (cudaMemcpy(&tab[i][(size_t)t * FFCU_FACE_C], src[t], FFCU_FACE_C * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return; }
-            if (bn) {
-                lut[i].resize(FFCU_FACE_C * 256);
-                if (cudaMemcpy(lut[i].data(), L.bn_lut, lut[i].size(), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return; }
+            for (int t = 0; t < 4 && ok; t++) ok = cudaMemcpy(&tab[i][t * C], src[t], C * sizeof(float), cudaMemcpyDeviceToHost) == cudaSuccess;
+            if (bn && ok) {
+                lut[i].resize(C * 256);
+                ok = cudaMemcpy(lut[i].data(), L.bn_lut, lut[i].size(), cudaMemcpyDeviceToHost) == cudaSuccess;
             }
             FaceLayerDesc& f = desc[i];
             f = {};
@@ -457,9 +458,9 @@ static void build_face(ffcu_ctx* c)
             f.res = res && from[i] < 0 ? c->bufs[L.d.res_buf] : nullptr;
             f.out = c->bufs[L.d.dst_buf]; f.out2 = bn ? c->bufs[L.d.bn2_dst_buf] : nullptr;
         }
-        c->face = ffcu_face_plan(c->max_batch, c->bufs[d[k].src_buf], desc.data(), n);
-        c->face_first = k; c->face_count = n;
-        return;
+        if (!ok) { cudaGetLastError(); continue; }
+        FacePlan* plan = ffcu_face_plan((int)C, d[k].H, c->max_batch, c->bufs[d[k].src_buf], desc.data(), n);
+        if (plan) c->runs.push_back({k, n, d[k].H, plan});
     }
 }
 
@@ -525,7 +526,7 @@ extern "C" int ffcu_finalize(ffcu_ctx* c)
     c->launches = 0;
     for (auto& L : c->layers) if (!L.skip) c->launches++;
     find_heads(c);
-    build_face(c);
+    build_face_runs(c);
     c->finalized = true;
     return 0;
 }
@@ -654,29 +655,43 @@ static const ffcu_ctx::Chain* chain_at(const ffcu_ctx* c, size_t k, int n, const
     return nullptr;
 }
 
-// (A context made for two or three faces keeps one launch per layer beyond a single face: chain_max_faces.)
-static bool face_takes(const ffcu_ctx* c, int n) { return c->face && (n == 1 || c->max_batch >= 4); }
-
-// The 14x14 stage's launches for n faces.  A few faces: a cluster each, while the device holds one for each.  More: a pair takes
-// two faces at a time through the stage, so whole rounds of two per pair go out as one launch, and what is left over in
-// clusters where it can, which is quicker than a round with one face per pair (149 / 160 / 300 faces: 1199 / 1245 / 2170 ->
-// 1174 / 1196 / 2110 us).
-static int launch_face_stage(ffcu_ctx* c, int n, int* launches)
+// The run of layers that starts at k and that a call of n faces takes face by face; NULL: none.  28x28 and 7x7 maps only while the
+// device holds a cluster for each: in rounds they lose to one launch per layer, as every CTA brings in all of its weights
+// (forward of 64 / 148 / 256 faces: 604 / 978 / 1655 us; 28x28 stage in rounds 599 / 1015 / 1718, 7x7 608 / 1051 / 1790).
+// A context made for two or three faces keeps one launch per layer beyond a single face (chain_max_faces), one for up to four
+// also on 28x28 maps: callers count a single face's 22 launches there (tests/test_gpu_parity.py).
+static const ffcu_ctx::FaceRun* run_at(const ffcu_ctx* c, size_t k, int n)
 {
-    int left = n % (2 * ffcu_face_pairs(c->face));
-    const int tiles = c->no_clusters ? 0 : ffcu_stage_row_tiles(c->face, left);
-    if (!tiles) left = 0;
+    for (const ffcu_ctx::FaceRun& r : c->runs) {
+        if (r.first != k) continue;
+        if (c->max_batch < 4 ? n > 1 || r.H == 28 : c->max_batch == 4 && r.H == 28) return nullptr;
+        return r.H == 14 || (!c->no_clusters && ffcu_stage_form(r.plan, n) >= 0) ? &r : nullptr;
+    }
+    return nullptr;
+}
+
+// Its launches; 1: refused, and not to be tried again.  A few faces: a cluster each, while the device holds one for each.  More
+// (14x14): a pair takes two faces at a time through the stage, so whole rounds of two per pair go out as one launch, and what
+// is left over in clusters where it can, which is quicker than a round with one face per pair (149 / 160 / 300 faces: 1199 /
+// 1245 / 2170 -> 1174 / 1196 / 2110 us).
+static int launch_run(ffcu_ctx* c, const ffcu_ctx::FaceRun& run, int n, int* launches)
+{
+    int left = run.H == 14 ? n % (2 * ffcu_face_pairs(run.plan)) : n;
+    const int form = c->no_clusters ? -1 : ffcu_stage_form(run.plan, left);
+    if (form < 0) left = 0;
     if (left < n) {
-        const int rc = ffcu_face_launch(c->face, 0, n - left, c->mode, c->d_err, c->stream);
+        const int rc = ffcu_face_launch(run.plan, 0, n - left, c->mode, c->d_err, c->stream);
         (*launches)++;
         if (rc != 0 || !left) return rc;
     }
     (*launches)++;
-    if (ffcu_stage_launch(c->face, tiles, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
+    if (ffcu_stage_launch(run.plan, form, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
     // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...): no more in this context
     cudaGetLastError();
     c->no_clusters = 1;
-    return ffcu_face_launch(c->face, n - left, left, c->mode, c->d_err, c->stream);
+    if (run.H == 14) return ffcu_face_launch(run.plan, n - left, left, c->mode, c->d_err, c->stream);
+    (*launches)--;
+    return 1;
 }
 
 // Layers [k0, k1) for faces b0 .. b0 + n - 1 (b0 > 0 within a head only); c->launches = the launches made.
@@ -686,11 +701,10 @@ static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
     const bool chain_call = n <= chain_max_faces(c);
     if (chain_call && !c->chains_built) build_chains(c);
     for (size_t k = k0; k < k1; k++) {
-        if (face_takes(c, n) && k == c->face_first && k + (size_t)c->face_count <= k1) {
-            const int rc = launch_face_stage(c, n, &launches);
-            if (rc != 0) return rc;
-            k += (size_t)c->face_count - 1;
-            continue;
+        if (const ffcu_ctx::FaceRun* run = run_at(c, k, n)) {
+            const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, &launches) : 1;
+            if (rc < 0) return rc;
+            if (rc == 0) { k += (size_t)run->count - 1; continue; }
         }
         if (chain_call && !c->no_chain) {
             const ChainPlan* plan = nullptr;
@@ -1074,15 +1088,16 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     if (rc != 0) return rc;
     std::vector<cudaEvent_t> ev(2 * nl);
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
-    // the 14x14 stage as the forward runs it: the time of its one or two launches, shared equally among its layers
-    const bool face = face_takes(c, n) && n > chain_max_faces(c);
-    const int f0 = (int)c->face_first, f1 = f0 + c->face_count;
+    // the 14x14 stage beyond the clusters' reach as the forward runs it: the time of its one or two launches, shared equally among its layers
+    const ffcu_ctx::FaceRun* face = nullptr;
+    for (const ffcu_ctx::FaceRun& r : c->runs) if (n > chain_max_faces(c) && run_at(c, r.first, n) == &r) face = &r;
+    const int f0 = face ? (int)face->first : nl, f1 = face ? f0 + face->count : nl;
     for (int k = 0; k < nl && rc == 0; k++) {
         DevLayer& M = c->layers[k];
-        if (face && k >= f0 && k < f1) {
+        if (k >= f0 && k < f1) {
             int launched = 0;
             FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
-            if (k == f0) for (int it = 0; it < iters && rc == 0; it++) rc = launch_face_stage(c, n, &launched);
+            if (k == f0) for (int it = 0; it < iters && rc == 0; it++) rc = launch_run(c, *face, n, &launched);
             FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
             continue;
         }
@@ -1107,7 +1122,7 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     int wrc = ffcu_wait(c);
     if (rc == 0) rc = wrc;
     for (int k = 0; k < nl && rc == 0; k++) FFCU_CHECK(cudaEventElapsedTime(&ms[k], ev[2 * k], ev[2 * k + 1]));
-    if (face && rc == 0) for (int k = f1 - 1; k >= f0; k--) ms[k] = ms[f0] / (float)c->face_count;
+    if (face && rc == 0) for (int k = f1 - 1; k >= f0; k--) ms[k] = ms[f0] / (float)face->count;
     for (auto& e : ev) cudaEventDestroy(e);
     return rc == 0 ? nl : rc;
 }

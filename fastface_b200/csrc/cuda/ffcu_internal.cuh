@@ -215,21 +215,23 @@ ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int
 int        ffcu_chain_clusters(const ChainPlan* p);
 void       ffcu_chain_free(ChainPlan* p);
 int        ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s);
-// 14x14 stage (a run of 3x3 stride-1 256 -> 256 convolutions: PReLU layers, and residual + fused BN ones), a CTA pair per face.
+// A stage (a run of 3x3 stride-1 C -> C convolutions: PReLU layers, and residual + fused BN ones) taken face by face: 128 channels on
+// 28x28 maps, 256 on 14x14, 512 on 7x7.
 #define FFCU_FACE_C 256
 struct FacePlan;
 struct FaceLayerDesc {
     const int8_t* w;                          // device
-    const float* tab; const int8_t* lut;      // host: [4][256], [256][256] or NULL
+    const float* tab; const int8_t* lut;      // host: [4][C], [C][256] or NULL
     const int8_t* res;                        // residual from outside; NULL in a layer with `lut`: the result of the one before it
     int8_t* out; int8_t* out2;                // result and its fused BN: stored for the last layer
 };
-FacePlan* ffcu_face_plan(int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers);
+FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers);
 void      ffcu_face_free(FacePlan* p);
-int       ffcu_face_pairs(const FacePlan* p);                             // pairs the device holds at once
-// Row tiles of the form with a cluster of two CTAs per row tile and face that the device holds `faces` clusters of (4 or 2; 0: none).
-int       ffcu_stage_row_tiles(const FacePlan* p, int faces);
-int       ffcu_stage_launch(const FacePlan* p, int row_tiles, int face0, int faces, int mode, int* d_err, cudaStream_t s);
+// With a cluster per face: the form (0, 1) the device holds `faces` clusters of, more and smaller tiles first; -1: none.
+int       ffcu_stage_form(const FacePlan* p, int faces);
+int       ffcu_stage_launch(const FacePlan* p, int form, int face0, int faces, int mode, int* d_err, cudaStream_t s);
+// 14x14, any number of faces, a CTA pair for two; pairs the device holds at once.
+int       ffcu_face_pairs(const FacePlan* p);
 int       ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_err, cudaStream_t s);
 struct TcPlan;   // opaque: tile shape, TMA descriptors, launch geometry for one layer
 int ffcu_stem_weight_k32(const int8_t* d_w, int8_t* d_wk, int Cout, cudaStream_t s);

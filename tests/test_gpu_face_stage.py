@@ -1,4 +1,5 @@
-"""The 14x14 stage as one launch with a CTA pair per face: same bytes as one launch per layer, and as the oracle."""
+"""Stages as one launch, the 14x14 one with a CTA pair per face, 28x28, 14x14 and 7x7 with a cluster per face: same bytes as one launch
+per layer, and as the oracle."""
 import ctypes as C
 
 import numpy as np
@@ -32,6 +33,31 @@ def test_stage_in_one_launch(built_lib, model_root, ffw4, oracle, monkeypatch, n
             bad = np.flatnonzero((got["1", mode, rep] != got["0", mode, 0]).any(axis=1))
             assert bad.size == 0, f"mode {mode} rep {rep}: faces {bad[:16].tolist()}"
         assert np.array_equal(got["1", mode, 0][sample], oracle.forward(faces[sample], mode))
+
+
+@pytest.mark.parametrize("max_batch,n", [(1, 1), (3, 1), (3, 2), (4, 4), (5, 1), (5, 5), (40, 2), (40, 14), (40, 15), (40, 16), (40, 17), (40, 20), (40, 21),
+                                         (40, 32), (40, 33), (40, 34)])
+def test_stages_in_clusters(built_lib, model_root, ffw4, oracle, monkeypatch, max_batch, n):
+    """A cluster per face, its two forms' last faces on a B200 and one more: eager, captured and replayed, both epilogue orders,
+    against one launch per layer (exact, as above)."""
+    faces = synth.faces(n, seed=900 + n)
+    got, launches = {}, {}
+    for flag in ("1", "0"):
+        monkeypatch.setenv("FF_FACE", flag)
+        monkeypatch.setenv("FF_CHAIN", flag)
+        with ff.FastFace(ffw4, cwd=model_root, max_batch=max_batch) as e:
+            for mode in (ffo.CONTRACT, ffo.STRICT):
+                e.set_epilogue_mode(mode)
+                for rep in range(3 if flag == "1" else 1):
+                    got[flag, mode, rep] = e.embed_batch(faces)
+            launches[flag] = e.launches_per_forward
+    # one launch for the 6 + 26 + 4 layers of the three stages
+    if max_batch > 4 and n <= 32:
+        assert launches["0"] - launches["1"] == 5 + 25 + 3, launches
+    for mode in (ffo.CONTRACT, ffo.STRICT):
+        for rep in range(3):
+            assert np.array_equal(got["1", mode, rep], got["0", mode, 0]), (mode, rep)
+        assert np.array_equal(got["1", mode, 0][[0, n - 1]], oracle.forward(faces[[0, n - 1]], mode))
 
 
 @pytest.mark.parametrize("n", [40, 80], ids=["one-face-a-pair", "two-faces-a-pair"])
