@@ -316,7 +316,7 @@ extern "C" void ffcu_test_arm_fc_timeout(int drop_step, long long wait_cycles)
 }
 
 // The FC as a split-K GEMM (conv_tc_fc.cu): `scratch` = tiles' tickets (FFCU_FC_TC_TICKETS ints) followed by
-// [rows][N] int32 sums, all zero between calls.  Returns 1 when this plan / batch does not take that kernel
+// int32 sums, 512 per face, all zero between calls.  Returns 1 when this plan / batch does not take that kernel
 // (the caller then launches the one-CTA-per-tile form), 0 on success, < 0 on error.
 int ffcu_fc_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, float* out, int* scratch, int scratch_rows,
                       int* d_err, cudaStream_t s)
@@ -327,17 +327,20 @@ int ffcu_fc_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t,
     if (!on || !scratch || !p->out_f32 || p->BN != 64 || p->KC != 128 || p->pair || p->ws || p->wsp) return 1;
     const ffcu_layer& d = p->d;
     const int kblocks = d.Cin_pad / 128;
-    const int tiles_n = d.Cout / 64, tiles_m = (batch + TC_TILE_M - 1) / TC_TILE_M;
-    if (batch < 1 || batch > p->max_batch || d.Cin_pad % 128 != 0 || tiles_m * TC_TILE_M > scratch_rows ||
+    // tiles of 128 outputs x equally many faces, at most 256
+    const int tiles_n = d.Cout / 128, tiles_m = (batch + 255) / 256;
+    const int n_cols = ((batch + tiles_m - 1) / tiles_m + 15) / 16 * 16;
+    if (batch < 1 || batch > p->max_batch || d.Cin_pad % 128 != 0 || d.Cout % 128 != 0 || batch > scratch_rows ||
         tiles_m * tiles_n > FFCU_FC_TC_TICKETS) return 1;
-    // K ranges: the most that divide the K loop, leave two K blocks per CTA and keep the grid within the SMs
+    // K ranges: the most that divide the K loop, leave two K blocks per CTA and keep the grid within the SMs (7 / 14 / 28 / 49 ranges: 64
+    // faces 13.1 / 9.6 / 8.3 / 13.3 us, 256 23.6 / 18.8 / 16.9 / 25.3, 1024 28.6 / 38.3 / 55.3 / 73.7)
     int splits = 1;
     for (int sp = 2; sp <= kblocks / 2; sp++)
         if (kblocks % sp == 0 && tiles_n * tiles_m * sp <= p->n_sm) splits = sp;
     { const char* e = getenv("FF_FC_SPLITS"); const int v = e ? atoi(e) : 0; if (v >= 1 && v <= kblocks / 2 && kblocks % v == 0) splits = v; }
     const int bps = kblocks / splits;
     if (d.Wo != 1 || d.Ho != 1 || d.W != 1 || d.H != 1) return 1;
-    const int TW = 1, TH = 1, TB = TC_TILE_M;              // a row tile = 128 consecutive faces
+    const int TW = 1, TH = 1, TB = n_cols;                 // a tile = consecutive faces
     TcGeom* g = nullptr;
     for (int i = 0; i < p->n_geoms; i++)
         if (p->geoms[i].TW == TW && p->geoms[i].TH == TH && p->geoms[i].TB == TB) g = &p->geoms[i];
@@ -353,20 +356,19 @@ int ffcu_fc_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t,
     prm.tickets = scratch; prm.sums = scratch + FFCU_FC_TC_TICKETS; prm.err = d_err;
     prm.batch = batch; prm.N = d.Cout;
     prm.tiles_n = tiles_n; prm.tiles_m = tiles_m; prm.splits = splits; prm.blocks_per_split = bps;
-    prm.group = (bps % 2 == 0) ? 2 : 1;
-    const int sub = (TC_TILE_M + 64) * 128;
-    int st = (232448 - (int)sizeof(TcShared) - 2048) / (prm.group * sub);
+    const int sub = (128 + n_cols) * 128, room = 232448 - (int)sizeof(TcShared) - 2048;
+    int st = room / sub;
     if (st > TC_MAX_STAGES) st = TC_MAX_STAGES;
-    if (st > bps / prm.group) st = bps / prm.group;
-    if (st < 1) return 1;
-    prm.stages = st;
+    if (st > bps) st = bps;
+    prm.n_cols = n_cols; prm.stages = st;
+    prm.ring_bytes = std::max(st * sub, n_cols * 128 * (int)sizeof(int));      // the partial sums take the ring's place
     prm.drop_step = -1; prm.wait_cycles = TC_WAIT_CYCLES;
     if (g_test_fc_drop_step >= 0) {                          // armed for this one launch by the timeout test
         prm.drop_step = g_test_fc_drop_step;
         if (g_test_fc_wait > 0) prm.wait_cycles = g_test_fc_wait;
         g_test_fc_drop_step = -1; g_test_fc_wait = 0;
     }
-    const int smem = st * prm.group * sub + (int)sizeof(TcShared) + 2048;
+    const int smem = prm.ring_bytes + (int)sizeof(TcShared) + 2048;
     return tc_launch_fc(mode, tiles_n * tiles_m * splits, smem, s, g->mapA, p->mapB, prm);
 }
 

@@ -99,7 +99,7 @@ struct ffcu_ctx {
     int mode = 1;
     int force_simt = 0;          // FF_CONV_IMPL=simt: every conv on the CUDA-core kernel
     int no_fc_small = 0;         // FF_FC_SMALL=0: small batches take the large-batch FC path too
-    int fc_small_max = 4;        // largest batch the CUDA-core FC kernel takes ($FF_FC_SMALL_MAX, at most 16): measured quicker than the split-K tensor-core FC up to 3 faces, equal at 4, slower from 6
+    int fc_small_max = 2;        // largest batch the CUDA-core FC kernel takes ($FF_FC_SMALL_MAX, at most 16); against the split-K tensor-core FC, 1 / 2 / 3 / 4 faces: 5.3 / 6.3 / 8.3 / 9.4 us, 6.3 each
     int* d_fc_tc_scratch = nullptr; // split-K tensor-core FC: FFCU_FC_TC_TICKETS counters + int32 [fc_tc_rows][512] sums (kept zero between calls)
     int fc_tc_rows = 0;
     int launches = 0;

@@ -1,0 +1,38 @@
+"""The split-K FC at the edges of its tiles: 128 outputs x up to 256 faces, faces in steps of 16."""
+import numpy as np
+import pytest
+
+import fastface_b200 as ff
+from fastface_b200 import synth
+from oracle import ffo
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [3, 4, 15, 16, 17, 47, 49, 112, 113, 240, 241, 256, 257, 272, 273, 289, 511, 512, 513, 529]
+
+
+@pytest.fixture(scope="module")
+def want(built_lib, model_root, ffw4):
+    """Two faces at a time: the CUDA-core FC.  Both forms add the same integers, so the comparison is exact."""
+    faces = synth.faces(max(SIZES), seed=73)
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=2) as e:
+        out = {}
+        for mode in (ffo.CONTRACT, ffo.STRICT):
+            e.set_epilogue_mode(mode)
+            out[mode] = e.embed_batch(faces)
+    return faces, out
+
+
+@pytest.mark.parametrize("room", [0, 100], ids=["full-context", "larger-context"])
+def test_tiles_of_faces(built_lib, model_root, ffw4, want, room):
+    """Whole and ragged tiles, one to three of them, calls in between that leave other faces in the buffers; twice each, so that
+    sums and tickets are seen to be left clean."""
+    faces, ref = want
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=max(SIZES) + room) as e:
+        for n in SIZES + SIZES[::-1]:
+            mode = (ffo.CONTRACT, ffo.STRICT)[n & 1]
+            e.set_epilogue_mode(mode)
+            for start in (0, max(SIZES) - n):
+                got = e.embed_batch(faces[start:start + n])
+                bad = np.flatnonzero((got != ref[mode][start:start + n]).any(axis=1))
+                assert bad.size == 0, f"{n} faces from {start}, mode {mode}: {bad[:8].tolist()} differ"
