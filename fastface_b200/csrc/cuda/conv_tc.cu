@@ -497,6 +497,7 @@ struct ScPlan {
     TcGeom geoms2[8];        // shortcut input boxes per tile geometry
     int n_geoms2;
     int kb_sc, stages, group, smem_bytes, lut_bytes;
+    int no_split;            // 1: a cluster launch was refused
 };
 
 static bool encode_A2(ScPlan* sp, TcGeom* g)
@@ -533,7 +534,7 @@ ScPlan* ffcu_sc_plan(const ffcu_layer& main, const ffcu_layer& sc, int max_batch
     TcPlan* mp = ffcu_tc_plan(main, max_batch, d_in_main, d_w_main, device, 64);
     if (!mp) return nullptr;
     ScPlan* sp = new ScPlan();
-    sp->main = mp; sp->d2 = sc; sp->d_in2 = d_in_sc; sp->n_geoms2 = 0;
+    sp->main = mp; sp->d2 = sc; sp->d_in2 = d_in_sc; sp->n_geoms2 = 0; sp->no_split = 0;
     const int KC = mp->KC;
     sp->kb_sc = (sc.Cin_pad + KC - 1) / KC;
     sp->lut_bytes = sc.bn2_dst_buf >= 0 ? 64 * 256 : 0;
@@ -622,7 +623,19 @@ int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, 
     ScParams q = {};
     q.t2 = t2; q.out_sc = out_sc; q.out2_sc = (out2_sc && t2.bn_lut && sp->lut_bytes) ? out2_sc : nullptr;
     q.kb_sc = sp->kb_sc; q.write_main = (write_main && out_main) ? 1 : 0; q.lut_bytes = q.out2_sc ? sp->lut_bytes : 0;
-    return tc_launch_sc(p->KC, mode, grid, sp->smem_bytes, s, g->mapA, p->mapB, g2->mapA, sp->mapB2, prm, q);
+    // Two CTAs per tile while the device has the SMs for them and each gets two steps of the K loop (conv_tc_sc.cu)
+    const int steps = prm.taps * prm.cin_blocks / prm.group, stage_bytes = prm.group * (128 + 64) * p->KC;
+    if (2 * prm.total_tiles <= p->n_sm && steps >= 4 && p->KC == 128 && !sp->no_split) {
+        TcParams half = prm;
+        half.stages = std::min(prm.stages, (steps + 1) / 2 + 1);
+        int smem = sp->smem_bytes - (prm.stages - half.stages) * stage_bytes + SC_RECV_BYTES(2);
+        for (; smem > 232448 && half.stages > 2; smem -= stage_bytes) half.stages--;
+        if (smem <= 232448 &&
+            tc_launch_sc(p->KC, mode, 2, prm.total_tiles, smem, s, g->mapA, p->mapB, g2->mapA, sp->mapB2, half, q) == 0) return 0;
+        cudaGetLastError();              // no clusters of two here and now: not again with this plan
+        sp->no_split = 1;
+    }
+    return tc_launch_sc(p->KC, mode, 1, grid, sp->smem_bytes, s, g->mapA, p->mapB, g2->mapA, sp->mapB2, prm, q);
 }
 
 // ---------------------------------------------------------------------------

@@ -867,7 +867,8 @@ struct ScParams {
     int write_main;          // 1: the main path's int8 output is stored too (TcParams::out): another layer reads it
     int lut_bytes;           // 64 * 256 when out2_sc comes through the byte table, else 0
 };
-int tc_launch_sc(int kc, int mode, int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB,
+#define SC_RECV_BYTES(S) (((S) - 1) * (4 / (S)) * 128 * 64)      // what a CTA gets from the others of its cluster
+int tc_launch_sc(int kc, int mode, int split, int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB,
                  const CUtensorMap& mapA2, const CUtensorMap& mapB2, const TcParams& prm, const ScParams& q);
 
 // Split-K FC (conv_tc_fc.cu)

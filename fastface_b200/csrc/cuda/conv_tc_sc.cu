@@ -10,6 +10,13 @@
 // layer reads it.  Used where the call's column tile is 64 channels wide: every down-sampling block at small batch
 // (a launch less per block: ~4 us of a 300 us forward each), the 112x112 one at any batch.
 //
+// At small batch a handful of tiles has a long K loop (7x7 maps: 36 K blocks, 885 KB through each of eight SMs for one face).  Where
+// the device holds two CTAs for each tile, a cluster of two shares it: each takes half of the main path's K loop and the whole
+// shortcut, sends its sums of the other's 32 columns into that one's shared memory and finishes its own.  512 channels, 1 / 8 / 17
+// faces: 12.0 / 12.3 / 12.4 -> 8.8 / 9.2 / 9.8 us, 256 channels 8.6 / 9.0 / 8.8 -> 6.9 / 7.3 / 8.8; forward of 1 / 3 / 8 / 12 / 17 faces 216.2 / 225.0 /
+// 245.7 / 262.3 / 327.6 -> 205.2 / 211.3 / 236.0 / 257.0 / 325.6 us.  Four CTAs a tile: 512 channels 7.1 / 8.1 us at 1 / 8 faces, but the forward
+// 205.8 / 236.4.
+//
 // Structure and bounded waits as conv_tc_kernel (conv_tc_generic.cu); 64-column tiles, four tile slots of two
 // accumulators in the 512 TMEM columns.
 #include "conv_tc_common.cuh"
@@ -29,7 +36,57 @@ __device__ __forceinline__ void sc_load_tables(float* tab, const EpiTables& t, i
     }
 }
 
-template <int KC, bool CONTRACT>
+// Sixteen channels of one pixel: main path's and shortcut's accumulators -> the block's output and its fused BN.
+template <bool CONTRACT>
+__device__ __forceinline__ void sc_finish16(const TcParams& p, const ScParams& q, const int (&va)[16], const int (&vb)[16], const float* tab1, const float* tab2,
+                                            uint32_t lut, bool has_slope1, bool has_slope2, bool has_bn2, bool valid, size_t o)
+{
+    int wm[4], wo[4], wo2[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        const float* t1 = tab1 + 4 * g;
+        const float* t2 = tab2 + 4 * g;
+        const float4 ws1 = *(const float4*)(t1), bi1 = *(const float4*)(t1 + TC_MAX_COUT), sl1 = *(const float4*)(t1 + 2 * TC_MAX_COUT);
+        const float4 iv1 = *(const float4*)(t1 + 4 * TC_MAX_COUT);
+        const float4 ws2 = *(const float4*)(t2), bi2 = *(const float4*)(t2 + TC_MAX_COUT), sl2 = *(const float4*)(t2 + 2 * TC_MAX_COUT);
+        const float4 rs2 = *(const float4*)(t2 + 3 * TC_MAX_COUT), iv2 = *(const float4*)(t2 + 4 * TC_MAX_COUT);
+        // the main path's int8 output, exactly as its own launch would have stored it
+        const float m0 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 0]), ws1.x, bi1.x, false, 0.0f, 0.0f, has_slope1, sl1.x);
+        const float m1 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 1]), ws1.y, bi1.y, false, 0.0f, 0.0f, has_slope1, sl1.y);
+        const float m2 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 2]), ws1.z, bi1.z, false, 0.0f, 0.0f, has_slope1, sl1.z);
+        const float m3 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 3]), ws1.w, bi1.w, false, 0.0f, 0.0f, has_slope1, sl1.w);
+        const int w1 = ffcu_pack4(ffcu_requant_nosat<false>(m0, iv1.x), ffcu_requant_nosat<false>(m1, iv1.y),
+                                  ffcu_requant_nosat<false>(m2, iv1.z), ffcu_requant_nosat<false>(m3, iv1.w));
+        wm[g] = w1;
+        // ... is the shortcut's residual
+        const uint32_t rx = (uint32_t)w1 ^ 0x80808080u;
+        const float f0 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 0]), ws2.x, bi2.x, true, ffcu_byte2f<0>(rx), rs2.x, has_slope2, sl2.x);
+        const float f1 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 1]), ws2.y, bi2.y, true, ffcu_byte2f<1>(rx), rs2.y, has_slope2, sl2.y);
+        const float f2 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 2]), ws2.z, bi2.z, true, ffcu_byte2f<2>(rx), rs2.z, has_slope2, sl2.z);
+        const float f3 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 3]), ws2.w, bi2.w, true, ffcu_byte2f<3>(rx), rs2.w, has_slope2, sl2.w);
+        const int w = ffcu_pack4(ffcu_requant_nosat<false>(f0, iv2.x), ffcu_requant_nosat<false>(f1, iv2.y),
+                                 ffcu_requant_nosat<false>(f2, iv2.z), ffcu_requant_nosat<false>(f3, iv2.w));
+        wo[g] = w;
+        wo2[g] = 0;
+        if (has_bn2) {
+            const uint32_t rowa = lut + (uint32_t)(4 * g) * 256u;
+            uint32_t b0, b1, b2, b3;
+            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b0) : "r"(rowa + ((uint32_t)w & 0xffu)));
+            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b1) : "r"(rowa + 256u + (((uint32_t)w >> 8) & 0xffu)));
+            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b2) : "r"(rowa + 512u + (((uint32_t)w >> 16) & 0xffu)));
+            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b3) : "r"(rowa + 768u + ((uint32_t)w >> 24)));
+            wo2[g] = (int)(b0 | (b1 << 8) | (b2 << 16) | (b3 << 24));
+        }
+    }
+    if (valid) {
+        if (q.write_main) *(int4*)((int8_t*)p.out + o) = make_int4(wm[0], wm[1], wm[2], wm[3]);
+        *(int4*)(q.out_sc + o) = make_int4(wo[0], wo[1], wo[2], wo[3]);
+        if (has_bn2) *(int4*)(q.out2_sc + o) = make_int4(wo2[0], wo2[1], wo2[2], wo2[3]);
+    }
+}
+
+// S > 1: a cluster of S CTAs shares a tile's K loop, its launch has one tile per cluster.
+template <int KC, bool CONTRACT, int S>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                const __grid_constant__ CUtensorMap mapA2, const __grid_constant__ CUtensorMap mapB2,
@@ -48,16 +105,20 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     float* tab1 = (float*)(smem + (size_t)p.stages * p.group * SUB_BYTES);     // main path: [5][TC_MAX_COUT]
     float* tab2 = tab1 + 5 * TC_MAX_COUT;                                       // shortcut:  [5][TC_MAX_COUT]
     uint8_t* lut = (uint8_t*)(tab2 + 5 * TC_MAX_COUT);                          // [64][256] fused-BN table of the block's output
-    TcShared* sh = (TcShared*)(lut + q.lut_bytes);
+    uint8_t* recv = lut + q.lut_bytes;          // S > 1: partial sums of this CTA's columns [other CTA][16 columns][four of them][row] from the others
+    TcShared* sh = (TcShared*)(recv + (S > 1 ? SC_RECV_BYTES(S) : 0));
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int kblocks = p.taps * p.cin_blocks;
     const int G = p.group;
-    const int n_steps = kblocks / G;
-    const int tn = blockIdx.x % p.tiles_n;
+    const int rank = S > 1 ? (int)cluster_ctarank() : 0;
+    const int step0 = kblocks / G * rank / S, n_steps = kblocks / G * (rank + 1) / S - step0;      // this CTA's part of the main path's K loop
+    const int tile0 = (int)blockIdx.x / S, tile_step = (int)gridDim.x / S;
+    const int tn = tile0 % p.tiles_n;
 
     tc_setup(sh, p.stages, TMEM_COLS, warp, p.epi_wps);
+    if (S > 1) cluster_sync_all();                          // the others have started: their memory may be written
     const uint32_t tmem_base = sh->tmem_base;
     volatile int* abort_flag = &sh->abort_flag;
     const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
@@ -74,12 +135,12 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const CUtensorMap* map = is_a ? &mapA : &mapB;
         const CUtensorMap* map2 = is_a ? &mapA2 : &mapB2;
         const uint32_t smem0 = smem_u32(smem) + (uint32_t)(g * SUB_BYTES) + (is_a ? 0u : (uint32_t)A_BYTES);
-        int c0_first = g * KC, kw_first = 0, kh_first = 0;
+        int c0_first = (step0 * G + g) * KC, kw_first = 0, kh_first = 0;
         while (c0_first >= p.Cp) { c0_first -= p.Cp; if (++kw_first == p.Kw) { kw_first = 0; kh_first++; } }
         tc_pdl_wait();
         TileWalk wk;
-        walk_init(wk, p, blockIdx.x / p.tiles_n, gridDim.x / p.tiles_n);
-        for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x, walk_next(wk, p)) {
+        walk_init(wk, p, tile0 / p.tiles_n, tile_step / p.tiles_n);
+        for (int tile = tile0; tile < p.total_tiles && ok; tile += tile_step, walk_next(wk, p)) {
             const int tw = wk.tw, th = wk.th, tb = wk.tb;
             const int x0 = tw * p.TW * p.stride - p.pad;
             const int y0 = th * p.TH * p.stride - p.pad;
@@ -117,7 +178,7 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const uint64_t da0 = smem_desc<KC>(smem_u32(smem));
         const uint64_t db0 = smem_desc<KC>(smem_u32(smem) + A_BYTES);
         uint32_t ready = 0;
-        for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+        for (int tile = tile0; tile < p.total_tiles && ok; tile += tile_step) {
             ok = mbar_wait(smem_u32(&sh->acc_empty[ts]), tphase ^ 1, abort_flag, p.err, FFCU_ERR_TMEM_TIMEOUT);
             if (!ok) break;
             tc_fence_after();
@@ -162,7 +223,7 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         asm volatile("bar.sync 1, 512;" ::: "memory");
         bool ok = !q.lut_bytes || mbar_wait(smem_u32(&sh->lut_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT);
         tc_pdl_wait();
-        const int wps = p.epi_wps;
+        const int wps = S > 1 ? 16 : p.epi_wps;
         const int sets = TC_EPI_TOTAL_WARPS / wps;
         const int cols = BN / (wps >> 2);
         const int n_chunks = cols >> 4;
@@ -180,9 +241,48 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         // this set's tiles: set, set + sets, ... of the CTA's; tile slot and phase follow the CTA's tile count
         int local = set;
         TileWalk wk;
-        walk_init(wk, p, (int)(blockIdx.x + set * gridDim.x) / p.tiles_n, (int)(gridDim.x * sets) / p.tiles_n);
-        for (int tile = blockIdx.x + set * gridDim.x; tile < p.total_tiles && ok;
-             tile += gridDim.x * sets, local += sets, walk_next(wk, p)) {
+        walk_init(wk, p, (tile0 + set * tile_step) / p.tiles_n, tile_step * sets / p.tiles_n);
+        if constexpr (S > 1) {
+            // Sixteen warps, sixteen columns each: those of another CTA's share are sent there, its own are finished when the
+            // others' sums are here.
+            const int ow = wk.tw * p.TW + iw, oh = wk.th * p.TH + ih, b = wk.tb * p.TB + ib;
+            const bool valid = (ow < p.Wo) && (oh < p.Ho) && (b < p.batch);
+            const size_t o0 = (((size_t)b * p.Ho + oh) * p.Wo + ow) * p.Cout + c0;
+            const int owner = cg * S / 4, part = cg % (4 / S);
+            const uint32_t taddr = tmem_base + (uint32_t)(cg * 16) + ((uint32_t)(qd * 32) << 16);
+            ok = ok && mbar_wait(smem_u32(&sh->acc_full[0]), 0, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT);
+            int va[16], vb[16];
+            if (ok) {
+                tc_fence_after();
+                tmem_ld16_issue(taddr, va);
+                tmem_ld16_issue(taddr + BN, vb);
+                tmem_ld_wait(va);
+                tmem_ld_wait(vb);
+                if (owner != rank && valid) {
+                    const uint32_t to = map_to_cta(smem_u32(recv) + (uint32_t)((((rank - owner + S - 1) % S * (4 / S) + part) * 4 * 128 + row) * 16), (uint32_t)owner);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(to + (uint32_t)(j * 128 * 16)), "r"(va[4 * j]), "r"(va[4 * j + 1]), "r"(va[4 * j + 2]), "r"(va[4 * j + 3]) : "memory");
+                }
+            }
+            __syncwarp();
+            cluster_sync_all();
+            if (ok && owner == rank) {
+#pragma unroll
+                for (int m = 0; m < S - 1; m++) {
+                    const int4* from = (const int4*)recv + (m * (4 / S) + part) * 4 * 128 + row;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const int4 x = from[j * 128];
+                        va[4 * j] += x.x; va[4 * j + 1] += x.y; va[4 * j + 2] += x.z; va[4 * j + 3] += x.w;
+                    }
+                }
+                sc_finish16<CONTRACT>(p, q, va, vb, tab1 + c0, tab2 + c0, lut0, has_slope1, has_slope2, has_bn2, valid, o0);
+            }
+        } else
+        for (int tile = tile0 + set * tile_step; tile < p.total_tiles && ok;
+             tile += tile_step * sets, local += sets, walk_next(wk, p)) {
             const int ow = wk.tw * p.TW + iw, oh = wk.th * p.TH + ih, b = wk.tb * p.TB + ib;
             const bool valid = (ow < p.Wo) && (oh < p.Ho) && (b < p.batch);
             const size_t o0 = (((size_t)b * p.Ho + oh) * p.Wo + ow) * p.Cout + c0;
@@ -200,63 +300,25 @@ conv_sc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 tmem_ld_wait(va);
                 tmem_ld_wait(vb);
                 const int cb = c0 + 16 * ch;
-                int wm[4], wo[4], wo2[4];
-#pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    const float* t1 = tab1 + cb + 4 * g;
-                    const float* t2 = tab2 + cb + 4 * g;
-                    const float4 ws1 = *(const float4*)(t1), bi1 = *(const float4*)(t1 + TC_MAX_COUT), sl1 = *(const float4*)(t1 + 2 * TC_MAX_COUT);
-                    const float4 iv1 = *(const float4*)(t1 + 4 * TC_MAX_COUT);
-                    const float4 ws2 = *(const float4*)(t2), bi2 = *(const float4*)(t2 + TC_MAX_COUT), sl2 = *(const float4*)(t2 + 2 * TC_MAX_COUT);
-                    const float4 rs2 = *(const float4*)(t2 + 3 * TC_MAX_COUT), iv2 = *(const float4*)(t2 + 4 * TC_MAX_COUT);
-                    // the main path's int8 output, exactly as its own launch would have stored it
-                    const float m0 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 0]), ws1.x, bi1.x, false, 0.0f, 0.0f, has_slope1, sl1.x);
-                    const float m1 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 1]), ws1.y, bi1.y, false, 0.0f, 0.0f, has_slope1, sl1.y);
-                    const float m2 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 2]), ws1.z, bi1.z, false, 0.0f, 0.0f, has_slope1, sl1.z);
-                    const float m3 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(va[4 * g + 3]), ws1.w, bi1.w, false, 0.0f, 0.0f, has_slope1, sl1.w);
-                    const int w1 = ffcu_pack4(ffcu_requant_nosat<false>(m0, iv1.x), ffcu_requant_nosat<false>(m1, iv1.y),
-                                              ffcu_requant_nosat<false>(m2, iv1.z), ffcu_requant_nosat<false>(m3, iv1.w));
-                    wm[g] = w1;
-                    // ... is the shortcut's residual
-                    const uint32_t rx = (uint32_t)w1 ^ 0x80808080u;
-                    const float f0 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 0]), ws2.x, bi2.x, true, ffcu_byte2f<0>(rx), rs2.x, has_slope2, sl2.x);
-                    const float f1 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 1]), ws2.y, bi2.y, true, ffcu_byte2f<1>(rx), rs2.y, has_slope2, sl2.y);
-                    const float f2 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 2]), ws2.z, bi2.z, true, ffcu_byte2f<2>(rx), rs2.z, has_slope2, sl2.z);
-                    const float f3 = ffcu_conv_fp_f<CONTRACT>(__int2float_rn(vb[4 * g + 3]), ws2.w, bi2.w, true, ffcu_byte2f<3>(rx), rs2.w, has_slope2, sl2.w);
-                    const int w = ffcu_pack4(ffcu_requant_nosat<false>(f0, iv2.x), ffcu_requant_nosat<false>(f1, iv2.y),
-                                             ffcu_requant_nosat<false>(f2, iv2.z), ffcu_requant_nosat<false>(f3, iv2.w));
-                    wo[g] = w;
-                    wo2[g] = 0;
-                    if (has_bn2) {
-                        const uint32_t rowa = lut0 + (uint32_t)(16 * ch + 4 * g) * 256u;
-                        uint32_t b0, b1, b2, b3;
-                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b0) : "r"(rowa + ((uint32_t)w & 0xffu)));
-                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b1) : "r"(rowa + 256u + (((uint32_t)w >> 8) & 0xffu)));
-                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b2) : "r"(rowa + 512u + (((uint32_t)w >> 16) & 0xffu)));
-                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b3) : "r"(rowa + 768u + ((uint32_t)w >> 24)));
-                        wo2[g] = (int)(b0 | (b1 << 8) | (b2 << 16) | (b3 << 24));
-                    }
-                }
-                if (valid) {
-                    const size_t o = o0 + 16 * ch;
-                    if (q.write_main) *(int4*)((int8_t*)p.out + o) = make_int4(wm[0], wm[1], wm[2], wm[3]);
-                    *(int4*)(q.out_sc + o) = make_int4(wo[0], wo[1], wo[2], wo[3]);
-                    if (has_bn2) *(int4*)(q.out2_sc + o) = make_int4(wo2[0], wo2[1], wo2[2], wo2[3]);
-                }
+                sc_finish16<CONTRACT>(p, q, va, vb, tab1 + cb, tab2 + cb, lut0 + (uint32_t)(16 * ch) * 256u, has_slope1, has_slope2, has_bn2, valid, o0 + 16 * ch);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_relaxed(smem_u32(&sh->acc_empty[ts]));
         }
     }
+    if (S > 1 && warp >= TC_EPI_TOTAL_WARPS) {
+        __syncwarp();
+        cluster_sync_all();                                 // (the epilogue's warps: above)
+    }
     tc_teardown(abort_flag, tmem_base, TMEM_COLS, warp);
 }
 
-template <int KC, bool CONTRACT>
+template <int KC, bool CONTRACT, int S>
 static int launch_sc(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB,
                      const CUtensorMap& mapA2, const CUtensorMap& mapB2, const TcParams& prm, const ScParams& q)
 {
-    auto kern = conv_sc_kernel<KC, CONTRACT>;
+    auto kern = conv_sc_kernel<KC, CONTRACT, S>;
     static int smem_set[64] = {};      // per device: the attribute belongs to the device's copy of the function
     int dev = 0;
     FFCU_CHECK(cudaGetDevice(&dev));
@@ -264,14 +326,16 @@ static int launch_sc(int grid, int smem, cudaStream_t s, const CUtensorMap& mapA
         FFCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         smem_set[dev & 63] = smem;
     }
-    return tc_launch_ex(kern, grid, smem, s, 1, mapA, mapB, mapA2, mapB2, prm, q);
+    return tc_launch_ex(kern, S * grid, smem, s, S, mapA, mapB, mapA2, mapB2, prm, q);
 }
 
-int tc_launch_sc(int kc, int mode, int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB,
+int tc_launch_sc(int kc, int mode, int split, int grid, int smem, cudaStream_t s, const CUtensorMap& mapA, const CUtensorMap& mapB,
                  const CUtensorMap& mapA2, const CUtensorMap& mapB2, const TcParams& prm, const ScParams& q)
 {
-    if (kc == 128) return mode ? launch_sc<128, true>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q)
-                               : launch_sc<128, false>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q);
-    return mode ? launch_sc<64, true>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q)
-                : launch_sc<64, false>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q);
+    if (kc == 128 && split == 2) return mode ? launch_sc<128, true, 2>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q)
+                                             : launch_sc<128, false, 2>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q);
+    if (kc == 128) return mode ? launch_sc<128, true, 1>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q)
+                               : launch_sc<128, false, 1>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q);
+    return mode ? launch_sc<64, true, 1>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q)
+                : launch_sc<64, false, 1>(grid, smem, s, mapA, mapB, mapA2, mapB2, prm, q);
 }

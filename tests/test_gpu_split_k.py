@@ -1,4 +1,5 @@
-"""The split-K FC at the edges of its tiles: 128 outputs x up to 256 faces, faces in steps of 16."""
+"""Kernels whose K loop several CTAs share: the FC at the edges of its tiles (128 outputs x up to 256 faces, faces in steps of 16),
+and the stride-2 convolutions of small batches."""
 import numpy as np
 import pytest
 
@@ -36,3 +37,22 @@ def test_tiles_of_faces(built_lib, model_root, ffw4, want, room):
                 got = e.embed_batch(faces[start:start + n])
                 bad = np.flatnonzero((got != ref[mode][start:start + n]).any(axis=1))
                 assert bad.size == 0, f"{n} faces from {start}, mode {mode}: {bad[:8].tolist()} differ"
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 7, 13, 18, 19, 20])
+def test_stride2_pairs_of_ctas(built_lib, model_root, ffw4, oracle, monkeypatch, n):
+    """A stride-2 convolution and its shortcut by two CTAs per tile, up to the last batch at which the device holds both (on a B200 18
+    faces on 14 x 14 -> 7 x 7 maps) and beyond, against two launches with whole K loops (exact: sums of integers)."""
+    faces = synth.faces(n, seed=90 + n)
+    got = {}
+    for flag in ("1", "0"):
+        monkeypatch.setenv("FF_FUSE_SC", flag)
+        with ff.FastFace(ffw4, cwd=model_root, max_batch=n) as e:
+            for mode in (ffo.CONTRACT, ffo.STRICT):
+                e.set_epilogue_mode(mode)
+                for rep in range(3 if flag == "1" else 1):
+                    got[flag, mode, rep] = e.embed_batch(faces)
+    for mode in (ffo.CONTRACT, ffo.STRICT):
+        for rep in range(3):
+            assert np.array_equal(got["1", mode, rep], got["0", mode, 0]), (mode, rep)
+        assert np.array_equal(got["1", mode, 0][[0, n - 1]], oracle.forward(faces[[0, n - 1]], mode))
