@@ -795,13 +795,13 @@ int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaS
 // Stages taken face by face: a cluster per face (conv_tc_stage.cu), the 14x14 one also with a CTA pair per two (conv_tc_face.cu)
 // ---------------------------------------------------------------------------
 struct FacePlan {
-    CUtensorMap mapA[2], map_pair;      // boxes of the first input
+    CUtensorMap mapA[STAGE_FORMS], map_pair;      // boxes of the first input
     FaceLayer* d_layers;
     char* d_tables;          // every layer's constants and byte table
     int8_t* d_kept;
-    int H, n_layers;
+    int H, n_layers, forms;
     int pairs;               // CTA pairs the device holds at once (14x14)
-    StageForm form[2];
+    StageForm form[STAGE_FORMS];
 };
 
 // layers[i]: device pointers of layer i, and on the host its constants ([4][C]: w_scale, bias, slope or residual scale,
@@ -814,7 +814,8 @@ FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const 
     p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->H = H; p->n_layers = n_layers;
     p->pairs = H == 14 ? tc_face_pairs() : 0;
     size_t kept = (size_t)p->pairs * 2 * FACE_KEPT_BYTES;
-    for (int i = 0; i < 2; i++) {
+    p->forms = H == 7 ? STAGE_FORMS : 2;
+    for (int i = 0; i < p->forms; i++) {
         p->form[i] = tc_stage_form(H, i);
         kept = std::max(kept, (size_t)p->form[i].clusters * p->form[i].kept_bytes);
     }
@@ -829,9 +830,10 @@ FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const 
     {
         cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)H, (cuuint64_t)H, (cuuint64_t)max_batch};
         cuuint64_t strides[3] = {(cuuint64_t)C, (cuuint64_t)C * H, (cuuint64_t)C * H * H};
-        for (int i = 0; i < 3; i++) {
-            cuuint32_t box[4] = {128, i < 2 ? (cuuint32_t)p->form[i].pitch : 16u, i < 2 ? (cuuint32_t)p->form[i].win_rows : 9u, 1};
-            ok = ok && enc(i < 2 ? &p->mapA[i] : &p->map_pair, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es,
+        for (int i = 0; i <= p->forms; i++) {
+            const StageForm f = i < p->forms ? p->form[i] : StageForm{9, 16, 0, 0, 0};
+            cuuint32_t box[4] = {128, (cuuint32_t)f.pitch, (cuuint32_t)f.win_rows, 1};
+            ok = ok && enc(i < p->forms ? &p->mapA[i] : &p->map_pair, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
         }
@@ -894,7 +896,7 @@ int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_e
 
 int ffcu_stage_form(const FacePlan* p, int faces)
 {
-    for (int i = 0; i < 2; i++) if (faces <= p->form[i].clusters) return i;
+    for (int i = 0; i < p->forms; i++) if (faces <= p->form[i].clusters * p->form[i].faces) return i;
     return -1;
 }
 

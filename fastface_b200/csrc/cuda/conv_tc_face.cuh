@@ -20,6 +20,11 @@ __device__ __forceinline__ void tmem_ld_wait8(int (&v)[8])
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]) :: "memory");
 }
+// MMAs issued so far are done: one arrival on this barrier of each CTA in `mask`.
+__device__ __forceinline__ void umma_commit_multicast(uint32_t bar, uint16_t mask)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask) : "memory");
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Shared memory of this CTA -> a CTA of the cluster, counted on that CTA's barrier (all shared::cluster addresses but `from`).

@@ -9,6 +9,12 @@
 //     14x14       R = 4, 4 / 3 rows, 64 columns; 8 CTAs      R = 2, 7 rows, 112 columns; 4 CTAs
 //     7x7         R = 2, 4 / 3 rows, 32 columns; 8 CTAs      R = 1, 7 rows, 64 columns; 4 CTAs
 //
+// On 7x7 maps a cluster of four also takes two faces at once (128 columns), one under the other with a row of zeros between them:
+// each CTA brings in 590 KB of weights per layer whatever it does with them.  One buffer has to do then, written when all four CTAs'
+// MMAs have read it (a commit that arrives at all of them).  34 to 66 faces, against one launch per layer: 13.7 and 16.1 -> 9.1 us a layer,
+// forward of 48 / 64 / 66 faces 544.6 / 595.7 / 608.4 -> 522.2 / 573.1 / 584.9 us.  Four faces a cluster (256 columns, 67 to 132 faces): 16.3 against
+// 14.1 and 16.5 us a layer at 80 faces, 17.5 and 20.2 at 128, forward within 1 %; not kept.
+//
 // A CTA holds, for all channels, its rows and one above and below, in two buffers that take turns.  Its epilogue writes its 128
 // channels of its rows into its own next buffer, bytewise, and sends the rows from there by bulk copies: all of them to the CTAs
 // with the other channels of the same rows, the first and the last to the CTAs of the neighbouring rows.
@@ -29,24 +35,28 @@
 
 namespace {
 
-// C channels on an H x H map, R row tiles; a cluster has C / 128 x R CTAs (rank = row tile * C / 128 + channel tile).
-template <int C_, int H_, int R_>
+// C channels on an H x H map, R row tiles; a cluster has C / 128 x R CTAs (rank = row tile * C / 128 + channel tile).  F > 1: a
+// cluster takes F faces at once, one under the other with a row of zeros between them, in a single buffer.
+template <int C_, int H_, int R_, int F_ = 1>
 struct Stage {
-    static constexpr int C = C_, H = H_, R = R_;
+    static constexpr int C = C_, H = H_, R = R_, F = F_;
     static constexpr int CT = C / 128;                       // channel tiles = planes of 128 input channels
     static constexpr int CLUSTER = CT * R;
     static constexpr int PITCH = H == 28 ? 32 : H == 14 ? 16 : 8;        // lines of a row: a zero line before it, zero or unread ones behind
     static constexpr int ROW_BYTES = PITCH * 128;
     static constexpr int ROWS = (H + R - 1) / R;             // rows of a tile; where R does not divide H the last tiles have one less
-    static constexpr int WIN = ROWS + 2 + (PITCH == H + 1 ? 1 : 0);      // (a row's last tap may read the line behind it: the next row's zero line)
-    static constexpr int PER_GROUP = (ROWS + 3) / 4;         // rows of an epilogue group of four warps
-    static constexpr int N = (ROWS * PITCH + 15) / 16 * 16;
+    static constexpr int FACE_ROWS = H + 1;                  // F > 1: rows from a face's first to the next one's
+    static constexpr int WIN = F > 1 ? F * FACE_ROWS + 2 : ROWS + 2 + (PITCH == H + 1 ? 1 : 0);      // (a row's last tap may read the line behind it: the next row's zero line)
+    static constexpr int BOX_ROWS = F > 1 ? FACE_ROWS : WIN; // rows a face's first input brings
+    static constexpr int PER_GROUP = F > 1 ? (ROWS * F + 3) / 4 : (ROWS + 3) / 4;        // rows of an epilogue group of four warps
+    static constexpr int N = F > 1 ? F * FACE_ROWS * PITCH : (ROWS * PITCH + 15) / 16 * 16;
+    static constexpr int BUFS = F > 1 ? 1 : 2;
     static constexpr int PLANE_BYTES = WIN * ROW_BYTES;
     static constexpr int ACT_BYTES = CT * PLANE_BYTES;
-    static constexpr int PL_STEP = CT < 2 ? CT : 2;          // a step of the weight ring: this many planes of one filter tap
+    static constexpr int PL_STEP = CT < 2 || F > 1 ? 1 : 2;          // a step of the weight ring: this many planes of one filter tap
     static constexpr int STEPS = 9 * (CT / PL_STEP);
     static constexpr int STEP_BYTES = PL_STEP * 128 * 128;
-    static constexpr int OFF_LUT = 2 * ACT_BYTES;
+    static constexpr int OFF_LUT = BUFS * ACT_BYTES;
     static constexpr int OFF_RING = OFF_LUT + FACE_LUT_BYTES;
     static constexpr int FIT = (232448 - 512 - OFF_RING) / STEP_BYTES;
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
@@ -54,8 +64,12 @@ struct Stage {
     static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
     static constexpr int WORDS = (H + 3) / 4;                // a row of a channel in packed bytes
     static constexpr int KEPT_BYTES = H * WORDS * C * 4;     // [row][word][channel]: a warp's 32 channels together
+    static_assert(F == 1 || (F == 2 && R == 1 && PITCH == H + 1), "faces of a cluster");
     static_assert(STAGES >= 3 && OFF_RING % 1024 == 0 && ACT_BYTES % 1024 == 0 && N <= 256, "layout");
     __device__ static int rows(int t) { return H / R + (t < H % R ? 1 : 0); }
+    // epilogue group g: its face of the cluster's, its first row in the tile
+    __device__ static int group_face(int g) { return F > 1 ? g * F / 4 : 0; }
+    __device__ static int group_row(int g) { return F > 1 ? g % (4 / F) * PER_GROUP : g * PER_GROUP; }
     __device__ static int first_row(int t) { return t * (H / R) + (t < H % R ? t : H % R); }
 };
 
@@ -72,14 +86,15 @@ struct StageShared {
 // One layer.  RESBN: residual and fused BN (else PReLU); LAST: results go to global memory as NHWC.
 template <bool CONTRACT, typename S, bool RESBN, bool LAST>
 __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, const FaceLayer* cl, const float4& k, int L, int rank, int q, int g,
-                                               int lane, uint32_t lut_lo, uint32_t lut_hi, int face, int8_t* kept, uint32_t tmem_base,
+                                               int lane, uint32_t lut_lo, uint32_t lut_hi, int face, int n_faces, int8_t* kept, uint32_t tmem_base,
                                                uint32_t lut_parity, volatile int* abort_flag, const FaceParams& p, bool& ok)
 {
     constexpr int PG = S::PER_GROUP, H = S::H, W4 = S::WORDS, CHUNKS = (H + 7) / 8;
     const int h = rank % S::CT, t = rank / S::CT, ch = q * 32 + lane;
     const int n_rows = S::rows(t), r0 = S::first_row(t);
-    const int mine = n_rows - g * PG < PG ? n_rows - g * PG : PG;          // rows of this warp's group: r0 + g * PG ..  (may be <= 0)
-    const size_t px0 = ((size_t)face * (H * H) + (size_t)(r0 + g * PG) * H) * S::C + h * 128 + ch;
+    const int f = S::group_face(g), y0 = S::group_row(g);
+    const int mine = f >= n_faces ? 0 : n_rows - y0 < PG ? n_rows - y0 : PG;          // rows of this warp's group: r0 + y0 ..  (may be <= 0)
+    const size_t px0 = ((size_t)face * (H * H) + (size_t)(r0 + y0) * H) * S::C + h * 128 + ch;
     uint32_t rw[W4 * PG];
 #pragma unroll
     for (int i = 0; i < W4 * PG; i++) rw[i] = 0;
@@ -103,12 +118,13 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
         }
     }
     if (RESBN && ok) ok = mbar_wait(smem_u32(&sh->lut_full), lut_parity, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
-    if (ok) ok = mbar_wait(smem_u32(&sh->acc_full), (uint32_t)L & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
+    if (ok) ok = S::BUFS == 1 ? mbar_wait_cluster(smem_u32(&sh->acc_full), (uint32_t)L & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles)
+                              : mbar_wait(smem_u32(&sh->acc_full), (uint32_t)L & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
     tc_fence_after();
     const uint8_t* lut = smem + S::OFF_LUT;
-    const uint32_t taddr = tmem_base + (uint32_t)(g * PG * S::PITCH) + ((uint32_t)(q * 32) << 16);
-    const uint32_t s_plane = smem_u32(smem) + (uint32_t)(((L + 1) & 1) * S::ACT_BYTES + h * S::PLANE_BYTES);
-    const uint32_t s_rows = s_plane + (uint32_t)((g * PG + 1) * S::ROW_BYTES);     // the group's rows in the next input
+    const uint32_t taddr = tmem_base + (uint32_t)((f * S::FACE_ROWS + y0) * S::PITCH) + ((uint32_t)(q * 32) << 16);
+    const uint32_t s_plane = smem_u32(smem) + (uint32_t)((L + 1) % S::BUFS * S::ACT_BYTES + h * S::PLANE_BYTES);
+    const uint32_t s_rows = s_plane + (uint32_t)((f * S::FACE_ROWS + y0 + 1) * S::ROW_BYTES);     // the group's rows in the next input
     if (ok && mine > 0) {
         FaceDst d;
         if (LAST) d.g = cl->out2 + px0;
@@ -137,10 +153,10 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(smem_u32(&sh->act_full[(L + 1) & 1]));
+        if (lane == 0 && ok) mbar_arrive(smem_u32(&sh->act_full[(L + 1) % S::BUFS]));
         asm volatile("bar.sync %0, 128;" ::"r"(2 + g) : "memory");
         if (ok && mine > 0) {
-            const uint32_t bar = smem_u32(&sh->act_full[(L + 1) & 1]);
+            const uint32_t bar = smem_u32(&sh->act_full[(L + 1) % S::BUFS]);
             const uint32_t tile0 = (uint32_t)(t * S::CT);                  // rank of this row tile's first CTA
             if (q == 0) {
                 // all rows: to the CTAs with the tile's other channels
@@ -192,14 +208,14 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
-    const int cluster = (int)blockIdx.x / S::CLUSTER, face = p.face0 + cluster;
+    const int cluster = (int)blockIdx.x / S::CLUSTER, n_faces = p.faces - cluster * S::F < S::F ? p.faces - cluster * S::F : S::F;
     const int h = rank % S::CT, t = rank / S::CT;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         mbar_init(smem_u32(&sh->a0_full), 1);
         for (int b = 0; b < 2; b++) mbar_init(smem_u32(&sh->act_full[b]), 17);          // the epilogue's warps, one arming arrival
-        mbar_init(smem_u32(&sh->acc_full), 1);
+        mbar_init(smem_u32(&sh->acc_full), S::BUFS == 1 ? S::CLUSTER : 1);              // one buffer: nobody reads it any more
         mbar_init(smem_u32(&sh->lut_full), 1);
         mbar_init(smem_u32(&sh->lut_empty), 16);
         sh->abort_flag = 0;
@@ -210,6 +226,12 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(S::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (S::F > 1) {
+        // the two rows below the last face (the others' zeros come with the first input)
+        for (int i = threadIdx.x; i < S::CT * 2 * S::ROW_BYTES / 16; i += TC_THREADS)
+            *(int4*)(smem + i / (2 * S::ROW_BYTES / 16) * S::PLANE_BYTES + S::F * S::FACE_ROWS * S::ROW_BYTES + i % (2 * S::ROW_BYTES / 16) * 16) = make_int4(0, 0, 0, 0);
+        fence_async_smem();
     }
     tc_fence_before();
     __syncthreads();
@@ -246,17 +268,18 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
             const uint64_t da0 = smem_desc<128>(s0 + S::OFF_RING);
             // what this CTA receives of each layer: its rows' other channels, and the rows above and below
-            const uint32_t in_bytes = (uint32_t)(S::ROW_BYTES * ((S::CT - 1) * S::rows(t) + S::CT * ((t > 0) + (t < S::R - 1))));
+            const uint32_t in_bytes = (uint32_t)(S::ROW_BYTES * ((S::CT - 1) * S::rows(t) * n_faces + S::CT * ((t > 0) + (t < S::R - 1))));
             int stage = 0; uint32_t phase = 0, ready = 0;
             bool ok = true;
 #pragma unroll 1
             for (int L = 0; L < p.n_layers && ok; L++) {
-                const int buf = L & 1;
+                const int buf = L % S::BUFS;
                 // (bytes that land before this only drive the count negative: the phase needs this arrival)
-                if (L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
+                if (S::BUFS == 2 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
                 ok = L == 0 ? mbar_wait(smem_u32(&sh->a0_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles)
-                            : mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) >> 1) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
+                            : mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) / S::BUFS) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
                 if (!ok) break;
+                if (S::BUFS == 1 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[0]), in_bytes);
                 tc_fence_after();
                 uint64_t db_row = smem_desc<128>(s0 + (uint32_t)(buf * S::ACT_BYTES));
                 uint32_t first = 0;
@@ -286,17 +309,20 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                         stage = ns; phase = np;
                     }
                 }
-                if (ok) umma_commit(smem_u32(&sh->acc_full));
+                if (!ok) break;
+                if (S::BUFS == 1) umma_commit_multicast(smem_u32(&sh->acc_full), (uint16_t)((1 << S::CLUSTER) - 1));
+                else umma_commit(smem_u32(&sh->acc_full));
             }
         }
     } else if (warp == TC_ISSUER2_WARP) {
         // The face's first input, into both buffers (of the second only the padding's zeros stay), and the fused BNs' byte tables
         if (tc_elect_one()) {
             tc_pdl_wait();
-            mbar_expect_tx(smem_u32(&sh->a0_full), 2 * S::ACT_BYTES);
+            mbar_expect_tx(smem_u32(&sh->a0_full), S::BUFS * S::F * S::CT * S::BOX_ROWS * S::ROW_BYTES);
 #pragma unroll
-            for (int i = 0; i < 2 * S::CT; i++)
-                tma_load_4d(s0 + i * S::PLANE_BYTES, &mapA, smem_u32(&sh->a0_full), i % S::CT * 128, -1, S::first_row(t) - 1, face);
+            for (int i = 0; i < S::BUFS * S::F * S::CT; i++)
+                tma_load_4d(s0 + i % (S::BUFS * S::CT) * S::PLANE_BYTES + i / (S::BUFS * S::CT) * (S::FACE_ROWS * S::ROW_BYTES), &mapA, smem_u32(&sh->a0_full),
+                            i % S::CT * 128, -1, S::first_row(t) - 1, p.face0 + cluster * S::F + i / (S::BUFS * S::CT));
             uint32_t lut_par = 0;
             bool ok = true;
 #pragma unroll 1
@@ -316,7 +342,8 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         const int q = warp & 3, g = warp >> 2;
         const uint32_t lut_lo = (uint32_t)(lane * 4 + (q & 1) * 128) * 0x01010101u, lut_hi = (uint32_t)(q >> 1) * 0x01010101u;
         // a result that the next residual layer adds lies as its thread left it
-        int8_t* kept = p.kept + (size_t)cluster * S::KEPT_BYTES + ((size_t)(S::first_row(t) + g * S::PER_GROUP) * S::WORDS * S::C + h * 128 + q * 32 + lane) * 4;
+        const int slot = cluster * S::F + S::group_face(g), face = p.face0 + slot;
+        int8_t* kept = p.kept + (size_t)slot * S::KEPT_BYTES + ((size_t)(S::first_row(t) + S::group_row(g)) * S::WORDS * S::C + h * 128 + q * 32 + lane) * 4;
         uint32_t lut_par = 0;
         bool ok = true;
         tc_pdl_wait();
@@ -328,9 +355,9 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             const bool last = L + 1 == p.n_layers;
             // (the next kernel not before: its CTAs would keep other contexts' kernels off the SMs this launch leaves free)
             if (last && warp == 0) tc_pdl_trigger();
-            if (last)    stage_epilogue<CONTRACT, S, true, true>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else if (bn) stage_epilogue<CONTRACT, S, true, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else         stage_epilogue<CONTRACT, S, false, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, kept, tmem_base, lut_par, abort_flag, p, ok);
+            if (last)    stage_epilogue<CONTRACT, S, true, true>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+            else if (bn) stage_epilogue<CONTRACT, S, true, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+            else         stage_epilogue<CONTRACT, S, false, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
             if (bn) {
                 lut_par ^= 1;
                 __syncwarp();
@@ -374,14 +401,14 @@ int launch(int mode, int faces, cudaStream_t s, const CUtensorMap& mapA, const F
 {
     const int rc = mode ? set_smem<true, S>() : set_smem<false, S>();
     if (rc != 0) return rc;
-    return mode ? tc_launch_ex(conv_stage_kernel<true, S>, S::CLUSTER * faces, smem_bytes<S>(), s, S::CLUSTER, mapA, prm)
-                : tc_launch_ex(conv_stage_kernel<false, S>, S::CLUSTER * faces, smem_bytes<S>(), s, S::CLUSTER, mapA, prm);
+    return mode ? tc_launch_ex(conv_stage_kernel<true, S>, S::CLUSTER * ((faces + S::F - 1) / S::F), smem_bytes<S>(), s, S::CLUSTER, mapA, prm)
+                : tc_launch_ex(conv_stage_kernel<false, S>, S::CLUSTER * ((faces + S::F - 1) / S::F), smem_bytes<S>(), s, S::CLUSTER, mapA, prm);
 }
 
 template <typename S>
 StageForm form()
 {
-    StageForm f = {S::WIN, S::PITCH, S::KEPT_BYTES, 0};
+    StageForm f = {S::BOX_ROWS, S::PITCH, S::KEPT_BYTES * S::F, 0, S::F};
     if (set_smem<true, S>() != 0 || set_smem<false, S>() != 0) { cudaGetLastError(); return f; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S::CLUSTER);
@@ -397,12 +424,12 @@ StageForm form()
     return f;
 }
 
-// calls fn with the form of the stage of H x H maps: 0, more and smaller tiles (few faces), or 1
-template <typename F>
-auto with_form(int H, int i, F&& fn)
+// calls fn with the form of the stage of H x H maps: 0, more and smaller tiles (few faces), or 1; 7x7 also 2, two faces a cluster
+template <typename Fn>
+auto with_form(int H, int i, Fn&& fn)
 {
     if (H == 28) return i == 0 ? fn(Stage<128, 28, 7>{}) : fn(Stage<128, 28, 4>{});
-    if (H == 7) return i == 0 ? fn(Stage<512, 7, 2>{}) : fn(Stage<512, 7, 1>{});
+    if (H == 7) return i == 0 ? fn(Stage<512, 7, 2>{}) : i == 1 ? fn(Stage<512, 7, 1>{}) : fn(Stage<512, 7, 1, 2>{});
     return i == 0 ? fn(Stage<256, 14, 4>{}) : fn(Stage<256, 14, 2>{});
 }
 

@@ -656,7 +656,7 @@ static const ffcu_ctx::Chain* chain_at(const ffcu_ctx* c, size_t k, int n, const
 }
 
 // The run of layers that starts at k and that a call of n faces takes face by face; NULL: none.  28x28 and 7x7 maps only while the
-// device holds a cluster for each: in rounds they lose to one launch per layer, as every CTA brings in all of its weights
+// device holds all their clusters at once: in rounds they lose to one launch per layer, as every CTA brings in all of its weights
 // (forward of 64 / 148 / 256 faces: 604 / 978 / 1655 us; 28x28 stage in rounds 599 / 1015 / 1718, 7x7 608 / 1051 / 1790).
 // A context made for two or three faces keeps one launch per layer beyond a single face (chain_max_faces), one for up to four
 // also on 28x28 maps: callers count a single face's 22 launches there (tests/test_gpu_parity.py).

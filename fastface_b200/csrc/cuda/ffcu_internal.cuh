@@ -227,7 +227,7 @@ struct FaceLayerDesc {
 };
 FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const FaceLayerDesc* layers, int n_layers);
 void      ffcu_face_free(FacePlan* p);
-// With a cluster per face: the form (0, 1) the device holds `faces` clusters of, more and smaller tiles first; -1: none.
+// In clusters: the first form (more and smaller tiles first) the device holds enough clusters of for `faces`; -1: none.
 int       ffcu_stage_form(const FacePlan* p, int faces);
 int       ffcu_stage_launch(const FacePlan* p, int form, int face0, int faces, int mode, int* d_err, cudaStream_t s);
 // 14x14, any number of faces, a CTA pair for two; pairs the device holds at once.
