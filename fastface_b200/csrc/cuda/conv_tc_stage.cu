@@ -53,13 +53,16 @@ struct Stage {
     static constexpr int BUFS = F > 1 ? 1 : 2;
     static constexpr int PLANE_BYTES = WIN * ROW_BYTES;
     static constexpr int ACT_BYTES = CT * PLANE_BYTES;
-    static constexpr int PL_STEP = CT < 2 || F > 1 ? 1 : 2;          // a step of the weight ring: this many planes of one filter tap
+    // A step of the weight ring: this many planes of one filter tap.  One plane (16 KB) keeps the ring fullest; where four MMAs take
+    // 128 cycles or less the issuer does not keep up with that many steps (14x14 with 64 columns: forward of one face 206 -> 215 us).
+    // On 7x7 maps with 64 columns and 14x14 with 112, one against two: forward of 16 / 17 / 24 / 33 faces 324 / 325 / 352 / 384 -> 308 / 310 / 337 / 370 us.
+    static constexpr int PL_STEP = CT > 1 && N <= (H == 7 ? 32 : 64) ? 2 : 1;
     static constexpr int STEPS = 9 * (CT / PL_STEP);
     static constexpr int STEP_BYTES = PL_STEP * 128 * 128;
     static constexpr int OFF_LUT = BUFS * ACT_BYTES;
     static constexpr int OFF_RING = OFF_LUT + FACE_LUT_BYTES;
     static constexpr int FIT = (232448 - 512 - OFF_RING) / STEP_BYTES;
-    static constexpr int STAGES = FIT < 8 ? FIT : 8;
+    static constexpr int STAGES = FIT < 12 ? FIT : 12;
     static constexpr int OFF_SH = OFF_RING + STAGES * STEP_BYTES;
     static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
     static constexpr int WORDS = (H + 3) / 4;                // a row of a channel in packed bytes
@@ -74,7 +77,7 @@ struct Stage {
 };
 
 struct StageShared {
-    uint64_t full[8], empty[8];
+    uint64_t full[12], empty[12];
     uint64_t a0_full;             // the first input has landed, and the padding's zeros in both buffers
     uint64_t act_full[2];         // buffer b holds the next layer's input: own rows (sixteen warps), and the bytes that come
     uint64_t acc_full;
@@ -242,7 +245,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     const uint32_t s0 = smem_u32(smem);
 
     if (warp == TC_PRODUCER_WARP) {
-        // Weight producer: a step is one or two planes of a filter tap, a box each (lane i: input channels 128 i .. of the step's)
+        // Weight producer: a plane is a box (lane i: input channels 128 i .. of the step's)
         int stage = 0, gs = 0; uint32_t phase = 0;
         bool ok = true;
 #pragma unroll 1
