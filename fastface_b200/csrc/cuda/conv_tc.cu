@@ -814,7 +814,7 @@ FacePlan* ffcu_face_plan(int C, int H, int max_batch, const int8_t* d_in, const 
     p->d_layers = nullptr; p->d_tables = nullptr; p->d_kept = nullptr; p->H = H; p->n_layers = n_layers;
     p->pairs = H == 14 ? tc_face_pairs() : 0;
     size_t kept = (size_t)p->pairs * 2 * FACE_KEPT_BYTES;
-    p->forms = H == 7 ? STAGE_FORMS : 2;
+    p->forms = H == 14 ? 2 : STAGE_FORMS;
     for (int i = 0; i < p->forms; i++) {
         p->form[i] = tc_stage_form(H, i);
         kept = std::max(kept, (size_t)p->form[i].clusters * p->form[i].kept_bytes);
@@ -896,7 +896,10 @@ int ffcu_face_launch(const FacePlan* p, int face0, int faces, int mode, int* d_e
 
 int ffcu_stage_form(const FacePlan* p, int faces)
 {
-    for (int i = 0; i < p->forms; i++) if (faces <= p->form[i].clusters * p->form[i].faces) return i;
+    // (28x28 in clusters of two takes one time up to 74 faces; as a launch per layer 34 to 48 faces are quicker.  Forward of 34 / 40 / 48 / 64 /
+    // 67 / 74 faces: 470 / 493 / 521 / 572 / 605 / 636 us by layers, 477 / 496 / 522 / 564 / 596 / 626 in clusters)
+    for (int i = 0; i < p->forms; i++)
+        if (faces <= p->form[i].clusters * p->form[i].faces) return p->H == 28 && i == 2 && faces <= 48 ? -1 : i;
     return -1;
 }
 

@@ -9,6 +9,8 @@
 //     14x14       R = 4, 4 / 3 rows, 64 columns; 8 CTAs      R = 2, 7 rows, 112 columns; 4 CTAs
 //     7x7         R = 2, 4 / 3 rows, 32 columns; 8 CTAs      R = 1, 7 rows, 64 columns; 4 CTAs
 //
+// From 49 to 74 faces the 28x28 stage also goes in clusters of two: 14 rows a CTA, as two accumulators of 224 columns from the same
+// weights, emptied one after the other (forward of 64 / 74 faces 572 / 636 -> 564 / 626 us).
 // On 7x7 maps a cluster of four also takes two faces at once (128 columns), one under the other with a row of zeros between them:
 // each CTA brings in 590 KB of weights per layer whatever it does with them.  One buffer has to do then, written when all four CTAs'
 // MMAs have read it (a commit that arrives at all of them).  34 to 66 faces, against one launch per layer: 13.7 and 16.1 -> 9.1 us a layer,
@@ -48,7 +50,9 @@ struct Stage {
     static constexpr int FACE_ROWS = H + 1;                  // F > 1: rows from a face's first to the next one's
     static constexpr int WIN = F > 1 ? F * FACE_ROWS + 2 : ROWS + 2 + (PITCH == H + 1 ? 1 : 0);      // (a row's last tap may read the line behind it: the next row's zero line)
     static constexpr int BOX_ROWS = F > 1 ? FACE_ROWS : WIN; // rows a face's first input brings
-    static constexpr int PER_GROUP = F > 1 ? (ROWS * F + 3) / 4 : (ROWS + 3) / 4;        // rows of an epilogue group of four warps
+    static constexpr int PARTS = ROWS * PITCH > 256 ? 2 : 1; // of a tile's rows: an MMA has up to 256 columns
+    static constexpr int PART_ROWS = ROWS / PARTS;
+    static constexpr int PER_GROUP = F > 1 ? (ROWS * F + 3) / 4 : (PART_ROWS + 3) / 4;   // rows of an epilogue group of four warps
     static constexpr int N = F > 1 ? F * FACE_ROWS * PITCH : (ROWS * PITCH + 15) / 16 * 16;
     static constexpr int BUFS = F > 1 ? 1 : 2;
     static constexpr int PLANE_BYTES = WIN * ROW_BYTES;
@@ -64,11 +68,11 @@ struct Stage {
     static constexpr int FIT = (232448 - 512 - OFF_RING) / STEP_BYTES;
     static constexpr int STAGES = FIT < 12 ? FIT : 12;
     static constexpr int OFF_SH = OFF_RING + STAGES * STEP_BYTES;
-    static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+    static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : N <= 256 ? 256 : 512;
     static constexpr int WORDS = (H + 3) / 4;                // a row of a channel in packed bytes
     static constexpr int KEPT_BYTES = H * WORDS * C * 4;     // [row][word][channel]: a warp's 32 channels together
     static_assert(F == 1 || (F == 2 && R == 1 && PITCH == H + 1), "faces of a cluster");
-    static_assert(STAGES >= 3 && OFF_RING % 1024 == 0 && ACT_BYTES % 1024 == 0 && N <= 256, "layout");
+    static_assert(STAGES >= 3 && OFF_RING % 1024 == 0 && ACT_BYTES % 1024 == 0 && N <= 256 * PARTS && ROWS % PARTS == 0, "layout");
     __device__ static int rows(int t) { return H / R + (t < H % R ? 1 : 0); }
     // epilogue group g: its face of the cluster's, its first row in the tile
     __device__ static int group_face(int g) { return F > 1 ? g * F / 4 : 0; }
@@ -86,18 +90,19 @@ struct StageShared {
     int abort_flag;
 };
 
-// One layer.  RESBN: residual and fused BN (else PReLU); LAST: results go to global memory as NHWC.
+// One layer, or one part of its rows.  RESBN: residual and fused BN (else PReLU); LAST: results go to global memory as NHWC.
 template <bool CONTRACT, typename S, bool RESBN, bool LAST>
-__device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, const FaceLayer* cl, const float4& k, int L, int rank, int q, int g,
+__device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, const FaceLayer* cl, const float4& k, int L, int rank, int part, int q, int g,
                                                int lane, uint32_t lut_lo, uint32_t lut_hi, int face, int n_faces, int8_t* kept, uint32_t tmem_base,
                                                uint32_t lut_parity, volatile int* abort_flag, const FaceParams& p, bool& ok)
 {
     constexpr int PG = S::PER_GROUP, H = S::H, W4 = S::WORDS, CHUNKS = (H + 7) / 8;
     const int h = rank % S::CT, t = rank / S::CT, ch = q * 32 + lane;
     const int n_rows = S::rows(t), r0 = S::first_row(t);
-    const int f = S::group_face(g), y0 = S::group_row(g);
-    const int mine = f >= n_faces ? 0 : n_rows - y0 < PG ? n_rows - y0 : PG;          // rows of this warp's group: r0 + y0 ..  (may be <= 0)
+    const int f = S::group_face(g), y0 = part * S::PART_ROWS + S::group_row(g), y1 = S::PARTS > 1 ? (part + 1) * S::PART_ROWS : n_rows;
+    const int mine = f >= n_faces ? 0 : y1 - y0 < PG ? y1 - y0 : PG;          // rows of this warp's group: r0 + y0 ..  (may be <= 0)
     const size_t px0 = ((size_t)face * (H * H) + (size_t)(r0 + y0) * H) * S::C + h * 128 + ch;
+    kept += (size_t)(part * S::PART_ROWS) * (W4 * S::C * 4);
     uint32_t rw[W4 * PG];
 #pragma unroll
     for (int i = 0; i < W4 * PG; i++) rw[i] = 0;
@@ -169,13 +174,13 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
                 }
             } else if (q == 1) {
                 // the first row is the row below the tile above's
-                if (g == 0 && t > 0 && lane < S::CT) {
+                if (y0 == 0 && t > 0 && lane < S::CT) {
                     const uint32_t to = tile0 - (uint32_t)(S::CT - lane);
                     bulk_send(map_to_cta(s_plane + (uint32_t)((S::rows(t - 1) + 1) * S::ROW_BYTES), to), s_rows, S::ROW_BYTES, map_to_cta(bar, to));
                 }
             } else if (q == 2) {
                 // the last one the row above the tile below's
-                if (g == (n_rows - 1) / PG && t < S::R - 1 && lane < S::CT) {
+                if (y0 + mine == n_rows && t < S::R - 1 && lane < S::CT) {
                     const uint32_t to = tile0 + (uint32_t)(S::CT + lane);
                     bulk_send(map_to_cta(s_plane, to), s_plane + (uint32_t)(n_rows * S::ROW_BYTES), S::ROW_BYTES, map_to_cta(bar, to));
                 }
@@ -217,7 +222,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         mbar_init(smem_u32(&sh->a0_full), 1);
-        for (int b = 0; b < 2; b++) mbar_init(smem_u32(&sh->act_full[b]), 17);          // the epilogue's warps, one arming arrival
+        for (int b = 0; b < 2; b++) mbar_init(smem_u32(&sh->act_full[b]), 16 * S::PARTS + 1);          // the epilogue's warps, one arming arrival
         mbar_init(smem_u32(&sh->acc_full), S::BUFS == 1 ? S::CLUSTER : 1);              // one buffer: nobody reads it any more
         mbar_init(smem_u32(&sh->lut_full), 1);
         mbar_init(smem_u32(&sh->lut_empty), 16);
@@ -267,7 +272,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         }
     } else if (warp == TC_ISSUER_WARP) {
         if (tc_elect_one()) {
-            constexpr uint32_t IDESC = idesc_i8(S::N);
+            constexpr uint32_t IDESC = idesc_i8(S::N / S::PARTS);
             const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
             const uint64_t da0 = smem_desc<128>(s0 + S::OFF_RING);
             // what this CTA receives of each layer: its rows' other channels, and the rows above and below
@@ -302,11 +307,14 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                         tc_fence_after();
                         const uint64_t da = da0 + (uint64_t)((uint32_t)(stage * S::STEP_BYTES) >> 4);
 #pragma unroll
-                        for (int pl = 0; pl < S::PL_STEP; pl++)
+                        for (int part = 0; part < S::PARTS; part++)
 #pragma unroll
-                            for (int k = 0; k < 4; k++)
-                                umma_i8(tmem_base, da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k),
-                                        db_row + (uint64_t)(((kw * 128 + (pl0 + pl) * S::PLANE_BYTES) >> 4) + 2 * k), IDESC, (kp | pl | k) ? 1u : first);
+                            for (int pl = 0; pl < S::PL_STEP; pl++)
+#pragma unroll
+                                for (int k = 0; k < 4; k++)
+                                    umma_i8(tmem_base + (uint32_t)(part * (S::N / S::PARTS)), da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k),
+                                            db_row + (uint64_t)(((kw * 128 + (pl0 + pl) * S::PLANE_BYTES + part * S::PART_ROWS * S::ROW_BYTES) >> 4) + 2 * k), IDESC,
+                                            (kp | pl | k) ? 1u : first);
                         first = 1;
                         umma_commit(empty0 + stage * 8);
                         stage = ns; phase = np;
@@ -346,7 +354,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         const uint32_t lut_lo = (uint32_t)(lane * 4 + (q & 1) * 128) * 0x01010101u, lut_hi = (uint32_t)(q >> 1) * 0x01010101u;
         // a result that the next residual layer adds lies as its thread left it
         const int slot = cluster * S::F + S::group_face(g), face = p.face0 + slot;
-        int8_t* kept = p.kept + (size_t)slot * S::KEPT_BYTES + ((size_t)(S::first_row(t) + S::group_row(g)) * S::WORDS * S::C + h * 128 + q * 32 + lane) * 4;
+        int8_t* kept = p.kept + (size_t)slot * S::KEPT_BYTES + ((size_t)(S::first_row(t) + S::group_row(g)) * S::WORDS * S::C + h * 128 + q * 32 + lane) * 4;      // (its first part's)
         uint32_t lut_par = 0;
         bool ok = true;
         tc_pdl_wait();
@@ -358,9 +366,12 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             const bool last = L + 1 == p.n_layers;
             // (the next kernel not before: its CTAs would keep other contexts' kernels off the SMs this launch leaves free)
             if (last && warp == 0) tc_pdl_trigger();
-            if (last)    stage_epilogue<CONTRACT, S, true, true>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else if (bn) stage_epilogue<CONTRACT, S, true, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
-            else         stage_epilogue<CONTRACT, S, false, false>(smem, sh, cl, k, L, rank, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+#pragma unroll 1
+            for (int part = 0; part < S::PARTS; part++) {
+                if (last)    stage_epilogue<CONTRACT, S, true, true>(smem, sh, cl, k, L, rank, part, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+                else if (bn) stage_epilogue<CONTRACT, S, true, false>(smem, sh, cl, k, L, rank, part, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+                else         stage_epilogue<CONTRACT, S, false, false>(smem, sh, cl, k, L, rank, part, q, g, lane, lut_lo, lut_hi, face, n_faces, kept, tmem_base, lut_par, abort_flag, p, ok);
+            }
             if (bn) {
                 lut_par ^= 1;
                 __syncwarp();
@@ -427,11 +438,12 @@ StageForm form()
     return f;
 }
 
-// calls fn with the form of the stage of H x H maps: 0, more and smaller tiles (few faces), or 1; 7x7 also 2, two faces a cluster
+// calls fn with the form of the stage of H x H maps: 0, more and smaller tiles (few faces), 1, or 2 (not 14x14; 7x7: two
+// faces a cluster)
 template <typename Fn>
 auto with_form(int H, int i, Fn&& fn)
 {
-    if (H == 28) return i == 0 ? fn(Stage<128, 28, 7>{}) : fn(Stage<128, 28, 4>{});
+    if (H == 28) return i == 0 ? fn(Stage<128, 28, 7>{}) : i == 1 ? fn(Stage<128, 28, 4>{}) : fn(Stage<128, 28, 2>{});
     if (H == 7) return i == 0 ? fn(Stage<512, 7, 2>{}) : i == 1 ? fn(Stage<512, 7, 1>{}) : fn(Stage<512, 7, 1, 2>{});
     return i == 0 ? fn(Stage<256, 14, 4>{}) : fn(Stage<256, 14, 2>{});
 }
