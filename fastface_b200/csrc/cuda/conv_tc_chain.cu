@@ -1,6 +1,7 @@
 // conv_tc_chain.cu -- small-batch latency path: a run of consecutive 3x3 stride-1 convolutions of one
 // shape (the 26 layers of the 14x14 stage, the 4 of the 7x7 stage) in ONE launch, one cluster of
-// eight or four CTAs per face, with the activations resident in shared memory.
+// eight or four CTAs per face, with the activations resident in shared memory.  The network's own stages go by
+// conv_tc_stage.cu; this kernel takes runs whose tensors between the layers are read from outside (it writes them all).
 //
 // Clusters share nothing but the weights (L2): n faces cost one face's time while all n clusters are resident at once
 // (26 layers of 14x14: 144 us at 1 face, 150 us at 8, against 205-208 us as one launch per layer), and twice that with
