@@ -19,7 +19,9 @@
 //
 // A CTA holds, for all channels, its rows and one above and below, in two buffers that take turns.  Its epilogue writes its 128
 // channels of its rows into its own next buffer, bytewise, and sends the rows from there by bulk copies: all of them to the CTAs
-// with the other channels of the same rows, the first and the last to the CTAs of the neighbouring rows.
+// with the other channels of the same rows, the first and the last to the CTAs of the neighbouring rows.  What a CTA has made itself is there some 1.5 thousand cycles before the others' bytes, so a layer begins with
+// the filter taps that read nothing else: the middle row of taps on its own plane, all nine where the rows are not split.
+// (Forward of 1 / 4 / 8 / 15 / 17 / 33 faces, all taps after the last byte -> this: 207 / 222 / 240 / 268 / 311 / 368 -> 201 / 212 / 231 / 259 / 304 / 361 us.)
 //
 // Bound: latency.  What passes between shared memories goes at 20 B per cycle and CTA whatever instruction sends it (measured:
 // 8 KB to 1 / 2 / 4 / 8 CTAs of a cluster of eight 710 / 1110 / 1920 / 3550 cycles by 16-byte st.async, 810 / 1210 / 2005 / 3790 by
@@ -61,11 +63,12 @@ struct Stage {
     // 128 cycles or less the issuer does not keep up with that many steps (14x14 with 64 columns: forward of one face 206 -> 215 us).
     // On 7x7 maps with 64 columns and 14x14 with 112, one against two: forward of 16 / 17 / 24 / 33 faces 324 / 325 / 352 / 384 -> 308 / 310 / 337 / 370 us.
     static constexpr int PL_STEP = CT > 1 && N <= (H == 7 ? 32 : 64) ? 2 : 1;
-    static constexpr int STEPS = 9 * (CT / PL_STEP);
+    static constexpr int UNITS = 9 * CT, STEPS = UNITS / PL_STEP;      // a unit: one plane of one tap
+    static constexpr int EARLY = R == 1 ? 9 : 3;             // units that read only what this CTA's epilogue has written: they come first
     static constexpr int STEP_BYTES = PL_STEP * 128 * 128;
     static constexpr int OFF_LUT = BUFS * ACT_BYTES;
     static constexpr int OFF_RING = OFF_LUT + FACE_LUT_BYTES;
-    static constexpr int FIT = (232448 - 512 - OFF_RING) / STEP_BYTES;
+    static constexpr int FIT = (232448 - 768 - OFF_RING) / STEP_BYTES;
     static constexpr int STAGES = FIT < 12 ? FIT : 12;
     static constexpr int OFF_SH = OFF_RING + STAGES * STEP_BYTES;
     static constexpr uint32_t TMEM_COLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : N <= 256 ? 256 : 512;
@@ -83,9 +86,11 @@ struct Stage {
 struct StageShared {
     uint64_t full[12], empty[12];
     uint64_t a0_full;             // the first input has landed, and the padding's zeros in both buffers
-    uint64_t act_full[2];         // buffer b holds the next layer's input: own rows (sixteen warps), and the bytes that come
+    uint64_t own_full;            // this CTA's results are in the next layer's input (sixteen warps, each part)
+    uint64_t act_full[2];         // the others' are in buffer b's
     uint64_t acc_full;
     uint64_t lut_full, lut_empty;
+    uint32_t unit_k[36], unit_db[36];      // of a layer's units in turn: where the weights start, where the activations do (>> 4)
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -161,7 +166,7 @@ __device__ __forceinline__ void stage_epilogue(uint8_t* smem, StageShared* sh, c
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(smem_u32(&sh->act_full[(L + 1) % S::BUFS]));
+        if (lane == 0 && ok) mbar_arrive(smem_u32(&sh->own_full));
         asm volatile("bar.sync %0, 128;" ::"r"(2 + g) : "memory");
         if (ok && mine > 0) {
             const uint32_t bar = smem_u32(&sh->act_full[(L + 1) % S::BUFS]);
@@ -222,7 +227,8 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) { mbar_init(smem_u32(&sh->full[s]), 1); mbar_init(smem_u32(&sh->empty[s]), 1); }
         mbar_init(smem_u32(&sh->a0_full), 1);
-        for (int b = 0; b < 2; b++) mbar_init(smem_u32(&sh->act_full[b]), 16 * S::PARTS + 1);          // the epilogue's warps, one arming arrival
+        mbar_init(smem_u32(&sh->own_full), 16 * S::PARTS);
+        for (int b = 0; b < 2; b++) mbar_init(smem_u32(&sh->act_full[b]), 1);          // the arming arrival
         mbar_init(smem_u32(&sh->acc_full), S::BUFS == 1 ? S::CLUSTER : 1);              // one buffer: nobody reads it any more
         mbar_init(smem_u32(&sh->lut_full), 1);
         mbar_init(smem_u32(&sh->lut_empty), 16);
@@ -234,6 +240,13 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&sh->tmem_base)), "r"(S::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + S::UNITS) {
+        // own plane first, of that the middle row of taps
+        const int u = (int)threadIdx.x - 32, t9 = u % 9, plane = (h + u / 9) % S::CT;
+        const int kh = u >= 9 || S::R == 1 ? t9 / 3 : t9 < 3 ? 1 : t9 < 6 ? 0 : 2, kw = t9 % 3;
+        sh->unit_k[u] = (uint32_t)(((kh * 3 + kw) * S::CT + plane) * 128);
+        sh->unit_db[u] = (uint32_t)((kh * S::ROW_BYTES + kw * 128 + plane * S::PLANE_BYTES) >> 4);
     }
     if (S::F > 1) {
         // the two rows below the last face (the others' zeros come with the first input)
@@ -250,7 +263,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     const uint32_t s0 = smem_u32(smem);
 
     if (warp == TC_PRODUCER_WARP) {
-        // Weight producer: a plane is a box (lane i: input channels 128 i .. of the step's)
+        // Weight producer: a unit is a box (lane i: the step's unit i)
         int stage = 0, gs = 0; uint32_t phase = 0;
         bool ok = true;
 #pragma unroll 1
@@ -266,7 +279,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                 // (drop_step: the timeout test's launch, CTA 0 leaves out this step)
                 if (lane < S::PL_STEP && (gs != p.drop_step || rank != 0))
                     tma_load_4d(s0 + S::OFF_RING + stage * S::STEP_BYTES + lane * (128 * 128), map, smem_u32(&sh->full[stage]),
-                                (st * S::PL_STEP + lane) * 128, h * 128, 0, 0);
+                                (int)sh->unit_k[st * S::PL_STEP + lane], h * 128, 0, 0);
                 if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -285,40 +298,40 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                 // (bytes that land before this only drive the count negative: the phase needs this arrival)
                 if (S::BUFS == 2 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[buf ^ 1]), in_bytes);
                 ok = L == 0 ? mbar_wait(smem_u32(&sh->a0_full), 0, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles)
-                            : mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) / S::BUFS) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
+                            : mbar_wait(smem_u32(&sh->own_full), (uint32_t)(L - 1) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
                 if (!ok) break;
-                if (S::BUFS == 1 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[0]), in_bytes);
                 tc_fence_after();
-                uint64_t db_row = smem_desc<128>(s0 + (uint32_t)(buf * S::ACT_BYTES));
-                uint32_t first = 0;
+                const uint64_t db0 = smem_desc<128>(s0 + (uint32_t)(buf * S::ACT_BYTES));
 #pragma unroll 1
-                for (int kh = 0; kh < 3 && ok; kh++, db_row += S::ROW_BYTES / 16) {
+                for (int u = 0; u < S::UNITS && ok;) {
+                    if (!ready) {
+                        ok = mbar_wait(full0 + stage * 8, phase, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
+                        if (!ok) break;
+                    }
+                    int ns = stage + 1; uint32_t np = phase;
+                    if (ns == S::STAGES) { ns = 0; np ^= 1; }
+                    ready = mbar_test(full0 + ns * 8, np);                       // used next round
+                    tc_fence_after();
+                    const uint64_t da = da0 + (uint64_t)((uint32_t)(stage * S::STEP_BYTES) >> 4);
 #pragma unroll
-                    for (int kp = 0; kp < 3 * (S::CT / S::PL_STEP); kp++) {      // (kw, planes of the step)
-                        constexpr int PS = S::CT / S::PL_STEP;
-                        const int kw = kp / PS, pl0 = kp % PS * S::PL_STEP;
-                        if (!ready) {
-                            ok = mbar_wait(full0 + stage * 8, phase, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
+                    for (int pl = 0; pl < S::PL_STEP; pl++, u++) {
+                        if (u == S::EARLY) {
+                            if (L) ok = mbar_wait_cluster(smem_u32(&sh->act_full[buf]), (uint32_t)((L - 1) / S::BUFS) & 1, abort_flag, p.err, FFCU_ERR_TMA_TIMEOUT, p.wait_cycles);
                             if (!ok) break;
+                            if (S::BUFS == 1 && L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->act_full[0]), in_bytes);
+                            tc_fence_after();
                         }
-                        int ns = stage + 1; uint32_t np = phase;
-                        if (ns == S::STAGES) { ns = 0; np ^= 1; }
-                        ready = mbar_test(full0 + ns * 8, np);                   // used next round
-                        tc_fence_after();
-                        const uint64_t da = da0 + (uint64_t)((uint32_t)(stage * S::STEP_BYTES) >> 4);
+                        const uint64_t db = db0 + sh->unit_db[u];
 #pragma unroll
                         for (int part = 0; part < S::PARTS; part++)
 #pragma unroll
-                            for (int pl = 0; pl < S::PL_STEP; pl++)
-#pragma unroll
-                                for (int k = 0; k < 4; k++)
-                                    umma_i8(tmem_base + (uint32_t)(part * (S::N / S::PARTS)), da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k),
-                                            db_row + (uint64_t)(((kw * 128 + (pl0 + pl) * S::PLANE_BYTES + part * S::PART_ROWS * S::ROW_BYTES) >> 4) + 2 * k), IDESC,
-                                            (kp | pl | k) ? 1u : first);
-                        first = 1;
-                        umma_commit(empty0 + stage * 8);
-                        stage = ns; phase = np;
+                            for (int k = 0; k < 4; k++)
+                                umma_i8(tmem_base + (uint32_t)(part * (S::N / S::PARTS)), da + (uint64_t)(pl * (128 * 128 >> 4) + 2 * k),
+                                        db + (uint64_t)((part * S::PART_ROWS * S::ROW_BYTES >> 4) + 2 * k), IDESC, (u | k) ? 1u : 0u);
                     }
+                    if (!ok) break;
+                    umma_commit(empty0 + stage * 8);
+                    stage = ns; phase = np;
                 }
                 if (!ok) break;
                 if (S::BUFS == 1) umma_commit_multicast(smem_u32(&sh->acc_full), (uint16_t)((1 << S::CLUSTER) - 1));
@@ -394,6 +407,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
     }
 }
 
+static_assert(sizeof(StageShared) <= 768, "StageShared: what the ring leaves");
 template <typename S>
 constexpr int smem_bytes() { return S::OFF_SH + (int)sizeof(StageShared); }
 
