@@ -351,11 +351,10 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             bool ok = true;
 #pragma unroll 1
             for (int L = 0; L < p.n_layers && ok; L++) {
-                // (a layer at a time, so that a launch that hangs does so at the wait that is to blame)
-                if (L) ok = mbar_wait(smem_u32(&sh->acc_full), (uint32_t)(L - 1) & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
                 const uint8_t* lut = p.layers[L].lut;
-                if (!lut || !ok) continue;
-                ok = mbar_wait(smem_u32(&sh->lut_empty), lut_par ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, p.wait_cycles);
+                if (!lut) continue;
+                // (twice the limit: whoever this wait depends on gives up first, and says where)
+                ok = mbar_wait(smem_u32(&sh->lut_empty), lut_par ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, 2 * p.wait_cycles);
                 lut_par ^= 1;
                 if (!ok) break;
                 mbar_expect_tx(smem_u32(&sh->lut_full), FACE_LUT_BYTES);
