@@ -876,6 +876,17 @@ void ffcu_face_free(FacePlan* p)
 
 int ffcu_face_pairs(const FacePlan* p) { return p->pairs; }
 
+// The next `launches` launches of a stage: the warp that loads first inputs and byte tables in the first CTA of each cluster stands still
+// for `cycles` in front of its first load and after each table (ordering tests: the results are the same).
+static int g_test_hold_launches = 0;
+static long long g_test_hold_cycles = 0;
+
+extern "C" void ffcu_test_hold_stage_loader(int launches, long long cycles)
+{
+    g_test_hold_launches = launches;
+    g_test_hold_cycles = cycles;
+}
+
 static FaceParams face_params(const FacePlan* p, int face0, int faces, int* d_err)
 {
     FaceParams prm = {};
@@ -886,6 +897,7 @@ static FaceParams face_params(const FacePlan* p, int face0, int faces, int* d_er
         if (g_test_chain_wait > 0) prm.wait_cycles = g_test_chain_wait;
         g_test_chain_drop_step = -1; g_test_chain_wait = 0;
     }
+    if (g_test_hold_launches > 0) { g_test_hold_launches--; prm.hold_cycles = g_test_hold_cycles; }
     return prm;
 }
 

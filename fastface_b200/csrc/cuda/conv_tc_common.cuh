@@ -144,6 +144,14 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Stands still for `cycles` (ordering tests; 0 elsewhere).
+__device__ __forceinline__ void tc_hold(long long cycles)
+{
+    if (cycles > 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < cycles) {}
+    }
+}
 // True in one lane of a converged warp, always the same one.
 __device__ __forceinline__ bool tc_elect_one()
 {
@@ -944,6 +952,7 @@ struct FaceParams {
     int n_layers, face0, faces;           // faces face0 .. face0 + faces - 1
     long long wait_cycles;                // limit of every barrier wait
     int drop_step;                        // >= 0: each pair's CTA 0 leaves out this ring step (timeout test); -1 otherwise
+    long long hold_cycles;                // > 0: the loader of each cluster's CTA 0 stands still this long at the places marked (ordering tests)
     int* err;
 };
 int tc_face_smem_bytes();

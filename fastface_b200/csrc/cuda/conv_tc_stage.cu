@@ -85,7 +85,7 @@ struct Stage {
 
 struct StageShared {
     uint64_t full[12], empty[12];
-    uint64_t a0_full;             // the first input has landed, and the padding's zeros in both buffers
+    uint64_t a0_full;             // the first input has landed
     uint64_t own_full;            // this CTA's results are in the next layer's input (sixteen warps, each part)
     uint64_t act_full[2];         // the others' are in buffer b's
     uint64_t acc_full;
@@ -248,6 +248,12 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         sh->unit_k[u] = (uint32_t)(((kh * 3 + kw) * S::CT + plane) * 128);
         sh->unit_db[u] = (uint32_t)((kh * S::ROW_BYTES + kw * 128 + plane * S::PLANE_BYTES) >> 4);
     }
+    if (S::BUFS == 2) {
+        // The second buffer's padding.  By stores in front of the cluster's barrier, not by a load of the first input as in the first buffer: the
+        // peers wait for their own loads only, and their first layer's rows may be here before a load of this CTA's has landed.
+        for (int i = threadIdx.x; i < S::ACT_BYTES / 16; i += TC_THREADS) *(int4*)(smem + S::ACT_BYTES + i * 16) = make_int4(0, 0, 0, 0);
+        fence_async_smem();
+    }
     if (S::F > 1) {
         // the two rows below the last face (the others' zeros come with the first input)
         for (int i = threadIdx.x; i < S::CT * 2 * S::ROW_BYTES / 16; i += TC_THREADS)
@@ -339,14 +345,16 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             }
         }
     } else if (warp == TC_ISSUER2_WARP) {
-        // The face's first input, into both buffers (of the second only the padding's zeros stay), and the fused BNs' byte tables
+        // The face's first input, and the fused BNs' byte tables
         if (tc_elect_one()) {
             tc_pdl_wait();
-            mbar_expect_tx(smem_u32(&sh->a0_full), S::BUFS * S::F * S::CT * S::BOX_ROWS * S::ROW_BYTES);
+            const long long hold = rank == 0 ? p.hold_cycles : 0;
+            tc_hold(hold);
+            mbar_expect_tx(smem_u32(&sh->a0_full), S::F * S::CT * S::BOX_ROWS * S::ROW_BYTES);
 #pragma unroll
-            for (int i = 0; i < S::BUFS * S::F * S::CT; i++)
-                tma_load_4d(s0 + i % (S::BUFS * S::CT) * S::PLANE_BYTES + i / (S::BUFS * S::CT) * (S::FACE_ROWS * S::ROW_BYTES), &mapA, smem_u32(&sh->a0_full),
-                            i % S::CT * 128, -1, S::first_row(t) - 1, p.face0 + cluster * S::F + i / (S::BUFS * S::CT));
+            for (int i = 0; i < S::F * S::CT; i++)
+                tma_load_4d(s0 + i % S::CT * S::PLANE_BYTES + i / S::CT * (S::FACE_ROWS * S::ROW_BYTES), &mapA, smem_u32(&sh->a0_full),
+                            i % S::CT * 128, -1, S::first_row(t) - 1, p.face0 + cluster * S::F + i / S::CT);
             uint32_t lut_par = 0;
             bool ok = true;
 #pragma unroll 1
@@ -359,6 +367,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                 if (!ok) break;
                 mbar_expect_tx(smem_u32(&sh->lut_full), FACE_LUT_BYTES);
                 bulk_load(s0 + S::OFF_LUT, lut + h * FACE_LUT_BYTES, FACE_LUT_BYTES, smem_u32(&sh->lut_full));
+                tc_hold(hold);
             }
         }
     } else {

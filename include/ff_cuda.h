@@ -157,6 +157,10 @@ void ffcu_test_arm_timeout(int drop_stage, long long full_wait_cycles);
  * sends, give up one limit later; all eight meet at the final cluster barrier, free their tensor memory
  * and return; the call reports 1000 + the error word.  Disarms itself after that one launch. */
 void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles);
+/* Ordering tests: in each of the next `launches` launches that take a stage in clusters (conv_tc_stage.cu) or CTA pairs
+ * (conv_tc_face.cu), the warp that loads first inputs and byte tables in the first CTA of every cluster stands still for `cycles`
+ * in front of its first load and after each table.  Results stay the same. */
+void ffcu_test_hold_stage_loader(int launches, long long cycles);
 /* The same for the split-K FC kernel: the activation box of K step drop_step never arrives in any CTA of the next FC
  * launch and every barrier wait of that launch is limited to wait_cycles; every CTA gives up, takes no ticket, frees
  * its tensor memory and returns; the call reports 1000 + the error word and clears the kernel's scratch sums. */
