@@ -46,6 +46,7 @@ struct FaceShared {
     uint64_t acc_full[2];         // slot's accumulator is complete
     uint64_t in_ready[2];         // (leader) both CTAs' own results are in place, and what came to CTA 1 from its peer
     uint64_t rx[2];               // what comes to this CTA from its peer has landed
+    uint64_t face_done[2];        // slot's last layer: its MMAs are done (for those who do not follow acc_full through all layers)
     uint64_t lut_full, lut_empty;
     uint32_t tmem_base;
     int abort_flag;
@@ -215,6 +216,7 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             mbar_init(smem_u32(&sh->acc_full[s]), 1);
             mbar_init(smem_u32(&sh->in_ready[s]), 33);        // both CTAs' epilogue warps, CTA 1's word that its rx is complete
             mbar_init(smem_u32(&sh->rx[s]), 1);
+            mbar_init(smem_u32(&sh->face_done[s]), 1);
         }
         mbar_init(smem_u32(&sh->lut_full), 1);
         mbar_init(smem_u32(&sh->lut_empty), 16);
@@ -325,6 +327,7 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                         // arm the barrier of what will come from the peer (bytes that land before this would only drive the
                         // count negative: the phase needs this arrival)
                         if (L + 1 < p.n_layers) mbar_expect_tx(smem_u32(&sh->rx[s]), STG_BYTES);
+                        else umma2_commit_both(smem_u32(&sh->face_done[s]));
                     }
                 }
             }
@@ -333,7 +336,7 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
         if (tc_elect_one()) {
             // CTA 1: tells the leader when what comes from it has landed
             const uint32_t leader_ready = map_to_cta(smem_u32(&sh->in_ready[0]), 0);
-            uint32_t rx_par = 0, acc_par = 0;
+            uint32_t rx_par = 0;
             bool ok = true;
 #pragma unroll 1
             for (int i = 0; i < rounds && ok; i++) {
@@ -348,17 +351,17 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
                             ok = mbar_wait_cluster(smem_u32(&sh->rx[s]), (rx_par >> s) & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
                             rx_par ^= bit;
                         } else {                              // nothing comes; not before the layer's own phase has begun, though
-                            ok = mbar_wait(smem_u32(&sh->acc_full[s]), (acc_par >> s) & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
+                            ok = mbar_wait(smem_u32(&sh->face_done[s]), (uint32_t)i & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
                         }
-                        acc_par ^= bit;
                         if (ok) mbar_arrive_release_cluster(leader_ready + (uint32_t)(s * 8));
                     }
                 }
             }
         }
     } else if (warp == TC_ISSUER2_WARP) {
-        // Faces' first inputs (a slot is free once its last face's MMAs are done) and the fused BNs' byte tables.  Goes through
-        // the accumulators in order: a parity says nothing about a phase that is two or more ahead.
+        // Faces' first inputs (a slot is free once its last face's MMAs are done) and the fused BNs' byte tables.  Waits only where the
+        // next phase needs what it does then: a parity says nothing about a phase that is two ahead, and the accumulators', which do
+        // not wait for this warp in a PReLU layer, could be.
         const uint32_t a0_leader = map_to_cta(smem_u32(&sh->a0_full[0]), 0);
         auto load_face = [&](int s, int j) {                  // the pair's j-th face
             if (lane == 0) {
@@ -369,32 +372,34 @@ conv_face_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             }
             __syncwarp();
         };
-        uint32_t acc_par = 0, lut_par = 0;
+        const long long hold = rank == 0 ? p.hold_cycles : 0;
+        uint32_t lut_par = 0;
         bool ok = true;
         tc_pdl_wait();
+        tc_hold(hold);
         for (int j = 0; j < 2 && j < nf; j++) load_face(j, j);
 #pragma unroll 1
         for (int i = 0; i < rounds && ok; i++) {
-            const int slots = nf - 2 * i < 2 ? 1 : 2;
 #pragma unroll 1
             for (int L = 0; L < p.n_layers && ok; L++) {
                 const uint8_t* lut = p.layers[L].lut;
-                if (lut) {
-                    ok = mbar_wait(smem_u32(&sh->lut_empty), lut_par ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, p.wait_cycles);
-                    lut_par ^= 1;
-                    if (ok && lane == 0) {
-                        mbar_expect_tx(smem_u32(&sh->lut_full), LUT_BYTES);
-                        bulk_load(s0 + OFF_LUT, lut + rank * LUT_BYTES, LUT_BYTES, smem_u32(&sh->lut_full));
-                    }
-                    __syncwarp();
+                if (!lut) continue;
+                // (twice the limit: whoever this wait depends on gives up first, and says where)
+                ok = mbar_wait(smem_u32(&sh->lut_empty), lut_par ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT, 2 * p.wait_cycles);
+                lut_par ^= 1;
+                if (ok && lane == 0) {
+                    mbar_expect_tx(smem_u32(&sh->lut_full), LUT_BYTES);
+                    bulk_load(s0 + OFF_LUT, lut + rank * LUT_BYTES, LUT_BYTES, smem_u32(&sh->lut_full));
                 }
+                __syncwarp();
+                tc_hold(hold);
+            }
 #pragma unroll 1
-                for (int s = 0; s < slots && ok; s++) {
-                    ok = mbar_wait(smem_u32(&sh->acc_full[s]), (acc_par >> s) & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, p.wait_cycles);
-                    acc_par ^= 1u << s;
-                    const int j = 2 * (i + 1) + s;
-                    if (ok && L + 1 == p.n_layers && j < nf) load_face(s, j);
-                }
+            for (int s = 0; s < 2 && ok; s++) {
+                const int j = 2 * (i + 1) + s;
+                if (j >= nf) break;
+                ok = mbar_wait(smem_u32(&sh->face_done[s]), (uint32_t)i & 1, abort_flag, p.err, FFCU_ERR_EPI_TIMEOUT, 2 * p.wait_cycles);
+                if (ok) load_face(s, j);
             }
         }
     } else {

@@ -82,7 +82,8 @@ def test_bounded_waits_run_out(built_lib, model_root, ffw4, oracle, n):
             assert np.array_equal(e.embed_batch(faces), want)
 
 
-@pytest.mark.parametrize("n", [1, 17, 64], ids=["clusters-of-eight", "clusters-of-four", "two-faces-a-cluster"])
+@pytest.mark.parametrize("n", [1, 17, 64, 80, 160, 296, 330], ids=["clusters-of-eight", "clusters-of-four", "two-faces-a-cluster", "a-pair-and-two-faces",
+                                                                   "pairs-and-clusters", "two-rounds", "three-rounds"])
 def test_a_late_loader_changes_nothing(built_lib, model_root, ffw4, oracle, n):
     """One CTA of each cluster loads its first input, and every byte table, several layers' time (a layer takes five to ten thousand
     cycles) after the others have theirs: neighbours' first results must not be overwritten by an input that lands after them, and
@@ -92,7 +93,7 @@ def test_a_late_loader_changes_nothing(built_lib, model_root, ffw4, oracle, n):
     lib.ffcu_test_hold_stage_loader.argtypes = [C.c_int, C.c_longlong]
     faces = synth.faces(n, seed=79)
     want = oracle.forward(faces[[0, n - 1]], ffo.CONTRACT)
-    with ff.FastFace(ffw4, cwd=model_root, max_batch=160) as e:
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=330) as e:
         lib.ffcu_test_hold_stage_loader(8, 40_000)              # a shape's first call runs eagerly
         held = e.embed_batch(faces)
         lib.ffcu_test_hold_stage_loader(0, 0)
