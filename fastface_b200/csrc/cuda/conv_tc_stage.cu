@@ -396,7 +396,7 @@ conv_stage_kernel(const __grid_constant__ CUtensorMap mapA, const FaceParams p)
             if (bn) {
                 lut_par ^= 1;
                 __syncwarp();
-                if (lane == 0) mbar_arrive_relaxed(smem_u32(&sh->lut_empty));
+                if (lane == 0) mbar_arrive(smem_u32(&sh->lut_empty));
             }
         }
     }
