@@ -326,6 +326,7 @@ static int launch_rows(int m, int n_sm)
 int CosWorkspace::run_pipeline(int n_sm, const float* ha, int n, const float* hb, int m, float* hout, bool in_a, bool in_b, bool out_staged)
 {
     const size_t in_bytes = (size_t)(n + m) * CS_DIM * 4, out_bytes = (size_t)n * m * 4;
+    pieces_in = 0;                                    // the last call has waited for its copies: the ring is free (and the count cannot run over)
     if (in_a && in_b && out_staged && in_bytes <= CS_PIECE && out_bytes <= CS_PIECE) {
         // a small matrix: both inputs in one copy, everything in order on one stream (1 x 100 / 1 x 300: 63 / 77 -> 53 / 60 us)
         if (!grow(&b, &cap_b, (size_t)(n + m) * CS_DIM) || !grow(&out, &cap_out, (size_t)n * m)) {
