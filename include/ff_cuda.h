@@ -185,7 +185,7 @@ int ffcu_fc_small_noalloc(const int8_t* act, const int8_t* w, const float* w_sca
 /* Cosine-similarity matrix out[n][m] of host embeddings a[n][512], b[m][512] with the float64
  * accumulation of the reference's Go wrapper (go/fastface/fastface.go:157-168), bit for bit. */
 int ffcu_cos_sim_matrix(int device, const float* a, int n, const float* b, int m, float* out);
-/* The same on the context's device, with device buffers (at most 57 MB, and 8 MB page-locked) that the context keeps from its first call to
+/* The same on the context's device, with device buffers (at most 68 MB, and 8 MB page-locked) that the context keeps from its first call to
  * ffcu_destroy.  May be called from several threads at once, also beside ffcu_submit. */
 int ffcu_ctx_cos_sim_matrix(ffcu_ctx* c, const float* a, int n, const float* b, int m, float* out);
 

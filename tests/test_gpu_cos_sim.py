@@ -98,7 +98,7 @@ def test_matrix_from_several_threads(engine):
     assert not bad
 
 
-@pytest.mark.parametrize("n,m,over", [(500, 5000, "b"), (2500, 520, "a"), (300, 600, "b")])
+@pytest.mark.parametrize("n,m,over", [(500, 5000, "b"), (2500, 520, "a"), (300, 600, "b"), (2048, 1400, "a"), (2048, 4096, "b")])
 def test_matrix_written_over_an_input(engine, n, m, over):
     """A result that takes the place of an input, also where the matrix goes in slices: the inputs are read first."""
     rng = np.random.default_rng(n + m)
