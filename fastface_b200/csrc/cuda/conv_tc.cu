@@ -1,5 +1,5 @@
 // conv_tc.cu -- host side of the tensor-core convolution: per-layer kernel choice, tile
-// geometry, TMA descriptors, launch.  The kernels live in conv_tc_{generic,ws,pair,k32}.cu.
+// geometry, TMA descriptors, launch.  The kernels live in conv_tc_*.cu.
 #include "conv_tc_common.cuh"
 #include <algorithm>
 #include <vector>
@@ -639,159 +639,6 @@ int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, 
 }
 
 // ---------------------------------------------------------------------------
-// Layer chain (conv_tc_chain.cu): plan = the first input's tensor map, the per-layer records in
-// device memory (weights' tensor map, table / buffer pointers) and the shared-memory budget
-// ---------------------------------------------------------------------------
-struct ChainPlan {
-    CUtensorMap mapA;
-    ChainLayer* d_layers;
-    ChainParams prm;
-    int smem_bytes;
-    int clusters;            // clusters the device holds at once
-    int bn;                  // output channels per CTA: 64 (eight CTAs per face) or 128 (four)
-};
-
-// layers[i]: device pointers of layer i (weights, tables, residual, outputs); all layers are 3x3 stride-1
-// pad-1 convolutions C -> C on an H x W map, layer i + 1 reading what layer i writes (its fused BN's
-// output where it has one).  d_in = the first layer's input (max_batch faces, NHWC; a launch of n faces reads the first n).
-// bn = output channels per CTA (64: clusters of eight, 128: of four).  NULL when the shape does
-// not fit the kernel (C / bn column tiles x row tiles of 128 positions must be exactly a cluster's CTAs).
-ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers)
-{
-    encode_tiled_fn enc = get_encode();
-    if (!enc || n_layers < 2 || C % 128 != 0 || C > TC_MAX_COUT) return nullptr;
-    // pitch: a power of two >= W + 1.  With P = W + 1 the right-hand padding of a row is the next row's
-    // left-hand slot, and the last tap of the last row reads one line past row H: one more (zero) row.
-    int P = 1;
-    while (P < W + 1) P <<= 1;
-    const int tiles_n = C / bn;
-    const int tiles_m = (H * P + TC_TILE_M - 1) / TC_TILE_M;
-    // rows a CTA holds: the padded rows its row tile's outputs read (first output row .. last + 2)
-    int rows = 0;
-    for (int t = 0; t < tiles_m; t++) {
-        const int olo = (t * TC_TILE_M) / P;
-        int ohi = (t * TC_TILE_M + TC_TILE_M - 1) / P;
-        if (ohi > H - 1) ohi = H - 1;
-        if (ohi - olo + 3 > rows) rows = ohi - olo + 3;
-    }
-    rows += (P == W + 1 ? 1 : 0);
-    if (tiles_n * tiles_m != CHAIN_CLUSTER_OF(bn) || P > 256 || P % 8 != 0 || rows > 256) return nullptr;
-    const int planes = C / 128;
-    if (planes != 2 && planes != 4) return nullptr;       // the issue loops are built for 256 and 512 channels
-    const int plane_bytes = P * rows * 128;
-    if (plane_bytes % 1024 != 0) return nullptr;
-    const int fixed = 2 * planes * plane_bytes + bn * 256 + 5 * bn * 4 + 512 /* barriers */ + 1024 /* alignment */;
-    // Filter taps per stage of the weight ring (1, or 3 where two such stages fit and $FF_CHAIN_TPS=3 asks for it).
-    int tps = 1;
-    { const char* e = getenv("FF_CHAIN_TPS"); if (e && (atoi(e) == 1 || atoi(e) == 3) && planes == 2) tps = atoi(e); }
-    while (tps > 1 && (232448 - fixed) / (tps * planes * bn * 128) < 2) tps /= 3;
-    const int stage_bytes = bn == 128 ? bn * 128 : tps * planes * bn * 128;
-    int stages = (232448 - fixed) / stage_bytes;
-    if (stages > CHAIN_MAX_STAGES) stages = CHAIN_MAX_STAGES;
-    stages &= ~1;                                         // two issuers on alternate stages: the ring must be even
-    if (stages < 2) return nullptr;
-    const int clusters = tc_chain_clusters(bn, fixed + stages * stage_bytes);
-    if (clusters < 1) return nullptr;                     // no room for a cluster on this device
-    ChainPlan* p = new ChainPlan();
-    p->d_layers = nullptr;
-    {
-        cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)max_batch};
-        cuuint64_t strides[3] = {(cuuint64_t)C, (cuuint64_t)C * W, (cuuint64_t)C * W * H};
-        cuuint32_t box[4] = {128, (cuuint32_t)P, (cuuint32_t)rows, 1};
-        cuuint32_t es[4] = {1, 1, 1, 1};
-        CUresult r = enc(&p->mapA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d_in, dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { ffcu_set_error("cuTensorMapEncodeTiled(chain A) failed: %d", (int)r); delete p; return nullptr; }
-    }
-    std::vector<ChainLayer> h((size_t)n_layers);
-    memset(h.data(), 0, h.size() * sizeof(ChainLayer));
-    for (int i = 0; i < n_layers; i++) {
-        const ChainLayerDesc& d = layers[i];
-        cuuint64_t Ktot = (cuuint64_t)9 * C;
-        cuuint64_t dims[4] = {Ktot, (cuuint64_t)C, 1, 1};
-        cuuint64_t strides[3] = {Ktot, Ktot * C, Ktot * C};
-        cuuint32_t box[4] = {128, (cuuint32_t)bn, 1, 1};
-        cuuint32_t es[4] = {1, 1, 1, 1};
-        CUresult r = enc(&h[i].mapB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)d.w, dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { ffcu_set_error("cuTensorMapEncodeTiled(chain B) failed: %d", (int)r); delete p; return nullptr; }
-        h[i].w_scale = d.t.w_scale; h[i].bias = d.t.bias; h[i].slope = d.t.slope;
-        h[i].res_scale = d.res ? d.t.res_scale : nullptr; h[i].inv_out = d.t.inv_out;
-        h[i].lut = (d.out2 && d.t.bn_lut) ? d.t.bn_lut : nullptr;
-        h[i].res = (d.res && d.t.res_scale) ? d.res : nullptr;
-        h[i].out = d.out; h[i].out2 = (d.out2 && d.t.bn_lut) ? d.out2 : nullptr;
-    }
-    if (cudaMalloc(&p->d_layers, h.size() * sizeof(ChainLayer)) != cudaSuccess ||
-        cudaMemcpy(p->d_layers, h.data(), h.size() * sizeof(ChainLayer), cudaMemcpyHostToDevice) != cudaSuccess) {
-        ffcu_set_error("layer chain: device allocation or upload failed");
-        cudaFree(p->d_layers); cudaGetLastError(); delete p; return nullptr;
-    }
-    p->prm.layers = p->d_layers; p->prm.n_layers = n_layers;
-    p->prm.H = H; p->prm.W = W; p->prm.P = P; p->prm.C = C;
-    p->prm.planes = planes; p->prm.plane_bytes = plane_bytes; p->prm.win_rows = rows; p->prm.tiles_n = tiles_n; p->prm.stages = stages; p->prm.tps = tps;
-    p->prm.err = nullptr;
-    p->smem_bytes = fixed + stages * stage_bytes;
-    p->clusters = clusters; p->bn = bn;
-    return p;
-}
-
-int ffcu_chain_clusters(const ChainPlan* p) { return p->clusters; }
-
-void ffcu_chain_free(ChainPlan* p)
-{
-    if (!p) return;
-    cudaFree(p->d_layers);
-    delete p;
-}
-
-// One-shot fault injection for the layer chain's timeout-path test: consumed by the next chain launch.
-static int g_test_chain_drop_step = -1;
-static long long g_test_chain_wait = 0;
-
-extern "C" void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles)
-{
-    g_test_chain_drop_step = drop_step;
-    g_test_chain_wait = wait_cycles;
-}
-
-int ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s)
-{
-    ChainParams prm = p->prm;
-    prm.err = d_err;
-    prm.wait_cycles = TC_WAIT_CYCLES; prm.drop_step = -1;
-    if (g_test_chain_drop_step >= 0) {                    // armed for this one launch
-        prm.drop_step = g_test_chain_drop_step;
-        if (g_test_chain_wait > 0) prm.wait_cycles = g_test_chain_wait;
-        g_test_chain_drop_step = -1; g_test_chain_wait = 0;
-    }
-#ifdef FF_TC_TIMING
-    // timing build, $FF_CHAIN_TS=1: the 30th launch of a chain prints CTA 0's per-layer time stamps
-    { static int dbg = -1; if (dbg < 0) { const char* e = getenv("FF_TC_DBG"); dbg = e ? atoi(e) : 0; } prm.dbg = dbg; }
-    static unsigned long long* d_ts = nullptr;
-    static int calls = 0;
-    prm.ts = nullptr;
-    if (getenv("FF_CHAIN_TS")) {
-        if (!d_ts) cudaMalloc(&d_ts, 64 * 4 * sizeof(unsigned long long));
-        prm.ts = d_ts;
-        if (++calls == 29 || calls == 30) {
-            int rc = tc_launch_chain(p->bn, mode, faces, p->smem_bytes, s, p->mapA, prm);
-            cudaStreamSynchronize(s);
-            unsigned long long h[256];
-            cudaMemcpy(h, d_ts, sizeof h, cudaMemcpyDeviceToHost);
-            for (int L = 0; L < prm.n_layers; L++)
-                fprintf(stderr, "chain L%d: in->mma_issued %lld, mma_issued->acc %lld, acc->sent %lld, sent->next_in %lld ns\n", L,
-                        (long long)(h[4 * L + 1] - h[4 * L]), (long long)(h[4 * L + 2] - h[4 * L + 1]), (long long)(h[4 * L + 3] - h[4 * L + 2]),
-                        L + 1 < prm.n_layers ? (long long)(h[4 * L + 4] - h[4 * L + 3]) : 0ll);
-            return rc;
-        }
-    }
-#endif
-    return tc_launch_chain(p->bn, mode, faces, p->smem_bytes, s, p->mapA, prm);
-}
-
-// ---------------------------------------------------------------------------
 // Stages taken face by face: a cluster per face (conv_tc_stage.cu), the 14x14 one also with a CTA pair per two (conv_tc_face.cu)
 // ---------------------------------------------------------------------------
 struct FacePlan {
@@ -876,6 +723,16 @@ void ffcu_face_free(FacePlan* p)
 
 int ffcu_face_pairs(const FacePlan* p) { return p->pairs; }
 
+// One-shot fault injection for the stages' timeout-path tests: consumed by the next launch of one.
+static int g_test_stage_drop_step = -1;
+static long long g_test_stage_wait = 0;
+
+extern "C" void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles)
+{
+    g_test_stage_drop_step = drop_step;
+    g_test_stage_wait = wait_cycles;
+}
+
 // The next `launches` launches of a stage: the warp that loads first inputs and byte tables in the first CTA of each cluster stands still
 // for `cycles` in front of its first load and after each table (ordering tests: the results are the same).
 static int g_test_hold_launches = 0;
@@ -892,10 +749,10 @@ static FaceParams face_params(const FacePlan* p, int face0, int faces, int* d_er
     FaceParams prm = {};
     prm.layers = p->d_layers; prm.kept = p->d_kept; prm.n_layers = p->n_layers; prm.face0 = face0; prm.faces = faces; prm.err = d_err;
     prm.wait_cycles = TC_WAIT_CYCLES; prm.drop_step = -1;
-    if (g_test_chain_drop_step >= 0) {                    // armed for this one launch
-        prm.drop_step = g_test_chain_drop_step;
-        if (g_test_chain_wait > 0) prm.wait_cycles = g_test_chain_wait;
-        g_test_chain_drop_step = -1; g_test_chain_wait = 0;
+    if (g_test_stage_drop_step >= 0) {                    // armed for this one launch
+        prm.drop_step = g_test_stage_drop_step;
+        if (g_test_stage_wait > 0) prm.wait_cycles = g_test_stage_wait;
+        g_test_stage_drop_step = -1; g_test_stage_wait = 0;
     }
     if (g_test_hold_launches > 0) { g_test_hold_launches--; prm.hold_cycles = g_test_hold_cycles; }
     return prm;

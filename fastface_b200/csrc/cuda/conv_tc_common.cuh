@@ -38,11 +38,6 @@
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ uint64_t globaltimer_ns()
-{
-    uint64_t t; asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)); return t;
-}
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -128,13 +123,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
                  "[%0], [%1, {%3, %4, %5, %6}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                 "[%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after()  { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -163,19 +151,6 @@ __device__ __forceinline__ bool tc_elect_one()
 __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&v)[32])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                   "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                   "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // ---- CTA-pair (cta_group::2) helpers: cluster of two CTAs on one TPC -------------------
@@ -208,12 +183,6 @@ __device__ __forceinline__ void tma2_load_4d(uint32_t dst, const CUtensorMap* ma
     asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
                  "[%0], [%1, {%3, %4, %5, %6}], [%2];"
                  ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void tma2_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1)
-{
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                 "[%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void umma2_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
@@ -259,18 +228,6 @@ __device__ __forceinline__ uint32_t mbar_test_cluster(uint32_t bar, uint32_t par
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, int (&v)[32]) { tmem_ld32(taddr, v); }
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, int (&v)[16]) { tmem_ld16(taddr, v); }
 
 // K-major shared-memory matrix descriptor: rows of ROWB bytes (= swizzle span), 8-row groups
 // 8*ROWB bytes apart, descriptor version 1 (sm_100), layout 2 = 128B swizzle / 4 = 64B swizzle.
@@ -366,7 +323,7 @@ enum { EPI_RUNTIME = 0, EPI_PLAIN = 1, EPI_SLOPE = 2, EPI_RES_BN = 3, EPI_RES = 
 // epilogue warps and back, so the issuer must be able to run several tiles ahead.
 #define TC_MAX_ACC 8
 #define TC_NACC(BN) (512 / (BN) > TC_MAX_ACC ? TC_MAX_ACC : 512 / (BN))
-// Warps 0 .. 15: epilogue, 16: TMA producer, 17: second MMA issuer (weight-stationary kernels, chains; the stem's second
+// Warps 0 .. 15: epilogue, 16: TMA producer, 17: second MMA issuer (weight-stationary kernels; the stem's second
 // producer; idle elsewhere), 18: MMA issuer.  The issuer shares its scheduler with four epilogue warps, and the scheduler
 // prefers the highest-numbered warp that is ready: with sixteen warps of independent FMAs beside it, one M = 256, N = 224
 // MMA was issued every 365 cycles by warp 1 and every 158 by warp 18 (110 alone, the tensor rate).  An issuer's loop
@@ -597,7 +554,7 @@ __device__ __forceinline__ void tc_fc16(const TcParams& p, const float* tab, con
 
 // Programmatic dependent launch.  Each tensor-core kernel is launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization.  tc_pdl_trigger, the kernel's first
-// statement (a layer chain's at its last layer), lets the NEXT kernel of the stream become resident at once (on SMs this one leaves
+// statement (in the stages' kernels at their last layer), lets the NEXT kernel of the stream become resident at once (on SMs this one leaves
 // free: always the case at small batch, where a launch is 8-16 CTAs), so that its launch latency
 // and set-up (barriers, TMEM, the per-channel tables, which no kernel writes) are hidden several
 // kernels deep.  tc_pdl_wait blocks until the PREVIOUS kernel has completed and its stores are
@@ -613,7 +570,7 @@ __device__ __forceinline__ void tc_pdl_wait()
 }
 
 // Launch with the programmatic-serialisation attribute, as clusters of `cluster` CTAs when that is
-// 2 or more (the CTA-pair kernels, the eight-CTA layer chain).  $FF_PDL=0 launches the plain way.
+// 2 or more (the CTA-pair kernels, the stages in clusters).  $FF_PDL=0 launches the plain way.
 template <typename... KArgs, typename... Args>
 static int tc_launch_ex(void (*kern)(KArgs...), int grid, int smem, cudaStream_t s, int cluster, Args&&... args)
 {
@@ -893,45 +850,6 @@ struct FcTcParams {
     long long wait_cycles;   // limit of every barrier wait
 };
 int tc_launch_fc(int mode, int grid, int smem, cudaStream_t s, const CUtensorMap& mapX, const CUtensorMap& mapW, const FcTcParams& prm);
-
-// Layer chain (conv_tc_chain.cu)
-#define CHAIN_BN 64                       // output channels per CTA: 64, or 128 in the wide form
-#define CHAIN_CLUSTER_OF(BN) (512 / (BN))   // CTAs per face: two row tiles of 256 channels, or one of 512
-#define CHAIN_MAX_STAGES 8
-#define CHAIN_EPI_WARPS 16
-#define CHAIN_EPI_THREADS (32 * CHAIN_EPI_WARPS)
-
-struct ChainLayer {                       // one layer of the chain, in global memory (256 bytes, 128-byte aligned)
-    CUtensorMap mapB;                     // weights [Cout][9 * C] K-major, box {128, 64 or 128}
-    const float* w_scale; const float* bias; const float* slope; const float* res_scale; const float* inv_out;
-    const int8_t* lut;                    // fused BN byte table [Cout][256], or NULL
-    const int8_t* res;                    // residual (NHWC int8), or NULL
-    int8_t* out;                          // NHWC int8 output
-    int8_t* out2;                         // fused BN second output, or NULL
-    uint8_t pad_[256 - 128 - 9 * 8];
-};
-static_assert(sizeof(ChainLayer) == 256, "ChainLayer layout");
-
-struct ChainParams {
-    const ChainLayer* layers;
-    int n_layers;
-    int H, W, P, C;                       // feature map, pitch in lines, channels (in = out)
-    int planes, plane_bytes;              // C / 128 planes of P * win_rows lines of 128 bytes
-    int win_rows;                         // padded rows a CTA holds (the rows its row tile reads)
-    int tiles_n;                          // C / 64 (wide form: / 128) column tiles
-    int stages;                           // weight ring (wide form: slots of one plane of one tap, two per step)
-    int tps;                              // filter taps per stage (1 or 3), planes x 8 KB each
-    long long wait_cycles;                // limit of every barrier wait (TC_WAIT_CYCLES unless a test shortened it)
-    int drop_step;                        // >= 0: CTA 0's producer leaves out this ring step (ffcu_test_arm_chain_timeout; -1 otherwise)
-    int* err;
-#ifdef FF_TC_TIMING
-    unsigned long long* ts;               // timing build: per layer 4 time stamps of CTA 0 (ns)
-    int dbg;                              // timing build: bit 0 = skip the weight loads (wrong results)
-#endif
-};
-
-int tc_launch_chain(int bn, int mode, int faces, int smem, cudaStream_t s, const CUtensorMap& mapA, const ChainParams& prm);
-int tc_chain_clusters(int bn, int smem);
 
 // 14x14 stage, a CTA pair per face (conv_tc_face.cu)
 #define FACE_C FFCU_FACE_C

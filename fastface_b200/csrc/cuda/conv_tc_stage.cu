@@ -1,4 +1,4 @@
-// conv_tc_stage.cu -- small batches: a stage (a run of 3x3 stride-1 C -> C convolutions) in ONE launch, a cluster of four to eight
+// conv_tc_stage.cu -- small batches: a stage (a run of 3x3 stride-1 C -> C convolutions) in ONE launch, a cluster of two to eight
 // CTAs per face, activations in shared memory: 128 channels on 28x28 maps, 256 on 14x14, 512 on 7x7.
 //
 // The operands as in conv_tc_face.cu (weights are the MMA's 128 rows, a row of the face 8, 16 or 32 of its columns), but every
@@ -26,7 +26,7 @@
 // Bound: latency.  What passes between shared memories goes at 20 B per cycle and CTA whatever instruction sends it (measured:
 // 8 KB to 1 / 2 / 4 / 8 CTAs of a cluster of eight 710 / 1110 / 1920 / 3550 cycles by 16-byte st.async, 810 / 1210 / 2005 / 3790 by
 // bulk copies), so the split is the one that sends least: at 14x14 16 KB per CTA and layer instead of 36 KB for 2 row tiles x 4
-// channel tiles (conv_tc_chain.cu).
+// channel tiles (an earlier kernel with positions as the MMA's rows, the "chain" below).
 // Forward of 1 / 4 / 8 / 15 faces, 14x14 stage by that chain -> clusters of eight: 273 / 287 / 309 / 349 -> 230 / 249 / 267 / 304 us; of
 // 16 / 17 / 24 / 33 faces, its wide form -> clusters of four: 409 / 413 / 445 / 487 -> 357 / 361 / 396 / 435 us (layers 5.1 -> 3.5 and 7 -> 5 us).
 // The 28x28 stage by one launch per layer and the 7x7 one by that chain (from 25 faces a launch per layer): forward of 1 / 8 / 15 /

@@ -110,14 +110,8 @@ struct ffcu_ctx {
     int graph_max_batch = 1 << 30;
     std::map<long long, cudaGraphExec_t> graphs;
     std::map<long long, int> graph_launches;
-    // Small batches: runs of same-shape 3x3 stride-1 convolutions (the 14x14 and 7x7 stages) go out as one
-    // launch each (conv_tc_chain.cu).  Found on the first such forward; FF_CHAIN=0 disables.
-    struct Chain { size_t first; int count; ChainPlan* plan[2]; };   // clusters of eight (64 channels per CTA), of four (128)
-    std::vector<Chain> chains;
-    bool chains_built = false;
-    int no_chain = 0;
     // The 28x28, 14x14 and 7x7 stages as one launch each, a cluster per face (conv_tc_stage.cu), beyond what the device holds
-    // clusters for a CTA pair per two faces of the 14x14 one (conv_tc_face.cu); FF_FACE=0 disables.
+    // clusters for a CTA pair per two faces of the 14x14 one (conv_tc_face.cu); FF_FACE=0 or FF_CHAIN=0 disables.
     struct FaceRun { size_t first; int count, H; FacePlan* plan; };
     std::vector<FaceRun> runs;
     int no_clusters = 0;         // a cluster launch was refused
@@ -218,7 +212,6 @@ extern "C" ffcu_ctx* ffcu_create(int device, int max_batch, int n_bufs, size_t b
     { const char* e = getenv("FF_FC_SMALL_MAX"); if (e && atoi(e) >= 0 && atoi(e) <= FFCU_FC_SMALL_MAX_BATCH) c->fc_small_max = atoi(e); }
     { const char* e = getenv("FF_GRAPH_MAX_BATCH"); if (e && atoi(e) > 0) c->graph_max_batch = atoi(e); }
     { const char* e = getenv("FF_GRAPH"); if (e && e[0] == '0') c->graph_max_batch = 0; }
-    { const char* e = getenv("FF_CHAIN"); c->no_chain = (e && e[0] == '0') ? 1 : 0; }
     { const char* e = getenv("FF_LEAN_MAX_BATCH"); if (e && atoi(e) >= 0) c->lean_max_batch = atoi(e); }
     if (!ok) {
         ffcu_set_error("device allocation failed on device %d: %s", device, cudaGetErrorString(cudaGetLastError()));
@@ -240,7 +233,6 @@ extern "C" void ffcu_destroy(ffcu_ctx* c)
         if (s && cudaStreamSynchronize(s) != cudaSuccess) done = false;
     for (int k = 0; k < 2 && done; k++) deliver(c, k);    // outputs nobody has waited for
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-    for (auto& ch : c->chains) for (ChainPlan* q : ch.plan) ffcu_chain_free(q);
     for (auto& run : c->runs) ffcu_face_free(run.plan);
     for (auto& L : c->layers) {
         for (TcPlan* q : L.tc_bn) if (q) ffcu_tc_free(q);      // L.tc is one of them
@@ -400,9 +392,9 @@ static void find_heads(ffcu_ctx* c)
     c->head_end[1] = 2;
 }
 
-// A layer the chain kernel can take: tensor-core 3x3 stride-1 pad-1 convolution C -> C (C = 256 or 512)
-// with the no-overflow proof, its fused BN (if any) as a byte table.
-static bool chain_eligible(const ffcu_ctx* c, const DevLayer& L)
+// A layer of a stage: tensor-core 3x3 stride-1 pad-1 convolution C -> C with the no-overflow proof, its fused BN (if any) as a
+// byte table.
+static bool stage_layer(const ffcu_ctx* c, const DevLayer& L)
 {
     const ffcu_layer& d = L.d;
     return d.kind == FFCU_CONV && L.tc && !L.skip && !L.fused_stem && !c->force_simt && d.Kh == 3 && d.Kw == 3 &&
@@ -410,12 +402,12 @@ static bool chain_eligible(const ffcu_ctx* c, const DevLayer& L)
            d.Ho == d.H && d.Wo == d.W && L.epi.no_overflow && (d.bn2_dst_buf < 0 || L.bn_lut != nullptr);
 }
 
-// End of the run of layers from k on that the chain kernels can take: one shape, each reading what the one before it wrote.
-static size_t chain_end(const ffcu_ctx* c, size_t k)
+// End of the run of such layers from k on: one shape, each reading what the one before it wrote.
+static size_t stage_end(const ffcu_ctx* c, size_t k)
 {
-    if (!chain_eligible(c, c->layers[k])) return k;
+    if (!stage_layer(c, c->layers[k])) return k;
     size_t e = k + 1;
-    for (; e < c->layers.size() && chain_eligible(c, c->layers[e]) && c->layers[e].d.H == c->layers[k].d.H &&
+    for (; e < c->layers.size() && stage_layer(c, c->layers[e]) && c->layers[e].d.H == c->layers[k].d.H &&
            c->layers[e].d.Cout == c->layers[k].d.Cout; e++) {
         const ffcu_layer& prev = c->layers[e - 1].d;
         if (c->layers[e].d.src_buf != (prev.bn2_dst_buf >= 0 ? prev.bn2_dst_buf : prev.dst_buf)) break;
@@ -426,13 +418,15 @@ static size_t chain_end(const ffcu_ctx* c, size_t k)
 // The stages that go face by face, which leaves only their last layers' tensors in memory (ff_plan_stage).
 static void build_face_runs(ffcu_ctx* c)
 {
-    const char* e = getenv("FF_FACE");
-    if (c->no_chain || (e && e[0] == '0')) return;
+    for (const char* name : {"FF_FACE", "FF_CHAIN"}) {
+        const char* e = getenv(name);
+        if (e && e[0] == '0') return;
+    }
     std::vector<ffcu_layer> d;
     for (const DevLayer& L : c->layers) d.push_back(L.d);
     size_t end;
     for (size_t k = 0; k < d.size(); k = end > k ? end : k + 1) {
-        end = chain_end(c, k);
+        end = stage_end(c, k);
         if (end < k + 2) continue;
         const int n = (int)(end - k);
         const size_t C = (size_t)d[k].Cout;
@@ -604,61 +598,10 @@ static int launch_layer(ffcu_ctx* c, size_t k, int n, int32_t* acc_dbg, bool unf
     return -1;
 }
 
-static void build_chains(ffcu_ctx* c)
-{
-    c->chains_built = true;
-    if (c->no_chain) return;
-    size_t k = 0;
-    while (k < c->layers.size()) {
-        const size_t e = chain_end(c, k);
-        if (e == k) { k++; continue; }
-        const int count = (int)(e - k);
-        if (count >= 2) {
-            std::vector<ChainLayerDesc> desc((size_t)count);
-            for (int i = 0; i < count; i++) {
-                const DevLayer& L = c->layers[k + i];
-                desc[i].w = L.w; desc[i].t = L.epi;
-                desc[i].res = L.d.res_buf >= 0 ? c->bufs[L.d.res_buf] : nullptr;
-                desc[i].out = c->bufs[L.d.dst_buf];
-                desc[i].out2 = L.d.bn2_dst_buf >= 0 ? c->bufs[L.d.bn2_dst_buf] : nullptr;
-            }
-            const ffcu_layer& d0 = c->layers[k].d;
-            ffcu_ctx::Chain ch = {k, count, {nullptr, nullptr}};
-            ch.plan[0] = ffcu_chain_plan(64, d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
-            // the wide form serves calls beyond what clusters of eight hold
-            if (ch.plan[0] && c->max_batch > ffcu_chain_clusters(ch.plan[0]))
-                ch.plan[1] = ffcu_chain_plan(128, d0.H, d0.W, d0.Cout, c->max_batch, c->bufs[d0.src_buf], desc.data(), count);
-            if (ch.plan[0]) c->chains.push_back(ch);
-        }
-        k = e;
-    }
-}
-
-// Largest call that takes the layer chains (each chain's own limit, the clusters the device holds at once, comes on
-// top: one cluster works on one face, and a second wave of clusters doubles the stage's time).  Measured, forward of
-// 2 / 4 / 8 / 12 faces, chains against one launch per layer: 300 / 311 / 332 / 363 us against 366 / 379 / 403 / 445; the wide
-// form's figures stand in conv_tc_chain.cu.  A context made for two or three faces keeps one launch per layer beyond a
-// single face, the launch count fastface_launches_per_forward has always given there.
-static int chain_max_faces(const ffcu_ctx* c)
-{
-    return c->max_batch >= 4 ? FFCU_CHAIN_MAX_FACES : 1;
-}
-
-// The chain that starts at layer k, in the narrowest clusters of which the device holds n at once; NULL: none.
-static const ffcu_ctx::Chain* chain_at(const ffcu_ctx* c, size_t k, int n, const ChainPlan** plan)
-{
-    *plan = nullptr;
-    for (const ffcu_ctx::Chain& ch : c->chains)
-        if (ch.first == k)
-            for (const ChainPlan* q : ch.plan)
-                if (!*plan && q && n <= ffcu_chain_clusters(q)) { *plan = q; return &ch; }
-    return nullptr;
-}
-
 // The run of layers that starts at k and that a call of n faces takes face by face; NULL: none.  28x28 and 7x7 maps only while the
 // device holds all their clusters at once: in rounds they lose to one launch per layer, as every CTA brings in all of its weights
 // (forward of 64 / 148 / 256 faces: 604 / 978 / 1655 us; 28x28 stage in rounds 599 / 1015 / 1718, 7x7 608 / 1051 / 1790).
-// A context made for two or three faces keeps one launch per layer beyond a single face (chain_max_faces), one for up to four
+// A context made for two or three faces keeps one launch per layer beyond a single face, one for up to four
 // also on 28x28 maps: callers count a single face's 22 launches there (tests/test_gpu_parity.py).
 static const ffcu_ctx::FaceRun* run_at(const ffcu_ctx* c, size_t k, int n)
 {
@@ -698,29 +641,11 @@ static int launch_run(ffcu_ctx* c, const ffcu_ctx::FaceRun& run, int n, int* lau
 static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
 {
     int launches = 0;
-    const bool chain_call = n <= chain_max_faces(c);
-    if (chain_call && !c->chains_built) build_chains(c);
     for (size_t k = k0; k < k1; k++) {
         if (const ffcu_ctx::FaceRun* run = run_at(c, k, n)) {
             const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, &launches) : 1;
             if (rc < 0) return rc;
             if (rc == 0) { k += (size_t)run->count - 1; continue; }
-        }
-        if (chain_call && !c->no_chain) {
-            const ChainPlan* plan = nullptr;
-            const ffcu_ctx::Chain* ch = chain_at(c, k, n, &plan);
-            if (ch) {
-                if (ffcu_chain_launch(plan, n, c->mode, c->d_err, c->stream) == 0) {
-                    launches++;
-                    k += (size_t)ch->count - 1;
-                    continue;
-                }
-                // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...):
-                // no more chains in this context (captured graphs may still hold launches of these plans: they stay until
-                // the context goes); go on with this layer as a launch of its own
-                cudaGetLastError();
-                c->no_chain = 1;
-            }
         }
         {
             DevLayer& M = c->layers[k];
@@ -1090,7 +1015,7 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
     // the 14x14 stage beyond the clusters' reach as the forward runs it: the time of its one or two launches, shared equally among its layers
     const ffcu_ctx::FaceRun* face = nullptr;
-    for (const ffcu_ctx::FaceRun& r : c->runs) if (n > chain_max_faces(c) && run_at(c, r.first, n) == &r) face = &r;
+    for (const ffcu_ctx::FaceRun& r : c->runs) if (n > 37 && run_at(c, r.first, n) == &r) face = &r;
     const int f0 = face ? (int)face->first : nl, f1 = face ? f0 + face->count : nl;
     for (int k = 0; k < nl && rc == 0; k++) {
         DevLayer& M = c->layers[k];

@@ -207,14 +207,6 @@ ScPlan* ffcu_sc_plan(const ffcu_layer& main, const ffcu_layer& sc, int max_batch
 void    ffcu_sc_free(ScPlan* sp);
 int     ffcu_sc_launch(const ScPlan* sp, int batch, int mode, const EpiTables& t1, const EpiTables& t2, int8_t* out_main,
                        int write_main, int8_t* out_sc, int8_t* out2_sc, int* d_err, cudaStream_t s, int b0 = 0);
-// Layer chain (small batches, one cluster of eight or four CTAs per face): consecutive 3x3 stride-1 C -> C convolutions of one feature-map size in one launch.
-#define FFCU_CHAIN_MAX_FACES 37     // 148 SMs hold at most 18 clusters of eight and 37 of four, fewer where GPCs are smaller
-struct ChainPlan;
-struct ChainLayerDesc { const int8_t* w; EpiTables t; const int8_t* res; int8_t* out; int8_t* out2; };
-ChainPlan* ffcu_chain_plan(int bn, int H, int W, int C, int max_batch, const int8_t* d_in, const ChainLayerDesc* layers, int n_layers);
-int        ffcu_chain_clusters(const ChainPlan* p);
-void       ffcu_chain_free(ChainPlan* p);
-int        ffcu_chain_launch(const ChainPlan* p, int faces, int mode, int* d_err, cudaStream_t s);
 // A stage (a run of 3x3 stride-1 C -> C convolutions: PReLU layers, and residual + fused BN ones) taken face by face: 128 channels on
 // 28x28 maps, 256 on 14x14, 512 on 7x7.
 #define FFCU_FACE_C 256

@@ -15,8 +15,8 @@ int32 accumulators) with its time beside it.
 
 runs the whole network instead (seeded synthetic model, seeded faces) through the public
 embed / embed_batch call --iters times and prints the launch count, the device time per forward and
-the wall-clock latency per call; at batch 1 the launch list is the small-batch one (layer chains,
-one-launch FC), so this is also the command the profiler captures those kernels under.  With
+the wall-clock latency per call; at batch 1 the launch list is the small-batch one (stages in
+clusters, one-launch FC), so this is also the command the profiler captures those kernels under.  With
 --cos-sim N it ends with one N x N similarity matrix of the last embeddings.
 """
 from __future__ import annotations

@@ -151,11 +151,11 @@ int ffcu_winograd_f23_once(int device, const int8_t* in, const int8_t* w_oihw, i
  * the launch returns; ffcu_conv_once / ffcu_wait report 1000 + the error word.  Nothing faults,
  * traps or spins without a limit, and the hook disarms itself after that one launch. */
 void ffcu_test_arm_timeout(int drop_stage, long long full_wait_cycles);
-/* The same for the batch-1 layer-chain kernel (a cluster of eight CTAs): CTA 0's weight producer leaves out
- * ring step drop_step of the next chain launch and every barrier wait of that launch is limited to
- * wait_cycles.  CTA 0's MMA issuer gives up first; the other seven, waiting for results CTA 0 never
- * sends, give up one limit later; all eight meet at the final cluster barrier, free their tensor memory
- * and return; the call reports 1000 + the error word.  Disarms itself after that one launch. */
+/* The same for the kernels that take a stage in one launch (conv_tc_stage.cu, conv_tc_face.cu): the first CTA of every cluster
+ * or pair of the next such launch leaves out ring step drop_step of its weights, and every barrier wait of that launch is limited
+ * to wait_cycles.  That CTA's MMA issuer gives up first; the others, waiting for results it never sends, one limit later; all
+ * meet at their cluster's final barrier, free their tensor memory and return; the call reports 1000 + the error word.  Disarms
+ * itself after that one launch. */
 void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles);
 /* Ordering tests: in each of the next `launches` launches that take a stage in clusters (conv_tc_stage.cu) or CTA pairs
  * (conv_tc_face.cu), the warp that loads first inputs and byte tables in the first CTA of every cluster stands still for `cycles`

@@ -1,4 +1,4 @@
-"""Layer-chain launches (runs of same-shape convolutions in one launch) beyond a single face: same bytes as one
+"""Stages of a small call in one launch each (runs of same-shape convolutions, conv_tc_stage.cu): same bytes as one
 launch per layer, and as the oracle."""
 import ctypes as C
 import os
@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n", [2, 4, 15, 16, 17, 24, 32, 33, 34, 35, 36, 37, 38])
 def test_small_batch_layer_chains(built_lib, model_root, ffw4, oracle, monkeypatch, n):
     """One cluster per face, for as many faces as the device holds clusters (of eight CTAs: 15-18, of four: 32-37, by
-    its GPC sizes; beyond that one launch per layer): eager, captured and replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
+    its GPC sizes; beyond that CTA pairs on 14x14 maps, two faces a cluster on 7x7 ones): eager, captured and replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
     faces = synth.faces(n, seed=500 + n)
     sample = sorted({0, n // 2, n - 1})
     got = {}
@@ -42,7 +42,7 @@ def test_small_batch_layer_chains(built_lib, model_root, ffw4, oracle, monkeypat
 @pytest.mark.parametrize("n", [8, 20], ids=["clusters-of-eight", "clusters-of-four"])
 def test_bounded_waits_run_out_with_several_clusters(built_lib, model_root, ffw4, oracle, n):
     """The timeout path with a cluster per face, without faulting anything: the hook makes the first CTA of every
-    cluster of the next chain launch leave out one step of its weights and limits every wait of that launch to two million
+    cluster of the next stage launch leave out one step of its weights and limits every wait of that launch to two million
     cycles.  All of them must give up, meet at their cluster's barrier and return; the call reports 1000 + the error word, and
     the same context then serves the same faces bit-exactly (eager, captured, replayed)."""
     lib = ff.load_library()
@@ -51,7 +51,7 @@ def test_bounded_waits_run_out_with_several_clusters(built_lib, model_root, ffw4
     faces = synth.faces(n, seed=77)
     want = oracle.forward(faces, ffo.CONTRACT)
     with ff.FastFace(ffw4, cwd=model_root, max_batch=40) as e:
-        lib.ffcu_test_arm_chain_timeout(12, 2_000_000)          # layer 1, fourth tap; a shape's first call runs eagerly
+        lib.ffcu_test_arm_chain_timeout(12, 2_000_000)          # second layer; a shape's first call runs eagerly
         with pytest.raises(RuntimeError) as ei:
             e.embed_batch(faces)
         assert "rc=1001" in str(ei.value) or "rc=1004" in str(ei.value), str(ei.value)
@@ -61,9 +61,9 @@ def test_bounded_waits_run_out_with_several_clusters(built_lib, model_root, ffw4
 
 
 def test_contexts_share_the_device(built_lib, model_root, ffw4):
-    """A chain keeps eight SMs per face for 150 us; the kernels queued behind it must not keep the others waiting with them.
+    """A stage keeps eight SMs per face for 90 us; the kernels queued behind it must not keep the others waiting with them.
     Four threads with a context each get 3.5 times one thread's single-face rate on an idle machine, and got 1.5 times with a
-    successor launched at the chain's start."""
+    successor launched at the stage's start."""
     if len(os.sched_getaffinity(0)) < 6:
         pytest.skip("needs a CPU for each of the calling threads")
     face = synth.faces(1, seed=8)[0]

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n", [34, 73, 74, 75, 147, 148, 149, 163, 164, 182, 190, 222, 223, 296, 297])
 def test_stage_in_one_launch(built_lib, model_root, ffw4, oracle, monkeypatch, n):
-    """One and two faces per pair, a round more, and what is left of a round in chains (74 pairs on a B200): eager, captured and
+    """One and two faces per pair, a round more, and what is left of a round in clusters (74 pairs on a B200): eager, captured and
     replayed, both epilogue orders.  The comparison is exact: integer accumulators and stated fp32 roundings."""
     faces = synth.faces(n, seed=700 + n)
     sample = sorted({0, n // 2, n - 1})

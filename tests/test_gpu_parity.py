@@ -409,7 +409,7 @@ def test_layer_microbench_reports_both_kernels(built_lib):
 
 
 def test_network_microbench_single_face(built_lib):
-    """`layer_bench --forward` at batch 1: the small-batch launch list (stem, layer chains, one-launch FC) through
+    """`layer_bench --forward` at batch 1: the small-batch launch list (stem, stages in clusters, one-launch FC) through
     the public call; the similarity matrix of an embedding with itself has a unit diagonal."""
     from fastface_b200 import layer_bench
     line = layer_bench.run_forward(1, 3, 4)
@@ -690,7 +690,7 @@ def test_network_trace_at_batch_64(built_lib, model_root, ffw4, oracle, mode, st
 def test_network_other_model_seeds(built_lib, tmp_path_factory, seed):
     """Synthetic models of seeds 1 and 2 (other weights, scales and calibration tables): every dump
     point at batch 3 against the C port, embeddings at batch 8 and 40 against port and live reference, single faces
-    (the layer-chain launch list) against the batch."""
+    (their own launch list) against the batch."""
     root = str(tmp_path_factory.mktemp(f"ffmodel_seed{seed}"))
     path = synth.materialize(root, seed)
     orc = ffo.Oracle(path, os.path.join(root, "models", "op_scales.bin"), os.path.join(root, "models", "op_scales_v2.bin"))
@@ -708,7 +708,7 @@ def test_network_other_model_seeds(built_lib, tmp_path_factory, seed):
         assert not first, "; ".join(first)
         got8 = e.embed_batch(faces[:8])
         got40 = e.embed_batch(faces)
-        got1 = [e.embed(faces[i]) for i in (0, 5, 0, 5)]        # single faces: layer chains, eager then captured
+        got1 = [e.embed(faces[i]) for i in (0, 5, 0, 5)]        # single faces: stages in clusters, eager then captured
     assert np.array_equal(got8, orc.forward(faces[:8], ffo.CONTRACT))
     assert all(np.array_equal(g, got8[i]) for g, i in zip(got1, (0, 5, 0, 5)))
     assert np.array_equal(got40[:8], got8)
@@ -826,8 +826,8 @@ def test_bounded_wait_runs_out_and_the_device_stays_usable(built_lib):
 
 
 def test_layer_chain_bounded_waits_run_out_and_the_device_stays_usable(built_lib, model_root, ffw4, oracle):
-    """The timeout path of the cluster-resident layer chain, exercised without faulting anything: the test hook makes
-    CTA 0's weight producer leave out one ring step of the next chain launch and limits every barrier wait of that
+    """The timeout path of a stage in clusters of eight, exercised without faulting anything: the test hook makes
+    CTA 0's weight producer leave out one ring step of the next stage launch and limits every barrier wait of that
     launch to two million cycles (about a millisecond).  CTA 0's issuer must give up, then the seven peers that wait
     for CTA 0's results, all eight must meet at the final cluster barrier and return; the call reports 1000 + the
     error word.  The same context must then serve the same face bit-exactly (eager, captured, replayed)."""
@@ -837,7 +837,7 @@ def test_layer_chain_bounded_waits_run_out_and_the_device_stays_usable(built_lib
     faces = synth.faces(2, seed=5)
     want = oracle.forward(faces, ffo.CONTRACT)
     with ff.FastFace(ffw4, cwd=model_root, max_batch=2) as e:
-        lib.ffcu_test_arm_chain_timeout(12, 2_000_000)          # layer 1, fourth tap
+        lib.ffcu_test_arm_chain_timeout(12, 2_000_000)          # second layer
         with pytest.raises(RuntimeError) as ei:
             e.embed(faces[0])
         # 1000 + the code of whichever wait ran out first: the issuer's for the missing stage (TMA, 1) or the epilogue
