@@ -601,13 +601,12 @@ static int launch_layer(ffcu_ctx* c, size_t k, int n, int32_t* acc_dbg, bool unf
 // The run of layers that starts at k and that a call of n faces takes face by face; NULL: none.  28x28 and 7x7 maps only while the
 // device holds all their clusters at once: in rounds they lose to one launch per layer, as every CTA brings in all of its weights
 // (forward of 64 / 148 / 256 faces: 604 / 978 / 1655 us; 28x28 stage in rounds 599 / 1015 / 1718, 7x7 608 / 1051 / 1790).
-// A context made for two or three faces keeps one launch per layer beyond a single face, one for up to four
-// also on 28x28 maps: callers count a single face's 22 launches there (tests/test_gpu_parity.py).
+// The rule asks for the call's faces only, not for the context's size (full calls of contexts for 1 / 2 / 3 / 4 faces that kept launches per layer: forward
+// 213.7 / 321.2 / 327.8 / 225.2 -> 200.3 / 203.4 / 207.2 / 214.9 us).
 static const ffcu_ctx::FaceRun* run_at(const ffcu_ctx* c, size_t k, int n)
 {
     for (const ffcu_ctx::FaceRun& r : c->runs) {
         if (r.first != k) continue;
-        if (c->max_batch < 4 ? n > 1 || r.H == 28 : c->max_batch == 4 && r.H == 28) return nullptr;
         return r.H == 14 || (!c->no_clusters && ffcu_stage_form(r.plan, n) >= 0) ? &r : nullptr;
     }
     return nullptr;

@@ -312,9 +312,9 @@ def test_unfused_plan_agrees(built_lib, model_root, ffw4, oracle, monkeypatch):
     monkeypatch.setenv("FF_FUSE_STEM", "0")
     with ff.FastFace(ffw4, cwd=model_root, max_batch=3) as e:
         assert np.array_equal(e.embed_batch(faces), want)
-        # fused: 1 stem launch, 52 convs (the four stride-2 conv + shortcut pairs one launch each at this batch), 1 FC;
-        # unfused: 1 quantise, 53 convs (same four pairs fused), 25 BN passes, 1 FC
-        assert e.launches_per_forward == 80 - 4 and n_fused == 54 - 4
+        # fused: 1 stem launch, 52 convs (the four stride-2 conv + shortcut pairs one launch each at this batch, so are the 28x28, 14x14 and
+        # 7x7 stages of 6, 26 and 4 layers), 1 FC; unfused: 1 quantise, 53 convs (same four pairs fused), 25 BN passes, 1 FC
+        assert e.launches_per_forward == 80 - 4 and n_fused == 54 - 4 - 5 - 25 - 3
 
 
 @pytest.mark.parametrize("case", LAYER_CASES[:4], ids=lambda c: c[0])
@@ -413,7 +413,7 @@ def test_network_microbench_single_face(built_lib):
     the public call; the similarity matrix of an embedding with itself has a unit diagonal."""
     from fastface_b200 import layer_bench
     line = layer_bench.run_forward(1, 3, 4)
-    assert line["launches_per_forward"] == 22 and line["device_ms_per_forward"] > 0
+    assert line["launches_per_forward"] == 17 and line["device_ms_per_forward"] > 0
     assert abs(line["cos_sim_matrix"]["diag_min"] - 1.0) < 1e-6
 
 
@@ -767,8 +767,8 @@ def test_single_face_layer_chains(built_lib, model_root, ffw4, oracle, monkeypat
                     got = e.embed(faces[i])
                     assert np.array_equal(got, want[i]), f"FF_CHAIN={flag} rep {rep} face {i}"
             counts[flag] = e.launches_per_forward
-            assert np.array_equal(e.embed_batch(faces), want)      # batch 4: per-layer launches in the same context
-    assert counts["0"] == 54 - 4 and counts["1"] == 54 - 4 - 26 - 4 + 2, counts
+            assert np.array_equal(e.embed_batch(faces), want)      # batch 4 in the same context
+    assert counts["0"] == 54 - 4 and counts["1"] == 54 - 4 - 5 - 25 - 3, counts
 
 
 @pytest.mark.parametrize("B", [1, 5, 32, 40, 64, 300])
@@ -846,7 +846,7 @@ def test_layer_chain_bounded_waits_run_out_and_the_device_stays_usable(built_lib
         for _ in range(3):
             assert np.array_equal(e.embed(faces[0]), want[0])
             assert np.array_equal(e.embed(faces[1]), want[1])
-        assert e.launches_per_forward == 22
+        assert e.launches_per_forward == 17
 
 
 def test_embed_and_embed_batch_agree_with_oracle(engine, oracle):
@@ -908,7 +908,7 @@ def test_stem_on_cuda_cores_agrees(built_lib, model_root, ffw4, oracle, monkeypa
         with ff.FastFace(ffw4, cwd=model_root, max_batch=3) as e:
             assert np.array_equal(e.embed_batch(faces), want), f"FF_STEM_TC={flag}"
             assert np.array_equal(e.embed_batch_u8(pix), want_u8), f"FF_STEM_TC={flag}, uint8 input"
-            assert e.launches_per_forward == 54 - 4
+            assert e.launches_per_forward == 17
 
 
 def test_network_with_the_large_batch_tiling(built_lib, model_root, ffw4, oracle, monkeypatch):
