@@ -486,6 +486,19 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
 }
 
 
+// The next `count` launches in clusters that have another way to go (stages, split shortcuts) are refused, as by a device that cannot place
+// them (for the test of those ways).
+static int g_test_refuse_clusters = 0;
+
+extern "C" void ffcu_test_refuse_clusters(int count) { g_test_refuse_clusters = count; }
+
+static bool cluster_refused()
+{
+    if (g_test_refuse_clusters < 1) return false;
+    g_test_refuse_clusters--;
+    return true;
+}
+
 // ---------------------------------------------------------------------------
 // Stride-2 convolution + the block's 1x1 stride-2 shortcut in one launch (conv_tc_sc.cu)
 // ---------------------------------------------------------------------------
@@ -630,7 +643,7 @@ int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, 
         half.stages = std::min(prm.stages, (steps + 1) / 2 + 1);
         int smem = sp->smem_bytes - (prm.stages - half.stages) * stage_bytes + SC_RECV_BYTES(2);
         for (; smem > 232448 && half.stages > 2; smem -= stage_bytes) half.stages--;
-        if (smem <= 232448 &&
+        if (smem <= 232448 && !cluster_refused() &&
             tc_launch_sc(p->KC, mode, 2, prm.total_tiles, smem, s, g->mapA, p->mapB, g2->mapA, sp->mapB2, half, q) == 0) return 0;
         cudaGetLastError();              // no clusters of two here and now: not again with this plan
         sp->no_split = 1;
@@ -774,6 +787,7 @@ int ffcu_stage_form(const FacePlan* p, int faces)
 
 int ffcu_stage_launch(const FacePlan* p, int form, int face0, int faces, int mode, int* d_err, cudaStream_t s)
 {
+    if (cluster_refused()) { ffcu_set_error("stage launch refused"); return -1; }
     return tc_launch_stage(p->H, form, mode, faces, s, p->mapA[form], face_params(p, face0, faces, d_err));
 }
 

@@ -157,6 +157,9 @@ void ffcu_test_arm_timeout(int drop_stage, long long full_wait_cycles);
  * meet at their cluster's final barrier, free their tensor memory and return; the call reports 1000 + the error word.  Disarms
  * itself after that one launch. */
 void ffcu_test_arm_chain_timeout(int drop_step, long long wait_cycles);
+/* The next `count` launches in clusters that have another way to go (a stage, a stride-2 convolution shared by two CTAs) are refused, as by a
+ * device that cannot place them; 0 disarms. */
+void ffcu_test_refuse_clusters(int count);
 /* Ordering tests: in each of the next `launches` launches that take a stage in clusters (conv_tc_stage.cu) or CTA pairs
  * (conv_tc_face.cu), the warp that loads first inputs and byte tables in the first CTA of every cluster stands still for `cycles`
  * in front of its first load and after each table.  Results stay the same. */

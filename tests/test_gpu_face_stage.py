@@ -99,3 +99,30 @@ def test_a_late_loader_changes_nothing(built_lib, model_root, ffw4, oracle, n):
         lib.ffcu_test_hold_stage_loader(0, 0)
         assert np.array_equal(held, e.embed_batch(faces))
     assert np.array_equal(held[[0, n - 1]], want)
+
+
+@pytest.mark.parametrize("at", [0, 1], ids=["first-call", "while-captured"])
+@pytest.mark.parametrize("refused", [1, 2, 1000], ids=["one", "two", "all"])
+@pytest.mark.parametrize("n", [1, 17, 64, 160])
+def test_refused_clusters(built_lib, model_root, ffw4, oracle, n, refused, at):
+    """A device that cannot place a cluster: the call goes on with CTA pairs on 14x14 maps, one launch per layer on the others, one CTA per tile
+    in the stride-2 convolutions, and does not ask again.  In the first (eager) call or in the one that is captured; exact, as above."""
+    lib = ff.load_library()
+    lib.ffcu_test_refuse_clusters.restype = None
+    lib.ffcu_test_refuse_clusters.argtypes = [C.c_int]
+    faces = synth.faces(n, seed=80)
+    want = oracle.forward(faces[[0, n - 1]], ffo.CONTRACT)
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=160) as e:
+        before = e.embed_batch(faces) if at else None
+        lib.ffcu_test_refuse_clusters(refused)
+        try:
+            got = [e.embed_batch(faces) for _ in range(4)]
+        finally:
+            lib.ffcu_test_refuse_clusters(0)
+        launches = e.launches_per_forward
+        got.append(e.embed_batch(faces))
+    for g in got + ([before] if at else []):
+        assert np.array_equal(g, got[0])
+    assert np.array_equal(got[0][[0, n - 1]], want)
+    if n <= 17 and refused == 1000 and not at:
+        assert launches == 54 - 4 - 25                             # all 54 but the shortcuts' and the 14x14 stage's
