@@ -698,14 +698,15 @@ static int run_forward(ffcu_ctx* c, int n, int slot, int k0 = 0)
     if (rc != 0 || e != cudaSuccess || !graph) {
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
-        c->graph_max_batch = 0;                     // capture not possible here: stay eager
-        return rc != 0 ? rc : launch_forward(c, n, k0);
+        c->graph_max_batch = 0;                     // capture not possible here: stay eager (nothing of it has run)
+        return launch_forward(c, n, k0);
     }
     cudaGraphExec_t exec = nullptr;
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess || !exec) { cudaGetLastError(); c->graph_max_batch = 0; return launch_forward(c, n, k0); }
     c->graphs[key] = exec;
+    c->graph_launches[key] = c->launches;           // (fewer clusters than the first time, where one was refused)
     FFCU_CHECK(cudaGraphLaunch(exec, c->stream));
     return 0;
 }

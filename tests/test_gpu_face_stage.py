@@ -124,5 +124,5 @@ def test_refused_clusters(built_lib, model_root, ffw4, oracle, n, refused, at):
     for g in got + ([before] if at else []):
         assert np.array_equal(g, got[0])
     assert np.array_equal(got[0][[0, n - 1]], want)
-    if n <= 17 and refused == 1000 and not at:
+    if n <= 17 and refused == 1000:
         assert launches == 54 - 4 - 25                             # all 54 but the shortcuts' and the 14x14 stage's
