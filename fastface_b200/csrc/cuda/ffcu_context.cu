@@ -636,35 +636,37 @@ static int launch_run(ffcu_ctx* c, const ffcu_ctx::FaceRun& run, int n, int* lau
     return 1;
 }
 
+// What a forward of n faces launches from layer k on, of the layers before k1: the stage that starts there, a stride-2 convolution with
+// its block's shortcut, or the layer alone.  How many layers that was, or < 0; the launches made are added to *launches.
+static int launch_next(ffcu_ctx* c, size_t k, int n, size_t k1, int b0, int* launches)
+{
+    if (const ffcu_ctx::FaceRun* run = run_at(c, k, n)) {
+        const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, launches) : 1;
+        if (rc <= 0) return rc < 0 ? rc : run->count;
+    }
+    DevLayer& M = c->layers[k];
+    if (M.sc && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64) {
+        DevLayer& S = c->layers[k + 1];
+        const size_t off = (size_t)b0 * out_bytes_per_face(S.d);
+        int8_t* out2 = S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] + off : nullptr;
+        const int rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf] + off, M.sc_write_main,
+                                      c->bufs[S.d.dst_buf] + off, out2, c->d_err, c->stream, b0);
+        (*launches)++;
+        return rc != 0 ? -std::abs(rc) : 2;
+    }
+    const int rc = launch_layer(c, k, n, nullptr, false, b0);
+    if (!M.skip) (*launches)++;
+    return rc != 0 ? -std::abs(rc) : 1;
+}
+
 // Layers [k0, k1) for faces b0 .. b0 + n - 1 (b0 > 0 within a head only); c->launches = the launches made.
 static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
 {
     int launches = 0;
-    for (size_t k = k0; k < k1; k++) {
-        if (const ffcu_ctx::FaceRun* run = run_at(c, k, n)) {
-            const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, &launches) : 1;
-            if (rc < 0) return rc;
-            if (rc == 0) { k += (size_t)run->count - 1; continue; }
-        }
-        {
-            DevLayer& M = c->layers[k];
-            if (M.sc && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64) {
-                // stride-2 conv + the block's shortcut, one launch
-                DevLayer& S = c->layers[k + 1];
-                const size_t off = (size_t)b0 * out_bytes_per_face(S.d);
-                int8_t* out2 = S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] + off : nullptr;
-                int rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf] + off, M.sc_write_main,
-                                        c->bufs[S.d.dst_buf] + off, out2, c->d_err, c->stream, b0);
-                if (rc != 0) return rc;
-                launches++;
-                k++;
-                continue;
-            }
-        }
-        int rc = launch_layer(c, k, n, nullptr, false, b0);
-        if (rc != 0) return rc;
-        const DevLayer& L = c->layers[k];
-        if (!L.skip) launches++;
+    for (size_t k = k0; k < k1; ) {
+        const int layers = launch_next(c, k, n, k1, b0, &launches);
+        if (layers < 0) return layers;
+        k += (size_t)layers;
     }
     c->launches = launches;
     return 0;
@@ -1013,41 +1015,29 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     if (rc != 0) return rc;
     std::vector<cudaEvent_t> ev(2 * nl);
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
-    // the 14x14 stage beyond the clusters' reach as the forward runs it: the time of its one or two launches, shared equally among its layers
-    const ffcu_ctx::FaceRun* face = nullptr;
-    for (const ffcu_ctx::FaceRun& r : c->runs) if (n > 37 && run_at(c, r.first, n) == &r) face = &r;
-    const int f0 = face ? (int)face->first : nl, f1 = face ? f0 + face->count : nl;
-    for (int k = 0; k < nl && rc == 0; k++) {
-        DevLayer& M = c->layers[k];
-        if (k >= f0 && k < f1) {
-            int launched = 0;
-            FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
-            if (k == f0) for (int it = 0; it < iters && rc == 0; it++) rc = launch_run(c, *face, n, &launched);
-            FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
-            continue;
-        }
-        // a stride-2 conv that shares its launch with the block's shortcut at this batch is timed as the forward runs
-        // it: the pair's one launch under the conv, nothing under the shortcut
-        const bool pair = M.sc && k + 1 < nl && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64;
+    std::vector<int> layers((size_t)nl, 0);               // of what starts at layer k
+    for (int k = 0; k < nl && rc == 0; k += layers[k]) {
         FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
         for (int it = 0; it < iters && rc == 0; it++) {
-            if (pair) {
-                DevLayer& S = c->layers[k + 1];
-                rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf], M.sc_write_main, c->bufs[S.d.dst_buf],
-                                    S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] : nullptr, c->d_err, c->stream);
-            } else rc = launch_layer(c, k, n, nullptr);
+            int made = 0;
+            const int m = launch_next(c, (size_t)k, n, (size_t)nl, 0, &made);
+            if (m < 0) rc = m;
+            else if (it && m != layers[k]) {              // a cluster launch was refused: timed anew, as the forward goes on
+                FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
+                it = -1;
+            }
+            layers[k] = m;
         }
         FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
-        if (pair) {
-            k++;
-            FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
-            FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
-        }
     }
     int wrc = ffcu_wait(c);
     if (rc == 0) rc = wrc;
-    for (int k = 0; k < nl && rc == 0; k++) FFCU_CHECK(cudaEventElapsedTime(&ms[k], ev[2 * k], ev[2 * k + 1]));
-    if (face && rc == 0) for (int k = f1 - 1; k >= f0; k--) ms[k] = ms[f0] / (float)face->count;
+    for (int k = 0; k < nl && rc == 0; k += layers[k]) {
+        FFCU_CHECK(cudaEventElapsedTime(&ms[k], ev[2 * k], ev[2 * k + 1]));
+        const bool pair = layers[k] == 2 && c->layers[k].sc;      // all of it under the convolution, nothing under the shortcut
+        for (int j = k + 1; j < k + layers[k]; j++) ms[j] = pair ? 0.0f : ms[k] / (float)layers[k];
+        if (!pair) ms[k] /= (float)layers[k];
+    }
     for (auto& e : ev) cudaEventDestroy(e);
     return rc == 0 ? nl : rc;
 }

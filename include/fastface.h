@@ -110,8 +110,9 @@ int fastface_bench_resident(FastFace* ff, const float* input_hwc, int n, int ite
  * fastface_layer_desc fills desc[12] = {kind (0 quantise, 1 conv, 2 BN, 3 FC), FFW4 op index,
  * Cin, Cout, Kh, Kw, stride, H, W, Ho, Wo, 1 if the tensor-core kernel runs it};
  * fastface_bench_layers times each layer `iters` times over n resident faces (ms[k] = total
- * CUDA-event milliseconds of layer k; where the forward runs the 14x14 stage as one launch, that
- * launch's time shared equally among its layers) and returns the layer count. */
+ * CUDA-event milliseconds of layer k) and returns the layer count.  What a forward of n faces runs as
+ * one is timed as one: a stage's time is shared equally among its layers, a stride-2 convolution's is
+ * that of its block's shortcut too, which then has 0. */
 int fastface_layer_count(const FastFace* ff);
 int fastface_layer_desc(const FastFace* ff, int k, int* desc12);
 int fastface_bench_layers(FastFace* ff, const float* input_hwc, int n, int iters, float* ms, int cap);

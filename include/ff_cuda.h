@@ -110,9 +110,10 @@ int ffcu_bench_resident(ffcu_ctx* c, const float* host_in, int n, int iters, flo
 /* Launches that every face of the last call went through (layers run in chunks count once). */
 int ffcu_launches_per_forward(const ffcu_ctx* c);
 
-/* Per-layer timing: after one full forward over n resident faces, each layer is
- * launched `iters` times back to back between two CUDA events on the compute stream;
- * ms[k] receives the total for layer k.  Returns the layer count (<0 on error). */
+/* Per-layer timing: after one full forward over n resident faces, what such a forward launches for
+ * each layer (a stage, a convolution with its shortcut, or the layer alone) is launched `iters` times
+ * back to back between two CUDA events on the compute stream; ms[k] receives the total for layer k, an
+ * equal share of a stage's, 0 for a shortcut that shares a launch.  Returns the layer count (<0 on error). */
 int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int iters, float* ms, int cap);
 
 /* Layer count and description of layer k (pointer members are NULL in *out);

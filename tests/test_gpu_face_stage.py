@@ -126,3 +126,43 @@ def test_refused_clusters(built_lib, model_root, ffw4, oracle, n, refused, at):
     assert np.array_equal(got[0][[0, n - 1]], want)
     if n <= 17 and refused == 1000:
         assert launches == 54 - 4 - 25                             # all 54 but the shortcuts' and the 14x14 stage's
+
+
+def stage_layers(layers):
+    """Map size -> its 3x3 stride-1 C -> C layers, C >= 128: those that a stage's launch takes."""
+    out = {}
+    for k, l in enumerate(layers):
+        if l["kind"] == 1 and l["Kh"] == 3 and l["stride"] == 1 and l["Cin"] == l["Cout"] >= 128:
+            out.setdefault(l["H"], []).append(k)
+    return out
+
+
+@pytest.mark.parametrize("n,shared", [(1, {28, 14, 7}), (17, {28, 14, 7}), (40, {14, 7}), (64, {28, 14, 7}), (160, {14})])
+def test_layer_timing_follows_the_forward(built_lib, model_root, ffw4, n, shared):
+    """bench_layers times the launches that a forward of n faces makes: a stage in one launch gives its layers equal shares, layers with
+    a launch each have times of their own (six equal event times in a row do not happen), and no layer is left out."""
+    faces = synth.faces(n, seed=81)
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=160) as e:
+        layers, ms = e.layers(), e.bench_layers(faces, 3)
+        stages = stage_layers(layers)
+        assert {h: len(k) for h, k in stages.items()} == {28: 6, 14: 26, 7: 4}
+        assert {h for h, k in stages.items() if len({ms[i] for i in k}) == 1} == shared
+        forward = e.bench_resident(faces, 20) / 20
+        assert 0.6 * forward < sum(ms) / 3 < 2.0 * forward, (sum(ms) / 3, forward)
+
+
+def test_layer_timing_with_refused_clusters(built_lib, model_root, ffw4):
+    """Refused in the forward before the timing: the layers' own launches are timed, and the count returned is that of the layers."""
+    lib = ff.load_library()
+    lib.ffcu_test_refuse_clusters.restype = None
+    lib.ffcu_test_refuse_clusters.argtypes = [C.c_int]
+    faces = synth.faces(64, seed=81)
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=64) as e:
+        lib.ffcu_test_refuse_clusters(1000)
+        try:
+            ms = e.bench_layers(faces, 3)
+        finally:
+            lib.ffcu_test_refuse_clusters(0)
+        stages = stage_layers(e.layers())
+        assert {h for h, k in stages.items() if len({ms[i] for i in k}) == 1} == {14}
+        assert all(ms[i] > 0 for k in stages.values() for i in k)
