@@ -84,6 +84,8 @@ def load_library() -> C.CDLL:
     L.fastface_layer_desc.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_int)]
     L.fastface_bench_layers.restype = C.c_int
     L.fastface_bench_layers.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_float), C.c_int]
+    L.fastface_layer_launches.restype = C.c_int
+    L.fastface_layer_launches.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_int)]
     L.ffcu_device_count.restype = C.c_int
     L.ffcu_conv_once.restype = C.c_int
     L.ffcu_conv_once.argtypes = [C.c_int, C.POINTER(FfcuLayer), C.c_int, C.c_int, C.c_int,
@@ -256,6 +258,17 @@ class FastFace:
         if rc != n:
             raise RuntimeError(f"fastface_bench_layers rc={rc}: " + self.lib.fastface_last_error().decode())
         return list(ms)
+
+    def layer_launches(self) -> List[dict]:
+        """What the last ``bench_layers`` launched for each layer: ``layers`` layers from it on (0: in an earlier one's launch), by
+        ``single`` launches (a layer, or a convolution and its shortcut), ``pairs`` and ``clusters`` (a stage)."""
+        out = []
+        for k in range(self.lib.fastface_layer_count(self.h)):
+            v = (C.c_int * 4)()
+            if self.lib.fastface_layer_launches(self.h, k, v) != 0:
+                raise RuntimeError("fastface_layer_launches failed: no bench_layers call yet")
+            out.append(dict(zip(("layers", "single", "pairs", "clusters"), list(v))))
+        return out
 
     @property
     def launches_per_forward(self) -> int:

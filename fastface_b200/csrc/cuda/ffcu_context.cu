@@ -115,6 +115,7 @@ struct ffcu_ctx {
     struct FaceRun { size_t first; int count, H; FacePlan* plan; };
     std::vector<FaceRun> runs;
     int no_clusters = 0;         // a cluster launch was refused
+    std::vector<ffcu_launches> made;     // by layer, what ffcu_bench_layers launched from there on
     // A whole call that is one step of fewer than CHUNK_MIN_FACES faces, and any submit of at most lean_max_batch
     // (FF_LEAN_MAX_BATCH, default 1), runs copy-in, forward and copy-out on the compute stream alone: it has nothing to overlap and
     // is spared the pipeline's two cross-stream hops.  Other submits go through the three-stream pipeline, where the next step's
@@ -616,57 +617,57 @@ static const ffcu_ctx::FaceRun* run_at(const ffcu_ctx* c, size_t k, int n)
 // (14x14): a pair takes two faces at a time through the stage, so whole rounds of two per pair go out as one launch, and what
 // is left over in clusters where it can, which is quicker than a round with one face per pair (149 / 160 / 300 faces: 1199 /
 // 1245 / 2170 -> 1174 / 1196 / 2110 us).
-static int launch_run(ffcu_ctx* c, const ffcu_ctx::FaceRun& run, int n, int* launches)
+static int launch_run(ffcu_ctx* c, const ffcu_ctx::FaceRun& run, int n, ffcu_launches* made)
 {
     int left = run.H == 14 ? n % (2 * ffcu_face_pairs(run.plan)) : n;
     const int form = c->no_clusters ? -1 : ffcu_stage_form(run.plan, left);
     if (form < 0) left = 0;
     if (left < n) {
         const int rc = ffcu_face_launch(run.plan, 0, n - left, c->mode, c->d_err, c->stream);
-        (*launches)++;
+        made->pairs++;
         if (rc != 0 || !left) return rc;
     }
-    (*launches)++;
-    if (ffcu_stage_launch(run.plan, form, n - left, left, c->mode, c->d_err, c->stream) == 0) return 0;
+    if (ffcu_stage_launch(run.plan, form, n - left, left, c->mode, c->d_err, c->stream) == 0) { made->clusters++; return 0; }
     // the cluster launch was refused (no eight free SMs in one GPC right now, a partitioned device ...): no more in this context
     cudaGetLastError();
     c->no_clusters = 1;
-    if (run.H == 14) return ffcu_face_launch(run.plan, n - left, left, c->mode, c->d_err, c->stream);
-    (*launches)--;
-    return 1;
+    if (run.H != 14) return 1;
+    made->pairs++;
+    return ffcu_face_launch(run.plan, n - left, left, c->mode, c->d_err, c->stream);
 }
 
 // What a forward of n faces launches from layer k on, of the layers before k1: the stage that starts there, a stride-2 convolution with
-// its block's shortcut, or the layer alone.  How many layers that was, or < 0; the launches made are added to *launches.
-static int launch_next(ffcu_ctx* c, size_t k, int n, size_t k1, int b0, int* launches)
+// its block's shortcut, or the layer alone.  0 or < 0; *made says how many layers that was, and by which launches.
+static int launch_next(ffcu_ctx* c, size_t k, int n, size_t k1, int b0, ffcu_launches* made)
 {
+    *made = {};
     if (const ffcu_ctx::FaceRun* run = run_at(c, k, n)) {
-        const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, launches) : 1;
-        if (rc <= 0) return rc < 0 ? rc : run->count;
+        const int rc = k + (size_t)run->count <= k1 ? launch_run(c, *run, n, made) : 1;
+        made->layers = run->count;
+        if (rc <= 0) return rc;
     }
     DevLayer& M = c->layers[k];
     if (M.sc && ffcu_tc_pick_bn(M.d, n, c->device, 1) == 64) {
         DevLayer& S = c->layers[k + 1];
         const size_t off = (size_t)b0 * out_bytes_per_face(S.d);
         int8_t* out2 = S.d.bn2_dst_buf >= 0 ? c->bufs[S.d.bn2_dst_buf] + off : nullptr;
-        const int rc = ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf] + off, M.sc_write_main,
-                                      c->bufs[S.d.dst_buf] + off, out2, c->d_err, c->stream, b0);
-        (*launches)++;
-        return rc != 0 ? -std::abs(rc) : 2;
+        made->layers = 2; made->single = 1;
+        return ffcu_sc_launch(M.sc, n, c->mode, M.epi, S.epi, c->bufs[M.d.dst_buf] + off, M.sc_write_main,
+                              c->bufs[S.d.dst_buf] + off, out2, c->d_err, c->stream, b0);
     }
-    const int rc = launch_layer(c, k, n, nullptr, false, b0);
-    if (!M.skip) (*launches)++;
-    return rc != 0 ? -std::abs(rc) : 1;
+    made->layers = 1; made->single = M.skip ? 0 : 1;
+    return launch_layer(c, k, n, nullptr, false, b0);
 }
 
 // Layers [k0, k1) for faces b0 .. b0 + n - 1 (b0 > 0 within a head only); c->launches = the launches made.
 static int launch_range(ffcu_ctx* c, int n, size_t k0, size_t k1, int b0)
 {
     int launches = 0;
-    for (size_t k = k0; k < k1; ) {
-        const int layers = launch_next(c, k, n, k1, b0, &launches);
-        if (layers < 0) return layers;
-        k += (size_t)layers;
+    ffcu_launches made;
+    for (size_t k = k0; k < k1; k += (size_t)made.layers) {
+        const int rc = launch_next(c, k, n, k1, b0, &made);
+        if (rc != 0) return rc;
+        launches += made.single + made.pairs + made.clusters;
     }
     c->launches = launches;
     return 0;
@@ -1015,31 +1016,38 @@ extern "C" int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int i
     if (rc != 0) return rc;
     std::vector<cudaEvent_t> ev(2 * nl);
     for (auto& e : ev) FFCU_CHECK(cudaEventCreate(&e));
-    std::vector<int> layers((size_t)nl, 0);               // of what starts at layer k
-    for (int k = 0; k < nl && rc == 0; k += layers[k]) {
+    std::vector<ffcu_launches> made((size_t)nl);          // by what starts at layer k
+    for (int k = 0; k < nl && rc == 0; k += made[k].layers) {
         FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
         for (int it = 0; it < iters && rc == 0; it++) {
-            int made = 0;
-            const int m = launch_next(c, (size_t)k, n, (size_t)nl, 0, &made);
-            if (m < 0) rc = m;
-            else if (it && m != layers[k]) {              // a cluster launch was refused: timed anew, as the forward goes on
+            const int was = made[k].layers;
+            rc = launch_next(c, (size_t)k, n, (size_t)nl, 0, &made[k]);
+            if (rc == 0 && it && made[k].layers != was) { // a cluster launch was refused: timed anew, as the forward goes on
                 FFCU_CHECK(cudaEventRecord(ev[2 * k], c->stream));
                 it = -1;
             }
-            layers[k] = m;
         }
         FFCU_CHECK(cudaEventRecord(ev[2 * k + 1], c->stream));
     }
     int wrc = ffcu_wait(c);
     if (rc == 0) rc = wrc;
-    for (int k = 0; k < nl && rc == 0; k += layers[k]) {
+    for (int k = 0; k < nl && rc == 0; k += made[k].layers) {
         FFCU_CHECK(cudaEventElapsedTime(&ms[k], ev[2 * k], ev[2 * k + 1]));
-        const bool pair = layers[k] == 2 && c->layers[k].sc;      // all of it under the convolution, nothing under the shortcut
-        for (int j = k + 1; j < k + layers[k]; j++) ms[j] = pair ? 0.0f : ms[k] / (float)layers[k];
-        if (!pair) ms[k] /= (float)layers[k];
+        const int layers = made[k].layers;
+        const bool pair = made[k].single && layers == 2;       // all of it under the convolution, nothing under the shortcut
+        for (int j = k + 1; j < k + layers; j++) ms[j] = pair ? 0.0f : ms[k] / (float)layers;
+        if (!pair) ms[k] /= (float)layers;
     }
+    if (rc == 0) c->made = made;
     for (auto& e : ev) cudaEventDestroy(e);
-    return rc == 0 ? nl : rc;
+    return rc == 0 ? nl : -std::abs(rc);                  // (a wait that ran out is 1000 + its word)
+}
+
+extern "C" int ffcu_layer_launches(const ffcu_ctx* c, int k, ffcu_launches* out)
+{
+    if (!c || !out || k < 0 || k >= (int)c->made.size()) return -1;
+    *out = c->made[k];
+    return 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -283,3 +283,12 @@ int fastface_bench_layers(FastFace* ff, const float* input_hwc, int n, int iters
     if (!ff || !input_hwc || !ms || n < 1 || n > ff->max_batch || iters < 1) return -1;
     return ffcu_bench_layers(ff->dev[0], input_hwc, n, iters, ms, cap);
 }
+
+int fastface_layer_launches(const FastFace* ff, int k, int* launches4)
+{
+    ffcu_launches l;
+    if (!ff || !launches4 || ffcu_layer_launches(ff->dev[0], k, &l) != 0) return -1;
+    int v[4] = { l.layers, l.single, l.pairs, l.clusters };
+    memcpy(launches4, v, sizeof v);
+    return 0;
+}

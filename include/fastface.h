@@ -116,6 +116,9 @@ int fastface_bench_resident(FastFace* ff, const float* input_hwc, int n, int ite
 int fastface_layer_count(const FastFace* ff);
 int fastface_layer_desc(const FastFace* ff, int k, int* desc12);
 int fastface_bench_layers(FastFace* ff, const float* input_hwc, int n, int iters, float* ms, int cap);
+/* What the last fastface_bench_layers launched for layer k: launches[4] = {layers from k on in these launches (0: in an earlier one's),
+ * launches of a layer or of a convolution and its shortcut, of a stage by CTA pairs, of a stage in clusters}.  0, or -1. */
+int fastface_layer_launches(const FastFace* ff, int k, int* launches4);
 
 /* Number of kernel launches a forward pass of the last embed/bench call consists of: what every face goes through.  A step of
  * 40 faces or more that finds the device idle runs its first layers in chunks; their launches count once here, not once per

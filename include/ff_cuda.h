@@ -116,6 +116,12 @@ int ffcu_launches_per_forward(const ffcu_ctx* c);
  * equal share of a stage's, 0 for a shortcut that shares a launch.  Returns the layer count (<0 on error). */
 int ffcu_bench_layers(ffcu_ctx* c, const float* host_in, int n, int iters, float* ms, int cap);
 
+/* What the last ffcu_bench_layers launched for layer k: `layers` layers from k on (0: in an earlier one's launch) in `single` launches of a
+ * layer, or of a convolution and its shortcut, `pairs` of a stage by CTA pairs (conv_tc_face.cu) and `clusters` of a stage in
+ * clusters (conv_tc_stage.cu). */
+typedef struct ffcu_launches { int layers, single, pairs, clusters; } ffcu_launches;
+int ffcu_layer_launches(const ffcu_ctx* c, int k, ffcu_launches* out);
+
 /* Layer count and description of layer k (pointer members are NULL in *out);
  * *uses_tc = 1 when the tensor-core implicit-GEMM kernel runs it. */
 int ffcu_layer_count(const ffcu_ctx* c);

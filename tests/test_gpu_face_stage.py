@@ -147,12 +147,18 @@ def test_layer_timing_follows_the_forward(built_lib, model_root, ffw4, n, shared
         stages = stage_layers(layers)
         assert {h: len(k) for h, k in stages.items()} == {28: 6, 14: 26, 7: 4}
         assert {h for h, k in stages.items() if len({ms[i] for i in k}) == 1} == shared
+        made = e.layer_launches()
+        assert sum(m["layers"] for m in made) == len(layers)
+        assert sum(m["single"] + m["pairs"] + m["clusters"] for m in made) == e.launches_per_forward
+        assert {h for h, k in stages.items() if made[k[0]]["pairs"] + made[k[0]]["clusters"]} == shared
+        assert made[stages[14][0]] == {"layers": 26, "single": 0, "pairs": int(n > 33), "clusters": int(n <= 33 or n == 160)}
         forward = e.bench_resident(faces, 20) / 20
         assert 0.6 * forward < sum(ms) / 3 < 2.0 * forward, (sum(ms) / 3, forward)
 
 
 def test_layer_timing_with_refused_clusters(built_lib, model_root, ffw4):
-    """Refused in the forward before the timing: the layers' own launches are timed, and the count returned is that of the layers."""
+    """Refused in the forward before the timing: the layers' own launches are timed, and the count returned is that of the layers.  A wait
+    that ran out is an error below zero, not a count."""
     lib = ff.load_library()
     lib.ffcu_test_refuse_clusters.restype = None
     lib.ffcu_test_refuse_clusters.argtypes = [C.c_int]
@@ -166,3 +172,10 @@ def test_layer_timing_with_refused_clusters(built_lib, model_root, ffw4):
         stages = stage_layers(e.layers())
         assert {h for h, k in stages.items() if len({ms[i] for i in k}) == 1} == {14}
         assert all(ms[i] > 0 for k in stages.values() for i in k)
+    lib.ffcu_test_arm_chain_timeout.restype = None
+    lib.ffcu_test_arm_chain_timeout.argtypes = [C.c_int, C.c_longlong]
+    with ff.FastFace(ffw4, cwd=model_root, max_batch=64) as e:
+        lib.ffcu_test_arm_chain_timeout(12, 2_000_000)
+        with pytest.raises(RuntimeError) as ei:
+            e.bench_layers(faces, 3)
+        assert "rc=-1001" in str(ei.value) or "rc=-1004" in str(ei.value), str(ei.value)
