@@ -258,10 +258,18 @@ def reference_extras(model_root, ffw4):
 
 
 def run_reference_arm(args, rank, world):
-    """--impl reference: the reference's own CPU implementation, rank 0 only."""
+    """--impl reference: the reference's own CPU implementation, rank 0 only; one line that says why where it cannot run
+    (this repository's port is no stand-in for it)."""
     if rank != 0:
         return
     from fastface_b200 import synth
+    from oracle import ffo
+    exe = os.path.join(ffo.REF_DIR, "fastface_int8_batched")
+    if not (ffo.ref_available() and os.path.exists(exe)):
+        why = ("the host's CPU lacks avx_vnni, which the reference's kernels are built for" if not ffo.host_has_avx_vnni()
+               else "the reference's binaries are not built (oracle/Makefile compiles them from its sources)")
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+        return
     batch = args.ref_batch
     per_step = 32                      # a step = 32 calls of the reference at its own batch size (256 faces)
     with tempfile.TemporaryDirectory() as root:

@@ -34,6 +34,18 @@ def test_reference_arm_other_ranks_exit_quietly():
     assert r.returncode == 0 and r.stdout.strip() == ""
 
 
+def test_reference_arm_without_the_reference(tmp_path):
+    """Where the reference's own binaries cannot run, --impl reference says so in its one line and exits 0: no other code is timed under
+    its name."""
+    code = (f"import sys; sys.path.insert(0, {ROOT!r}); from oracle import ffo; ffo.REF_DIR = {str(tmp_path)!r}; import bench; "
+            "sys.argv = ['bench.py', '--impl', 'reference', '--steps', '1']; bench.main()")
+    env = {k: v for k, v in os.environ.items() if k not in ("RANK", "LOCAL_RANK", "WORLD_SIZE")}
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+    d = json.loads(r.stdout)
+    assert set(d) == {"impl", "unavailable"} and d["impl"] == "reference" and len(d["unavailable"]) > 10
+
+
 def test_shard_plan(built_lib):
     lib = ff.load_library()
     lib.fastface_shard_plan.restype = C.c_int
