@@ -379,10 +379,6 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
     if (batch < 1 || b0 < 0 || batch > p->max_batch - b0) { ffcu_set_error("tc launch: batch out of range"); return -1; }
     if (b0 && (p->pair || p->wsp || p->out_f32)) { ffcu_set_error("tc launch: this kernel starts at face 0"); return -1; }
     const ffcu_layer& d = p->d;
-#ifdef FF_TC_TIMING
-    static int dbg = -1;
-    if (dbg < 0) { const char* e = getenv("FF_TC_DBG"); dbg = e ? atoi(e) : 0; }
-#endif
     const bool has_res = res && t.res_scale, has_slope = t.slope != nullptr, has_bn2 = out_bn2 && t.bn_in;
     int epi = EPI_RUNTIME;
     if (p->out_f32 || (!has_res && !has_slope && !has_bn2)) epi = EPI_PLAIN;
@@ -406,9 +402,6 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
         prm.total_tiles = prm.tiles_w * prm.tiles_h * batch;
         prm.stages = p->ws_stages; prm.group = 1; prm.lut_bytes = p->lut_bytes; prm.ntab = p->ntab;
         prm.full_wait = TC_WAIT_CYCLES; prm.drop_stage = -1;
-#ifdef FF_TC_TIMING
-        prm.dbg = dbg;
-#endif
         int grid = prm.total_tiles < p->n_sm ? prm.total_tiles : p->n_sm;
         prm.epi_wps = tc_epi_wps(p->BN, prm.total_tiles / grid);
         return tc_launch_ws(p->BN, mode, epi, grid, p->ws_smem_bytes, s, p->mapA_ws, p->mapB, prm);
@@ -426,9 +419,6 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
         prm.total_tiles = (images / 2) * p->wsp_tiles_per_image;
         prm.stages = p->wsp_stages; prm.group = 1; prm.lut_bytes = p->lut_bytes; prm.ntab = p->ntab;
         prm.full_wait = TC_WAIT_CYCLES; prm.drop_stage = -1;
-#ifdef FF_TC_TIMING
-        prm.dbg = dbg;
-#endif
         const int max_pairs = p->n_sm / 2;
         const int npairs = prm.total_tiles < max_pairs ? prm.total_tiles : max_pairs;
         prm.epi_wps = tc_epi_wps(p->BN, prm.total_tiles / npairs);
@@ -458,9 +448,6 @@ int ffcu_tc_launch(const TcPlan* cp, int batch, int mode, const EpiTables& t, co
     prm.total_tiles = prm.tiles_w * prm.tiles_h * prm.tiles_b * prm.tiles_n;
     prm.stages = p->stages; prm.group = p->group; prm.lut_bytes = p->lut_bytes; prm.ntab = p->ntab;
     prm.full_wait = TC_WAIT_CYCLES; prm.drop_stage = -1;
-#ifdef FF_TC_TIMING
-    prm.dbg = dbg;
-#endif
     { const char* e = getenv("FF_TC_STAGES"); if (e && atoi(e) >= 2 && atoi(e) < prm.stages) prm.stages = atoi(e); }
     if (p->pair) {
         const int m_tiles = prm.tiles_w * prm.tiles_h * prm.tiles_b;
@@ -627,9 +614,6 @@ int ffcu_sc_launch(const ScPlan* csp, int batch, int mode, const EpiTables& t1, 
     prm.total_tiles = prm.tiles_w * prm.tiles_h * prm.tiles_b * prm.tiles_n;
     prm.stages = sp->stages; prm.group = sp->group; prm.lut_bytes = 0; prm.ntab = 5;
     prm.full_wait = TC_WAIT_CYCLES; prm.drop_stage = -1;
-#ifdef FF_TC_TIMING
-    prm.dbg = 0;
-#endif
     int grid = prm.total_tiles < p->n_sm ? prm.total_tiles : p->n_sm;
     if (grid > prm.tiles_n) grid -= grid % prm.tiles_n;
     prm.epi_wps = tc_epi_wps(64, prm.total_tiles / grid);
@@ -842,9 +826,6 @@ int ffcu_stem_fused_launch(const StemTcPlan* p, const void* in_any, int in_u8, c
     prm.total_tiles = prm.tiles_w * prm.tiles_h * batch;
     prm.stages = p->stages; prm.group = 1; prm.lut_bytes = has_bn2 ? p->lut_bytes : 0; prm.ntab = 5;
     prm.full_wait = TC_WAIT_CYCLES; prm.drop_stage = -1;
-#ifdef FF_TC_TIMING
-    { static int dbg = -1; if (dbg < 0) { const char* e = getenv("FF_TC_DBG"); dbg = e ? atoi(e) : 0; } prm.dbg = dbg; }
-#endif
     const int grid = prm.total_tiles < p->n_sm ? prm.total_tiles : p->n_sm;
     prm.epi_wps = tc_epi_wps(64, prm.total_tiles / grid);
     return tc_launch_stem(mode, epi, in_u8, grid, p->smem_bytes, s, p->mapB, prm, in_any, inv3);

@@ -298,15 +298,7 @@ struct TcParams {
     long long full_wait;     // cycle limit of the MMA issuer's wait for a pipeline stage's data (TC_WAIT_CYCLES)
     int drop_stage;          // >= 0: the producer neither arms nor loads this K step of its first tile, so the
                              // issuer's wait for it must run out (ffcu_test_arm_timeout; -1 in every other launch)
-#ifdef FF_TC_TIMING
-    int dbg;                 // timing experiments: bit 0 = skip the TMA loads, bit 1 = skip the MMAs, bit 2 = no global memory in the epilogue, bit 3 = no epilogue arithmetic
-#endif
 };
-#ifdef FF_TC_TIMING
-#define TC_DBG(p, bit) ((p).dbg & (bit))
-#else
-#define TC_DBG(p, bit) 0
-#endif
 
 // Epilogue variants.  All but EPI_RUNTIME fix the presence of PReLU / residual / fused BN at
 // compile time, which turns the per-element code into one straight-line block the scheduler
@@ -520,9 +512,6 @@ __device__ __forceinline__ void tc_epilogue16(const TcParams& p, const float* ta
                                 ffcu_bn_q_nosat<CHECK>(a2, b_in.z, b_sc.z, b_of.z, b_iv.z),
                                 ffcu_bn_q_nosat<CHECK>(a3, b_in.w, b_sc.w, b_of.w, b_iv.w));
         } else if (has_bn2) {
-#ifdef FF_TC_TIMING
-            if (TC_DBG(p, 32)) { ow2[g] = w ^ 0x01010101; return; }     // timing experiment: no table look-ups (wrong results)
-#endif
             // BN of the four int8 results just packed: one table row per channel, indexed by the byte
             constexpr int R = CI * 16 + 4 * g;
             const uint32_t b0 = tc_lut_byte<0, R + 0>((uint32_t)w, lut_pr), b1 = tc_lut_byte<1, R + 1>((uint32_t)w, lut_pr);
@@ -698,7 +687,7 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
         int rw[8], rn[8];
 #pragma unroll
         for (int g = 0; g < 8; g++) { rw[g] = 0; rn[g] = 0; }
-        if (has_res && valid && !TC_DBG(p, 4)) {
+        if (has_res && valid) {
             ld_global_32B(p.res + o0, rw);
             if (n_pairs > 1) ld_global_32B(p.res + o0 + 32, rn);
         }
@@ -717,7 +706,7 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
             const uint32_t lut_pr = lut0 + (uint32_t)pr * (32u * 256u);
             tmem_ld16_issue(taddr + (uint32_t)(pr * 32 + 16), v1);            // lands while v0 is computed
             int w0[4], w0b[4], w1[4], w1b[4];
-            if (valid && !TC_DBG(p, 8)) {
+            if (valid) {
                 if (dump) {
                     const int d0[8] = {v0[0], v0[1], v0[2], v0[3], v0[4], v0[5], v0[6], v0[7]};
                     const int d1[8] = {v0[8], v0[9], v0[10], v0[11], v0[12], v0[13], v0[14], v0[15]};
@@ -730,7 +719,7 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
             }
             tmem_ld_wait(v1);
             if (more) tmem_ld16_issue(taddr + (uint32_t)(pr * 32 + 32), v0);  // lands while v1 is computed
-            if (valid && !TC_DBG(p, 8)) {
+            if (valid) {
                 if (dump) {
                     const int d0[8] = {v1[0], v1[1], v1[2], v1[3], v1[4], v1[5], v1[6], v1[7]};
                     const int d1[8] = {v1[8], v1[9], v1[10], v1[11], v1[12], v1[13], v1[14], v1[15]};
@@ -741,19 +730,17 @@ __device__ __forceinline__ void tc_epilogue_role(const TcParams& p, float* tab, 
                 else {
                     if (check) tc_epilogue16<CONTRACT, EPI, true, 1, false, CT, BN>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
                     else       tc_epilogue16<CONTRACT, EPI, false, 1, ACC22, CT, BN>(p, tab, ct, lut_pr, v1, rw + 4, cb + 16, has_res, has_slope, has_bn2, w1, w1b);
-                    if (!TC_DBG(p, 4)) {
-                        const int w8[8] = {w0[0], w0[1], w0[2], w0[3], w1[0], w1[1], w1[2], w1[3]};
-                        st_global_32B((int8_t*)p.out + o, w8);
-                        if (has_bn2) {
-                            const int w8b[8] = {w0b[0], w0b[1], w0b[2], w0b[3], w1b[0], w1b[1], w1b[2], w1b[3]};
-                            st_global_32B(p.out2 + o, w8b);
-                        }
+                    const int w8[8] = {w0[0], w0[1], w0[2], w0[3], w1[0], w1[1], w1[2], w1[3]};
+                    st_global_32B((int8_t*)p.out + o, w8);
+                    if (has_bn2) {
+                        const int w8b[8] = {w0b[0], w0b[1], w0b[2], w0b[3], w1b[0], w1b[1], w1b[2], w1b[3]};
+                        st_global_32B(p.out2 + o, w8b);
                     }
                 }
             }
 #pragma unroll
             for (int g = 0; g < 8; g++) rw[g] = rn[g];
-            if (has_res && pr + 2 < n_pairs && valid && !TC_DBG(p, 4)) ld_global_32B(p.res + o + 64, rn);   // two pairs ahead
+            if (has_res && pr + 2 < n_pairs && valid) ld_global_32B(p.res + o + 64, rn);   // two pairs ahead
             if (more) tmem_ld_wait(v0);
         }
         // this warp's TMEM reads are complete (the last tcgen05.wait::ld has returned)

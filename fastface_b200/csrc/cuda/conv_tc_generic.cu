@@ -60,7 +60,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             // first steps (as many as the ring holds) are requested before the programmatic-dependency
             // wait, the activation boxes after it.  Each slot's byte count is armed here for both.
             int pre = 0;
-            if ((int)blockIdx.x < p.total_tiles && !TC_DBG(p, 1)) {
+            if ((int)blockIdx.x < p.total_tiles) {
                 pre = n_steps < p.stages ? n_steps : p.stages;
                 int c0 = c0_first, kw = kw_first, kh = kh_first;
 #pragma unroll 1
@@ -89,8 +89,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
                         if (!ok) break;
                     }
-                    if (TC_DBG(p, 1)) { if (lane == 0) mbar_arrive(full0 + stage * 8); }
-                    else if (tile == (int)blockIdx.x && it == p.drop_stage) {
+                    if (tile == (int)blockIdx.x && it == p.drop_stage) {
                         // armed by ffcu_test_arm_timeout for one launch: this step's data never arrives
                     } else {
                         if (!first_fill) {
@@ -141,7 +140,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     tc_fence_after();
                     {
                         uint32_t soff = (uint32_t)((stage * stage_bytes) >> 4);
-                        if (!TC_DBG(p, 2))
 #pragma unroll 1
                         for (int g = 0; g < G; g++, soff += (uint32_t)(SUB_BYTES >> 4)) {
 #pragma unroll

@@ -95,7 +95,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             // tiles only: forward of 48 / 64 / 100 faces 718 / 778 / 1068 -> 710 / 770 / 1048 us; 128-column tiles, whose launches
             // leave hardly an SM free, lose by it (34 / 40 faces 588 / 648 -> 594 / 655).
             int pre = 0;
-            if (BN == 256 && pair_id < total && !TC_DBG(p, 1)) {
+            if (BN == 256 && pair_id < total) {
                 pre = n_steps < p.stages ? n_steps : p.stages;
 #pragma unroll 1
                 for (int it = 0; it < pre; it++) {
@@ -118,16 +118,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                         ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
                         if (!ok) break;
                     }
-                    if (TC_DBG(p, 1)) { if (rank == 0 && lane == 0) mbar_arrive(full0 + stage * 8); }
-                    else {
-                        if (!first_fill) {
-                            if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * G * SUB_BYTES);
-                            __syncwarp();                       // the byte count is armed before any copy can land
-                        }
-                        const int tapk = (kh * p.Kw + kw) * p.Cp + c0;
-                        if (issuer && (is_a || !first_fill)) tma2_load_4d(smem0 + stage * stage_bytes, map, full0_leader + stage * 8,
-                                    is_a ? c0 : tapk, is_a ? x0 + kw : tn * BN + (int)rank * (BN / 2), is_a ? y0 + kh : 0, c3);
+                    if (!first_fill) {
+                        if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * G * SUB_BYTES);
+                        __syncwarp();                       // the byte count is armed before any copy can land
                     }
+                    const int tapk = (kh * p.Kw + kw) * p.Cp + c0;
+                    if (issuer && (is_a || !first_fill)) tma2_load_4d(smem0 + stage * stage_bytes, map, full0_leader + stage * 8,
+                                is_a ? c0 : tapk, is_a ? x0 + kw : tn * BN + (int)rank * (BN / 2), is_a ? y0 + kh : 0, c3);
                     c0 += G * KC;
                     while (c0 >= p.Cp) { c0 -= p.Cp; if (++kw == p.Kw) { kw = 0; kh++; } }
                     if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -167,7 +164,6 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                     tc_fence_after();
                     {
                         uint32_t soff = (uint32_t)((stage * stage_bytes) >> 4);
-                        if (!TC_DBG(p, 2))
 #pragma unroll 1
                         for (int g = 0; g < G; g++, soff += (uint32_t)(SUB_BYTES >> 4)) {
 #pragma unroll

@@ -180,7 +180,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap mapB, const TcParams p, con
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
             const uint64_t da = smem_desc_sw32(smem_u32(s_a + (size_t)stage * STEM_A_BYTES));
-            if (!TC_DBG(p, 2)) umma_i8(d_tmem, da, dw, IDESC, 0u);
+            umma_i8(d_tmem, da, dw, IDESC, 0u);
             umma_commit(smem_u32(&sh->empty[stage]));
             umma_commit(smem_u32(&sh->acc_full[a]));
         }

@@ -61,7 +61,6 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (!ok) break;
                 const uint32_t bar = smem_u32(&sh->full[stage]);
                 const uint32_t sa = smem_u32(s_a + (size_t)stage * WS_A_BYTES);
-                if (TC_DBG(p, 1)) { if (lane == 0) mbar_arrive(bar); if (++stage == p.stages) { stage = 0; phase ^= 1; } continue; }
                 if (lane == 0) {
                     mbar_expect_tx(bar, WS_BOX_ROWS * 64);
                     tma_load_4d(sa, &mapA, bar, 0, tw * WS_TW - 1, th * WS_TH - 1, b);
@@ -105,7 +104,6 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
                 const uint64_t da0 = smem_desc_sbo<KC>(smem_u32(s_a + (size_t)stage * WS_A_BYTES), WS_PITCH * 64);
                 {
-                if (!TC_DBG(p, 2))
 #pragma unroll
                 for (int kw = 0; kw < 3; kw++)
 #pragma unroll

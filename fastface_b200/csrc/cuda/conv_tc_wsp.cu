@@ -94,13 +94,10 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             const int base_row = (t * TC_TILE_M) / P - 1;
             ok = mbar_wait(empty0 + stage * 8, phase ^ 1, abort_flag, p.err, FFCU_ERR_EMPTY_TIMEOUT);
             if (!ok) break;
-            if (TC_DBG(p, 1)) { if (rank == 0 && lane == 0) mbar_arrive(full0 + stage * 8); }
-            else {
-                if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * box_bytes);
-                __syncwarp();
-                if (lane == 0) tma2_load_4d(smem_u32(s_a + (size_t)stage * a_stride + WSP_GUARD_BYTES), &mapA,
-                                            full0_leader + stage * 8, 0, -1, base_row, b);
-            }
+            if (rank == 0 && lane == 0) mbar_expect_tx(full0 + stage * 8, 2 * box_bytes);
+            __syncwarp();
+            if (lane == 0) tma2_load_4d(smem_u32(s_a + (size_t)stage * a_stride + WSP_GUARD_BYTES), &mapA,
+                                        full0_leader + stage * 8, 0, -1, base_row, b);
             __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -145,19 +142,17 @@ conv_wsp_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 const int t = wk.th;
                 const int off = t * TC_TILE_M - ((t * TC_TILE_M) / P - 1) * P;
                 const uint64_t da0 = smem_desc<KC>(smem_u32(s_a + (size_t)stage * a_stride + WSP_GUARD_BYTES));
-                if (!TC_DBG(p, 2)) {
 #pragma unroll 1
-                    for (int kh = 0; kh < 3; kh++)
+                for (int kh = 0; kh < 3; kh++)
 #pragma unroll
-                        for (int kw = 0; kw < 3; kw++) {
-                            const int line = off + (kh - 1) * P + (kw - 1);        // >= -1: the guard in front of the box
-                            const uint64_t da = da0 + (uint64_t)(int64_t)((line * KC) >> 4);
-                            const uint64_t db = dw + (uint64_t)(((kh * 3 + kw) * W_TAP_BYTES) >> 4);
+                    for (int kw = 0; kw < 3; kw++) {
+                        const int line = off + (kh - 1) * P + (kw - 1);        // >= -1: the guard in front of the box
+                        const uint64_t da = da0 + (uint64_t)(int64_t)((line * KC) >> 4);
+                        const uint64_t db = dw + (uint64_t)(((kh * 3 + kw) * W_TAP_BYTES) >> 4);
 #pragma unroll
-                            for (int k = 0; k < KC / 32; k++)
-                                umma2_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kh | kw | k) ? 1u : 0u);
-                        }
-                }
+                        for (int k = 0; k < KC / 32; k++)
+                            umma2_i8(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC, (kh | kw | k) ? 1u : 0u);
+                    }
                 umma2_commit_both(smem_u32(&sh->empty[stage]));
                 umma2_commit_both(smem_u32(&sh->acc_full[a]));
             }
