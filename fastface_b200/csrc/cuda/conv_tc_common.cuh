@@ -863,7 +863,7 @@ struct FaceParams {
 int tc_face_smem_bytes();
 int tc_face_pairs();
 int tc_launch_face(int mode, int pairs, cudaStream_t s, const CUtensorMap& mapA, const FaceParams& prm);
-// Stages of 28x28, 14x14 and 7x7 maps for a handful of faces, a cluster per face, in two forms (conv_tc_stage.cu)
+// Stages of 28x28, 14x14 and 7x7 maps for a handful of faces, a cluster per face, in two or three forms (conv_tc_stage.cu)
 #define STAGE_FORMS 3                     // 14x14: two
 struct StageForm { int win_rows, pitch, kept_bytes, clusters, faces; };      // box of the first input; FaceParams::kept per cluster; clusters the device holds; faces of each
 StageForm tc_stage_form(int H, int i);

@@ -1,5 +1,5 @@
-// conv_tc_face.cuh -- what the kernels that take a face through the 14x14 stage share: the epilogue of one output channel per
-// thread (weights are the MMA's rows, a row of the face is 16 of its columns).
+// conv_tc_face.cuh -- what the kernels that take a face through a stage share: the epilogue of one output channel per
+// thread (weights are the MMA's rows, a row of the face 8, 16 or 32 of its columns).
 #pragma once
 #include "conv_tc_common.cuh"
 

@@ -3,7 +3,7 @@
 // The weights are the MMA's rows: a tile is 128 outputs x up to 256 faces (N = the faces, rounded up to 16), so a small call
 // moves and computes little for faces that are not there, and each weight passes through shared memory once per 256 faces.  A
 // tile is cut into `splits` K ranges, one CTA each: 4 tiles x 28 ranges = 112 CTAs up to 256 faces, 7 K blocks of 128 each, all
-// of them requested at once up to 112 faces (the weights before the programmatic-dependency wait).  A CTA lays its int32 partial sums
+// of them requested at once up to 128 faces (the weights before the programmatic-dependency wait).  A CTA lays its int32 partial sums
 // [face][128 outputs] into shared memory as its threads hold them (a thread is an output: 32 lanes, 32 consecutive words),
 // where a bulk reduction adds them to a scratch array (integer addition, so any order gives the same bits); the CTA that
 // takes the last ticket of its tile turns the sums into floats exactly as the one-CTA form does (reference
